@@ -38,6 +38,7 @@ struct MsCtrl {
     uint32_t touched;         // touched vertices of a push superstep
     uint32_t active;          // frontier vertices after the superstep
     unsigned long long active_edges;
+    unsigned long long live, live_next;  // sources with a frontier: of this superstep, of the next
     int32_t cur;              // queue / front buffer of the current frontier
     int32_t step;
     int32_t mode;             // 0: queue frontier (push next), 1: dense (pull next)
@@ -75,6 +76,12 @@ __device__ __forceinline__ void ms_count_launch(const MsArgs &a) {
 }
 
 __device__ __forceinline__ int32_t push_level(const MsArgs &a) { return a.c->step + 1; }
+
+__device__ __forceinline__ unsigned long long warp_or64(unsigned long long x) {
+    const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)x);
+    const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(x >> 32));
+    return ((unsigned long long)hi << 32) | lo;
+}
 
 // Record the level of every source in `bits` for vertex v.
 __device__ __forceinline__ void write_levels(const MsArgs &a, int32_t v, unsigned long long bits,
@@ -132,6 +139,8 @@ __global__ void k_ms_init(MsArgs a, const int32_t *sources) {
     c->active_edges = m;
     c->reached = nr;
     c->reached_edges = mr;
+    c->live = a.all;
+    c->live_next = 0ull;
     c->done = n == 0;
 }
 
@@ -219,7 +228,7 @@ __global__ void k_ms_commit(MsArgs a) {
     const int64_t total = (int64_t)nold + nt;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     uint32_t nr = 0;
-    unsigned long long mr = 0;
+    unsigned long long mr = 0, lv = 0;
     for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < total;
          base += warps * 32) {
         const int64_t i = base + lane;
@@ -239,6 +248,7 @@ __global__ void k_ms_commit(MsArgs a) {
                     mr += (uint32_t)a.outdeg[v];
                 }
                 a.seen[v] = old | nb;
+                lv |= nb;
                 front_nx[v] = nb;
                 write_levels(a, v, nb, lvl);
                 deg = (uint32_t)a.outdeg[v];
@@ -250,38 +260,199 @@ __global__ void k_ms_commit(MsArgs a) {
     }
     nr = warp_sum(nr);
     mr = warp_sum(mr);
+    lv = warp_or64(lv);
     if (lane == 0 && nr) {
         atomicAdd(&c->reached, nr);
         atomicAdd(&c->reached_edges, mr);
     }
+    if (lane == 0 && lv) atomicOr(&c->live_next, lv);
 }
 
 // pull: every vertex still missing some sources ORs its in-neighbours'
 // frontier masks (early exit once covered); writes the whole next buffer.
+// Bound by the random 8-byte mask gathers (one 32-byte L2 sector each), so
+// the mapping keeps many in flight and none serial: one warp per 32
+// consecutive vertices; a lane walks the first kMsLaneCap in-edges of its own
+// vertex, kMsLaneU gathers at a time; longer lists are finished by the whole
+// warp, and lists past kMsHubMin by one CTA each in a second kernel
+// (k_ms_pull_hub).  With one thread per list, a hub's list was one lane's
+// chain of dependent gathers and set the length of the superstep.  Only
+// sources that still have a frontier (c->live) are looked for: a source that
+// died out would otherwise keep every vertex scanning its whole list.
+// Measured, 64 sources on R-MAT 2^22 / 2^26: 6.69 -> 3.97 ms a call, the
+// levels' fill before the run (now k_ms_stats) included.
+constexpr int kMsLaneCap = 16;
+constexpr int kMsLaneU = 4;
+constexpr int32_t kMsHubMin = 4096;
+constexpr int kMsHubThreads = 512;
+constexpr int kMsHubU = 4;
+
+// Levels of 32 consecutive vertices (lane l: vertex v, new sources `bits`),
+// source by source, so that a store covers consecutive vertices.
+__device__ __forceinline__ void write_levels_warp(const MsArgs &a, int32_t v, unsigned long long bits,
+                                                  int32_t lvl) {
+    unsigned long long any = warp_or64(bits);
+    while (any) {
+        const int s = __ffsll((long long)any) - 1;
+        any &= any - 1;
+        if ((bits >> s) & 1ull) a.levels[(size_t)s * a.V + v] = lvl;
+    }
+}
+
+// Counters of a pull (all 32 lanes; one set of atomics per warp).
+__device__ __forceinline__ void ms_pull_counts(MsCtrl *c, uint32_t act, unsigned long long act_e, uint32_t nr,
+                                               unsigned long long mr, unsigned long long live) {
+    act = warp_sum(act);
+    act_e = warp_sum(act_e);
+    nr = warp_sum(nr);
+    mr = warp_sum(mr);
+    live = warp_or64(live);
+    if ((threadIdx.x & 31) != 0) return;
+    if (act) {
+        atomicAdd(&c->active, act);
+        atomicAdd(&c->active_edges, act_e);
+    }
+    if (nr) {
+        atomicAdd(&c->reached, nr);
+        atomicAdd(&c->reached_edges, mr);
+    }
+    if (live) atomicOr(&c->live_next, live);
+}
+
 __global__ void __launch_bounds__(256) k_ms_pull(MsArgs a) {
     MsCtrl *c = a.c;
     const int cur = c->cur;
     const unsigned long long *front = cur ? a.front[1] : a.front[0];
     unsigned long long *front_nx = cur ? a.front[0] : a.front[1];
+    const unsigned long long live = c->live;
     const int32_t lvl = push_level(a);
+    const int lane = threadIdx.x & 31;
     ms_count_launch(a);
     uint32_t act = 0, nr = 0;
-    unsigned long long act_e = 0, mr = 0;
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < a.V;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long old = a.seen[v];
-        const unsigned long long need = a.all & ~old;
+    unsigned long long act_e = 0, mr = 0, lv = 0;
+    const int64_t words = ((int64_t)a.V + 31) / 32;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < words; w += warps) {
+        const int32_t v = (int32_t)(w * 32 + lane);
+        const bool in = v < a.V;
+        const unsigned long long old = in ? a.seen[v] : ~0ull;
+        const unsigned long long need = live & ~old;
         unsigned long long acc = 0ull;
+        int32_t j = 0, je = 0;
+        bool hub = false;
         if (need) {
-            const int32_t jb = a.rrow[v], je = a.rrow[v + 1];
-            for (int32_t j = jb; j < je; j++) {
-                acc |= front[__ldg(&a.rcol[j])];
-                if ((acc & need) == need) break;
+            j = a.rrow[v];
+            je = a.rrow[v + 1];
+            hub = je - j > kMsHubMin;
+            if (hub) je = j;  // left to k_ms_pull_hub
+        }
+        const unsigned hubs = __ballot_sync(0xffffffffu, hub);
+        if (hubs) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&c->touched, (uint32_t)__popc(hubs));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (hub) a.touched[base + __popc(hubs & lanemask_lt())] = v;
+        }
+        const int32_t jcap = min(je, j + kMsLaneCap);
+        while (j < jcap) {
+            int32_t u[kMsLaneU];
+            unsigned long long f[kMsLaneU];
+#pragma unroll
+            for (int r = 0; r < kMsLaneU; r++) u[r] = j + r < jcap ? __ldg(&a.rcol[j + r]) : -1;
+#pragma unroll
+            for (int r = 0; r < kMsLaneU; r++) f[r] = u[r] >= 0 ? __ldg(&front[u[r]]) : 0ull;
+#pragma unroll
+            for (int r = 0; r < kMsLaneU; r++) acc |= f[r];
+            j += kMsLaneU;
+            if ((acc & need) == need) je = j;  // covered: nothing left
+            if (j >= je) break;
+        }
+        // longer lists, the whole warp on one at a time
+        unsigned pend = __ballot_sync(0xffffffffu, j < je && (acc & need) != need);
+        while (pend) {
+            const int l = __ffs(pend) - 1;
+            pend &= pend - 1;
+            const int32_t pj = __shfl_sync(0xffffffffu, j, l), pje = __shfl_sync(0xffffffffu, je, l);
+            const unsigned long long pneed = __shfl_sync(0xffffffffu, need & ~acc, l);
+            unsigned long long got = 0ull;
+            for (int32_t b = pj; b < pje; b += 64) {
+                const int32_t j0 = b + lane, j1 = b + 32 + lane;
+                const int32_t u0 = j0 < pje ? __ldg(&a.rcol[j0]) : -1;
+                const int32_t u1 = j1 < pje ? __ldg(&a.rcol[j1]) : -1;
+                const unsigned long long f0 = u0 >= 0 ? __ldg(&front[u0]) : 0ull;
+                const unsigned long long f1 = u1 >= 0 ? __ldg(&front[u1]) : 0ull;
+                got |= warp_or64(f0 | f1);
+                if ((got & pneed) == pneed) break;
             }
-            acc &= need;
+            if (lane == l) acc |= got;
+        }
+        acc &= need;
+        if (acc) {
+            a.seen[v] = old | acc;
+            const uint32_t d = (uint32_t)a.outdeg[v];
+            if (old == 0ull) {
+                nr++;
+                mr += d;
+            }
+            if (d > 0) {
+                act++;
+                act_e += d;
+            }
+            lv |= acc;
+        }
+        if (in && !hub) front_nx[v] = acc;
+        write_levels_warp(a, v, acc, lvl);
+    }
+    ms_pull_counts(c, act, act_e, nr, mr, lv);
+}
+
+// The hubs k_ms_pull left (c->touched of them): one CTA per in-list,
+// kMsHubU gathers of each thread in flight, early exit once covered.
+__global__ void __launch_bounds__(kMsHubThreads) k_ms_pull_hub(MsArgs a) {
+    __shared__ unsigned long long s_or[kMsHubThreads / 32];
+    MsCtrl *c = a.c;
+    ms_count_launch(a);
+    const int cur = c->cur;
+    const unsigned long long *front = cur ? a.front[1] : a.front[0];
+    unsigned long long *front_nx = cur ? a.front[0] : a.front[1];
+    const unsigned long long live = c->live;
+    const int32_t lvl = push_level(a);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t n = c->touched;
+    uint32_t act = 0, nr = 0;
+    unsigned long long act_e = 0, mr = 0, lv = 0;
+    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+        const int32_t v = a.touched[i];
+        const unsigned long long old = a.seen[v], need = live & ~old;
+        const int32_t jb = a.rrow[v], je = a.rrow[v + 1];
+        unsigned long long acc = 0ull;
+        for (int32_t b = jb; b < je; b += kMsHubThreads * kMsHubU) {
+            unsigned long long f[kMsHubU];
+            int32_t u[kMsHubU];
+#pragma unroll
+            for (int r = 0; r < kMsHubU; r++) {
+                const int64_t j = (int64_t)b + r * kMsHubThreads + threadIdx.x;
+                u[r] = j < je ? __ldg(&a.rcol[j]) : -1;
+            }
+#pragma unroll
+            for (int r = 0; r < kMsHubU; r++) f[r] = u[r] >= 0 ? __ldg(&front[u[r]]) : 0ull;
+            unsigned long long x = 0ull;
+#pragma unroll
+            for (int r = 0; r < kMsHubU; r++) x |= f[r];
+            x = warp_or64(x);
+            if (lane == 0) s_or[wid] = x;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kMsHubThreads / 32; k++) acc |= s_or[k];
+            __syncthreads();
+            if ((acc & need) == need) break;  // the same for every thread
+            if (je - b <= kMsHubThreads * kMsHubU) break;  // b + step could pass 2^31
+        }
+        acc &= need;
+        if (threadIdx.x == 0) {
+            front_nx[v] = acc;
             if (acc) {
                 a.seen[v] = old | acc;
-                write_levels(a, (int32_t)v, acc, lvl);
                 const uint32_t d = (uint32_t)a.outdeg[v];
                 if (old == 0ull) {
                     nr++;
@@ -291,39 +462,23 @@ __global__ void __launch_bounds__(256) k_ms_pull(MsArgs a) {
                     act++;
                     act_e += d;
                 }
+                lv |= acc;
             }
         }
-        front_nx[v] = acc;
+        if (threadIdx.x < 64 && ((acc >> threadIdx.x) & 1ull)) a.levels[(size_t)threadIdx.x * a.V + v] = lvl;
     }
-    act = warp_sum(act);
-    act_e = warp_sum(act_e);
-    nr = warp_sum(nr);
-    mr = warp_sum(mr);
-    if ((threadIdx.x & 31) == 0 && act) {
-        atomicAdd(&c->active, act);
-        atomicAdd(&c->active_edges, act_e);
-    }
-    if ((threadIdx.x & 31) == 0 && nr) {
-        atomicAdd(&c->reached, nr);
-        atomicAdd(&c->reached_edges, mr);
-    }
+    if (wid == 0) ms_pull_counts(c, act, act_e, nr, mr, lv);
 }
 
-// after a pull: clear the old front buffer
-__global__ void k_ms_clear_front(MsArgs a) {
-    ms_count_launch(a);
-    unsigned long long *f = a.c->cur ? a.front[1] : a.front[0];
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < a.V;
-         v += (int64_t)gridDim.x * blockDim.x)
-        f[v] = 0ull;
-}
-
-// dense front -> queue of the vertices with a nonzero mask (for a push)
+// dense front -> queue of the vertices with a nonzero mask (for a push); the
+// other buffer, still holding the frontier before the pull, is cleared for
+// the push's commit (a pull writes its whole next buffer and needs no clear)
 __global__ void k_ms_dense2q(MsArgs a) {
     MsCtrl *c = a.c;
     ms_count_launch(a);
     const int cur = c->cur;
     const unsigned long long *front = cur ? a.front[1] : a.front[0];
+    unsigned long long *front_nx = cur ? a.front[0] : a.front[1];
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < a.V;
@@ -331,6 +486,7 @@ __global__ void k_ms_dense2q(MsArgs a) {
         const int64_t v = base + lane;
         uint32_t deg = 0;
         bool in = false;
+        if (v < a.V) front_nx[v] = 0ull;
         if (v < a.V && front[v]) {
             deg = (uint32_t)a.outdeg[v];
             in = deg > 0;
@@ -345,6 +501,7 @@ __device__ void ms_begin(MsCtrl *c, int pull) {
     if (pull) {
         c->active = 0;
         c->active_edges = 0ull;
+        c->touched = 0;  // the hubs the pull leaves to k_ms_pull_hub
     } else {
         c->touched = 0;
         c->q[c->cur ^ 1] = 0ull;
@@ -367,6 +524,8 @@ __device__ void ms_end(MsCtrl *c, int pull) {
         c->active_edges = (uint32_t)qn;
         c->pushes++;
     }
+    c->live = c->live_next;
+    c->live_next = 0ull;
     c->step++;
     c->supersteps++;
     c->done = c->active == 0;
@@ -444,13 +603,19 @@ __global__ void k_ms_select(MsArgs a, int cap, cudaGraphConditionalHandle h_cont
     if (use_handles) cudaGraphSetConditional(h_branch, (unsigned)c->branch);
 }
 
-// per-source traversal count: sum over v of popc(seen[v]) * outdeg[v]
+// per-source traversal count: sum over v of popc(seen[v]) * outdeg[v]; and
+// the -1 of every (source, vertex) not reached, so that the levels need no
+// fill of nsrc * V entries before the run
 __global__ void k_ms_stats(MsArgs a, unsigned long long *out) {
     ms_count_launch(a);
     unsigned long long er = 0, vr = 0;
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < a.V;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const int p = __popcll(a.seen[v]);
+    for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll; b < a.V;
+         b += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = b + (threadIdx.x & 31);
+        const unsigned long long sn = v < a.V ? a.seen[v] : a.all;
+        write_levels_warp(a, (int32_t)v, a.all & ~sn, -1);
+        if (v >= a.V) continue;
+        const int p = __popcll(sn);
         vr += p;
         er += (unsigned long long)p * (uint32_t)a.outdeg[v];
     }
@@ -526,7 +691,6 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
         MB_CUDA(cudaMemsetAsync(a.front[0], 0, 8 * vb, cs));
         MB_CUDA(cudaMemsetAsync(a.front[1], 0, 8 * vb, cs));
         MB_CUDA(cudaMemsetAsync(a.nxt, 0, 8 * vb, cs));
-        MB_CUDA(cudaMemsetAsync(levels_dev, 0xff, sizeof(int32_t) * vb * nsrc, cs));
         MB_CUDA(cudaMemsetAsync(st.stats.p, 0, 2 * sizeof(unsigned long long), cs));
         k_ms_init<<<1, 32, 0, cs>>>(a, st.srcs.as<int32_t>());
         MB_CHECK_LAUNCH();
@@ -534,7 +698,7 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
     auto branch = [&](int b, cudaStream_t cs) {
         if (b == kMsBranchPull) {
             k_ms_pull<<<gv, 256, 0, cs>>>(a);
-            k_ms_clear_front<<<gv, 256, 0, cs>>>(a);
+            if (g.max_indeg > kMsHubMin) k_ms_pull_hub<<<ctx.num_sms * 2, kMsHubThreads, 0, cs>>>(a);
         } else {
             if (b == kMsBranchDensePush) k_ms_dense2q<<<gv, 256, 0, cs>>>(a);
             k_ms_push<<<gp, kPushThreads, 0, cs>>>(a);
