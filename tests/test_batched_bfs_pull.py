@@ -4,6 +4,7 @@ list covered by its last edge only."""
 import numpy as np
 import pytest
 
+from medusa_b200 import api
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -38,7 +39,7 @@ def star_graph(rng, first_hit):
 
 @pytest.mark.parametrize("direction", [None, 4], ids=["fixed", "pull"])
 @pytest.mark.parametrize("first_hit", [True, False], ids=["first", "late"])
-def test_pull_list_lengths(gpu_ctx, api, direction, first_hit):
+def test_pull_list_lengths(gpu_ctx, direction, first_hit):
     V, src, dst, sources = star_graph(np.random.default_rng(5), first_hit)
     g = gpu_ctx.graph_from_edges(V, src, dst)
     if direction is not None:
