@@ -17,8 +17,8 @@
 // reference counterpart exists for the batching itself (the reference's
 // "MBFS" app is multi-GPU BFS).
 //
-// The loop is one CUDA graph (WHILE over a SWITCH of three branches: push,
-// dense->queue + push, pull).  A one-warp select kernel at the top of each
+// The loop is one CUDA graph (WHILE over a SWITCH of five branches: push
+// and wide push, each also after a dense->queue conversion, and pull).  A one-warp select kernel at the top of each
 // iteration finishes the superstep that ran and picks the direction of the
 // next one: the fixed rule (pull once the union frontier's out-edges pass
 // E/16), a forced or replayed schedule, or the learned scheduler's MLP
@@ -47,19 +47,33 @@ struct MsCtrl {
     int32_t pushes, pulls;
     int32_t pending;          // a superstep ran since the last select
     int32_t last_pull;        // its direction
+    int32_t last_wide;        // it left a dense frontier (a pull, or a wide push)
+    int32_t nkeep;            // frontiers kept for the levels (keep_lvl of them)
+    int32_t keep_lvl[8];
     int32_t iter, err, branch, sched;
     uint32_t reached;         // vertices seen by at least one source
     unsigned long long reached_edges;  // their out-edges
     float skew;               // log2(max out-degree / mean), scheduler feature
     float feat[8];            // features of the last decision
 };
-constexpr int kMsBranchPush = 0, kMsBranchPull = 1, kMsBranchDensePush = 2, kMsBranches = 3;
+constexpr int kMsBranchPush = 0, kMsBranchPull = 1, kMsBranchDensePush = 2, kMsBranchWidePush = 3,
+              kMsBranchDenseWidePush = 4, kMsBranches = 5;
+// Frontiers of dense supersteps kept for the levels (k_ms_finish): 8 masks of
+// 8 bytes per vertex.  Past them a superstep stores its levels itself.
+constexpr int kMsKeep = 8;
+// A push whose frontier has at least V / kMsWideDiv out-edges is wide: it
+// touches so many vertices that a list of them (an atomic append each, and
+// a commit in list order with a scattered store per level) costs more than
+// one pass over all masks.  64 sources on R-MAT 2^22 / 2^26, the superstep
+// with 1.7M frontier edges: 0.48 ms as a list, 0.10 wide.
+constexpr int kMsWideDiv = 8;
 
 struct MsArgs {
     int32_t V;
     int64_t E;
     const int32_t *row, *col, *rrow, *rcol, *outdeg;
     unsigned long long *seen, *front[2], *nxt;
+    unsigned long long *keep;  // kMsKeep frontiers of V masks
     int32_t *touched;
     int32_t *qv[2];
     uint32_t *qo[2];
@@ -83,7 +97,7 @@ __device__ __forceinline__ unsigned long long warp_or64(unsigned long long x) {
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// Record the level of every source in `bits` for vertex v.
+// Record the level of every source in `bits` for vertex v (list supersteps).
 __device__ __forceinline__ void write_levels(const MsArgs &a, int32_t v, unsigned long long bits,
                                              int32_t lvl) {
     while (bits) {
@@ -141,6 +155,8 @@ __global__ void k_ms_init(MsArgs a, const int32_t *sources) {
     c->reached_edges = mr;
     c->live = a.all;
     c->live_next = 0ull;
+    c->nkeep = 0;
+    c->last_wide = 0;
     c->done = n == 0;
 }
 
@@ -151,7 +167,9 @@ struct MsPushSmem {
 };
 
 // push: next[v] |= front[u] & ~seen[v] over the frontier queue's edges
-// (merge-path tiles, one search per thread over consecutive edges)
+// (merge-path tiles, one search per thread over consecutive edges).  kWide:
+// no list of the touched vertices, so the masks' atomics return nothing.
+template <bool kWide>
 __global__ void __launch_bounds__(kPushThreads) k_ms_push(MsArgs a) {
     __shared__ MsPushSmem sm;
     MsCtrl *c = a.c;
@@ -196,8 +214,12 @@ __global__ void __launch_bounds__(kPushThreads) k_ms_push(MsArgs a) {
             bool first = false;
             if (v[r] >= 0) {
                 const unsigned long long bits = f[r] & ~__ldcg(&a.seen[v[r]]);
-                if (bits) first = atomicOr(&a.nxt[v[r]], bits) == 0ull;
+                if (bits) {
+                    if (kWide) atomicOr(&a.nxt[v[r]], bits);
+                    else first = atomicOr(&a.nxt[v[r]], bits) == 0ull;
+                }
             }
+            if (kWide) continue;
             // warp-aggregated append of first touches
             const unsigned mask = __ballot_sync(0xffffffffu, first);
             if (mask) {
@@ -280,9 +302,9 @@ __global__ void k_ms_commit(MsArgs a) {
 // sources that still have a frontier (c->live) are looked for: a source that
 // died out would otherwise keep every vertex scanning its whole list.
 // Measured, 64 sources on R-MAT 2^22 / 2^26: 6.69 -> 3.97 ms a call, the
-// levels' fill before the run (now k_ms_stats) included.
+// levels' fill before the run (now k_ms_finish) included.
 constexpr int kMsLaneCap = 16;
-constexpr int kMsLaneU = 4;
+constexpr int kMsLaneU = 4;  // 8, or one 16-byte index load for 4: the same time
 constexpr int32_t kMsHubMin = 4096;
 constexpr int kMsHubThreads = 512;
 constexpr int kMsHubU = 4;
@@ -297,6 +319,13 @@ __device__ __forceinline__ void write_levels_warp(const MsArgs &a, int32_t v, un
         any &= any - 1;
         if ((bits >> s) & 1ull) a.levels[(size_t)s * a.V + v] = lvl;
     }
+}
+
+// Where a dense superstep keeps its new frontier for the levels, or null
+// once kMsKeep are kept.
+__device__ __forceinline__ unsigned long long *ms_keep(const MsArgs &a) {
+    const int k = a.c->nkeep;
+    return k < kMsKeep ? a.keep + (size_t)k * a.V : nullptr;
 }
 
 // Counters of a pull (all 32 lanes; one set of atomics per warp).
@@ -325,6 +354,7 @@ __global__ void __launch_bounds__(256) k_ms_pull(MsArgs a) {
     const unsigned long long *front = cur ? a.front[1] : a.front[0];
     unsigned long long *front_nx = cur ? a.front[0] : a.front[1];
     const unsigned long long live = c->live;
+    unsigned long long *keep = ms_keep(a);
     const int32_t lvl = push_level(a);
     const int lane = threadIdx.x & 31;
     ms_count_launch(a);
@@ -401,7 +431,8 @@ __global__ void __launch_bounds__(256) k_ms_pull(MsArgs a) {
             lv |= acc;
         }
         if (in && !hub) front_nx[v] = acc;
-        write_levels_warp(a, v, acc, lvl);
+        if (!keep) write_levels_warp(a, v, acc, lvl);
+        else if (in && !hub) keep[v] = acc;
     }
     ms_pull_counts(c, act, act_e, nr, mr, lv);
 }
@@ -416,6 +447,7 @@ __global__ void __launch_bounds__(kMsHubThreads) k_ms_pull_hub(MsArgs a) {
     const unsigned long long *front = cur ? a.front[1] : a.front[0];
     unsigned long long *front_nx = cur ? a.front[0] : a.front[1];
     const unsigned long long live = c->live;
+    unsigned long long *keep = ms_keep(a);
     const int32_t lvl = push_level(a);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n = c->touched;
@@ -451,6 +483,7 @@ __global__ void __launch_bounds__(kMsHubThreads) k_ms_pull_hub(MsArgs a) {
         acc &= need;
         if (threadIdx.x == 0) {
             front_nx[v] = acc;
+            if (keep) keep[v] = acc;
             if (acc) {
                 a.seen[v] = old | acc;
                 const uint32_t d = (uint32_t)a.outdeg[v];
@@ -465,9 +498,51 @@ __global__ void __launch_bounds__(kMsHubThreads) k_ms_pull_hub(MsArgs a) {
                 lv |= acc;
             }
         }
-        if (threadIdx.x < 64 && ((acc >> threadIdx.x) & 1ull)) a.levels[(size_t)threadIdx.x * a.V + v] = lvl;
+        if (!keep && threadIdx.x < 64 && ((acc >> threadIdx.x) & 1ull)) a.levels[(size_t)threadIdx.x * a.V + v] = lvl;
     }
     if (wid == 0) ms_pull_counts(c, act, act_e, nr, mr, lv);
+}
+
+// commit after a wide push: one pass over every vertex's new bits (bound by
+// streaming seen and nxt), leaving a dense frontier as a pull does.
+__global__ void __launch_bounds__(256) k_ms_commit_wide(MsArgs a) {
+    MsCtrl *c = a.c;
+    ms_count_launch(a);
+    unsigned long long *front_nx = c->cur ? a.front[0] : a.front[1];
+    unsigned long long *keep = ms_keep(a);
+    const int32_t lvl = push_level(a);
+    const int lane = threadIdx.x & 31;
+    uint32_t act = 0, nr = 0;
+    unsigned long long act_e = 0, mr = 0, lv = 0;
+    for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll; b < a.V;
+         b += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = b + lane;
+        const bool in = v < a.V;
+        const unsigned long long nx = in ? a.nxt[v] : 0ull;
+        unsigned long long nb = 0ull;
+        if (nx) {
+            const unsigned long long old = a.seen[v];
+            nb = nx & ~old;
+            a.nxt[v] = 0ull;
+            if (nb) {
+                a.seen[v] = old | nb;
+                const uint32_t d = (uint32_t)a.outdeg[v];
+                if (old == 0ull) {
+                    nr++;
+                    mr += d;
+                }
+                if (d > 0) {
+                    act++;
+                    act_e += d;
+                }
+                lv |= nb;
+            }
+        }
+        if (in) front_nx[v] = nb;
+        if (!keep) write_levels_warp(a, (int32_t)v, nb, lvl);
+        else if (in) keep[v] = nb;
+    }
+    ms_pull_counts(c, act, act_e, nr, mr, lv);
 }
 
 // dense front -> queue of the vertices with a nonzero mask (for a push); the
@@ -496,25 +571,26 @@ __global__ void k_ms_dense2q(MsArgs a) {
     }
 }
 
-// superstep bookkeeping (one thread) before and after a push or a pull
-__device__ void ms_begin(MsCtrl *c, int pull) {
-    if (pull) {
+// superstep bookkeeping (one thread) before and after a push or a pull;
+// wide: the superstep leaves a dense frontier (a pull, or a wide push)
+__device__ void ms_begin(MsCtrl *c, int pull, int wide) {
+    c->touched = 0;  // a push's touched vertices, or the hubs a pull leaves to k_ms_pull_hub
+    if (wide) {
         c->active = 0;
         c->active_edges = 0ull;
-        c->touched = 0;  // the hubs the pull leaves to k_ms_pull_hub
-    } else {
-        c->touched = 0;
+    }
+    if (!pull) {
         c->q[c->cur ^ 1] = 0ull;
         if (c->mode == 1) c->q[c->cur] = 0ull;  // refilled by k_ms_dense2q
     }
 }
 
-__device__ void ms_end(MsCtrl *c, int pull) {
-    if (pull) {
+__device__ void ms_end(MsCtrl *c, int pull, int wide) {
+    if (wide) {
+        if (c->nkeep < kMsKeep) c->keep_lvl[c->nkeep++] = c->step + 1;
         c->cur ^= 1;
         c->mode = 1;
         c->q[0] = c->q[1] = 0ull;
-        c->pulls++;
     } else {
         const unsigned long long qn = ldg2(&c->q[c->cur ^ 1]);
         c->q[c->cur] = 0ull;
@@ -522,8 +598,9 @@ __device__ void ms_end(MsCtrl *c, int pull) {
         c->mode = 0;
         c->active = (uint32_t)(qn >> 32);
         c->active_edges = (uint32_t)qn;
-        c->pushes++;
     }
+    if (pull) c->pulls++;
+    else c->pushes++;
     c->live = c->live_next;
     c->live_next = 0ull;
     c->step++;
@@ -549,7 +626,7 @@ __global__ void k_ms_select(MsArgs a, int cap, cudaGraphConditionalHandle h_cont
         c->p.launches++;
         if (c->pending) {
             c->pending = 0;
-            ms_end(c, c->last_pull);
+            ms_end(c, c->last_pull, c->last_wide);
         }
         c->iter++;
         if (c->iter > cap && !c->done) {
@@ -596,32 +673,67 @@ __global__ void k_ms_select(MsArgs a, int cap, cudaGraphConditionalHandle h_cont
     }
     const int pull = pull_family(s);
     c->sched = pull ? MB_SCHED_PULL_THREAD : MB_SCHED_PUSH_EDGE_QUEUE;
-    c->branch = pull ? kMsBranchPull : (c->mode == 1 ? kMsBranchDensePush : kMsBranchPush);
-    ms_begin(c, pull);
+    const int wide = pull || (unsigned long long)c->active_edges * kMsWideDiv >= (unsigned long long)a.V;
+    c->branch = pull ? kMsBranchPull
+                     : wide ? (c->mode == 1 ? kMsBranchDenseWidePush : kMsBranchWidePush)
+                            : (c->mode == 1 ? kMsBranchDensePush : kMsBranchPush);
+    ms_begin(c, pull, wide);
     c->last_pull = pull;
+    c->last_wide = wide;
     c->pending = 1;
     if (use_handles) cudaGraphSetConditional(h_branch, (unsigned)c->branch);
 }
 
-// per-source traversal count: sum over v of popc(seen[v]) * outdeg[v]; and
-// the -1 of every (source, vertex) not reached, so that the levels need no
-// fill of nsrc * V entries before the run
-__global__ void k_ms_stats(MsArgs a, unsigned long long *out) {
+// End of a run.  The levels of the kept frontiers, and -1 of every (source,
+// vertex) not reached: each line of the output is written once, source by
+// source over 32 consecutive vertices, where a store per superstep wrote the
+// same lines in parts several times over (and a fill before the run once
+// more).  A vertex's bit is set in at most one kept frontier, so the index
+// of that frontier is three bit planes over the sources (the levels' stores in
+// the pulls were 1.1 ms of 3.9 on R-MAT 2^22 / 2^26 with 64 sources).  Then the
+// per-source traversal count, the sum over v of popc(seen[v]) * outdeg[v].
+__global__ void __launch_bounds__(256) k_ms_finish(MsArgs a, unsigned long long *out) {
     ms_count_launch(a);
+    static_assert(kMsKeep == 8, "three bit planes");
+    const int lane = threadIdx.x & 31;
+    const int nkeep = a.c->nkeep;
+    const int32_t my_lvl = lane < nkeep ? a.c->keep_lvl[lane] : -1;  // lane 8 and past: -1 (not reached)
     unsigned long long er = 0, vr = 0;
     for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll; b < a.V;
          b += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = b + (threadIdx.x & 31);
-        const unsigned long long sn = v < a.V ? a.seen[v] : a.all;
-        write_levels_warp(a, (int32_t)v, a.all & ~sn, -1);
-        if (v >= a.V) continue;
-        const int p = __popcll(sn);
-        vr += p;
-        er += (unsigned long long)p * (uint32_t)a.outdeg[v];
+        const int64_t v = b + lane;
+        const bool in = v < a.V;
+        const unsigned long long sn = in ? a.seen[v] : a.all;
+        unsigned long long m[kMsKeep];
+#pragma unroll
+        for (int p = 0; p < kMsKeep; p++) m[p] = in && p < nkeep ? a.keep[(size_t)p * a.V + v] : 0ull;
+        const unsigned long long b0 = m[1] | m[3] | m[5] | m[7], b1 = m[2] | m[3] | m[6] | m[7],
+                                 b2 = m[4] | m[5] | m[6] | m[7];
+        const unsigned long long none = a.all & ~sn;  // no plane has these bits
+        const unsigned long long set = m[0] | b0 | b1 | b2 | none;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t p0 = (uint32_t)(b0 >> (32 * h)), p1 = (uint32_t)(b1 >> (32 * h)),
+                           p2 = (uint32_t)(b2 >> (32 * h)), p3 = (uint32_t)(none >> (32 * h)),
+                           st = (uint32_t)(set >> (32 * h));
+            const int n = min(32, a.nsrc - 32 * h);
+            int32_t *lp = a.levels + (size_t)(32 * h) * a.V + v;
+            for (int s = 0; s < n; s++, lp += a.V) {
+                const int k = (int)(((p0 >> s) & 1u) | (((p1 >> s) & 1u) << 1) | (((p2 >> s) & 1u) << 2) |
+                                    (((p3 >> s) & 1u) << 3));
+                const int32_t lvl = __shfl_sync(0xffffffffu, my_lvl, k);
+                if ((st >> s) & 1u) *lp = lvl;
+            }
+        }
+        if (in) {
+            const int p = __popcll(sn);
+            vr += p;
+            er += (unsigned long long)p * (uint32_t)a.outdeg[v];
+        }
     }
     er = warp_sum(er);
     vr = warp_sum(vr);
-    if ((threadIdx.x & 31) == 0 && (er | vr)) {
+    if (lane == 0 && (er | vr)) {
         atomicAdd(&out[0], er);
         atomicAdd(&out[1], vr);
     }
@@ -639,6 +751,7 @@ void MsBfsState::ensure(const Graph &g) {
     front[0].reserve(8 * vb);
     front[1].reserve(8 * vb);
     nxt.reserve(8 * vb);
+    keep.reserve(8 * vb * kMsKeep);
     touched.reserve(4 * vb);
     const size_t tiles = (size_t)(E / kTile) + 2;
     for (int i = 0; i < 2; i++) {
@@ -670,6 +783,7 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
     a.front[0] = st.front[0].as<unsigned long long>();
     a.front[1] = st.front[1].as<unsigned long long>();
     a.nxt = st.nxt.as<unsigned long long>();
+    a.keep = st.keep.as<unsigned long long>();
     a.touched = st.touched.as<int32_t>();
     for (int i = 0; i < 2; i++) {
         a.qv[i] = st.qv[i].as<int32_t>();
@@ -700,14 +814,19 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
             k_ms_pull<<<gv, 256, 0, cs>>>(a);
             if (g.max_indeg > kMsHubMin) k_ms_pull_hub<<<ctx.num_sms * 2, kMsHubThreads, 0, cs>>>(a);
         } else {
-            if (b == kMsBranchDensePush) k_ms_dense2q<<<gv, 256, 0, cs>>>(a);
-            k_ms_push<<<gp, kPushThreads, 0, cs>>>(a);
-            k_ms_commit<<<gv, 256, 0, cs>>>(a);
+            if (b == kMsBranchDensePush || b == kMsBranchDenseWidePush) k_ms_dense2q<<<gv, 256, 0, cs>>>(a);
+            if (b == kMsBranchWidePush || b == kMsBranchDenseWidePush) {
+                k_ms_push<true><<<gp, kPushThreads, 0, cs>>>(a);
+                k_ms_commit_wide<<<gv, 256, 0, cs>>>(a);
+            } else {
+                k_ms_push<false><<<gp, kPushThreads, 0, cs>>>(a);
+                k_ms_commit<<<gv, 256, 0, cs>>>(a);
+            }
         }
         MB_CHECK_LAUNCH();
     };
     auto epilogue = [&](cudaStream_t cs) {
-        k_ms_stats<<<gv, 256, 0, cs>>>(a, st.stats.as<unsigned long long>());
+        k_ms_finish<<<gv, 256, 0, cs>>>(a, st.stats.as<unsigned long long>());
         MB_CHECK_LAUNCH();
     };
 

@@ -10,7 +10,7 @@ struct MsBfsState {
     bool built = false;
     int32_t V = 0;
     int64_t E = 0;
-    DevBuf seen, front[2], nxt, touched, qv[2], qo[2], tf[2], ctrl, stats, srcs, out;
+    DevBuf seen, front[2], nxt, keep, touched, qv[2], qo[2], tf[2], ctrl, stats, srcs, out;
     // the loop graph and what it was built for (output buffer, batch size, weights)
     LoopGraph lg;
     const void *key_levels = nullptr;
@@ -20,7 +20,8 @@ struct MsBfsState {
     void release() {
         lg.reset();
         key_levels = nullptr;
-        seen.release(); front[0].release(); front[1].release(); nxt.release(); touched.release();
+        seen.release(); front[0].release(); front[1].release(); nxt.release(); keep.release();
+        touched.release();
         for (int i = 0; i < 2; i++) { qv[i].release(); qo[i].release(); tf[i].release(); }
         ctrl.release(); stats.release(); srcs.release(); out.release();
         built = false;
