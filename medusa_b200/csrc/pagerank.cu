@@ -11,12 +11,11 @@
 //
 // The sum runs in the fixed order of pr_order.cuh, the same for every
 // schedule, so schedules never change a bit of the result.  Work mapping:
-//   light vertices (in-degree <= kPrLight): their in-edge sources are copied
-//     once per graph into a compacted list; one warp per 32 x VPL (1, 2 or
-//     4) consecutive light vertices streams their in-edges through a
-//     shared-memory window (coalesced) and each lane folds its own vertices
-//     (k_pr_light; the message-reading schedule uses k_pr_pull over the
-//     full reverse CSR);
+//   light vertices (in-degree <= kPrLight): a sliced ELL (PrSell, k_pr_sell),
+//     vertices sorted by in-degree, 32 per group, row j holding slot j of
+//     each, so a warp reads a row of in-edge sources with one coalesced load
+//     and lane l folds its own vertex (the message-reading schedule uses
+//     k_pr_pull over the full reverse CSR);
 //   heavier vertices: their kPrBlock-edge blocks form a work list built once
 //     per graph, one 16-byte item per block (edge range, vertex, slot); one
 //     warp per long item, or 1, 2 or 4 short items per warp
@@ -39,14 +38,16 @@ namespace {
 constexpr int kWin = 512;                // edges staged per warp per window
 constexpr int kPrWarps = 8;              // warps per CTA
 constexpr int kPrThreads = kPrWarps * 32;
-
 struct PrArgs {
     int32_t V;
     int64_t E;
-    const int32_t *rrow, *rcol, *outdeg, *row, *mslot;  // rcol/mslot: of the order in use
-    const float *contrib_in;   // rank[u]/outdeg[u] of the previous superstep
+    const int32_t *rrow, *outdeg, *row, *mslot;  // mslot: of the order in use
+    // contributions by position (k_pos): rank[u]/outdeg[u] of the previous
+    // superstep at pos[u]
+    const int32_t *pos;
+    const float *contrib_in;
     float *contrib_out;
-    float *rank_out;
+    float *rank_out;           // null but in the last superstep: no other reads the ranks
     float *msg;                // E-slot message array (schedule 6)
     const int4 *items;           // heavy blocks: {j0, j1, vertex, hub slot or -1}
     int32_t nitems;
@@ -55,20 +56,21 @@ struct PrArgs {
     int32_t nhub;
     float *blk_sum;              // per-slot block sums of the hubs
     int32_t nlong;               // items [0, nlong) are longer than kPrShortItem
-    const int32_t *light_v;      // light vertices, id order
-    const int32_t *light_row;    // their in-edge offsets into light_col (nlight+1)
-    const int32_t *light_col;    // their in-edge sources, reverse-CSR order
-    int32_t nlight;
+    const int32_t *hcol;         // positions of the in-edge sources, reverse-CSR order
 };
 
-__device__ __forceinline__ void pr_write(const PrArgs &a, int32_t v, float sum, int32_t d) {
+// New rank and contribution of a vertex at position p (-1: no out-edges) with
+// out-degree d; MPG/CPUFunctorHoster.cpp:80-82.
+template <class Args>
+__device__ __forceinline__ void pr_write(const Args &a, int32_t v, float sum, int32_t p, int32_t d) {
     const float r = pr_update(sum);
-    a.rank_out[v] = r;
-    a.contrib_out[v] = d > 0 ? r / (float)d : 0.0f;  // MPG/CPUFunctorHoster.cpp:80-82
+    if (a.rank_out) a.rank_out[v] = r;
+    if (p >= 0) a.contrib_out[p] = r / (float)d;
 }
 
-__device__ __forceinline__ void pr_write(const PrArgs &a, int32_t v, float sum) {
-    pr_write(a, v, sum, a.outdeg[v]);
+template <class Args>
+__device__ __forceinline__ void pr_write(const Args &a, int32_t v, float sum) {
+    pr_write(a, v, sum, a.pos[v], a.outdeg[v]);
 }
 
 // Streamed index arrays (read once per superstep) bypass L1, which is left
@@ -81,12 +83,19 @@ __device__ __forceinline__ int32_t ld_stream(const int32_t *p) {
     return v;
 }
 
-__device__ __forceinline__ float ld_gather(const float *p) { return __ldg(p); }
+// The gathers of contributions are what bounds a superstep: a random 4-byte
+// load is one L1 lookup, and where it misses one request and 32-byte sector
+// from L2 (measured on tables of 4 to 64 MB: 285 G loads/s, one per clock
+// and SM; 800 from L1).  Holding the hottest 32K contributions in shared
+// memory (1300 G loads/s) instead made these kernels slower: one CTA of 1024
+// threads per SM keeps too few gathers in flight (R-MAT 2^24 / 2^28: 1.13
+// against 1.09 ms a superstep; 2^20.3 / 17M: 0.081 against 0.074).
+__device__ __forceinline__ float ld_gather(const float *c, int32_t i) { return __ldg(c + i); }
 
 template <bool kFromMsg>
 __device__ __forceinline__ float edge_val(const PrArgs &a, int64_t j) {
     if (kFromMsg) return a.msg[j];
-    return ld_gather(&a.contrib_in[ld_stream(&a.rcol[j])]);
+    return ld_gather(a.contrib_in, ld_stream(&a.hcol[j]));
 }
 
 // Heavy-vertex blocks (<= kPrBlock in-edges each), summed exactly as
@@ -111,7 +120,7 @@ __host__ __device__ __forceinline__ int64_t heavy_units(int32_t nitems, int32_t 
 
 __device__ __forceinline__ void heavy_finish(const PrArgs &a, const int4 &it, float acc, int32_t d) {
     if (it.w == -2) return;  // past the list
-    if (it.w < 0) pr_write(a, it.z, 0.f + acc, d);  // one block sum folded from 0
+    if (it.w < 0) pr_write(a, it.z, 0.f + acc, __ldg(&a.pos[it.z]), d);  // one block sum folded from 0
     else a.blk_sum[it.w] = acc;
 }
 
@@ -244,146 +253,259 @@ __global__ void __launch_bounds__(kPrThreads) k_pr_pull(PrArgs a) {
     }
 }
 
-// Fused combine+update of the light vertices (in-degree <= kPrLight) from
-// the compacted light lists: one warp per group of 32 * kVPL consecutive
-// light vertices (lane l owns the group's vertices l, l+32, ...).  The warp
-// streams the group's in-edge sources (contiguous in light_col) through a
-// shared-memory window of gathered contributions, every load of a window in
-// flight at once, and each lane folds its vertices' parts of the window in
-// order: the sequential fold of pr_order.cuh.
-template <int kVPL>
-__global__ void __launch_bounds__(kPrThreads) k_pr_light(PrArgs a) {
-    __shared__ float win[kPrWarps][kWin];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float *wv = win[wid];
-    constexpr int kG = 32 * kVPL;
-    const int64_t ngroups = ((int64_t)a.nlight + kG - 1) / kG;
-    const int64_t warps = (int64_t)gridDim.x * kPrWarps;
-    for (int64_t grp = (int64_t)blockIdx.x * kPrWarps + wid; grp < ngroups; grp += warps) {
-        const int32_t i0 = (int32_t)(grp * kG);
-        const int32_t iend = (int32_t)min((int64_t)i0 + kG, (int64_t)a.nlight);
-        int32_t v[kVPL], b[kVPL], e[kVPL], d[kVPL];
-        float sum[kVPL];
+// ---- sliced ELL ------------------------------------------------------------------
+// Vertices sorted by in-degree (largest first), 32 per group: a group's rows
+// are its first vertex's in-degree, at most 31 slots of padding per group.
+// Light vertices in both orders, and mid vertices (up to hub_min in-edges) in
+// the reference's order.
+struct SellArgs {
+    const int32_t *v;       // 32 per group (-1: padding)
+    const int2 *pd;         // their contribution positions and out-degrees
+    const int32_t *rows;    // rows of each group
+    const uint32_t *base;   // rows before it
+    const int32_t *src;     // position of group g, row j, lane l's source at 32 (base[g] + j) + l (-1: padding)
+    int32_t ngroups, nlong; // groups [0, nlong) have more than kSellShort rows
+    const float *contrib_in;
+    float *contrib_out, *rank_out;
+    uint32_t *ctr;          // units taken by late warps, zero before the launch
+};
+constexpr int kSellShort = 8;
+// Two builds of the kernel: 16 rows in flight and at least 5 CTAs per SM, or
+// 8 and 8 CTAs, which every unit of a small graph fits into at once (R-MAT
+// 2^24 / 2^28: 0.955 against 1.011 ms a superstep; uniform 2^18 / 2^22: 25.8
+// against 22.8 us).
+constexpr int kSellU = 16, kSellCtas = 5, kSellUSmall = 8, kSellCtasSmall = 8;
+
+// One group: kSellU rows (coalesced index loads, then the gathers) in
+// flight; each lane folds its own vertex's slots in order.  Padding slots
+// (-1) read 0, and s + 0 = s, so they change no bit.
+template <int kSellU>
+__device__ __forceinline__ void sell_long(const SellArgs &a, int64_t g) {
+    const int lane = threadIdx.x & 31;
+    const int32_t rows = __ldg(&a.rows[g]);
+    const int2 pd = __ldg(&a.pd[g * 32 + lane]);
+    const int32_t *src = a.src + (int64_t)__ldg(&a.base[g]) * 32 + lane;
+    float sum = 0.f;
+    // the next rows' indices load while this block's gathers are in flight
+    int32_t nxt[kSellU];
 #pragma unroll
-        for (int i = 0; i < kVPL; i++) {
-            const int32_t idx = i0 + 32 * i + lane;
-            v[i] = -1;
-            b[i] = e[i] = 0;
-            sum[i] = 0.f;
-            if (idx < iend) {
-                v[i] = ld_stream(&a.light_v[idx]);
-                b[i] = ld_stream(&a.light_row[idx]);
-                e[i] = ld_stream(&a.light_row[idx + 1]);
+    for (int u = 0; u < kSellU; u++) nxt[u] = u < rows ? ld_stream(src + (int64_t)u * 32) : -1;
+    for (int32_t j0 = 0; j0 < rows; j0 += kSellU) {
+        int32_t idx[kSellU];
+#pragma unroll
+        for (int u = 0; u < kSellU; u++) idx[u] = nxt[u];
+#pragma unroll
+        for (int u = 0; u < kSellU; u++) {
+            const int32_t j = j0 + kSellU + u;
+            nxt[u] = j < rows ? ld_stream(src + (int64_t)j * 32) : -1;
+        }
+        float x[kSellU];
+#pragma unroll
+        for (int u = 0; u < kSellU; u++) x[u] = idx[u] >= 0 ? ld_gather(a.contrib_in, idx[u]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < kSellU; u++) sum += x[u];
+    }
+    const int32_t v = a.rank_out ? a.v[g * 32 + lane] : 0;
+    if (v >= 0) pr_write(a, v, sum, pd.x, pd.y);
+}
+
+// kG consecutive groups of at most kSellShort rows at once: a group alone
+// would leave a lane with a handful of gathers in flight.
+template <int kG>
+__device__ __forceinline__ void sell_short(const SellArgs &a, int64_t g0) {
+    constexpr int kR = 16 / kG;
+    const int lane = threadIdx.x & 31;
+    int32_t rows[kG];
+    int2 pd[kG];
+    const int32_t *src[kG];
+    float sum[kG];
+#pragma unroll
+    for (int i = 0; i < kG; i++) {
+        const bool in = g0 + i < a.ngroups;
+        rows[i] = in ? __ldg(&a.rows[g0 + i]) : 0;
+        pd[i] = in ? __ldg(&a.pd[(g0 + i) * 32 + lane]) : make_int2(-1, 0);
+        src[i] = a.src + (in ? (int64_t)__ldg(&a.base[g0 + i]) * 32 + lane : 0);
+        sum[i] = 0.f;
+    }
+    const int32_t rmax = rows[0];
+    for (int32_t j0 = 0; j0 < rmax; j0 += kR) {
+        int32_t idx[kG][kR];
+        float x[kG][kR];
+#pragma unroll
+        for (int i = 0; i < kG; i++)
+#pragma unroll
+            for (int u = 0; u < kR; u++)
+                idx[i][u] = j0 + u < rows[i] ? ld_stream(src[i] + (int64_t)(j0 + u) * 32) : -1;
+#pragma unroll
+        for (int i = 0; i < kG; i++)
+#pragma unroll
+            for (int u = 0; u < kR; u++) x[i][u] = idx[i][u] >= 0 ? ld_gather(a.contrib_in, idx[i][u]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < kG; i++)
+#pragma unroll
+            for (int u = 0; u < kR; u++) sum[i] += x[i][u];
+    }
+#pragma unroll
+    for (int i = 0; i < kG; i++) {
+        if (g0 + i >= a.ngroups) break;
+        const int32_t v = a.rank_out ? a.v[(g0 + i) * 32 + lane] : 0;
+        if (v >= 0) pr_write(a, v, sum[i], pd[i].x, pd[i].y);
+    }
+}
+
+// A warp's first unit is its number; the next ones come from the counter, so
+// that CTAs which start late (the hub scans hold SMs) take no share of their
+// own.  Longest groups first.
+template <int kG, bool kSmall>
+__global__ void __launch_bounds__(256, kSmall ? kSellCtasSmall : kSellCtas) k_pr_sell(SellArgs a) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t units = (uint32_t)a.nlong + (uint32_t)(a.ngroups - a.nlong + kG - 1) / kG;
+    uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    while (u < units) {
+        uint32_t t = 0;  // the next unit's number is on its way during this one
+        if ((threadIdx.x & 31) == 0 && warps < units) t = atomicAdd(a.ctr, 1u);
+        if (u < (uint32_t)a.nlong) sell_long<kSmall ? kSellUSmall : kSellU>(a, u);
+        else sell_short<kG>(a, a.nlong + (int64_t)(u - a.nlong) * kG);
+        if (warps >= units) break;
+        u = warps + __shfl_sync(0xffffffffu, t, 0);
+    }
+}
+
+// All supersteps in one cooperative launch, for graphs whose groups fit one
+// to a resident warp and that have no other vertices: the group's head and
+// the first rows' indices are loaded before the barrier between two
+// supersteps, and no superstep waits for a launch.  Contributions are read
+// with plain loads (other SMs write them during the launch; the barrier's
+// acquire drops stale L1 lines).  A barrier that gives up writes *err (host
+// memory) and ends the launch.  Uniform 2^18 / 2^22, ten supersteps: 20.4 us
+// each, against 22.8 in launches of their own (the gathers alone: 14).
+constexpr int kResThreads = 1024, kResCtas = 2;  // 32 registers: 64 warps per SM
+constexpr int kResU = 8;
+struct ResidentArgs {
+    float *contrib[2], *rank;
+    const int32_t *zv;  // vertices without in-edges
+    const int2 *zpd;
+    int32_t nz, iters;
+    uint32_t *bar;      // arrivals, zero before the launch; top bit: a wait gave up
+    volatile int *err;
+    long polls;
+};
+__device__ __forceinline__ bool resident_sync(const ResidentArgs &a, uint32_t target) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        constexpr uint32_t kGaveUp = 1u << 31;
+        __threadfence();
+        atomicAdd(a.bar, 1u);
+        int ok = 0;
+        for (long it = 0;; it++) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+            if (v >= kGaveUp) break;
+            if (v >= target) {
+                ok = 1;
+                break;
+            }
+            if (it >= a.polls) {
+                *a.err = 1;
+                atomicOr(a.bar, kGaveUp);
+                break;
             }
         }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok;
+}
+__global__ void __launch_bounds__(kResThreads, kResCtas) k_pr_resident(SellArgs a, ResidentArgs r) {
+    const int lane = threadIdx.x & 31;
+    // the longest groups spread over the CTAs
+    const int32_t g = (int32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+    const bool in = g < a.ngroups;
+    const int32_t rows = in ? __ldg(&a.rows[g]) : 0;
+    const int2 pd = in ? __ldg(&a.pd[(int64_t)g * 32 + lane]) : make_int2(-1, 0);
+    const int32_t *src = a.src + (in ? (int64_t)__ldg(&a.base[g]) * 32 + lane : 0);
+    uint32_t target = 0;
+    for (int it = 0; it < r.iters; it++) {
+        int32_t idx[kResU];
 #pragma unroll
-        for (int i = 0; i < kVPL; i++) d[i] = v[i] >= 0 ? __ldg(&a.outdeg[v[i]]) : 0;
-        const int32_t g0 = __ldg(&a.light_row[i0]), g1 = __ldg(&a.light_row[iend]);
-        for (int32_t w0 = g0; w0 < g1; w0 += kWin) {
-            const int32_t w1 = min(w0 + kWin, g1);
-            int32_t src[kWin / 32];
-#pragma unroll
-            for (int r = 0; r < kWin / 32; r++) {
-                const int32_t j = w0 + lane + 32 * r;
-                src[r] = j < w1 ? ld_stream(&a.light_col[j]) : -1;
-            }
-            float vals[kWin / 32];
-#pragma unroll
-            for (int r = 0; r < kWin / 32; r++) vals[r] = src[r] >= 0 ? ld_gather(&a.contrib_in[src[r]]) : 0.f;
-#pragma unroll
-            for (int r = 0; r < kWin / 32; r++) wv[lane + 32 * r] = vals[r];
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < kVPL; i++) {
-                const int32_t lo = max(b[i], w0), hi = min(e[i], w1);
-                for (int32_t j = lo; j < hi; j++) sum[i] += wv[j - w0];
-            }
-            __syncwarp();
+        for (int u = 0; u < kResU; u++) idx[u] = u < rows ? __ldg(src + u * 32) : -1;
+        if (it > 0) {
+            target += gridDim.x;
+            if (!resident_sync(r, target)) return;
         }
+        const float *cin = it & 1 ? r.contrib[1] : r.contrib[0];
+        float *cout = it & 1 ? r.contrib[0] : r.contrib[1];
+        float *rank = it == r.iters - 1 ? r.rank : nullptr;
+        float sum = 0.f;
+        for (int32_t j0 = 0; j0 < rows; j0 += kResU) {
+            float x[kResU];
 #pragma unroll
-        for (int i = 0; i < kVPL; i++)
-            if (v[i] >= 0) pr_write(a, v[i], sum[i], d[i]);
+            for (int u = 0; u < kResU; u++) x[u] = idx[u] >= 0 ? cin[idx[u]] : 0.f;
+#pragma unroll
+            for (int u = 0; u < kResU; u++) {
+                const int32_t j = j0 + kResU + u;
+                idx[u] = j < rows ? __ldg(src + j * 32) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < kResU; u++) sum += x[u];
+        }
+        if (rows) {
+            const float nr = pr_update(sum);
+            if (pd.x >= 0) cout[pd.x] = nr / (float)pd.y;
+            if (rank) {
+                const int32_t v = a.v[(int64_t)g * 32 + lane];
+                if (v >= 0) rank[v] = nr;
+            }
+        }
+        if (it < 2 || rank) {
+            const float zr = pr_update(0.f);
+            for (int32_t i = blockIdx.x * kResThreads + threadIdx.x; i < r.nz; i += gridDim.x * kResThreads) {
+                const int2 p = r.zpd[i];
+                if (it < 2 && p.x >= 0) cout[p.x] = zr / (float)p.y;
+                if (rank) rank[r.zv[i]] = zr;
+            }
+        }
+    }
+}
+
+// Vertices without in-edges: their sum is 0 in every superstep, so their
+// contributions are written once to each of the two buffers.
+__global__ void k_pr_zero(const int32_t *v, const int2 *pd, int32_t n, float *contrib, float *rank) {
+    const float r = pr_update(0.f);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int2 p = pd[i];
+        if (contrib && p.x >= 0) contrib[p.x] = r / (float)p.y;
+        if (rank) rank[v[i]] = r;
     }
 }
 
 // ---- the reference's order (MB_PR_ORDER_REFERENCE), in parallel -------------
 // Every vertex's sum is the reference's sequential float fold over its MEG
-// slots, bit for bit (pr_order.cuh).  Three mappings by in-degree n:
-//   n <= kPrLight: k_pr_light over light lists copied from the MEG order;
-//   kPrLight < n <= hub_min: sliced ELL -- vertices sorted by in-degree, 32
-//     per group; row j of a group holds slot j of each of its vertices, so a
-//     warp reads a row with one coalesced load and lane l folds its own
-//     vertex in order (k_pr_sell, on a second side stream beside the light
-//     kernel);
+// slots, bit for bit (pr_order.cuh).  Two mappings by in-degree n:
+//   n <= hub_min: the sliced ELL above, filled in MEG slot order;
 //   n > hub_min: the contributions staged by every SM into one contiguous run
-//     per vertex (k_pr_hub_stage), then one CTA per vertex runs the parallel
-//     integer scan of pr_order.cuh over it (k_pr_hub_exact), on a side
-//     stream beside the others.
-#ifndef MB_SELL_U
-#define MB_SELL_U 16
-#endif
-constexpr int kSellU = MB_SELL_U;               // rows of a group in flight
+//     per vertex (k_pr_hub_stage), then one warp or CTA per vertex runs the
+//     parallel integer scan of pr_order.cuh over it (k_pr_hub_warp,
+//     k_pr_hub_exact), on side streams beside the sliced ELL.
 constexpr int kHubK = 16;                       // consecutive slots per thread
 constexpr int kHubBig = 16384;                  // in-degree above which a hub gets the big CTA
 constexpr int kHubMinDefault = 2048;
 
 struct ExactArgs {
-    const int32_t *rrow, *meg_src, *outdeg;
+    const int32_t *rrow, *outdeg;
+    const int32_t *pos;          // contribution positions, as in PrArgs
     const float *contrib_in;
     float *contrib_out, *rank_out;
-    const int32_t *sell_v;       // 32 vertices per group (-1: padding), sorted by in-degree
-    const int64_t *sell_base;    // first element of each group in sell_src
-    const int32_t *sell_rows;    // rows of each group (its largest in-degree)
-    const int32_t *sell_src;     // group g, row j, lane l at sell_base[g] + 32 j + l (-1: padding)
-    int32_t ngroups;
     const int32_t *hub_v;        // hubs, largest in-degree first
     int32_t nhub;
     float *x_stage;              // every hub's contributions, in MEG slot order
     const int64_t *stage_off;    // where hub h's run starts (16-byte aligned)
-    const int4 *stage_items;     // staging work: {stage offset, meg_src offset, length, 0}
+    const int32_t *stage_src;    // positions of their sources, at the same offsets
+    const int2 *stage_items;     // staging work: {offset, length}
     int32_t nstage_items;
 };
-
-__device__ __forceinline__ void x_write(const ExactArgs &a, int32_t v, float sum, int32_t d) {
-    const float r = pr_update(sum);
-    a.rank_out[v] = r;
-    a.contrib_out[v] = d > 0 ? r / (float)d : 0.0f;
-}
-
-// Sliced ELL: one warp per group, kSellU rows (coalesced index loads, then
-// the gathers) in flight; each lane folds its own vertex's slots in order.
-// Padding slots (-1) read 0, and s + 0 = s, so they change no bit.
-__global__ void __launch_bounds__(256) k_pr_sell(ExactArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < a.ngroups; g += warps) {
-        const int32_t v = __ldg(&a.sell_v[g * 32 + lane]);
-        const int32_t rows = __ldg(&a.sell_rows[g]);
-        const int32_t d = v >= 0 ? __ldg(&a.outdeg[v]) : 0;
-        const int32_t *src = a.sell_src + __ldg(&a.sell_base[g]) + lane;
-        float sum = 0.f;
-        // the next rows' indices load while this block's gathers are in flight
-        int32_t nxt[kSellU];
-#pragma unroll
-        for (int u = 0; u < kSellU; u++) nxt[u] = u < rows ? ld_stream(src + (int64_t)u * 32) : -1;
-        for (int32_t j0 = 0; j0 < rows; j0 += kSellU) {
-            int32_t idx[kSellU];
-#pragma unroll
-            for (int u = 0; u < kSellU; u++) idx[u] = nxt[u];
-#pragma unroll
-            for (int u = 0; u < kSellU; u++) {
-                const int32_t j = j0 + kSellU + u;
-                nxt[u] = j < rows ? ld_stream(src + (int64_t)j * 32) : -1;
-            }
-            float x[kSellU];
-#pragma unroll
-            for (int u = 0; u < kSellU; u++) x[u] = idx[u] >= 0 ? ld_gather(&a.contrib_in[idx[u]]) : 0.f;
-#pragma unroll
-            for (int u = 0; u < kSellU; u++) sum += x[u];
-        }
-        if (v >= 0) x_write(a, v, sum, d);
-    }
-}
 
 // Staging: every hub's contributions gathered, in MEG slot order, into one
 // contiguous run per hub (x_stage), by all SMs at once: one warp per item of
@@ -393,36 +515,41 @@ __global__ void __launch_bounds__(256) k_pr_sell(ExactArgs a) {
 #ifndef MB_STAGE_ITEM
 #define MB_STAGE_ITEM 1024
 #endif
-// The sliced ELL runs on its own stream beside the light kernel and the hub
-// scans, on half its resident grid.  Measured per 20 supersteps against the
-// three in line on one stream: C5 27.7 against 28.0 ms, the C5 generator
-// at 2^21 / 2^25 3.77 against 4.60, R-MAT 2^20 / 2^24 1.00 against 1.23
-// (forked before the staging kernel instead, C5 lost 7%: the staging that
-// the big hubs' scans wait for ran slower).
-constexpr int kSellGridDiv = 2;  // C5: 24.0 ms per 20 supersteps, against 25.1 at 1 and 28.0 at 3
 constexpr int kStageItem = MB_STAGE_ITEM;
 constexpr int kStageU = 8;
-__global__ void __launch_bounds__(256) k_pr_hub_stage(ExactArgs a) {
+__device__ __forceinline__ void stage_item(const ExactArgs &a, int64_t it) {
     const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < a.nstage_items; it += warps) {
-        const int4 item = __ldg(&a.stage_items[it]);
-        float *dst = a.x_stage + (uint32_t)item.x;
-        const int32_t *src = a.meg_src + (uint32_t)item.y;
-        for (int32_t k0 = 0; k0 < item.z; k0 += 32 * kStageU) {
-            float x[kStageU];
+    const int2 item = __ldg(&a.stage_items[it]);
+    float *dst = a.x_stage + (uint32_t)item.x;
+    const int32_t *src = a.stage_src + (uint32_t)item.x;
+    // the next indices load while these gathers are in flight
+    int32_t nxt[kStageU];
 #pragma unroll
-            for (int u = 0; u < kStageU; u++) {
-                const int32_t k = k0 + 32 * u + lane;
-                x[u] = k < item.z ? ld_gather(&a.contrib_in[ld_stream(src + k)]) : 0.f;
-            }
+    for (int u = 0; u < kStageU; u++) nxt[u] = 32 * u + lane < item.y ? ld_stream(src + 32 * u + lane) : -1;
+    for (int32_t k0 = 0; k0 < item.y; k0 += 32 * kStageU) {
+        int32_t idx[kStageU];
 #pragma unroll
-            for (int u = 0; u < kStageU; u++) {
-                const int32_t k = k0 + 32 * u + lane;
-                if (k < item.z) dst[k] = x[u];
-            }
+        for (int u = 0; u < kStageU; u++) idx[u] = nxt[u];
+#pragma unroll
+        for (int u = 0; u < kStageU; u++) {
+            const int32_t k = k0 + 32 * (kStageU + u) + lane;
+            nxt[u] = k < item.y ? ld_stream(src + k) : -1;
+        }
+        float x[kStageU];
+#pragma unroll
+        for (int u = 0; u < kStageU; u++) x[u] = idx[u] >= 0 ? ld_gather(a.contrib_in, idx[u]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < kStageU; u++) {
+            const int32_t k = k0 + 32 * u + lane;
+            if (k < item.y) dst[k] = x[u];
         }
     }
+}
+
+__global__ void __launch_bounds__(256) k_pr_hub_stage(ExactArgs a) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < a.nstage_items; it += warps)
+        stage_item(a, it);
 }
 
 // Scan thread t's kHubK consecutive staged values of the chunk at `pos`
@@ -543,7 +670,7 @@ __global__ void __launch_bounds__(kT) k_pr_hub_exact(ExactArgs a, int32_t h0, in
                 if (start >= kT) break;
             }
         }
-        if (tid == 0) x_write(a, v, s, __ldg(&a.outdeg[v]));
+        if (tid == 0) pr_write(a, v, s);
         __syncthreads();  // head and s_sh are reused by the next hub
     }
 }
@@ -609,34 +736,120 @@ __global__ void __launch_bounds__(256) k_pr_hub_warp(ExactArgs a, int32_t h0, in
                 if (start >= 32) break;
             }
         }
-        if (lane == 0) x_write(a, v, s, __ldg(&a.outdeg[v]));
+        if (lane == 0) pr_write(a, v, s);
     }
 }
 
-// Group g of the sliced ELL: row j, lane l <- slot j of the group's vertex l.
-__global__ void k_sell_fill(const int32_t *sell_v, const int64_t *sell_base, const int32_t *sell_rows,
-                            int32_t ngroups, const int32_t *rrow, const int32_t *meg_src, int32_t *sell_src) {
+// ---- building the sliced ELL (once per graph and order) ------------------------
+// Sort keys: vertices of more than max_rows in-edges first, then by in-degree
+// (largest first), those without in-edges last; counts[0], [1]: the first and
+// the last of these.
+__global__ void k_sell_keys(const int32_t *rrow, int32_t V, int32_t max_rows, uint32_t *key, uint32_t *val,
+                            uint32_t *counts) {
+    uint32_t nh = 0, nz = 0;
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t d = rrow[v + 1] - rrow[v];
+        key[v] = d > max_rows ? 0u : (uint32_t)(max_rows - d) + 1u;
+        val[v] = (uint32_t)v;
+        nh += d > max_rows;
+        nz += d == 0;
+    }
+    nh = __reduce_add_sync(0xffffffffu, nh);
+    nz = __reduce_add_sync(0xffffffffu, nz);
+    if ((threadIdx.x & 31) == 0) {
+        if (nh) atomicAdd(&counts[0], nh);
+        if (nz) atomicAdd(&counts[1], nz);
+    }
+}
+// rows of each group of the n vertices in `order`; counts[0]: groups longer than kSellShort
+__global__ void k_sell_rows(const uint32_t *order, int32_t n, int32_t ngroups, const int32_t *rrow, int32_t *rows,
+                            uint32_t *counts) {
+    uint32_t nl = 0;
+    for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gridDim.x * blockDim.x) {
+        const uint32_t v = order[(int64_t)g * 32];
+        const int32_t r = rrow[v + 1] - rrow[v];
+        rows[g] = r;
+        nl += r > kSellShort;
+    }
+    nl = __reduce_add_sync(0xffffffffu, nl);
+    if ((threadIdx.x & 31) == 0 && nl) atomicAdd(&counts[0], nl);
+}
+// Group g: row j, lane l <- position of slot j of the group's vertex l
+// (src: the slots of each destination, in the order of the sums).
+__global__ void k_sell_fill(const uint32_t *order, int32_t n, int32_t ngroups, const int32_t *rows,
+                            const uint32_t *base, const int32_t *rrow, const int32_t *src, const int32_t *pos,
+                            const int32_t *outdeg, int32_t *sell_v, int2 *sell_pd, int32_t *sell_src) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups; g += warps) {
-        const int32_t v = sell_v[g * 32 + lane];
-        const int32_t rows = sell_rows[g];
-        const int64_t b = v >= 0 ? rrow[v] : 0;
-        const int32_t n = v >= 0 ? rrow[v + 1] - (int32_t)b : 0;
-        int32_t *dst = sell_src + sell_base[g] + lane;
-        for (int32_t j = 0; j < rows; j++) dst[(int64_t)j * 32] = j < n ? meg_src[b + j] : -1;
+        const int64_t i = g * 32 + lane;
+        const int32_t v = i < n ? (int32_t)order[i] : -1;
+        sell_v[i] = v;
+        sell_pd[i] = v >= 0 ? make_int2(pos[v], outdeg[v]) : make_int2(-1, 0);
+        const int32_t b = v >= 0 ? rrow[v] : 0;
+        const int32_t m = v >= 0 ? rrow[v + 1] - b : 0;
+        int32_t *dst = sell_src + (int64_t)base[g] * 32 + lane;
+        const int32_t r = rows[g];
+        for (int32_t j = 0; j < r; j++) dst[(int64_t)j * 32] = j < m ? pos[src[b + j]] : -1;
+    }
+}
+__global__ void k_zero_fill(const uint32_t *order, int32_t n, const int32_t *pos, const int32_t *outdeg, int32_t *zv,
+                            int2 *zpd) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t v = (int32_t)order[i];
+        zv[i] = v;
+        zpd[i] = make_int2(pos[v], outdeg[v]);
+    }
+}
+// {first slot, in-degree} of the hubs
+__global__ void k_hub_info(const uint32_t *order, int32_t n, const int32_t *rrow, int2 *info) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t v = order[i];
+        info[i] = make_int2(rrow[v], rrow[v + 1] - rrow[v]);
     }
 }
 
-// Copy each light vertex's in-edge sources out of the reverse CSR.
-__global__ void k_light_copy(const int32_t *light_v, const int32_t *light_row, int32_t nlight,
-                             const int32_t *rrow, const int32_t *rcol, int32_t *light_col) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nlight;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t v = light_v[i], o = light_row[i];
-        const int32_t b = rrow[v], n = rrow[v + 1] - b;
-        for (int32_t k = 0; k < n; k++) light_col[o + k] = rcol[b + k];
+// Positions of the staged hubs' sources: item {stage offset, length} of the
+// slots from meg_off[item] on.
+__global__ void k_stage_fill(const int2 *items, const int32_t *meg_off, int32_t nitems, const int32_t *meg_src,
+                             const int32_t *pos, int32_t *stage_src) {
+    for (int32_t i = blockIdx.x; i < nitems; i += gridDim.x) {
+        const int2 it = items[i];
+        const int32_t o = meg_off[i];
+        for (int32_t k = threadIdx.x; k < it.y; k += blockDim.x)
+            stage_src[(int64_t)it.x + k] = pos[meg_src[(int64_t)o + k]];
     }
+}
+
+// ---- contribution layout ------------------------------------------------------
+// Sort key of a vertex: its out-degree class, four per octave, the largest
+// degrees first; vertices without out-edges last.
+constexpr int kDegClasses = 128;
+__host__ __device__ inline uint32_t degree_key(uint32_t d) {
+    if (d == 0) return kDegClasses;
+    uint32_t e = 0;
+    while (e < 31 && (d >> (e + 1))) e++;
+    const uint32_t frac = e >= 2 ? (d >> (e - 2)) & 3u : (d << (2 - e)) & 3u;
+    return kDegClasses - 1 - (4 * e + frac);
+}
+__global__ void k_deg_keys(const int32_t *outdeg, int32_t V, uint32_t *key, uint32_t *val) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        key[v] = degree_key((uint32_t)outdeg[v]);
+        val[v] = (uint32_t)v;
+    }
+}
+__global__ void k_pos(const uint32_t *key, const uint32_t *val, int32_t V, int32_t *pos) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V;
+         i += (int64_t)gridDim.x * blockDim.x)
+        pos[val[i]] = key[i] < kDegClasses ? (int32_t)i : -1;
+}
+
+__global__ void k_map_pos(const int32_t *src, int64_t E, const int32_t *pos, int32_t *out) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
+         e += (int64_t)gridDim.x * blockDim.x)
+        out[e] = pos[src[e]];
 }
 
 // Schedule 6, send (SendMsgAA, MPG/UserOperators.h:48-70): every vertex
@@ -644,25 +857,28 @@ __global__ void k_light_copy(const int32_t *light_v, const int32_t *light_row, i
 __global__ void k_pr_send(PrArgs a) {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < a.V;
          u += (int64_t)gridDim.x * blockDim.x) {
-        const float m = a.contrib_in[u];
-        for (int32_t e = a.row[u]; e < a.row[u + 1]; e++) a.msg[a.mslot[e]] = m;
+        const int32_t b = a.row[u], n = a.row[u + 1] - b;
+        if (n == 0) continue;
+        const float m = a.contrib_in[a.pos[u]];
+        for (int32_t e = b; e < b + n; e++) a.msg[a.mslot[e]] = m;
     }
 }
 
-__global__ void k_pr_init(const int32_t *outdeg, int32_t V, float init, float *contrib) {
+__global__ void k_pr_init(const int32_t *outdeg, const int32_t *pos, int32_t V, float init, float *contrib) {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < V;
          u += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = outdeg[u];
-        contrib[u] = d > 0 ? init / (float)d : 0.0f;
+        if (d > 0) contrib[pos[u]] = init / (float)d;
     }
 }
 
 // The first superstep's contributions from a given rank vector.
-__global__ void k_pr_init_vec(const int32_t *outdeg, int32_t V, const float *init, float *contrib) {
+__global__ void k_pr_init_vec(const int32_t *outdeg, const int32_t *pos, int32_t V, const float *init,
+                              float *contrib) {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < V;
          u += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = outdeg[u];
-        contrib[u] = d > 0 ? init[u] / (float)d : 0.0f;
+        if (d > 0) contrib[pos[u]] = init[u] / (float)d;
     }
 }
 
@@ -779,7 +995,30 @@ void PrState::ensure(Context &ctx, const Graph &g) {
     rank.reserve(sizeof(float) * (size_t)V);
     contrib[0].reserve(sizeof(float) * (size_t)V);
     contrib[1].reserve(sizeof(float) * (size_t)V);
-    msg.reserve(sizeof(float) * (size_t)std::max<int64_t>(E, 1));
+    // contribution layout: by out-degree class, id order within a class;
+    // vertices without out-edges send nothing and have no position
+    cudaStream_t s = ctx.stream;
+    const int gridV = grid_for(V, 256, ctx.num_sms * 16);
+    DevBuf key, val;
+    try {
+        key.reserve(sizeof(uint32_t) * (size_t)V);
+        val.reserve(sizeof(uint32_t) * (size_t)V);
+        pos.reserve(sizeof(int32_t) * (size_t)V);
+        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), V, key.as<uint32_t>(), val.as<uint32_t>());
+        MB_CHECK_LAUNCH();
+        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8, s);
+        k_pos<<<gridV, 256, 0, s>>>(key.as<uint32_t>(), val.as<uint32_t>(), V, pos.as<int32_t>());
+        MB_CUDA(cudaStreamSynchronize(s));
+    } catch (...) {
+        key.release(); val.release();
+        throw;
+    }
+    key.release(); val.release();
+    built = true;
+}
+
+void PrState::ensure_fixed(Context &ctx, const Graph &g) {
+    if (fixed_built) return;
     // heavy-vertex work list, built once per graph from the in-degree offsets:
     // one item per block; hubs (more than one block) get block-sum slots
     std::vector<int32_t> rrow(V + 1);
@@ -816,131 +1055,148 @@ void PrState::ensure(Context &ctx, const Graph &g) {
     copy_sync(ctx.stream, items.p, it.data(), sizeof(int4) * it.size());
     copy_sync(ctx.stream, hub_v.p, hv.data(), 4 * hv.size());
     copy_sync(ctx.stream, hub_first.p, hf.data(), 4 * hf.size());
-    // light lists: the vertices with in-degree <= kPrLight and their in-edges
-    std::vector<int32_t> lv, lr(1, 0);
-    lv.reserve((size_t)V);
-    lr.reserve((size_t)V + 1);
-    for (int32_t v = 0; v < V; v++) {
-        const int32_t d = rrow[v + 1] - rrow[v];
-        if (d > kPrLight) continue;
-        lv.push_back(v);
-        lr.push_back(lr.back() + d);
-    }
-    nlight = (int32_t)lv.size();
-    light_v.reserve(sizeof(int32_t) * std::max<size_t>(lv.size(), 1));
-    light_row.reserve(sizeof(int32_t) * lr.size());
-    light_col.reserve(sizeof(int32_t) * std::max<size_t>((size_t)lr.back(), 1));
-    if (nlight) {
-        copy_sync(ctx.stream, light_v.p, lv.data(), 4 * lv.size());
-        copy_sync(ctx.stream, light_row.p, lr.data(), 4 * lr.size());
-        k_light_copy<<<grid_for(nlight, 256, ctx.num_sms * 16), 256, 0, ctx.stream>>>(
-            light_v.as<int32_t>(), light_row.as<int32_t>(), nlight, g.rrow.as<int32_t>(),
-            g.rcol.as<int32_t>(), light_col.as<int32_t>());
+    if (nitems) {
+        hcol.reserve(sizeof(int32_t) * (size_t)E);
+        k_map_pos<<<grid_for(E, 256, ctx.num_sms * 16), 256, 0, ctx.stream>>>(
+            g.rcol.as<int32_t>(), E, pos.as<int32_t>(), hcol.as<int32_t>());
         MB_CHECK_LAUNCH();
-        MB_CUDA(cudaStreamSynchronize(ctx.stream));
     }
-    built = true;
+    build_sell(ctx, g, kPrLight, g.rcol.as<int32_t>(), light, nullptr);
+    fixed_built = true;
+}
+
+// The sliced ELL of the vertices with 1 to max_rows in-edges, the list of
+// those without any, and (hubs, when not null) the others' {vertex, first
+// slot, in-degree} in id order.
+void PrState::build_sell(Context &ctx, const Graph &g, int32_t max_rows, const int32_t *src, PrSell &out,
+                         std::vector<HubInfo> *hubs) {
+    cudaStream_t s = ctx.stream;
+    const int gridV = grid_for(V, 256, ctx.num_sms * 16);
+    max_rows = std::min(max_rows, g.max_indeg);
+    int bits = 1;
+    while (bits < 32 && ((int64_t)1 << bits) < (int64_t)max_rows + 2) bits++;
+    DevBuf key, val, cnt;
+    auto drop = [&] { key.release(); val.release(); cnt.release(); };
+    try {
+        key.reserve(sizeof(uint32_t) * (size_t)V);
+        val.reserve(sizeof(uint32_t) * (size_t)V);
+        cnt.reserve(4 * sizeof(uint32_t));
+        MB_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * sizeof(uint32_t), s));
+        k_sell_keys<<<gridV, 256, 0, s>>>(g.rrow.as<int32_t>(), V, max_rows, key.as<uint32_t>(), val.as<uint32_t>(),
+                                          cnt.as<uint32_t>());
+        MB_CHECK_LAUNCH();
+        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, bits, s);
+        uint32_t c[2] = {0, 0};
+        copy_sync(s, c, cnt.p, sizeof(c));
+        const int32_t nh = (int32_t)c[0], n = V - nh - (int32_t)c[1];
+        const uint32_t *order = val.as<uint32_t>();
+        out.nz = (int32_t)c[1];
+        out.ngroups = (int32_t)(((int64_t)n + 31) / 32);
+        out.nlong = 0;
+        if (hubs) {
+            hubs->resize((size_t)nh);
+            if (nh) {
+                std::vector<int32_t> hv((size_t)nh);
+                std::vector<int2> info((size_t)nh);
+                DevBuf hi;
+                hi.reserve(sizeof(int2) * (size_t)nh);
+                k_hub_info<<<grid_for(nh, 256, ctx.num_sms * 4), 256, 0, s>>>(order, nh, g.rrow.as<int32_t>(),
+                                                                              hi.as<int2>());
+                copy_sync(s, info.data(), hi.p, sizeof(int2) * (size_t)nh);
+                copy_sync(s, hv.data(), order, sizeof(int32_t) * (size_t)nh);
+                hi.release();
+                for (int32_t i = 0; i < nh; i++) (*hubs)[i] = HubInfo{hv[i], info[i].x, info[i].y};
+            }
+        }
+        if (out.ngroups) {
+            out.rows.reserve(sizeof(int32_t) * (size_t)out.ngroups);
+            out.base.reserve(sizeof(uint32_t) * (size_t)out.ngroups);
+            out.v.reserve(sizeof(int32_t) * 32 * (size_t)out.ngroups);
+            out.pd.reserve(sizeof(int2) * 32 * (size_t)out.ngroups);
+            k_sell_rows<<<grid_for(out.ngroups, 256, ctx.num_sms * 16), 256, 0, s>>>(
+                order + nh, n, out.ngroups, g.rrow.as<int32_t>(), out.rows.as<int32_t>(), cnt.as<uint32_t>() + 2);
+            MB_CHECK_LAUNCH();
+            scan_exclusive_u32(ctx, out.rows.as<uint32_t>(), out.base.as<uint32_t>(), out.ngroups,
+                               cnt.as<uint32_t>() + 3, s);
+            uint32_t t[2] = {0, 0};
+            copy_sync(s, t, cnt.as<uint32_t>() + 2, sizeof(t));
+            out.nlong = (int32_t)t[0];
+            out.src.reserve(sizeof(int32_t) * 32 * (size_t)t[1]);
+            k_sell_fill<<<grid_for((int64_t)out.ngroups * 32, 256, ctx.num_sms * 16), 256, 0, s>>>(
+                order + nh, n, out.ngroups, out.rows.as<int32_t>(), out.base.as<uint32_t>(), g.rrow.as<int32_t>(),
+                src, pos.as<int32_t>(), g.outdeg.as<int32_t>(), out.v.as<int32_t>(), out.pd.as<int2>(),
+                out.src.as<int32_t>());
+            MB_CHECK_LAUNCH();
+        }
+        if (out.nz) {
+            out.zv.reserve(sizeof(int32_t) * (size_t)out.nz);
+            out.zpd.reserve(sizeof(int2) * (size_t)out.nz);
+            k_zero_fill<<<grid_for(out.nz, 256, ctx.num_sms * 16), 256, 0, s>>>(
+                order + nh + n, out.nz, pos.as<int32_t>(), g.outdeg.as<int32_t>(), out.zv.as<int32_t>(),
+                out.zpd.as<int2>());
+            MB_CHECK_LAUNCH();
+        }
+        MB_CUDA(cudaStreamSynchronize(s));
+    } catch (...) {
+        drop();
+        throw;
+    }
+    drop();
 }
 
 void PrState::ensure_exact(Context &ctx, const Graph &g, int32_t hub_min) {
     if (exact_built && x_hub_min == hub_min) return;
     build_meg_order(ctx, g, *this);
     release_exact();
-    const int32_t V = g.V;
     cudaStream_t s = ctx.stream;
-    std::vector<int32_t> rrow((size_t)V + 1);
-    copy_sync(s, rrow.data(), g.rrow.p, sizeof(int32_t) * ((size_t)V + 1));
-    // light vertices in id order, their sources copied out of the MEG order
-    std::vector<int32_t> lv, lr(1, 0);
-    // mid vertices by in-degree, largest first (ties in id order): a
-    // counting sort over in-degrees kPrLight+1 .. hub_min
-    std::vector<int64_t> cnt((size_t)hub_min + 2, 0);
-    std::vector<int32_t> hubs;
-    for (int32_t v = 0; v < V; v++) {
-        const int32_t d = rrow[v + 1] - rrow[v];
-        if (d <= kPrLight) {
-            lv.push_back(v);
-            lr.push_back(lr.back() + d);
-        } else if (d <= hub_min) {
-            cnt[d]++;
-        } else {
-            hubs.push_back(v);
-        }
-    }
-    std::stable_sort(hubs.begin(), hubs.end(), [&](int32_t x, int32_t y) {
-        return rrow[x + 1] - rrow[x] > rrow[y + 1] - rrow[y];
-    });
-    std::vector<int64_t> at((size_t)hub_min + 2, 0);
-    int64_t nmid = 0;
-    for (int32_t d = hub_min; d > kPrLight; d--) {
-        at[d] = nmid;
-        nmid += cnt[d];
-    }
-    std::vector<int32_t> mid((size_t)nmid);
-    for (int32_t v = 0; v < V; v++) {
-        const int32_t d = rrow[v + 1] - rrow[v];
-        if (d > kPrLight && d <= hub_min) mid[at[d]++] = v;
-    }
-    ngroups = (int32_t)((nmid + 31) / 32);
-    std::vector<int32_t> sv((size_t)ngroups * 32, -1), rows((size_t)ngroups);
-    std::vector<int64_t> sbase((size_t)ngroups);
-    int64_t total = 0;
-    for (int32_t gi = 0; gi < ngroups; gi++) {
-        for (int l = 0; l < 32 && (int64_t)gi * 32 + l < nmid; l++) sv[(size_t)gi * 32 + l] = mid[(size_t)gi * 32 + l];
-        const int32_t v0 = sv[(size_t)gi * 32];
-        rows[gi] = rrow[v0 + 1] - rrow[v0];
-        sbase[gi] = total;
-        total += (int64_t)rows[gi] * 32;
-    }
-    x_nlight = (int32_t)lv.size();
-    x_light_v.reserve(sizeof(int32_t) * std::max<size_t>(lv.size(), 1));
-    x_light_row.reserve(sizeof(int32_t) * lr.size());
-    x_light_col.reserve(sizeof(int32_t) * std::max<size_t>((size_t)lr.back(), 1));
-    sell_v.reserve(sizeof(int32_t) * std::max<size_t>(sv.size(), 1));
-    sell_rows.reserve(sizeof(int32_t) * std::max<size_t>(rows.size(), 1));
-    sell_base.reserve(sizeof(int64_t) * std::max<size_t>(sbase.size(), 1));
-    sell_src.reserve(sizeof(int32_t) * (size_t)std::max<int64_t>(total, 1));
+    std::vector<HubInfo> hubs;
+    build_sell(ctx, g, hub_min, meg_src.as<int32_t>(), sell, &hubs);
+    std::stable_sort(hubs.begin(), hubs.end(), [](const HubInfo &x, const HubInfo &y) { return x.n > y.n; });
     x_nhub = (int32_t)hubs.size();
+    std::vector<int32_t> hv((size_t)x_nhub);
+    for (int32_t h = 0; h < x_nhub; h++) hv[h] = hubs[h].v;
     x_hub_v.reserve(sizeof(int32_t) * std::max<size_t>(hubs.size(), 1));
-    if (x_nlight) {
-        copy_sync(s, x_light_v.p, lv.data(), 4 * lv.size());
-        copy_sync(s, x_light_row.p, lr.data(), 4 * lr.size());
-        k_light_copy<<<grid_for(x_nlight, 256, ctx.num_sms * 16), 256, 0, s>>>(
-            x_light_v.as<int32_t>(), x_light_row.as<int32_t>(), x_nlight, g.rrow.as<int32_t>(),
-            meg_src.as<int32_t>(), x_light_col.as<int32_t>());
-        MB_CHECK_LAUNCH();
-    }
-    if (ngroups) {
-        copy_sync(s, sell_v.p, sv.data(), 4 * sv.size());
-        copy_sync(s, sell_rows.p, rows.data(), 4 * rows.size());
-        copy_sync(s, sell_base.p, sbase.data(), 8 * sbase.size());
-        k_sell_fill<<<grid_for((int64_t)ngroups * 32, 256, ctx.num_sms * 16), 256, 0, s>>>(
-            sell_v.as<int32_t>(), sell_base.as<int64_t>(), sell_rows.as<int32_t>(), ngroups,
-            g.rrow.as<int32_t>(), meg_src.as<int32_t>(), sell_src.as<int32_t>());
-        MB_CHECK_LAUNCH();
-    }
-    if (x_nhub) copy_sync(s, x_hub_v.p, hubs.data(), 4 * hubs.size());
+    copy_sync(s, x_hub_v.p, hv.data(), 4 * hv.size());
     x_nbig = 0;  // the hubs are sorted: the big ones come first
-    while (x_nbig < x_nhub && rrow[hubs[x_nbig] + 1] - rrow[hubs[x_nbig]] > kHubBig) x_nbig++;
+    while (x_nbig < x_nhub && hubs[x_nbig].n > kHubBig) x_nbig++;
     // staging: hub h's run at a multiple of 4 floats, items of kStageItem slots
     std::vector<int64_t> soff((size_t)std::max<int32_t>(x_nhub, 1), 0);
-    std::vector<int4> items;
+    std::vector<int2> items;
+    std::vector<int32_t> meg_off;
     int64_t staged = 0;
     for (int32_t h = 0; h < x_nhub; h++) {
-        const int32_t v = hubs[h];
-        const int32_t n = rrow[v + 1] - rrow[v];
+        const int32_t n = hubs[h].n;
         soff[h] = staged;
-        for (int32_t j0 = 0; j0 < n; j0 += kStageItem)
-            items.push_back(make_int4((int32_t)(staged + j0), rrow[v] + j0, std::min(kStageItem, n - j0), 0));
+        for (int32_t j0 = 0; j0 < n; j0 += kStageItem) {
+            items.push_back(make_int2((int32_t)(staged + j0), std::min(kStageItem, n - j0)));
+            meg_off.push_back(hubs[h].first + j0);
+        }
         staged += ((int64_t)n + 3) & ~(int64_t)3;
     }
     if (staged > 0x7fffffffll) fail(MB_ERR_UNSUPPORTED, "PageRank: hub staging exceeds 2^31 slots");
     nstage_items = (int32_t)items.size();
     x_stage.reserve(sizeof(float) * (size_t)std::max<int64_t>(staged, 1));
     stage_off.reserve(sizeof(int64_t) * soff.size());
-    stage_items.reserve(sizeof(int4) * std::max<size_t>(items.size(), 1));
+    stage_items.reserve(sizeof(int2) * std::max<size_t>(items.size(), 1));
     copy_sync(s, stage_off.p, soff.data(), 8 * soff.size());
-    if (nstage_items) copy_sync(s, stage_items.p, items.data(), sizeof(int4) * items.size());
+    if (nstage_items) {
+        stage_src.reserve(sizeof(int32_t) * (size_t)staged);
+        copy_sync(s, stage_items.p, items.data(), sizeof(int2) * items.size());
+        DevBuf off;
+        off.reserve(sizeof(int32_t) * meg_off.size());
+        try {
+            copy_sync(s, off.p, meg_off.data(), sizeof(int32_t) * meg_off.size());
+            k_stage_fill<<<std::min(nstage_items, ctx.num_sms * 8), 256, 0, s>>>(
+                stage_items.as<int2>(), off.as<int32_t>(), nstage_items, meg_src.as<int32_t>(), pos.as<int32_t>(),
+                stage_src.as<int32_t>());
+            MB_CHECK_LAUNCH();
+            MB_CUDA(cudaStreamSynchronize(s));
+        } catch (...) {
+            off.release();
+            throw;
+        }
+        off.release();
+    }
     MB_CUDA(cudaStreamSynchronize(s));
     ensure_streams();
     x_hub_min = hub_min;
@@ -957,20 +1213,24 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                                 : kHubMinDefault;
     if (ref_order) build_meg_order(ctx, g, st);
     if (ref_order && !unfused) st.ensure_exact(ctx, g, hub_min);
+    if (!ref_order) st.ensure_fixed(ctx, g);
+    if (unfused) st.msg.reserve(sizeof(float) * (size_t)std::max<int64_t>(g.E, 1));
     st.ensure_streams();
     cudaStream_t s = ctx.stream;
-    auto args = [&](int parity) {
+    auto args = [&](int it) {
+        const int parity = it & 1;
         PrArgs a;
         a.V = g.V;
         a.E = g.E;
         a.rrow = g.rrow.as<int32_t>();
-        a.rcol = ref_order ? st.meg_src.as<int32_t>() : g.rcol.as<int32_t>();
         a.outdeg = g.outdeg.as<int32_t>();
         a.row = g.row.as<int32_t>();
         a.mslot = ref_order ? st.meg_slot.as<int32_t>() : g.mslot.as<int32_t>();
         a.contrib_in = st.contrib[parity].as<float>();
         a.contrib_out = st.contrib[parity ^ 1].as<float>();
-        a.rank_out = st.rank.as<float>();
+        a.rank_out = it == iters - 1 ? st.rank.as<float>() : nullptr;
+        a.pos = st.pos.as<int32_t>();
+        a.hcol = st.hcol.as<int32_t>();
         a.msg = st.msg.as<float>();
         a.items = st.items.as<int4>();
         a.nitems = st.nitems;
@@ -979,10 +1239,6 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         a.nhub = st.nhub;
         a.blk_sum = st.blk_sum.as<float>();
         a.nlong = st.nlong;
-        a.light_v = st.light_v.as<int32_t>();
-        a.light_row = st.light_row.as<int32_t>();
-        a.light_col = st.light_col.as<int32_t>();
-        a.nlight = st.nlight;
         return a;
     };
     // grids of exactly the resident blocks (grid-stride loops: no tail wave)
@@ -991,16 +1247,9 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0));
         return ctx.num_sms * std::max(per_sm, 1);
     };
-    const int grid_pull = resident((const void *)k_pr_pull<false>, kPrThreads);
-    // light vertices per lane: the tunable, else 2 (measured best from 2^22
-    // to 2^28 edges) while every resident warp still gets four groups
-    int vpl = (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL];
-    if (vpl <= 0) {
-        vpl = 2;
-        const int64_t warps = (int64_t)resident((const void *)k_pr_light<1>, kPrThreads) * kPrWarps;
-        const int64_t nl = ref_order && !unfused ? st.x_nlight : st.nlight;
-        while (vpl > 1 && nl < (int64_t)32 * vpl * 4 * warps) vpl >>= 1;
-    }
+    const int grid_pull = resident((const void *)k_pr_pull<true>, kPrThreads);
+    // short sliced-ELL groups a warp takes at once: the tunable, else 4
+    const int vpl = ctx.tunable[MB_TUNE_PR_LIGHT_VPL] > 0 ? (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL] : 4;
     const int pair = ctx.tunable[MB_TUNE_PR_SHORT_PAIR] > 0 ? (int)ctx.tunable[MB_TUNE_PR_SHORT_PAIR]
                                                              : kShortPairDefault;
     // each variant's grid is its own resident block count (registers differ)
@@ -1008,25 +1257,49 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                                    (const void *)k_heavy_blocks<false, 4>},
                                   {(const void *)k_heavy_blocks<true, 1>, (const void *)k_heavy_blocks<true, 2>,
                                    (const void *)k_heavy_blocks<true, 4>}};
-    const void *light_fn[3] = {(const void *)k_pr_light<1>, (const void *)k_pr_light<2>,
-                               (const void *)k_pr_light<4>};
+    const void *sell_fn[2][3] = {
+        {(const void *)k_pr_sell<1, false>, (const void *)k_pr_sell<2, false>, (const void *)k_pr_sell<4, false>},
+        {(const void *)k_pr_sell<1, true>, (const void *)k_pr_sell<2, true>, (const void *)k_pr_sell<4, true>}};
     const int pi = pair == 1 ? 0 : pair == 2 ? 1 : 2, vi = vpl == 1 ? 0 : vpl == 2 ? 1 : 2;
     const int64_t heavy_threads = heavy_units(st.nitems, st.nlong, pair) * 32;
     const int grid_heavy[2] = {grid_for(heavy_threads, 256, resident(heavy_fn[0][pi], 256)),
                                grid_for(heavy_threads, 256, resident(heavy_fn[1][pi], 256))};
-    const int grid_light = resident(light_fn[vi], kPrThreads);
+    const int grid_sell[2] = {resident(sell_fn[0][vi], 256), resident(sell_fn[1][vi], 256)};
     auto heavy = [&](bool from_msg, cudaStream_t cs, const PrArgs &a) {
         PrArgs arg = a;
         void *params[] = {&arg};
         MB_CUDA(cudaLaunchKernel(heavy_fn[from_msg][pi], grid_heavy[from_msg], 256, params, 0, cs));
     };
-    auto light = [&](cudaStream_t cs, const PrArgs &a) {
-        PrArgs arg = a;
-        void *params[] = {&arg};
-        MB_CUDA(cudaLaunchKernel(light_fn[vi], grid_light, kPrThreads, params, 0, cs));
+    auto sell_args = [&](const PrSell &l) {
+        SellArgs a{};
+        a.v = l.v.as<int32_t>();
+        a.pd = l.pd.as<int2>();
+        a.rows = l.rows.as<int32_t>();
+        a.base = l.base.as<uint32_t>();
+        a.src = l.src.as<int32_t>();
+        a.ngroups = l.ngroups;
+        a.nlong = l.nlong;
+        return a;
+    };
+    // one superstep of the vertices of a sliced ELL, those without in-edges included
+    auto sell_step = [&](cudaStream_t cs, const PrSell &l, const PrArgs &p, int it) {
+        if (l.nz && (it < 2 || p.rank_out)) {
+            k_pr_zero<<<grid_for(l.nz, 256, ctx.num_sms * 8), 256, 0, cs>>>(
+                l.zv.as<int32_t>(), l.zpd.as<int2>(), l.nz, it < 2 ? p.contrib_out : nullptr, p.rank_out);
+            MB_CHECK_LAUNCH();
+        }
+        if (!l.ngroups) return;
+        SellArgs a = sell_args(l);
+        a.contrib_in = p.contrib_in;
+        a.contrib_out = p.contrib_out;
+        a.rank_out = p.rank_out;
+        a.ctr = st.ctr.as<uint32_t>() + it;
+        void *params[] = {&a};
+        const int64_t units = (int64_t)l.nlong + (l.ngroups - l.nlong + vpl - 1) / vpl;
+        const int small = units <= (int64_t)grid_sell[1] * (256 / 32);
+        MB_CUDA(cudaLaunchKernel(sell_fn[small][vi], grid_for(units * 32, 256, grid_sell[small]), 256, params, 0, cs));
     };
     const int grid_vtx = ctx.num_sms * 8;
-    const int grid_sell = resident((const void *)k_pr_sell, 256);
     const int hub_ctas = ctx.tunable[MB_TUNE_PR_HUB_CTAS] > 0 ? (int)ctx.tunable[MB_TUNE_PR_HUB_CTAS]
                                                                : std::max(ctx.num_sms / 4, 1);
     const int grid_hub_warp = std::max(resident((const void *)k_pr_hub_warp, 256) / 2, 1);
@@ -1035,32 +1308,60 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     auto exact_args = [&](const PrArgs &a) {
         ExactArgs x;
         x.rrow = g.rrow.as<int32_t>();
-        x.meg_src = st.meg_src.as<int32_t>();
+        x.pos = st.pos.as<int32_t>();
+        x.stage_src = st.stage_src.as<int32_t>();
         x.outdeg = g.outdeg.as<int32_t>();
         x.contrib_in = a.contrib_in;
         x.contrib_out = a.contrib_out;
         x.rank_out = a.rank_out;
-        x.sell_v = st.sell_v.as<int32_t>();
-        x.sell_base = st.sell_base.as<int64_t>();
-        x.sell_rows = st.sell_rows.as<int32_t>();
-        x.sell_src = st.sell_src.as<int32_t>();
-        x.ngroups = st.ngroups;
         x.hub_v = st.x_hub_v.as<int32_t>();
         x.nhub = st.x_nhub;
         x.x_stage = st.x_stage.as<float>();
         x.stage_off = st.stage_off.as<int64_t>();
-        x.stage_items = st.stage_items.as<int4>();
+        x.stage_items = st.stage_items.as<int2>();
         x.nstage_items = st.nstage_items;
         return x;
     };
+    st.ctr.reserve(sizeof(uint32_t) * (size_t)std::max(iters, 1));
+    // all supersteps in one launch (k_pr_resident)
+    const PrSell &all = ref_order ? st.sell : st.light;
+    int grid_res = 0;
+    volatile int *res_err = (volatile int *)ctx.ctrl_readback();
+    *res_err = 0;
+    if (!unfused && iters > 1 && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
+        const int64_t warps = kResThreads / 32;
+        grid_res = (int)std::min<int64_t>((all.ngroups + warps - 1) / warps, INT32_MAX);
+        if (grid_res > resident((const void *)k_pr_resident, kResThreads)) grid_res = 0;
+    }
     auto emit = [&](cudaStream_t cs) {
+        MB_CUDA(cudaMemsetAsync(st.ctr.p, 0, sizeof(uint32_t) * (size_t)std::max(iters, 1), cs));
         if (init_vec)
-            k_pr_init_vec<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), g.V, init_vec, st.contrib[0].as<float>());
+            k_pr_init_vec<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), st.pos.as<int32_t>(), g.V, init_vec,
+                                                    st.contrib[0].as<float>());
         else
-            k_pr_init<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), g.V, init, st.contrib[0].as<float>());
+            k_pr_init<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), st.pos.as<int32_t>(), g.V, init,
+                                                st.contrib[0].as<float>());
         MB_CHECK_LAUNCH();
+        if (grid_res) {
+            SellArgs a = sell_args(all);
+            ResidentArgs r;
+            r.contrib[0] = st.contrib[0].as<float>();
+            r.contrib[1] = st.contrib[1].as<float>();
+            r.rank = st.rank.as<float>();
+            r.zv = all.zv.as<int32_t>();
+            r.zpd = all.zpd.as<int2>();
+            r.nz = all.nz;
+            r.iters = iters;
+            r.bar = st.ctr.as<uint32_t>();
+            r.err = res_err;
+            r.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : 1l << 22;
+            void *params[] = {&a, &r};
+            MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pr_resident, dim3(grid_res), dim3(kResThreads), params,
+                                                0, cs));
+            return;
+        }
         for (int it = 0; it < iters; it++) {
-            PrArgs a = args(it & 1);
+            PrArgs a = args(it);
             if (ref_order && unfused) {
                 // the reference's send -> combine split over the message array,
                 // each vertex folded serially in MEG order
@@ -1103,31 +1404,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                     }
                     MB_CHECK_LAUNCH();
                 }
-                // the sliced ELL on its own stream with half the GPU: its
-                // longest groups (sequential folds) set its length, and the
-                // light kernel fills the SMs its tail leaves idle
-                if (st.ngroups) {
-                    MB_CUDA(cudaEventRecord(st.ev_fork2, cs));
-                    MB_CUDA(cudaStreamWaitEvent(st.side2, st.ev_fork2, 0));
-                    k_pr_sell<<<std::max(grid_sell / kSellGridDiv, 1), 256, 0, st.side2>>>(x);
-                    MB_CHECK_LAUNCH();
-                }
-                if (st.x_nlight) {
-                    PrArgs la = a;
-                    la.light_v = st.x_light_v.as<int32_t>();
-                    la.light_row = st.x_light_row.as<int32_t>();
-                    la.light_col = st.x_light_col.as<int32_t>();
-                    la.nlight = st.x_nlight;
-                    light(cs, la);
-                }
+                sell_step(cs, st.sell, a, it);
                 MB_CHECK_LAUNCH();
                 if (st.x_nhub) {
                     MB_CUDA(cudaEventRecord(st.ev_join, st.side));
                     MB_CUDA(cudaStreamWaitEvent(cs, st.ev_join, 0));
-                }
-                if (st.ngroups) {
-                    MB_CUDA(cudaEventRecord(st.ev_join2, st.side2));
-                    MB_CUDA(cudaStreamWaitEvent(cs, st.ev_join2, 0));
                 }
                 continue;
             }
@@ -1137,7 +1418,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                 k_pr_pull<true><<<grid_pull, kPrThreads, 0, cs>>>(a);
             } else {
                 if (a.nitems) heavy(false, cs, a);
-                if (a.nlight) light(cs, a);
+                sell_step(cs, st.light, a, it);
             }
             if (a.nhub) k_hub_finalize<<<grid_for(a.nhub, 128, ctx.num_sms * 4), 128, 0, cs>>>(a);
             MB_CHECK_LAUNCH();
@@ -1186,6 +1467,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             MB_CUDA(cudaEventRecord(e1, s));
         }
         MB_CUDA(cudaEventSynchronize(e1));
+        if (grid_res && *res_err) fail(MB_ERR_TIMEOUT, "pagerank: a barrier between two supersteps timed out");
         float ms = 0;
         MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         if (stats) {
@@ -1196,13 +1478,16 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             stats->device_ms = ms;
             stats->schedule_count[unfused ? MB_SCHED_PUSH_UNFUSED : MB_SCHED_PUSH_EDGE_QUEUE] = iters;
             stats->edges_scanned = (int64_t)iters * g.E;
-            int64_t per_step;
+            const PrSell &l = ref_order ? st.sell : st.light;
+            int64_t per_step, zeros = 0;
             if (ref_order && unfused) per_step = 2;
-            else if (ref_order)
-                per_step = (st.x_nhub > 0) + (st.x_nbig > 0) + (st.x_nhub > st.x_nbig) + (st.ngroups > 0) +
-                           (st.x_nlight > 0);
-            else per_step = (unfused ? 2 : st.nlight > 0) + (st.nitems > 0) + (st.nhub > 0);
-            stats->kernel_launches = 1 + (int64_t)iters * per_step + (iters == 0);
+            else if (unfused) per_step = 2 + (st.nitems > 0) + (st.nhub > 0);
+            else {
+                per_step = (l.ngroups > 0) + (ref_order ? (st.x_nhub > 0) + (st.x_nbig > 0) + (st.x_nhub > st.x_nbig)
+                                                        : (st.nitems > 0) + (st.nhub > 0));
+                if (l.nz) zeros = std::min(iters, 3);  // the first two supersteps and the last
+            }
+            stats->kernel_launches = grid_res ? 2 : 1 + (int64_t)iters * per_step + zeros + (iters == 0);
         }
     } catch (...) {
         cudaEventDestroy(e0);

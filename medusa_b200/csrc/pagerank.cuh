@@ -4,43 +4,54 @@
 
 namespace mb {
 
+// A sliced ELL over the vertices of some in-degree range (pagerank.cu), and
+// the vertices without in-edges.
+struct PrSell {
+    DevBuf v, pd, rows, base, src, zv, zpd;
+    int32_t ngroups = 0, nlong = 0, nz = 0;
+    void release() {
+        v.release(); pd.release(); rows.release(); base.release(); src.release();
+        zv.release(); zpd.release();
+        ngroups = nlong = nz = 0;
+    }
+};
+struct HubInfo {
+    int32_t v, first, n;
+};
+
 struct PrState {
     bool built = false;
     int32_t V = 0;
     int64_t E = 0;
     DevBuf rank, contrib[2], msg, items, hub_v, hub_first, blk_sum;
     DevBuf init_stage;  // host initial ranks of mb_pagerank_from, staged
+    // where each vertex's contribution sits in contrib[] (-1: no out-edges):
+    // ordered by out-degree class, the sources with the most out-edges first
+    DevBuf pos;
+    DevBuf ctr;  // the sliced ELL's work counters, one per superstep
+    bool fixed_built = false;  // the fixed order's lists below
     int32_t nitems = 0, nhub = 0;
     int32_t nlong = 0;  // items longer than kPrShortItem (the head of the list)
-    // light vertices (in-degree <= kPrLight) in id order, with their in-edge
-    // sources copied out of the reverse CSR: the fused pull streams only
-    // these edges (the heavy vertices' edges never enter its windows)
-    DevBuf light_v, light_row, light_col;
-    int32_t nlight = 0;
+    DevBuf hcol;   // positions of all in-edge sources (the heavy vertices' blocks read theirs)
+    PrSell light;  // vertices of 1 to kPrLight in-edges, slots in reverse-CSR order
     // the reference's MEG order (built on first use): in-edge sources per
     // destination in MEG slot order, and each CSR edge's slot in it
     bool meg_built = false;
     DevBuf meg_src, meg_slot;
-    // the reference's order computed in parallel (built on first use): light
-    // lists copied from the MEG order, the mid vertices' sliced ELL, the hubs
+    // the reference's order computed in parallel (built on first use): the
+    // sliced ELL of 1 to x_hub_min in-edges, slots in MEG order, and the hubs
     bool exact_built = false;
     int32_t x_hub_min = 0;  // in-degree above which a vertex is a hub
-    DevBuf x_light_v, x_light_row, x_light_col;
-    int32_t x_nlight = 0;
-    DevBuf sell_v, sell_base, sell_rows, sell_src;
-    int32_t ngroups = 0;
+    PrSell sell;
     DevBuf x_hub_v;
     int32_t x_nhub = 0;
     int32_t x_nbig = 0;  // hubs [0, x_nbig) have more than kHubBig in-edges
-    DevBuf x_stage, stage_off, stage_items;  // the hubs' staged contributions
+    DevBuf x_stage, stage_src, stage_off, stage_items;  // the hubs' staged contributions
     int32_t nstage_items = 0;
     // the hub kernel runs on a side stream beside the others (fork / join)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    // the sliced-ELL kernel on a second side stream beside the others
-    cudaStream_t side2 = nullptr;
-    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
-    // the warp-per-hub scans on a third, beside the big hubs' CTAs
+    // the warp-per-hub scans on another, beside the big hubs' CTAs
     cudaStream_t side3 = nullptr;
     cudaEvent_t ev_join3 = nullptr;
     cudaGraphExec_t exec = nullptr;  // captured run (init + iters supersteps)
@@ -53,9 +64,6 @@ struct PrState {
         if (!side) MB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         if (!ev_fork) MB_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
         if (!ev_join) MB_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-        if (!side2) MB_CUDA(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
-        if (!ev_fork2) MB_CUDA(cudaEventCreateWithFlags(&ev_fork2, cudaEventDisableTiming));
-        if (!ev_join2) MB_CUDA(cudaEventCreateWithFlags(&ev_join2, cudaEventDisableTiming));
         if (!side3) MB_CUDA(cudaStreamCreateWithFlags(&side3, cudaStreamNonBlocking));
         if (!ev_join3) MB_CUDA(cudaEventCreateWithFlags(&ev_join3, cudaEventDisableTiming));
     }
@@ -66,31 +74,32 @@ struct PrState {
         g_iters = -1;
         rank.release(); contrib[0].release(); contrib[1].release(); msg.release();
         init_stage.release();
+        pos.release(); hcol.release(); light.release(); ctr.release();
+        fixed_built = false;
         items.release(); hub_v.release(); hub_first.release(); blk_sum.release();
-        light_v.release(); light_row.release(); light_col.release();
         meg_src.release(); meg_slot.release();
         meg_built = false;
         release_exact();
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (side) cudaStreamDestroy(side);
-        if (ev_fork2) cudaEventDestroy(ev_fork2);
-        if (ev_join2) cudaEventDestroy(ev_join2);
-        if (side2) cudaStreamDestroy(side2);
         if (ev_join3) cudaEventDestroy(ev_join3);
         if (side3) cudaStreamDestroy(side3);
-        ev_fork = ev_join = ev_fork2 = ev_join2 = ev_join3 = nullptr;
-        side = side2 = side3 = nullptr;
+        ev_fork = ev_join = ev_join3 = nullptr;
+        side = side3 = nullptr;
         built = false;
     }
     void release_exact() {
-        x_light_v.release(); x_light_row.release(); x_light_col.release();
-        sell_v.release(); sell_base.release(); sell_rows.release(); sell_src.release();
+        sell.release();
         x_hub_v.release();
-        x_stage.release(); stage_off.release(); stage_items.release();
+        x_stage.release(); stage_src.release(); stage_off.release(); stage_items.release();
         exact_built = false;
     }
     void ensure(Context &ctx, const Graph &g);
+    // the structures of the fixed order
+    void ensure_fixed(Context &ctx, const Graph &g);
+    void build_sell(Context &ctx, const Graph &g, int32_t max_rows, const int32_t *src, PrSell &out,
+                    std::vector<HubInfo> *hubs);
     // the structures of the parallel reference-order sum (meg order included)
     void ensure_exact(Context &ctx, const Graph &g, int32_t hub_min);
 };
