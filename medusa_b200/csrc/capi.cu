@@ -71,7 +71,10 @@ int guarded(mb_ctx *ctx, F &&f) {
     }
 }
 
-void use_device(mb_ctx *ctx) { MB_CUDA(cudaSetDevice(ctx->c.device)); }
+void use_device(mb_ctx *ctx) {
+    MB_CUDA(cudaSetDevice(ctx->c.device));
+    mb::pool_use_stream(ctx->c.stream);
+}
 
 mb::AppStates &apps(mb_graph *g) {
     if (!g->g.apps) g->g.apps = new mb::AppStates();
@@ -115,8 +118,11 @@ int mb_create(int device, mb_ctx **out) {
         MB_CUDA(cudaGetDeviceProperties(&prop, device));
         if (prop.major < 10) mb::fail(MB_ERR_UNSUPPORTED, "this build targets sm_100a (B200)");
         ctx->c.device = device;
+        mb::pool_context(device, 1);
+        ctx->c.pool_counted = true;
         ctx->c.num_sms = prop.multiProcessorCount;
         MB_CUDA(cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking));
+        mb::pool_use_stream(ctx->c.stream);
         MB_CUDA(cudaMallocHost((void **)&ctx->c.pinned_small, mb::Context::kSmallBytes));
         for (mb::DevBuf &b : ctx->c.mlp) {
             b.reserve(sizeof(float) * mb::kModelFloats);
@@ -137,8 +143,13 @@ int mb_destroy(mb_ctx *ctx) {
     if (!ctx) return MB_OK;
     cudaSetDevice(ctx->c.device);
     if (ctx->c.stream) cudaStreamSynchronize(ctx->c.stream);
-    for (auto &b : ctx->c.scratch) b.release();
-    for (mb::DevBuf &b : ctx->c.mlp) b.release();
+    mb::pool_use_stream(nullptr);
+    {
+        mb::PoolIdle idle;
+        for (auto &b : ctx->c.scratch) b.release();
+        for (mb::DevBuf &b : ctx->c.mlp) b.release();
+    }
+    if (ctx->c.pool_counted) mb::pool_context(ctx->c.device, -1);
     if (ctx->c.pinned) cudaFreeHost(ctx->c.pinned);
     if (ctx->c.pinned_small) cudaFreeHost(ctx->c.pinned_small);
     if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
@@ -623,6 +634,7 @@ int mb_graph_destroy(mb_graph *g) {
     if (!g) return MB_OK;
     cudaSetDevice(g->g.device);
     cudaDeviceSynchronize();
+    mb::PoolIdle idle;
     delete g->g.apps;
     g->g.apps = nullptr;
     g->g.release();
@@ -722,6 +734,7 @@ int mb_batch_destroy(mb_batch *b) {
     if (!b) return MB_OK;
     cudaSetDevice(b->device);
     cudaDeviceSynchronize();
+    mb::PoolIdle idle;
     b->b.release();
     delete b;
     return MB_OK;

@@ -49,12 +49,25 @@ struct ApiError {
 
 [[noreturn]] inline void fail(int code, const std::string &msg) { throw ApiError{code, msg}; }
 
+// Device memory (pool.cu).  pool_free waits for the calling context's stream
+// (pool_use_stream, set at every entry point) before it hands memory on, or,
+// under a PoolIdle, for nothing: the caller has waited for the device.
+void *pool_alloc(size_t n);
+void pool_free(void *p);
+void pool_use_stream(cudaStream_t s);
+void pool_context(int device, int delta);  // a context of the device is made (+1) or destroyed (-1)
+struct PoolIdle {
+    bool was;
+    PoolIdle();
+    ~PoolIdle();
+};
+
 // A device buffer owned by a context or graph.
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     void release() {
-        if (p) cudaFree(p);
+        if (p) pool_free(p);
         p = nullptr;
         bytes = 0;
     }
@@ -63,7 +76,7 @@ struct DevBuf {
         if (n <= bytes && p) return p;
         release();
         size_t want = n < 256 ? 256 : n;
-        MB_CUDA(cudaMalloc(&p, want));
+        p = pool_alloc(want);
         bytes = want;
         return p;
     }
@@ -112,6 +125,7 @@ void graph_from_gtgraph(Context &ctx, Graph &g, const char *text, int64_t len, u
 // ---- context ------------------------------------------------------------------
 struct Context {
     int device = 0;
+    bool pool_counted = false;  // counted among the device's contexts (pool.cu)
     cudaStream_t stream = nullptr;
     int num_sms = 148;
     std::string last_error;
