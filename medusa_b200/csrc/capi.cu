@@ -208,9 +208,16 @@ int mb_set_persistent_grid(mb_ctx *ctx, int enable) {
 }
 
 namespace {
-// n bytes from host or device memory into a device buffer (returns the pointer to use)
+// n bytes from host or device memory, to be read by kernels: this device's
+// memory in place, anything else (host, another GPU) by a copy into b
 const void *stage_in(mb::DevBuf &b, const void *p, size_t n, cudaStream_t s) {
-    if (mb::is_device_ptr(p)) return p;
+    if (mb::is_device_ptr(p)) {
+        cudaPointerAttributes a;
+        int device = 0;
+        MB_CUDA(cudaPointerGetAttributes(&a, p));
+        MB_CUDA(cudaGetDevice(&device));
+        if (a.type == cudaMemoryTypeManaged || a.device == device) return p;
+    }
     b.reserve(std::max<size_t>(n, 1));
     mb::copy_sync(s, b.p, p, n);
     return b.p;
@@ -473,17 +480,14 @@ int mb_graph_from_edges(mb_ctx *ctx, int32_t V, int64_t E, const int32_t *src, c
         use_device(ctx);
         mb::DevBuf bs, bd, bw;
         try {
-            const size_t eb = sizeof(uint32_t) * (size_t)std::max<int64_t>(E, 1);
-            bs.reserve(eb);
-            bd.reserve(eb);
-            if (w) bw.reserve(eb);
-            if (E > 0) {
-                mb::copy_sync(ctx->c.stream, bs.p, src, 4 * (size_t)E);
-                mb::copy_sync(ctx->c.stream, bd.p, dst, 4 * (size_t)E);
-                if (w) mb::copy_sync(ctx->c.stream, bw.p, w, 4 * (size_t)E);
-            }
-            mb::graph_build_from_device_edges(ctx->c, g->g, V, E, bs.as<uint32_t>(),
-                                              bd.as<uint32_t>(), w ? bw.as<float>() : nullptr, flags);
+            // device arrays are read in place
+            const size_t n = 4 * (size_t)E;
+            const void *ps = E > 0 ? stage_in(bs, src, n, ctx->c.stream) : nullptr;
+            const void *pd = E > 0 ? stage_in(bd, dst, n, ctx->c.stream) : nullptr;
+            // a weight array makes the graph weighted even when it is empty
+            const void *pw = !w ? nullptr : E > 0 ? stage_in(bw, w, n, ctx->c.stream) : (const void *)w;
+            mb::graph_build_from_device_edges(ctx->c, g->g, V, E, (const uint32_t *)ps, (const uint32_t *)pd,
+                                              (const float *)pw, flags);
         } catch (...) {
             bs.release(); bd.release(); bw.release();
             throw;

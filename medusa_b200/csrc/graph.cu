@@ -6,16 +6,16 @@
 // SSSP/VertexDataType.cu:64-85) and then copies them to the GPU
 // (D_EdgeArray::Fill, SSSP/EdgeDataType.cu:364-391).  Here the edge list goes
 // to the device once and every array is built there:
-//   1. stable radix sort of (src, edge#) -> CSR order.  With
-//      MB_ORDER_REFERENCE the edge numbers are taken in reverse, which puts
+//   1. stable radix sort by src, dst and weight along -> CSR order.  With
+//      MB_ORDER_REFERENCE the edges are taken in reverse, which puts
 //      each source's edges in the reverse of insertion order, as GraphIR's
 //      prepend-and-walk does;
-//   2. row[] = exclusive scan of out-degrees (the reference's edge_index);
-//   3. stable radix sort of (dst, csr#) -> reverse CSR.  Stability keeps the
+//   2. row[] = the boundaries of the sorted sources (the reference's edge_index);
+//   3. stable radix sort of the CSR by dst -> reverse CSR.  Stability keeps the
 //      in-edges of each destination in CSR order, which is the order the
 //      reference's per-destination cursor hands out message slots in
 //      (msgDstID, SSSP/EdgeDataType.cu:181-182); mslot[] is that permutation;
-//   4. rrow[] = exclusive scan of in-degrees (the reference's msg_index).
+//   4. rrow[] = the boundaries of the sorted destinations (the reference's msg_index).
 #include <algorithm>
 #include <cmath>
 #include "mb_internal.cuh"
@@ -107,52 +107,10 @@ __global__ void k_check_ids(const uint32_t *src, const uint32_t *dst, int64_t E,
         if (src[e] >= V || dst[e] >= V) *bad = 1;
 }
 
-__global__ void k_iota(uint32_t *vals, int64_t n, int reverse) {
+__global__ void k_fill_f32(float *x, int64_t n, float v) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        vals[i] = reverse ? (uint32_t)(n - 1 - i) : (uint32_t)i;
-}
-
-// keys[i] <-> keys[n-1-i]: with the edge numbers also reversed, a stable
-// sort then leaves each source's edges in reverse insertion order
-__global__ void k_reverse(uint32_t *keys, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 2;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = keys[i];
-        keys[i] = keys[n - 1 - i];
-        keys[n - 1 - i] = t;
-    }
-}
-
-__global__ void k_hist(const uint32_t *keys, int64_t n, uint32_t *cnt) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[keys[i]], 1u);
-}
-
-// CSR arrays from the sorted (src, edge#) pairs.
-__global__ void k_gather_csr(const uint32_t *sorted_src, const uint32_t *perm,
-                             const uint32_t *dst_in, const float *w_in, int64_t E,
-                             int32_t *esrc, int32_t *col, float *wt) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < E;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t e = perm[k];
-        esrc[k] = (int32_t)sorted_src[k];
-        col[k] = (int32_t)dst_in[e];
-        wt[k] = w_in ? w_in[e] : 1.0f;
-    }
-}
-
-// reverse-CSR arrays from the sorted (dst, csr#) pairs.
-__global__ void k_gather_csc(const uint32_t *perm, const int32_t *esrc, const float *wt,
-                             int64_t E, int32_t *rcol, float *rwt, int32_t *mslot) {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < E;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t k = perm[j];
-        rcol[j] = esrc[k];
-        rwt[j] = wt[k];
-        mslot[k] = (int32_t)j;
-    }
+        x[i] = v;
 }
 
 __global__ void k_degrees(const int32_t *row, const int32_t *rrow, int32_t V, int32_t *outdeg,
@@ -184,7 +142,7 @@ int bits_for(uint32_t V) {
 }  // namespace
 
 void graph_build_from_device_edges(Context &ctx, Graph &g, int32_t V, int64_t E,
-                                   uint32_t *d_src, uint32_t *d_dst, float *d_w,
+                                   const uint32_t *d_src, const uint32_t *d_dst, const float *d_w,
                                    uint32_t flags) {
     cudaStream_t s = ctx.stream;
     const int gridE = grid_for(E, 256, ctx.num_sms * 16);
@@ -204,7 +162,7 @@ void graph_build_from_device_edges(Context &ctx, Graph &g, int32_t V, int64_t E,
     g.rwt.reserve(eb);
     g.mslot.reserve(eb);
 
-    DevBuf cnt, vals, flag;
+    DevBuf key, flag;
     try {
         flag.reserve(4 * sizeof(int));
         MB_CUDA(cudaMemsetAsync(flag.p, 0, 4 * sizeof(int), s));
@@ -217,44 +175,51 @@ void graph_build_from_device_edges(Context &ctx, Graph &g, int32_t V, int64_t E,
             if (bad) fail(MB_ERR_INVALID, "edge endpoint outside [0, num_vertices)");
         }
         const int bits = bits_for((uint32_t)V);
-        cnt.reserve(sizeof(uint32_t) * (size_t)(V + 1));
-        vals.reserve(eb);
-
-        // 1-2. CSR
-        MB_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(uint32_t) * (V + 1), s));
         if (E > 0) {
-            k_hist<<<gridE, 256, 0, s>>>(d_src, E, cnt.as<uint32_t>());
-            MB_CHECK_LAUNCH();
-        }
-        scan_exclusive_u32(ctx, cnt.as<uint32_t>(), (uint32_t *)g.row.p, V + 1, nullptr, s);
-        if (E > 0) {
-            const int rev = (flags & MB_ORDER_REFERENCE) ? 1 : 0;
-            k_iota<<<gridE, 256, 0, s>>>(vals.as<uint32_t>(), E, rev);
-            if (rev) k_reverse<<<gridE, 256, 0, s>>>(d_src, E);
-            MB_CHECK_LAUNCH();
-            radix_sort_pairs(ctx, d_src, vals.as<uint32_t>(), E, bits, s);
-            k_gather_csr<<<gridE, 256, 0, s>>>(d_src, vals.as<uint32_t>(), d_dst, d_w, E,
-                                               g.esrc.as<int32_t>(), g.col.as<int32_t>(),
-                                               g.wt.as<float>());
-            MB_CHECK_LAUNCH();
-        }
-        // 3-4. reverse CSR (reuse d_dst as the key buffer, vals as the permutation)
-        MB_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(uint32_t) * (V + 1), s));
-        if (E > 0) {
-            MB_CUDA(cudaMemcpyAsync(d_dst, g.col.p, sizeof(uint32_t) * E,
-                                    cudaMemcpyDeviceToDevice, s));
-            k_hist<<<gridE, 256, 0, s>>>(d_dst, E, cnt.as<uint32_t>());
-            MB_CHECK_LAUNCH();
-        }
-        scan_exclusive_u32(ctx, cnt.as<uint32_t>(), (uint32_t *)g.rrow.p, V + 1, nullptr, s);
-        if (E > 0) {
-            k_iota<<<gridE, 256, 0, s>>>(vals.as<uint32_t>(), E, 0);
-            MB_CHECK_LAUNCH();
-            radix_sort_pairs(ctx, d_dst, vals.as<uint32_t>(), E, bits, s);
-            k_gather_csc<<<gridE, 256, 0, s>>>(vals.as<uint32_t>(), g.esrc.as<int32_t>(),
-                                               g.wt.as<float>(), E, g.rcol.as<int32_t>(),
-                                               g.rwt.as<float>(), g.mslot.as<int32_t>());
-            MB_CHECK_LAUNCH();
+            // 1-2. CSR: the edges sorted by source, destination and weight
+            // along; the reverse of the input order first where each source's
+            // edges are to end up in the reverse of insertion order
+            SortJob c;
+            c.key_in = d_src;
+            c.key_out = (uint32_t *)g.esrc.p;
+            c.pay_in[0] = d_dst;
+            c.pay_out[0] = (uint32_t *)g.col.p;
+            c.npay = 1;
+            if (d_w) {
+                c.pay_in[1] = (const uint32_t *)d_w;
+                c.pay_out[1] = (uint32_t *)g.wt.p;
+                c.npay = 2;
+            }
+            c.reverse = (flags & MB_ORDER_REFERENCE) != 0;
+            radix_sort(ctx, c, E, bits, s);
+            key_offsets(ctx, (const uint32_t *)g.esrc.p, E, V, (uint32_t *)g.row.p, s);
+            // 3-4. reverse CSR: the CSR sorted by destination, source and
+            // weight along; a CSR edge's position is its message slot
+            key.reserve(eb);
+            SortJob r;
+            r.key_in = (const uint32_t *)g.col.p;
+            r.key_out = key.as<uint32_t>();
+            r.pay_in[0] = (const uint32_t *)g.esrc.p;
+            r.pay_out[0] = (uint32_t *)g.rcol.p;
+            r.npay = 1;
+            if (d_w) {
+                r.pay_in[1] = (const uint32_t *)g.wt.p;
+                r.pay_out[1] = (uint32_t *)g.rwt.p;
+                r.npay = 2;
+            }
+            r.npay++;
+            r.iota = true;
+            r.slot_out = (uint32_t *)g.mslot.p;
+            radix_sort(ctx, r, E, bits, s);
+            key_offsets(ctx, key.as<uint32_t>(), E, V, (uint32_t *)g.rrow.p, s);
+            if (!d_w) {
+                k_fill_f32<<<gridE, 256, 0, s>>>(g.wt.as<float>(), E, 1.0f);
+                k_fill_f32<<<gridE, 256, 0, s>>>(g.rwt.as<float>(), E, 1.0f);
+                MB_CHECK_LAUNCH();
+            }
+        } else {
+            MB_CUDA(cudaMemsetAsync(g.row.p, 0, sizeof(int32_t) * (V + 1), s));
+            MB_CUDA(cudaMemsetAsync(g.rrow.p, 0, sizeof(int32_t) * (V + 1), s));
         }
         MB_CUDA(cudaMemsetAsync(flag.p, 0, 2 * sizeof(int), s));
         k_degrees<<<gridV, 256, 0, s>>>(g.row.as<int32_t>(), g.rrow.as<int32_t>(), V,
@@ -266,10 +231,10 @@ void graph_build_from_device_edges(Context &ctx, Graph &g, int32_t V, int64_t E,
         g.max_outdeg = md[0];
         g.max_indeg = md[1];
     } catch (...) {
-        cnt.release(); vals.release(); flag.release();
+        key.release(); flag.release();
         throw;
     }
-    cnt.release(); vals.release(); flag.release();
+    key.release(); flag.release();
 }
 
 // CSR -> edge list: edge e's source is the last v with row[v] <= e (row
@@ -288,7 +253,7 @@ __global__ void k_csr_expand(const int32_t *row, int32_t V, int64_t E, uint32_t 
 }
 
 void graph_build_from_device_csr(Context &ctx, Graph &g, int32_t V, int64_t E, const int32_t *d_row,
-                                 uint32_t *d_col, float *d_w) {
+                                 const uint32_t *d_col, const float *d_w) {
     DevBuf src;
     try {
         src.reserve(sizeof(uint32_t) * (size_t)std::max<int64_t>(E, 1));

@@ -111,14 +111,28 @@ void scan_exclusive_u32(Context &ctx, const uint32_t *in, uint32_t *out, int64_t
 void radix_sort_pairs(Context &ctx, uint32_t *keys, uint32_t *vals, int64_t n, int bits,
                       cudaStream_t s);
 
+// Stable sort by the low `bits` bits of a key that carries up to three values
+// along.  The inputs are only read; every output is written.
+struct SortJob {
+    const uint32_t *key_in = nullptr, *pay_in[3] = {nullptr, nullptr, nullptr};
+    uint32_t *key_out = nullptr, *pay_out[3] = {nullptr, nullptr, nullptr};
+    int npay = 0;
+    bool reverse = false;          // the elements in reverse order
+    bool iota = false;             // the last value is the element's number
+    uint32_t *slot_out = nullptr;  // instead of the last value: its inverse, slot_out[value] = position
+};
+void radix_sort(Context &ctx, const SortJob &job, int64_t n, int bits, cudaStream_t s);
+// out[v] = first position of a key >= v among the n sorted keys (all < V), v in [0, V].
+void key_offsets(Context &ctx, const uint32_t *key, int64_t n, int32_t V, uint32_t *out, cudaStream_t s);
+
 // ---- graph construction (graph.cu) ------------------------------------------
+// Edge arrays (device, only read) -> graph.
 void graph_build_from_device_edges(Context &ctx, Graph &g, int32_t V, int64_t E,
-                                   uint32_t *d_src, uint32_t *d_dst, float *d_w,
+                                   const uint32_t *d_src, const uint32_t *d_dst, const float *d_w,
                                    uint32_t flags);
-// A caller's CSR (row checked on the host) -> graph; each row keeps its
-// order.  d_col is used as scratch.
+// A caller's CSR (row checked on the host) -> graph; each row keeps its order.
 void graph_build_from_device_csr(Context &ctx, Graph &g, int32_t V, int64_t E, const int32_t *d_row,
-                                 uint32_t *d_col, float *d_w);
+                                 const uint32_t *d_col, const float *d_w);
 // GTgraph text (host or device bytes) -> graph (gtgraph.cu).
 void graph_from_gtgraph(Context &ctx, Graph &g, const char *text, int64_t len, uint32_t flags);
 
