@@ -6,6 +6,7 @@
 #include <cstring>
 #include <new>
 #include "bfs.cuh"
+#include "bfs_coop.cuh"
 #include "learn.cuh"
 #include "msbfs.cuh"
 #include "multigraph.cuh"
@@ -17,6 +18,9 @@
 namespace mb {
 struct AppStates {
     BfsState bfs;
+    BfsCoopState bfs_coop;
+    DevBuf bfs_out;  // levels of a whole run for a host array
+    ~AppStates() { bfs_out.release(); }
     SsspState bfs_async;  // the asynchronous BFS's unit-weight runs (MB_TUNE_BFS_ASYNC)
     MsBfsState msbfs;
     SsspState sssp;
@@ -81,10 +85,21 @@ mb::AppStates &apps(mb_graph *g) {
     return *g->g.apps;
 }
 
+// Memory that kernels on the current device may use in place.
+bool on_this_device(const void *p) {
+    if (!mb::is_device_ptr(p)) return false;
+    cudaPointerAttributes a;
+    int device = 0;
+    MB_CUDA(cudaPointerGetAttributes(&a, p));
+    MB_CUDA(cudaGetDevice(&device));
+    return a.type == cudaMemoryTypeManaged || a.device == device;
+}
+
 // Copy n int32 from a host or device pointer to host.
 std::vector<int32_t> fetch_i32(const int32_t *p, int64_t n) {
     std::vector<int32_t> out((size_t)n);
-    if (n > 0) MB_CUDA(cudaMemcpy(out.data(), p, sizeof(int32_t) * (size_t)n, cudaMemcpyDefault));
+    if (n > 0 && !mb::is_device_ptr(p)) std::memcpy(out.data(), p, sizeof(int32_t) * (size_t)n);
+    else if (n > 0) MB_CUDA(cudaMemcpy(out.data(), p, sizeof(int32_t) * (size_t)n, cudaMemcpyDefault));
     return out;
 }
 
@@ -152,6 +167,8 @@ int mb_destroy(mb_ctx *ctx) {
     if (ctx->c.pool_counted) mb::pool_context(ctx->c.device, -1);
     if (ctx->c.pinned) cudaFreeHost(ctx->c.pinned);
     if (ctx->c.pinned_small) cudaFreeHost(ctx->c.pinned_small);
+    for (cudaEvent_t e : ctx->c.events)
+        if (e) cudaEventDestroy(e);
     if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
     delete ctx;
     return MB_OK;
@@ -211,13 +228,7 @@ namespace {
 // n bytes from host or device memory, to be read by kernels: this device's
 // memory in place, anything else (host, another GPU) by a copy into b
 const void *stage_in(mb::DevBuf &b, const void *p, size_t n, cudaStream_t s) {
-    if (mb::is_device_ptr(p)) {
-        cudaPointerAttributes a;
-        int device = 0;
-        MB_CUDA(cudaPointerGetAttributes(&a, p));
-        MB_CUDA(cudaGetDevice(&device));
-        if (a.type == cudaMemoryTypeManaged || a.device == device) return p;
-    }
+    if (on_this_device(p)) return p;
     b.reserve(std::max<size_t>(n, 1));
     mb::copy_sync(s, b.p, p, n);
     return b.p;
@@ -788,9 +799,24 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                                (ctx->c.schedule_policy == MB_POLICY_FIXED ||
                                 ctx->c.schedule_policy == MB_POLICY_LEARNED) &&
                                !ctx->c.persist;
+        const bool coop = !bfs_async && mb::bfs_coop_applies(ctx->c);
+        const bool out_here = coop && on_this_device(levels_out);
         if (bfs_async) apps(g).bfs.ensure(g->g);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};
+            if (coop) {
+                int32_t *out = levels_out + (size_t)i * V;
+                const size_t bytes = sizeof(int32_t) * (size_t)V;
+                // a small graph's levels go to a host array through pinned memory
+                const bool pinned = !out_here && !mb::is_device_ptr(levels_out) && mb::bfs_small(g->g);
+                int32_t *dev = out_here ? out : pinned ? (int32_t *)ctx->c.pinned_reserve(bytes)
+                                                       : (int32_t *)apps(g).bfs_out.reserve(bytes);
+                const mb::EmitFn copy = [&](cudaStream_t s) {
+                    MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(int32_t) * (size_t)V, cudaMemcpyDefault, s));
+                };
+                mb::run_bfs_coop(ctx->c, g->g, apps(g).bfs_coop, src[i], dev, &st, out_here || pinned ? nullptr : &copy);
+                if (pinned) std::memcpy(out, dev, bytes);
+            } else {
             // the levels' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {
                 MB_CUDA(cudaMemcpyAsync(levels_out + (size_t)i * V, apps(g).bfs.level.p,
@@ -801,6 +827,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                              apps(g).bfs.level.as<int32_t>(), &copy_out);
             else
                 mb::run_bfs(ctx->c, g->g, apps(g).bfs, src[i], &st, mb::LOOP_ALL, -1, nullptr, &copy_out);
+            }
             total.supersteps = std::max(total.supersteps, st.supersteps);
             total.status_flags |= st.status_flags;
             total.edges_traversed += st.edges_traversed;

@@ -160,6 +160,28 @@ __device__ __forceinline__ int upper_bound_minus1(const uint32_t *s, int n, uint
     return lo;
 }
 
+// The elements of x (n of them, 16-byte aligned) at positions [j, je) within
+// the aligned group of four that holds j, -1 elsewhere; returns the group's
+// first position.  One 16-byte load, except in a last group cut short by n.
+__device__ __forceinline__ int32_t load4_from(const int32_t *x, int32_t j, int32_t je, int64_t n,
+                                              int32_t (&u)[4]) {
+    const int32_t b = j & ~3;
+    if ((int64_t)b + 4 <= n) {
+        const int4 q = __ldg(reinterpret_cast<const int4 *>(x + b));
+        u[0] = q.x;
+        u[1] = q.y;
+        u[2] = q.z;
+        u[3] = q.w;
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; r++) u[r] = (int64_t)b + r < n ? __ldg(&x[b + r]) : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+        if (b + r < j || b + r >= je) u[r] = -1;
+    return b;
+}
+
 // x[i] for a two-element parameter array, without dynamic indexing (which
 // would copy the kernel parameter array to local memory).
 template <class T>

@@ -184,6 +184,12 @@ struct Context {
         uint64_t m;
     };
     std::vector<TraceRec> trace;
+    // timing events of a run, made once
+    cudaEvent_t events[2] = {nullptr, nullptr};
+    cudaEvent_t event(int i) {
+        if (!events[i]) MB_CUDA(cudaEventCreate(&events[i]));
+        return events[i];
+    }
     void *ctrl_readback() { return pinned_small + kCtrlOff; }
     void *pinned_reserve(size_t n) {
         if (n <= pinned_bytes && pinned) return pinned;
