@@ -25,6 +25,7 @@
 // latency of their first list entries); first calls 5.9 -> 0.6 ms, for there is
 // no graph to instantiate.
 #include "bfs_coop.cuh"
+#include "coop.cuh"
 
 namespace mb {
 namespace {
@@ -41,7 +42,7 @@ constexpr int kCoopItems = 2;
 constexpr int kCoopTile = kCoopThreads * kCoopItems;  // edges of a tile
 static_assert(kCoopTile == kBfsCoopTile, "the tile tables are sized by it");
 
-struct CoopCtr {  // one per superstep in turn, three in all
+struct alignas(128) CoopCtr {  // one per superstep in turn, three in all
     unsigned long long q;  // queued vertices << 32 | their out-edges
     uint32_t n, pad;       // a pull's new vertices
     unsigned long long m;  // and their out-edges
@@ -50,7 +51,8 @@ struct CoopShared {  // device memory of a run, zero before it
     CoopCtr ctr[3];
     unsigned long long toq;  // the queue built from a pull's vertices
     unsigned long long reached;
-    uint32_t bar, ticket;
+    uint32_t ticket;
+    alignas(128) uint32_t bar;  // polled: a line of its own
 };
 
 struct CoopArgs {
@@ -191,31 +193,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(CoopArgs a) {
 // ---- one cooperative grid -----------------------------------------------------------
 
 __device__ __forceinline__ bool coop_sync(const CoopArgs &a, uint32_t target) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        constexpr uint32_t kGaveUp = 1u << 31;
-        __threadfence();
-        atomicAdd(&a.sh->bar, 1u);
-        int ok = 0;
-        for (long it = 0;; it++) {
-            const uint32_t v = ld_acquire_gpu(&a.sh->bar);
-            if (v >= kGaveUp) break;
-            if (v >= target) {
-                ok = 1;
-                break;
-            }
-            if (it >= a.polls) {
-                a.out->err = ERR_BARRIER;
-                atomicOr(&a.sh->bar, kGaveUp);
-                break;
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok;
+    return coop_barrier(&a.sh->bar, target, a.polls, &a.out->err);
 }
 
 struct CoopSmem {
@@ -423,7 +401,9 @@ __device__ __forceinline__ void coop_pull(const CoopArgs &a, const uint32_t *vis
 }
 
 // The vertices a pull added (now, not before) -> queue: every warp gathers
-// them in a buffer of its own and appends full buffers with one atomic.
+// them in a buffer of its own and appends full buffers with one atomic (260k
+// vertices of 2^24: 28 us; four words a round and one atomic per CTA and round,
+// as sssp_coop.cu does on its denser bitmaps: 52).
 constexpr int kToqBuf = 64;
 __device__ __forceinline__ void coop_toq(const CoopArgs &a, CoopSmem &sm, const uint32_t *now, const uint32_t *before,
                                          unsigned long long *ctr, uint2 *q, int32_t *tf) {
@@ -647,7 +627,9 @@ void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int3
             int per_sm = 0;
             MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_coop, kCoopThreads, 0));
             if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative BFS kernel does not fit on an SM");
-            const int grid = ctx.num_sms * std::min(per_sm, kBfsCoopCtas);
+            // no more CTAs than tiles: fewer arrive at the barriers of small graphs
+            const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kBfsCoopCtas),
+                                                    std::max<int64_t>(g.E / kCoopTile, 16));
             MB_CUDA(cudaEventRecord(e0, s));
             MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(CoopShared), s));
             void *params[] = {&a};

@@ -14,13 +14,15 @@
 #include "pagerank.cuh"
 #include "sched.cuh"
 #include "sssp.cuh"
+#include "sssp_coop.cuh"
 
 namespace mb {
 struct AppStates {
     BfsState bfs;
     BfsCoopState bfs_coop;
-    DevBuf bfs_out;  // levels of a whole run for a host array
-    ~AppStates() { bfs_out.release(); }
+    SsspCoopState sssp_coop;
+    DevBuf run_out;  // levels or distances of a one-launch run for a host array
+    ~AppStates() { run_out.release(); }
     SsspState bfs_async;  // the asynchronous BFS's unit-weight runs (MB_TUNE_BFS_ASYNC)
     MsBfsState msbfs;
     SsspState sssp;
@@ -810,7 +812,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                 // a small graph's levels go to a host array through pinned memory
                 const bool pinned = !out_here && !mb::is_device_ptr(levels_out) && mb::bfs_small(g->g);
                 int32_t *dev = out_here ? out : pinned ? (int32_t *)ctx->c.pinned_reserve(bytes)
-                                                       : (int32_t *)apps(g).bfs_out.reserve(bytes);
+                                                       : (int32_t *)apps(g).run_out.reserve(bytes);
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(int32_t) * (size_t)V, cudaMemcpyDefault, s));
                 };
@@ -882,14 +884,25 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
+        const bool coop = mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop);
+        const bool out_here = coop && on_this_device(dist_out);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};
+            if (coop) {
+                float *out = dist_out + (size_t)i * V;
+                float *dev = out_here ? out : (float *)apps(g).run_out.reserve(sizeof(float) * (size_t)V);
+                const mb::EmitFn copy = [&](cudaStream_t s) {
+                    MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(float) * (size_t)V, cudaMemcpyDefault, s));
+                };
+                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, src[i], dev, &st, out_here ? nullptr : &copy);
+            } else {
             // the distances' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {
                 MB_CUDA(cudaMemcpyAsync(dist_out + (size_t)i * V, apps(g).sssp.dist.p,
                                         sizeof(float) * (size_t)V, cudaMemcpyDefault, s));
             };
             mb::run_sssp(ctx->c, g->g, apps(g).sssp, src[i], &st, mb::LOOP_ALL, -1, nullptr, nullptr, &copy_out);
+            }
             total.supersteps = std::max(total.supersteps, st.supersteps);
             total.status_flags |= st.status_flags;
             total.edges_traversed += st.edges_traversed;

@@ -1,0 +1,496 @@
+// sssp_coop.cu -- a whole SSSP in one launch, for graphs with hubs under the
+// fixed rule.
+//
+// Frontier Bellman-Ford relaxes 3.7 to 6 edges per reached edge on R-MAT
+// graphs.  Distance buckets (near-far: Davidson, Baxter, Garland & Owens,
+// IPDPS 2014) cut that to 1.3 to 2, but need three to five times the
+// supersteps, which the loop graph's 12-17 us per superstep made a loss.
+// Here the supersteps follow one another inside one cooperative grid with one
+// barrier each (6-8 us for a small one), so the buckets pay.
+//
+// A superstep relaxes the out-edges of the near queue.  A vertex whose
+// distance drops below the threshold T joins the next queue, once per
+// superstep (a claim bit; two claim bitmaps in turn, so that a bit is cleared
+// while the vertex is expanded and no superstep claims in it); one that drops
+// to T or above gets a bit in the far bitmap.  When the queue runs dry, T
+// rises by delta, past the least distance the last split kept (the same rules
+// as choose_next, engine.cuh), and a split moves the far vertices now below T
+// to the queue; one that is below the old T was expanded at that distance
+// already and only loses its bit.  Every order reaches the same fixpoint,
+// the exact distances; with weights that are not integers too, since a float
+// sum along a path is monotone in its start.
+// A superstep of at least kBmMin edges claims without asking for the result and
+// builds the queue from the claim bitmap in a pass of its own: an append per
+// tile costs more there than the pass.
+#include "coop.cuh"
+#include "sssp.cuh"
+#include "sssp_coop.cuh"
+
+namespace mb {
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kItems = 2;
+constexpr int kTileE = kThreads * kItems;
+static_assert(kTileE >= kSsspCoopTile, "the tile tables are sized by it");
+constexpr int kCtas = 3;  // per SM; 2: 0.82 / 4.3 ms, 4 (32 registers, spills): slower on both
+constexpr uint32_t kInf = 0x7f800000u;
+constexpr uint32_t kBmMin = 1 << 20;  // 2^19 and less: 2-4% slower
+// Bucket width in mean weights.  0.5 / 0.7 / 0.85 / 1 / 1.5 / none, ms: mild R-MAT
+// 2^20 / 2^24 0.90 / 0.79 / 0.79 / 0.86 / 1.08 / 1.22; 2^23 / 10^8 3.31 / 3.80 / 3.43 /
+// 2.96 / 4.6 / 6.7; the skewed one 2^20 / 2^24 1.05 / 0.95 / 0.99 / 0.99 / 0.98 / 0.96.
+// Below kBucketMinE edges the supersteps saved by no buckets are worth more
+// (10^4 / 10^5: 0.118 without, 0.146 with).
+constexpr float kBucketWidth = 0.85f;
+constexpr int64_t kBucketMinE = 1 << 18;
+
+__device__ __forceinline__ float inf_f() { return __uint_as_float(kInf); }
+
+struct alignas(128) SCtr {  // one per iteration in turn, three in all
+    unsigned long long q;  // queued vertices << 32 | their out-edges
+    uint32_t far;          // a vertex was put off
+    uint32_t far_min;      // split: float bits of the least distance kept
+};
+struct SShared {  // device memory of a run, zero before it
+    SCtr ctr[3];
+    unsigned long long reached, edges;
+    uint32_t ticket;
+    alignas(128) uint32_t bar;  // polled: a line of its own
+};
+
+struct SArgs {
+    int32_t V;
+    int64_t W;
+    const int32_t *row, *col;
+    const float *wt;
+    float *dist;
+    uint32_t *claim[2], *far;
+    uint2 *q[2];      // {first edge less the out-edges queued before it, those}
+    int32_t *qv[2];   // vertices
+    int32_t *tf[2];   // first entry of each tile
+    SShared *sh;
+    SsspCoopOut *out;  // host memory
+    int32_t source, cap;
+    float delta;       // 0: no buckets
+    long polls;
+};
+
+struct SSmem {
+    uint32_t off[kTileE + 1];
+    int32_t row[kTileE + 1];
+    float du[kTileE + 1];
+    uint2 out[kTileE];  // found vertices: {first edge, out-edges}
+    int32_t outv[kTileE];
+    uint32_t nout;
+    uint32_t wtot[kThreads / 32];
+    unsigned long long base;
+};
+
+__device__ __forceinline__ void write_entry(const SArgs &a, int nx, uint32_t pos, int32_t v, uint32_t rs, uint32_t d,
+                                            uint32_t off) {
+    pick(a.q, nx)[pos] = make_uint2(rs - off, off);
+    pick(a.qv, nx)[pos] = v;
+    int32_t *tf = pick(a.tf, nx);
+    const uint32_t t0 = (off + kTileE - 1) / kTileE, t1 = (off + d - 1) / kTileE;
+    for (uint32_t t = t0; t <= t1; t++) tf[t] = (int32_t)pos;
+}
+
+__device__ __forceinline__ void found(SSmem &sm, bool pred, int32_t v, int32_t rs, uint32_t d) {
+    const unsigned mask = __ballot_sync(0xffffffffu, pred);
+    if (!mask) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(&sm.nout, (uint32_t)__popc(mask));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (pred) {
+        const uint32_t i = base + __popc(mask & lanemask_lt());
+        sm.out[i] = make_uint2((uint32_t)rs, d);
+        sm.outv[i] = v;
+    }
+}
+
+// The tile's found vertices -> the next queue, one atomic per tile.
+__device__ __forceinline__ void flush(const SArgs &a, SSmem &sm, unsigned long long *ctr, int nx) {
+    __syncthreads();
+    const uint32_t n = sm.nout;
+    if (n == 0) return;  // the same for every thread
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t i0 = threadIdx.x * kItems;
+    uint2 e[kItems];
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+        e[k] = i0 + k < n ? sm.out[i0 + k] : make_uint2(0u, 0u);
+        sum += e[k].y;
+    }
+    const uint32_t incl = warp_incl_scan_u32(sum);
+    if (lane == 31) sm.wtot[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+        constexpr int kW = kThreads / 32;
+        const uint32_t t = lane < kW ? sm.wtot[lane] : 0u;
+        const uint32_t ti = warp_incl_scan_u32(t);
+        if (lane < kW) sm.wtot[lane] = ti - t;
+        if (lane == kW - 1) {
+            sm.base = atomicAdd(ctr, ((unsigned long long)n << 32) | ti);
+            sm.nout = 0;
+        }
+    }
+    __syncthreads();
+    const unsigned long long base = sm.base;
+    uint32_t off = (uint32_t)base + sm.wtot[wid] + incl - sum;
+#pragma unroll
+    for (int k = 0; k < kItems; k++)
+        if (i0 + k < n) {
+            write_entry(a, nx, (uint32_t)(base >> 32) + i0 + k, sm.outv[i0 + k], e[k].x, e[k].y, off);
+            off += e[k].y;
+        }
+}
+
+// par: the claim bitmap of this superstep.
+template <bool kBm>
+__device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_t n, uint32_t m, float T, int par,
+                                     SCtr *ctr) {
+    const uint32_t tiles = (m + kTileE - 1) / kTileE;
+    const uint2 *q = pick(a.q, cur);
+    const int32_t *qv = pick(a.qv, cur), *tf = pick(a.tf, cur);
+    uint32_t *claim = pick(a.claim, par), *old = pick(a.claim, par ^ 1);
+    bool far = false;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const uint32_t c0 = t * kTileE, c1 = min(c0 + kTileE, m);
+        const int32_t i0 = __ldcg(&tf[t]);
+        const int32_t i1 = t + 1 < tiles ? __ldcg(&tf[t + 1]) : (int32_t)n - 1;
+        const int k = i1 - i0 + 1;
+        for (int j = threadIdx.x; j < k; j += kThreads) {
+            const uint2 e = __ldcg(&q[i0 + j]);
+            const int32_t u = __ldcg(&qv[i0 + j]);
+            sm.off[j] = e.y;
+            sm.row[j] = (int32_t)e.x;
+            sm.du[j] = __ldcg(&a.dist[u]);
+            old[u >> 5] = 0u;  // every bit set there is of a vertex in this queue
+        }
+        __syncthreads();
+        int32_t v[kItems];
+        float nd[kItems], dv[kItems];
+        {
+            const uint32_t e0 = c0 + threadIdx.x * kItems;
+            int j = e0 < c1 ? upper_bound_minus1(sm.off, k, e0) : 0;
+#pragma unroll
+            for (int r = 0; r < kItems; r++) {
+                const uint32_t e = e0 + r;
+                v[r] = -1;
+                nd[r] = 0.f;
+                if (e < c1) {
+                    while (j + 1 < k && sm.off[j + 1] <= e) j++;
+                    const int32_t at = sm.row[j] + (int32_t)e;
+                    v[r] = __ldg(&a.col[at]);
+                    nd[r] = sm.du[j] + __ldg(&a.wt[at]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kItems; r++) dv[r] = v[r] >= 0 ? __ldcg(&a.dist[v[r]]) : 0.f;
+#pragma unroll
+        for (int r = 0; r < kItems; r++) {
+            bool own = false;
+            int32_t rs = 0, re = 0;
+            if (nd[r] < dv[r]) {
+                atomicMin((unsigned *)&a.dist[v[r]], __float_as_uint(nd[r]));
+                const uint32_t bit = 1u << (v[r] & 31);
+                if (nd[r] >= T) {
+                    far = true;
+                    atomicOr(&a.far[v[r] >> 5], bit);  // a test of the bit first costs more
+                } else if (kBm) {
+                    atomicOr(&claim[v[r] >> 5], bit);
+                } else {
+                    rs = __ldg(&a.row[v[r]]);
+                    re = __ldg(&a.row[v[r] + 1]);
+                    own = !(atomicOr(&claim[v[r] >> 5], bit) & bit);
+                }
+            }
+            if (!kBm) found(sm, own && re > rs, v[r], rs, (uint32_t)(re - rs));
+        }
+        if (kBm) __syncthreads();  // the tile's entries are reloaded next
+        else flush(a, sm, &ctr->q, cur ^ 1);
+    }
+    // one store per CTA at most: the same address from every warp queues up
+    if (__syncthreads_or(far) && threadIdx.x == 0) ctr->far = 1u;
+}
+
+// Vertices of a bitmap -> queue nx.  A warp takes four words (128 vertices) a
+// round, their loads in flight together and the next round's words on their
+// way; the CTA appends a round with one atomic.  (Word after word, each with
+// its own chain of loads and an atomic, a warp's share of a 2^20-vertex bitmap
+// took 30 to 60 us.)  kSplit: the far bitmap -- those below T leave it, and of
+// these the ones not below T0 are queued; the least distance kept goes to
+// ctr->far_min.  Else a claim bitmap, cleared.
+template <bool kSplit>
+__device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t *bm, float T0, float T, int nx,
+                                         SCtr *ctr) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t units = a.W / 4, step = (int64_t)gridDim.x * (kThreads / 32);
+    const int64_t first = (int64_t)blockIdx.x * (kThreads / 32);
+    uint32_t kept = kInf;
+    auto words = [&](int64_t u) {
+        return u < units ? __ldcg(reinterpret_cast<const uint4 *>(bm) + u) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    uint4 next = words(first + wid);
+    for (int64_t c = first; c < units; c += step) {
+        const int64_t u = c + wid;
+        const uint32_t x[4] = {next.x, next.y, next.z, next.w};
+        next = words(u + step);
+        if (!__syncthreads_or((x[0] | x[1] | x[2] | x[3]) != 0u)) continue;
+        const int32_t v0 = (int32_t)(u * 128) + lane;
+        bool take[4];
+        if (kSplit) {
+            float d[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) d[k] = (x[k] >> lane) & 1u ? __ldcg(&a.dist[v0 + 32 * k]) : inf_f();
+            uint32_t keep[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const bool has = (x[k] >> lane) & 1u;
+                take[k] = has && d[k] < T && d[k] >= T0;
+                const bool stay = has && !(d[k] < T);
+                if (stay) kept = min(kept, __float_as_uint(d[k]));
+                keep[k] = __ballot_sync(0xffffffffu, stay);
+            }
+            if (lane == 0 && (keep[0] != x[0] || keep[1] != x[1] || keep[2] != x[2] || keep[3] != x[3]))
+                reinterpret_cast<uint4 *>(bm)[u] = make_uint4(keep[0], keep[1], keep[2], keep[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) take[k] = (x[k] >> lane) & 1u;
+            if (lane == 0 && (x[0] | x[1] | x[2] | x[3]) != 0u)
+                reinterpret_cast<uint4 *>(bm)[u] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        int32_t rs[4];
+        uint32_t dg[4], sum = 0, cnt = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            rs[k] = 0;
+            dg[k] = 0;
+            if (take[k]) {
+                rs[k] = __ldg(&a.row[v0 + 32 * k]);
+                dg[k] = (uint32_t)(__ldg(&a.row[v0 + 32 * k + 1]) - rs[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            sum += dg[k];
+            cnt += dg[k] > 0;
+        }
+        const unsigned long long base = coop_round_append(cr, cnt, sum, &ctr->q);
+        uint32_t pos = (uint32_t)(base >> 32), off = (uint32_t)base;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (dg[k] > 0) {
+                write_entry(a, nx, pos, v0 + 32 * k, (uint32_t)rs[k], dg[k], off);
+                pos++;
+                off += dg[k];
+            }
+    }
+    if (kSplit) {
+        kept = __reduce_min_sync(0xffffffffu, kept);
+        if (lane == 0 && kept < kInf) atomicMin(&ctr->far_min, kept);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
+    __shared__ SSmem sm;
+    __shared__ CoopRound cr;
+    __shared__ unsigned long long s_n[kThreads / 32], s_m[kThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t gt = (int64_t)blockIdx.x * kThreads + tid, gn = (int64_t)gridDim.x * kThreads;
+    const float inf = inf_f();
+    uint32_t target = 0;
+    auto sync = [&] {
+        target += gridDim.x;
+        return coop_barrier(&a.sh->bar, target, a.polls, &a.out->err);
+    };
+    int cur = 0, par = 0, it = 0, supersteps = 0, splits = 0, err = 0;
+    const int32_t rs0 = __ldg(&a.row[a.source]), deg0 = __ldg(&a.row[a.source + 1]) - rs0;
+    for (int64_t v = gt; v < a.V; v += gn) a.dist[v] = v == a.source ? 0.f : kMedusaMax;
+    for (int64_t w = gt; w < a.W; w += gn) {
+        a.claim[0][w] = 0u;
+        a.claim[1][w] = 0u;
+        a.far[w] = 0u;
+    }
+    for (int64_t t = gt; t * kTileE < deg0; t += gn) a.tf[0][t] = 0;
+    if (gt == 0) {
+        a.q[0][0] = make_uint2((uint32_t)rs0, 0u);
+        a.qv[0][0] = a.source;
+        a.sh->ctr[0] = SCtr{0ull, 0u, kInf};
+    }
+    if (tid == 0) sm.nout = 0;
+    uint32_t n = deg0 > 0 ? 1u : 0u, m = (uint32_t)deg0;
+    unsigned long long work = 0;
+    float T = a.delta > 0.f ? a.delta : inf, fmin = inf;
+    bool far = false;
+    if (!sync()) return;
+    for (;; it++) {
+        if (n == 0 && !far) break;
+        if (it >= a.cap) {
+            err = ERR_STEP_CAP;
+            break;
+        }
+        SCtr *ctr = &a.sh->ctr[it % 3];
+        // last read before the barrier just passed
+        if (gt == 0) a.sh->ctr[(it + 1) % 3] = SCtr{0ull, 0u, kInf};
+        if (n == 0) {  // next bucket
+            const float T0 = T;
+            T = T0 + a.delta;
+            if (fmin < inf) T = fmaxf(T, fmin + a.delta);
+            if (!(T > T0)) T = __uint_as_float(__float_as_uint(T0) + 1u);
+            if (fmin < inf && !(T > fmin)) T = __uint_as_float(__float_as_uint(fmin) + 1u);
+            to_queue<true>(a, cr, a.far, T0, T, cur, ctr);
+            if (!sync()) return;
+            fmin = __uint_as_float(__ldcg(&ctr->far_min));
+            far = fmin < inf;
+            splits++;
+        } else {
+            work += m;
+            const bool bm = m >= kBmMin;
+            if (bm) {
+                push<true>(a, sm, cur, n, m, T, par, ctr);
+                if (!sync()) return;
+                to_queue<false>(a, cr, pick(a.claim, par), 0.f, 0.f, cur ^ 1, ctr);
+            } else {
+                push<false>(a, sm, cur, n, m, T, par, ctr);
+            }
+            if (!sync()) return;
+            far = far || __ldcg(&ctr->far) != 0u;
+            cur ^= 1;
+            par ^= 1;
+            supersteps++;
+        }
+        const unsigned long long c = __ldcg(&ctr->q);
+        n = (uint32_t)(c >> 32);
+        m = (uint32_t)c;
+    }
+    // reached vertices and their out-edges
+    unsigned long long rn = 0, rm = 0;
+    for (int64_t v = gt; v < a.V; v += gn)
+        if (__ldcg(&a.dist[v]) < kMedusaMax) {
+            rn++;
+            rm += (uint32_t)(__ldg(&a.row[v + 1]) - __ldg(&a.row[v]));
+        }
+    rn = warp_sum(rn);
+    rm = warp_sum(rm);
+    if (lane == 0) {
+        s_n[tid >> 5] = rn;
+        s_m[tid >> 5] = rm;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        rn = rm = 0;
+        for (int w = 0; w < kThreads / 32; w++) {
+            rn += s_n[w];
+            rm += s_m[w];
+        }
+        if (rn) {
+            atomicAdd(&a.sh->reached, rn);
+            atomicAdd(&a.sh->edges, rm);
+        }
+        __threadfence();
+        if (atomicAdd(&a.sh->ticket, 1u) == gridDim.x - 1) {  // the last CTA reports
+            a.out->supersteps = supersteps;
+            a.out->splits = splits;
+            a.out->reached = atomicAdd(&a.sh->reached, 0ull);
+            a.out->edges = atomicAdd(&a.sh->edges, 0ull);
+            a.out->work = work;
+            if (err) a.out->err = err;
+        }
+    }
+}
+
+}  // namespace
+
+void SsspCoopState::ensure(const Graph &g) {
+    if (built) return;
+    const size_t tiles = (size_t)(g.E / kSsspCoopTile) + 2, W = (((size_t)g.V + 31) / 32 + 3) & ~(size_t)3;
+    for (int i = 0; i < 2; i++) {
+        claim[i].reserve(sizeof(uint32_t) * W);
+        q[i].reserve(sizeof(uint2) * (size_t)g.V);
+        qv[i].reserve(sizeof(int32_t) * (size_t)g.V);
+        tf[i].reserve(sizeof(int32_t) * tiles);
+    }
+    far.reserve(sizeof(uint32_t) * W);
+    sh.reserve(sizeof(SShared));
+    double mean = 0.0;
+    bool bad = false;
+    sssp_weight_stats(g, &mean, &bad);
+    mean_w = (float)mean;
+    weights_ok = !bad;
+    built = true;
+}
+
+bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st) {
+    // the loop graph's and the asynchronous kernel's own parameters ask for them
+    for (int t : {MB_TUNE_SSSP_BM_PUSH_MIN, MB_TUNE_PUSH_BLOCKS_PER_SM, MB_TUNE_VERTEX_BLOCKS_PER_SM,
+                  MB_TUNE_TAIL_EDGES, MB_TUNE_BULK_STAGE, MB_TUNE_SMALL_PUSH_EDGES, MB_TUNE_SSSP_ASYNC,
+                  MB_TUNE_ASYNC_DELTA, MB_TUNE_ASYNC_BLOCKS_PER_SM, MB_TUNE_ASYNC_BELOW})
+        if (ctx.tunable[t] >= 0) return false;
+    if (ctx.schedule_policy != MB_POLICY_FIXED || !ctx.use_graphs || ctx.tracing || ctx.persist || !ctx.tail ||
+        ctx.max_step >= 0 || ctx.sssp_delta != 0.f)
+        return false;
+    if (async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
+    st.ensure(g);
+    return st.weights_ok;
+}
+
+void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, int32_t source, float *dist, mb_stats *stats,
+                   const EmitFn *after) {
+    static_assert(sizeof(SsspCoopOut) <= Context::kSmallBytes - Context::kCtrlOff, "readback too small");
+    cudaStream_t s = ctx.stream;
+    volatile SsspCoopOut *out = (volatile SsspCoopOut *)ctx.ctrl_readback();
+    out->err = 0;
+    SArgs a{};
+    a.V = g.V;
+    a.W = ((((int64_t)g.V + 31) / 32) + 3) & ~3ll;  // whole units of to_queue
+    a.row = g.row.as<int32_t>();
+    a.col = g.col.as<int32_t>();
+    a.wt = g.wt.as<float>();
+    a.dist = dist;
+    for (int i = 0; i < 2; i++) {
+        a.claim[i] = st.claim[i].as<uint32_t>();
+        a.q[i] = st.q[i].as<uint2>();
+        a.qv[i] = st.qv[i].as<int32_t>();
+        a.tf[i] = st.tf[i].as<int32_t>();
+    }
+    a.far = st.far.as<uint32_t>();
+    a.sh = st.sh.as<SShared>();
+    a.out = (SsspCoopOut *)ctx.ctrl_readback();
+    a.source = source;
+    a.cap = step_cap(ctx, (int64_t)g.V * 4 + 16);
+    a.delta = g.E >= kBucketMinE ? kBucketWidth * st.mean_w : 0.f;
+    a.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
+    int per_sm = 0;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sssp_coop, kThreads, 0));
+    if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative SSSP kernel does not fit on an SM");
+    // no more CTAs than tiles: fewer arrive at the barriers of small graphs
+    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kCtas), std::max<int64_t>(g.E / kTileE, 16));
+    const cudaEvent_t e0 = ctx.event(0), e1 = ctx.event(1);
+    MB_CUDA(cudaEventRecord(e0, s));
+    MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(SShared), s));
+    void *params[] = {&a};
+    MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_sssp_coop, dim3(grid), dim3(kThreads), params, 0, s));
+    MB_CUDA(cudaEventRecord(e1, s));
+    if (after) (*after)(s);
+    MB_CUDA(cudaStreamSynchronize(s));
+    float ms = 0;
+    MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if (out->err & ERR_BARRIER) fail(MB_ERR_TIMEOUT, "sssp: a grid barrier timed out");
+    if (out->err & ERR_STEP_CAP) fail(MB_ERR_TIMEOUT, "sssp: superstep cap reached");
+    if (stats) {
+        *stats = mb_stats{};
+        stats->supersteps = out->supersteps + out->splits;
+        stats->edges_traversed = (int64_t)out->edges;
+        stats->vertices_reached = (int64_t)out->reached;
+        stats->device_ms = ms;
+        stats->schedule_count[MB_SCHED_PUSH_EDGE_QUEUE] = out->supersteps;
+        stats->kernel_launches = 1;
+        stats->edges_scanned = (int64_t)out->work;
+    }
+}
+
+}  // namespace mb
