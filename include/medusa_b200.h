@@ -366,7 +366,7 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                 at least E / gamma out-edges (default 16; 0: no floor) */
 #define MB_TUNE_PR_HUB_MIN 12 /* PageRank in the reference's order: in-degree above
                                 which one CTA sums a vertex by the parallel
-                                integer scan (default 2048; at least 64) */
+                                integer scan (default E / 2^14 within 512 .. 2048; at least 64) */
 #define MB_TUNE_WAIT_POLLS 13 /* polls before a bounded device wait gives up -- the grid
                                 barrier of the persistent kernels, the team barrier of the
                                 many-graph kernel, the bulk-copy wait of the staged push

@@ -267,11 +267,29 @@ struct SellArgs {
     int32_t ngroups, nlong; // groups [0, nlong) have more than kSellShort rows
     const float *contrib_in;
     float *contrib_out, *rank_out;
-    uint32_t *ctr;          // units taken by late warps, zero before the launch
+    uint32_t *ctr;          // units taken by late warps, zero before the launch (null: every unit has its warp)
+    // vertices without in-edges: their sum is 0 in every superstep, so their
+    // contributions are written once to each of the two buffers (zfirst), their
+    // ranks with the others'
+    const int32_t *zv;
+    const int2 *zpd;
+    int32_t nz;
+    int32_t zfirst;
 };
+
+__device__ __forceinline__ void zero_vertices(const SellArgs &a) {
+    if (!a.zfirst && !a.rank_out) return;
+    const float r = pr_update(0.f);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.nz; i += (int64_t)gridDim.x * blockDim.x) {
+        const int2 p = a.zpd[i];
+        if (a.zfirst && p.x >= 0) a.contrib_out[p.x] = r / (float)p.y;
+        if (a.rank_out) a.rank_out[a.zv[i]] = r;
+    }
+}
 constexpr int kSellShort = 8;
 // Two builds of the kernel: 16 rows in flight and at least 5 CTAs per SM, or
-// 8 and 8 CTAs, which every unit of a small graph fits into at once (R-MAT
+// 8 and 8 CTAs, where that takes every unit at once and the first does not (light
+// vertices only: a long group's chain wants the deeper prefetch; R-MAT
 // 2^24 / 2^28: 0.955 against 1.011 ms a superstep; uniform 2^18 / 2^22: 25.8
 // against 22.8 us).
 constexpr int kSellU = 16, kSellCtas = 5, kSellUSmall = 8, kSellCtasSmall = 8;
@@ -361,12 +379,13 @@ __global__ void __launch_bounds__(256, kSmall ? kSellCtasSmall : kSellCtas) k_pr
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t units = (uint32_t)a.nlong + (uint32_t)(a.ngroups - a.nlong + kG - 1) / kG;
     uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    zero_vertices(a);
     while (u < units) {
         uint32_t t = 0;  // the next unit's number is on its way during this one
-        if ((threadIdx.x & 31) == 0 && warps < units) t = atomicAdd(a.ctr, 1u);
+        if ((threadIdx.x & 31) == 0 && a.ctr) t = atomicAdd(a.ctr, 1u);
         if (u < (uint32_t)a.nlong) sell_long<kSmall ? kSellUSmall : kSellU>(a, u);
         else sell_short<kG>(a, a.nlong + (int64_t)(u - a.nlong) * kG);
-        if (warps >= units) break;
+        if (!a.ctr) break;
         u = warps + __shfl_sync(0xffffffffu, t, 0);
     }
 }
@@ -379,14 +398,16 @@ __global__ void __launch_bounds__(256, kSmall ? kSellCtasSmall : kSellCtas) k_pr
 // acquire drops stale L1 lines).  A barrier that gives up writes *err (host
 // memory) and ends the launch.  Uniform 2^18 / 2^22, ten supersteps: 20.4 us
 // each, against 22.8 in launches of their own (the gathers alone: 14).
-constexpr int kResThreads = 1024, kResCtas = 2;  // 32 registers: 64 warps per SM
-constexpr int kResU = 8;
+// 8 rows in flight at 32 registers (64 warps per SM), or 16 where half the
+// warps are enough: the fewer rounds, the shorter a small graph's superstep.
+constexpr int kResThreads = 1024;
 struct ResidentArgs {
     float *contrib[2], *rank;
     const int32_t *zv;  // vertices without in-edges
     const int2 *zpd;
     int32_t nz, iters;
-    uint32_t *bar;      // arrivals, zero before the launch; top bit: a wait gave up
+    uint32_t *bar;      // arrivals (top bit: a wait gave up), and CTAs done, on lines of their own;
+                        // zero before the launch, which leaves them so
     volatile int *err;
     long polls;
 };
@@ -418,7 +439,8 @@ __device__ __forceinline__ bool resident_sync(const ResidentArgs &a, uint32_t ta
     __syncthreads();
     return s_ok;
 }
-__global__ void __launch_bounds__(kResThreads, kResCtas) k_pr_resident(SellArgs a, ResidentArgs r) {
+template <int kResU>
+__global__ void __launch_bounds__(kResThreads, kResU == 8 ? 2 : 1) k_pr_resident(SellArgs a, ResidentArgs r) {
     const int lane = threadIdx.x & 31;
     // the longest groups spread over the CTAs
     const int32_t g = (int32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
@@ -461,25 +483,21 @@ __global__ void __launch_bounds__(kResThreads, kResCtas) k_pr_resident(SellArgs 
         }
         if (it < 2 || rank) {
             const float zr = pr_update(0.f);
-            for (int32_t i = blockIdx.x * kResThreads + threadIdx.x; i < r.nz; i += gridDim.x * kResThreads) {
+            for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < r.nz; i += gridDim.x * blockDim.x) {
                 const int2 p = r.zpd[i];
                 if (it < 2 && p.x >= 0) cout[p.x] = zr / (float)p.y;
                 if (rank) rank[r.zv[i]] = zr;
             }
         }
     }
-}
-
-// Vertices without in-edges: their sum is 0 in every superstep, so their
-// contributions are written once to each of the two buffers.
-__global__ void k_pr_zero(const int32_t *v, const int2 *pd, int32_t n, float *contrib, float *rank) {
-    const float r = pr_update(0.f);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int2 p = pd[i];
-        if (contrib && p.x >= 0) contrib[p.x] = r / (float)p.y;
-        if (rank) rank[v[i]] = r;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&r.bar[32], 1u) == gridDim.x - 1) {  // no CTA waits any more
+        r.bar[0] = 0u;
+        r.bar[32] = 0u;
     }
 }
+
+__global__ void k_pr_zero(SellArgs a) { zero_vertices(a); }  // a graph without any in-edge list
 
 // ---- the reference's order (MB_PR_ORDER_REFERENCE), in parallel -------------
 // Every vertex's sum is the reference's sequential float fold over its MEG
@@ -491,7 +509,13 @@ __global__ void k_pr_zero(const int32_t *v, const int2 *pd, int32_t n, float *co
 //     k_pr_hub_exact), on side streams beside the sliced ELL.
 constexpr int kHubK = 16;                       // consecutive slots per thread
 constexpr int kHubBig = 16384;                  // in-degree above which a hub gets the big CTA
-constexpr int kHubMinDefault = 2048;
+// In-degree above which a vertex is a hub by default: E / 2^14 within these.  A
+// sliced-ELL group is a chain of gathers as long as its rows (2048 rows: some
+// 150 us), which has to stay short against the superstep; a scan costs more
+// per slot.  us per superstep at 512 / 1024 / 2048: skewed R-MAT 10^5 / 2^20 61 /
+// 61 / 89, 0.6M / 11M 138 / 124 / 177, 2^21 / 2^25 220 / 212 / 186, 2^23 / 2^27 702 /
+// 500 / 500.
+constexpr int kHubMinLeast = 512, kHubMinMost = 2048;
 
 struct ExactArgs {
     const int32_t *rrow, *outdeg;
@@ -1073,6 +1097,7 @@ void PrState::build_sell(Context &ctx, const Graph &g, int32_t max_rows, const i
     cudaStream_t s = ctx.stream;
     const int gridV = grid_for(V, 256, ctx.num_sms * 16);
     max_rows = std::min(max_rows, g.max_indeg);
+    out.max_rows = max_rows;
     int bits = 1;
     while (bits < 32 && ((int64_t)1 << bits) < (int64_t)max_rows + 2) bits++;
     DevBuf key, val, cnt;
@@ -1210,7 +1235,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     const bool unfused = sched == MB_SCHED_PUSH_UNFUSED;
     const int32_t hub_min = ctx.tunable[MB_TUNE_PR_HUB_MIN] > 0
                                 ? (int32_t)std::min<int64_t>(ctx.tunable[MB_TUNE_PR_HUB_MIN], 0x7fffffff)
-                                : kHubMinDefault;
+                                : (int32_t)std::min<int64_t>(std::max<int64_t>(g.E >> 14, kHubMinLeast), kHubMinMost);
     if (ref_order) build_meg_order(ctx, g, st);
     if (ref_order && !unfused) st.ensure_exact(ctx, g, hub_min);
     if (!ref_order) st.ensure_fixed(ctx, g);
@@ -1283,21 +1308,26 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     };
     // one superstep of the vertices of a sliced ELL, those without in-edges included
     auto sell_step = [&](cudaStream_t cs, const PrSell &l, const PrArgs &p, int it) {
-        if (l.nz && (it < 2 || p.rank_out)) {
-            k_pr_zero<<<grid_for(l.nz, 256, ctx.num_sms * 8), 256, 0, cs>>>(
-                l.zv.as<int32_t>(), l.zpd.as<int2>(), l.nz, it < 2 ? p.contrib_out : nullptr, p.rank_out);
-            MB_CHECK_LAUNCH();
-        }
-        if (!l.ngroups) return;
         SellArgs a = sell_args(l);
         a.contrib_in = p.contrib_in;
         a.contrib_out = p.contrib_out;
         a.rank_out = p.rank_out;
-        a.ctr = st.ctr.as<uint32_t>() + it;
+        a.zv = l.zv.as<int32_t>();
+        a.zpd = l.zpd.as<int2>();
+        a.nz = l.nz;
+        a.zfirst = it < 2;
+        if (!l.ngroups) {
+            k_pr_zero<<<grid_for(l.nz, 256, ctx.num_sms * 8), 256, 0, cs>>>(a);
+            MB_CHECK_LAUNCH();
+            return;
+        }
         void *params[] = {&a};
         const int64_t units = (int64_t)l.nlong + (l.ngroups - l.nlong + vpl - 1) / vpl;
-        const int small = units <= (int64_t)grid_sell[1] * (256 / 32);
-        MB_CUDA(cudaLaunchKernel(sell_fn[small][vi], grid_for(units * 32, 256, grid_sell[small]), 256, params, 0, cs));
+        const int small = l.max_rows <= kPrLight && units > (int64_t)grid_sell[0] * (256 / 32) &&
+                          units <= (int64_t)grid_sell[1] * (256 / 32);
+        const int grid = grid_for(units * 32, 256, grid_sell[small]);
+        a.ctr = (int64_t)grid * (256 / 32) < units ? st.ctr.as<uint32_t>() + it : nullptr;
+        MB_CUDA(cudaLaunchKernel(sell_fn[small][vi], grid, 256, params, 0, cs));
     };
     const int grid_vtx = ctx.num_sms * 8;
     const int hub_ctas = ctx.tunable[MB_TUNE_PR_HUB_CTAS] > 0 ? (int)ctx.tunable[MB_TUNE_PR_HUB_CTAS]
@@ -1322,19 +1352,29 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         x.nstage_items = st.nstage_items;
         return x;
     };
-    st.ctr.reserve(sizeof(uint32_t) * (size_t)std::max(iters, 1));
     // all supersteps in one launch (k_pr_resident)
     const PrSell &all = ref_order ? st.sell : st.light;
-    int grid_res = 0;
+    int grid_res = 0, res_threads = kResThreads;
+    const void *res_fn = (const void *)k_pr_resident<16>;
     volatile int *res_err = (volatile int *)ctx.ctrl_readback();
     *res_err = 0;
     if (!unfused && iters > 1 && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
-        const int64_t warps = kResThreads / 32;
+        // small graphs in smaller CTAs, one per SM: 177 groups in 6 CTAs of 32
+        // warps were bound by 6 SMs' gathers
+        const int64_t warps = std::min<int64_t>(kResThreads / 32,
+                                                std::max<int64_t>(4, (all.ngroups + ctx.num_sms - 1) / ctx.num_sms));
+        res_threads = (int)warps * 32;
         grid_res = (int)std::min<int64_t>((all.ngroups + warps - 1) / warps, INT32_MAX);
-        if (grid_res > resident((const void *)k_pr_resident, kResThreads)) grid_res = 0;
+        if (grid_res > resident(res_fn, res_threads)) res_fn = (const void *)k_pr_resident<8>;
+        if (grid_res > resident(res_fn, res_threads)) grid_res = 0;
+    }
+    st.ctr.reserve(sizeof(uint32_t) * (size_t)std::max(iters, 1));
+    if (grid_res && !st.bar.p) {
+        st.bar.reserve(256);
+        MB_CUDA(cudaMemsetAsync(st.bar.p, 0, 256, s));
     }
     auto emit = [&](cudaStream_t cs) {
-        MB_CUDA(cudaMemsetAsync(st.ctr.p, 0, sizeof(uint32_t) * (size_t)std::max(iters, 1), cs));
+        if (!unfused && !grid_res) MB_CUDA(cudaMemsetAsync(st.ctr.p, 0, sizeof(uint32_t) * (size_t)std::max(iters, 1), cs));
         if (init_vec)
             k_pr_init_vec<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), st.pos.as<int32_t>(), g.V, init_vec,
                                                     st.contrib[0].as<float>());
@@ -1352,11 +1392,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             r.zpd = all.zpd.as<int2>();
             r.nz = all.nz;
             r.iters = iters;
-            r.bar = st.ctr.as<uint32_t>();
+            r.bar = st.bar.as<uint32_t>();
             r.err = res_err;
             r.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : 1l << 22;
             void *params[] = {&a, &r};
-            MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pr_resident, dim3(grid_res), dim3(kResThreads), params,
+            MB_CUDA(cudaLaunchCooperativeKernel(res_fn, dim3(grid_res), dim3(res_threads), params,
                                                 0, cs));
             return;
         }
@@ -1417,8 +1457,20 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                 if (a.nitems) heavy(true, cs, a);
                 k_pr_pull<true><<<grid_pull, kPrThreads, 0, cs>>>(a);
             } else {
-                if (a.nitems) heavy(false, cs, a);
+                // the heavy blocks beside the light vertices: neither waits for
+                // the other's last warps (us per superstep, in line / beside:
+                // R-MAT 10^4 / 10^5 11.2 / 6.5, 1.3M / 17M 58.7 / 48.8, 2^23 / 2^26
+                // 225 / 204)
+                if (a.nitems) {
+                    MB_CUDA(cudaEventRecord(st.ev_fork, cs));
+                    MB_CUDA(cudaStreamWaitEvent(st.side, st.ev_fork, 0));
+                }
+                if (a.nitems) heavy(false, st.side, a);
                 sell_step(cs, st.light, a, it);
+                if (a.nitems) {
+                    MB_CUDA(cudaEventRecord(st.ev_join, st.side));
+                    MB_CUDA(cudaStreamWaitEvent(cs, st.ev_join, 0));
+                }
             }
             if (a.nhub) k_hub_finalize<<<grid_for(a.nhub, 128, ctx.num_sms * 4), 128, 0, cs>>>(a);
             MB_CHECK_LAUNCH();
@@ -1467,6 +1519,10 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             MB_CUDA(cudaEventRecord(e1, s));
         }
         MB_CUDA(cudaEventSynchronize(e1));
+        if (grid_res && *res_err) {
+            MB_CUDA(cudaMemsetAsync(st.bar.p, 0, 256, s));
+            MB_CUDA(cudaStreamSynchronize(s));
+        }
         if (grid_res && *res_err) fail(MB_ERR_TIMEOUT, "pagerank: a barrier between two supersteps timed out");
         float ms = 0;
         MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -1479,15 +1535,14 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             stats->schedule_count[unfused ? MB_SCHED_PUSH_UNFUSED : MB_SCHED_PUSH_EDGE_QUEUE] = iters;
             stats->edges_scanned = (int64_t)iters * g.E;
             const PrSell &l = ref_order ? st.sell : st.light;
-            int64_t per_step, zeros = 0;
+            int64_t per_step;
             if (ref_order && unfused) per_step = 2;
             else if (unfused) per_step = 2 + (st.nitems > 0) + (st.nhub > 0);
             else {
-                per_step = (l.ngroups > 0) + (ref_order ? (st.x_nhub > 0) + (st.x_nbig > 0) + (st.x_nhub > st.x_nbig)
+                per_step = 1 + (ref_order ? (st.x_nhub > 0) + (st.x_nbig > 0) + (st.x_nhub > st.x_nbig)
                                                         : (st.nitems > 0) + (st.nhub > 0));
-                if (l.nz) zeros = std::min(iters, 3);  // the first two supersteps and the last
             }
-            stats->kernel_launches = grid_res ? 2 : 1 + (int64_t)iters * per_step + zeros + (iters == 0);
+            stats->kernel_launches = grid_res ? 2 : 1 + (int64_t)iters * per_step + (iters == 0);
         }
     } catch (...) {
         cudaEventDestroy(e0);

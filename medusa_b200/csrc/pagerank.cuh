@@ -9,6 +9,7 @@ namespace mb {
 struct PrSell {
     DevBuf v, pd, rows, base, src, zv, zpd;
     int32_t ngroups = 0, nlong = 0, nz = 0;
+    int32_t max_rows = 0;  // no vertex in it has more in-edges
     void release() {
         v.release(); pd.release(); rows.release(); base.release(); src.release();
         zv.release(); zpd.release();
@@ -29,6 +30,7 @@ struct PrState {
     // ordered by out-degree class, the sources with the most out-edges first
     DevBuf pos;
     DevBuf ctr;  // the sliced ELL's work counters, one per superstep
+    DevBuf bar;  // the one-launch run's barrier
     bool fixed_built = false;  // the fixed order's lists below
     int32_t nitems = 0, nhub = 0;
     int32_t nlong = 0;  // items longer than kPrShortItem (the head of the list)
@@ -74,7 +76,7 @@ struct PrState {
         g_iters = -1;
         rank.release(); contrib[0].release(); contrib[1].release(); msg.release();
         init_stage.release();
-        pos.release(); hcol.release(); light.release(); ctr.release();
+        pos.release(); hcol.release(); light.release(); ctr.release(); bar.release();
         fixed_built = false;
         items.release(); hub_v.release(); hub_first.release(); blk_sum.release();
         meg_src.release(); meg_slot.release();
