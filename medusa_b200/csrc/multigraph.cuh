@@ -1,7 +1,9 @@
 // multigraph.cuh -- many independent graphs in one persistent launch (internal).
 #pragma once
+#include <memory>
 #include <vector>
-#include "mb_internal.cuh"
+#include "bfs_coop.cuh"
+#include "pagerank.cuh"
 
 namespace mb {
 
@@ -24,7 +26,20 @@ struct TeamState {
     unsigned long long reached;        // BFS: reached vertices
 };
 
+// The batch's graphs as one graph, with what its runs need (made on the first).
+struct BatchUnion {
+    Graph g;  // row, col, rrow, rcol, outdeg
+    PrState pr;
+    BfsCoopState bfs;
+    DevBuf src, c0, slot_hub, hub_done, front, sources;
+    ~BatchUnion() {
+        g.release();
+        src.release(); c0.release(); slot_hub.release(); hub_done.release(); front.release(); sources.release();
+    }
+};
+
 struct Batch {
+    std::unique_ptr<BatchUnion> uni;
     std::vector<Graph> graphs;        // built with the single-graph builder
     std::vector<int64_t> vbase;       // n+1 prefix of vertex counts
     int64_t total_V = 0, total_E = 0;
@@ -33,6 +48,7 @@ struct Batch {
     int64_t desc_gen = -1;            // tunables generation the entries were built for
     ~Batch() { release(); }
     void release() {
+        uni.reset();
         for (auto &g : graphs) g.release();
         graphs.clear();
         desc.release(); team.release(); entries.release();
