@@ -857,6 +857,30 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
         for (int32_t s : src)
             if (s < 0 || s >= V) mb::fail(MB_ERR_INVALID, "source vertex out of range");
         mb_stats total{};
+        if (nsrc > 1 && ctx->c.batching && mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop, nsrc)) {
+            const bool here = on_this_device(dist_out);
+            const int32_t most = mb::sssp_coop_sources(g->g);
+            for (int32_t b0 = 0; b0 < nsrc; b0 += most) {
+                const int32_t nb = std::min(most, nsrc - b0);
+                const size_t bytes = sizeof(float) * (size_t)nb * V;
+                float *out = dist_out + (size_t)b0 * V;
+                float *dev = here ? out : (float *)apps(g).run_out.reserve(bytes);
+                const mb::EmitFn copy = [&](cudaStream_t s) {
+                    MB_CUDA(cudaMemcpyAsync(out, dev, bytes, cudaMemcpyDefault, s));
+                };
+                mb_stats st{};
+                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, src.data() + b0, nb, dev, &st, here ? nullptr : &copy);
+                total.supersteps = std::max(total.supersteps, st.supersteps);
+                total.edges_traversed += st.edges_traversed;
+                total.vertices_reached += st.vertices_reached;
+                total.device_ms += st.device_ms;
+                total.kernel_launches += st.kernel_launches;
+                total.edges_scanned += st.edges_scanned;
+                for (int k = 0; k < MB_NUM_SCHEDULES; k++) total.schedule_count[k] += st.schedule_count[k];
+            }
+            if (stats) *stats = total;
+            return;
+        }
         if (nsrc > 1 && ctx->c.batching) {
             // batches of up to 32 sources, one masked traversal each
             mb::MsSsspState &ms = apps(g).mssssp;
@@ -884,7 +908,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
-        const bool coop = mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop);
+        const bool coop = mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop, 1);
         const bool out_here = coop && on_this_device(dist_out);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};
@@ -894,7 +918,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(float) * (size_t)V, cudaMemcpyDefault, s));
                 };
-                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, src[i], dev, &st, out_here ? nullptr : &copy);
+                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, &src[i], 1, dev, &st, out_here ? nullptr : &copy);
             } else {
             // the distances' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {

@@ -22,6 +22,13 @@
 // A superstep of at least kBmMin edges claims without asking for the result and
 // builds the queue from the claim bitmap in a pass of its own: an append per
 // tile costs more there than the pass.
+//
+// Several sources run in the same launch as (source, vertex) pairs, whatever
+// the graph: a superstep's own cost is shared by all of them, and distances
+// come out source by source.  The lines of 32 distances per vertex (mssssp.cu)
+// relax an edge for all sources at once, but with buckets only 2 or 3 of the 32
+// have it in their frontier.  32 sources on the mild R-MAT 2^20 / 2^24: 13.2 ms,
+// against 29.4; uniform 5 10^5 / 6 10^6 x 9 1.5 against 5.8; grid 700^2 x 20 3.5 against 12.
 #include "coop.cuh"
 #include "sssp.cuh"
 #include "sssp_coop.cuh"
@@ -43,6 +50,24 @@ constexpr uint32_t kBmMin = 1 << 20;  // 2^19 and less: 2-4% slower
 // (10^4 / 10^5: 0.118 without, 0.146 with).
 constexpr float kBucketWidth = 0.85f;
 constexpr int64_t kBucketMinE = 1 << 18;
+// Several sources: (source, vertex) pairs of a run, 128 MB of distances.
+// 32 sources at 2^23 / 2^24 / 2^25 pairs: mild R-MAT 2^20 / 2^24 15.7 / 14.1 / 13.2 ms,
+// 2^22 / 2^26 59.0 / 55.6 / 54.0.
+constexpr int64_t kPairs = 1 << 25;
+// Bucket width in mean weights with several sources.  The more out-edges a
+// run's frontiers hold, the less a superstep's own cost matters, and the
+// narrower the best bucket; a sparse graph without hubs (roads) needs
+// supersteps by the hundred at any width.  Measured best: mild R-MAT 2^20 and
+// 2^22 x 32 0.4 (13.2 ms; 25.8 at 2.5), 10^5 x 32 0.7 (1.5; 1.6 at 1.2), uniform 5 10^5 x 9
+// 1.2 (1.5; 1.7 at 0.4), 5 10^4 x 32 2.5 (0.63; 1.0 at 0.4), grid 700^2 x 20 5 (3.5; 10.3 at
+// 0.4), skewed R-MAT 5 10^3 x 32 5 (0.24; 0.79 at 0.4).
+inline float pairs_width(const Graph &g, int32_t nsrc) {
+    const double e = (double)g.E * nsrc;
+    if (async_by_default(g, true)) return 5.f;  // hub-free, at most 6 out-edges per vertex
+    if (e >= (double)(1 << 27)) return 0.4f;
+    if (e >= (double)(1 << 25)) return 0.9f;
+    return e >= (double)(1 << 23) ? 2.5f : 5.f;
+}
 
 __device__ __forceinline__ float inf_f() { return __uint_as_float(kInf); }
 
@@ -58,9 +83,15 @@ struct SShared {  // device memory of a run, zero before it
     alignas(128) uint32_t bar;  // polled: a line of its own
 };
 
+// kMulti: nsrc sources at once.  A vertex is then a (source, vertex) pair,
+// p = source * V + vertex: the index of its distance and of its bits.
 struct SArgs {
     int32_t V;
-    int64_t W;
+    int64_t W;         // bitmap words, whole units of to_queue
+    int32_t nsrc;
+    const int32_t *sources;  // kMulti (device)
+    uint8_t *qs[2];          // kMulti: the entries' sources
+    unsigned long long *front;  // kMulti: the first queue's count << 32 | out-edges
     const int32_t *row, *col;
     const float *wt;
     float *dist;
@@ -75,27 +106,33 @@ struct SArgs {
     long polls;
 };
 
+template <bool kMulti>
 struct SSmem {
     uint32_t off[kTileE + 1];
     int32_t row[kTileE + 1];
     float du[kTileE + 1];
+    uint32_t pb[kMulti ? kTileE + 1 : 1];  // source * V
     uint2 out[kTileE];  // found vertices: {first edge, out-edges}
     int32_t outv[kTileE];
+    uint8_t outs[kMulti ? kTileE : 1];
     uint32_t nout;
     uint32_t wtot[kThreads / 32];
     unsigned long long base;
 };
 
-__device__ __forceinline__ void write_entry(const SArgs &a, int nx, uint32_t pos, int32_t v, uint32_t rs, uint32_t d,
-                                            uint32_t off) {
+template <bool kMulti>
+__device__ __forceinline__ void write_entry(const SArgs &a, int nx, uint32_t pos, int32_t v, uint32_t src, uint32_t rs,
+                                            uint32_t d, uint32_t off) {
     pick(a.q, nx)[pos] = make_uint2(rs - off, off);
     pick(a.qv, nx)[pos] = v;
+    if (kMulti) pick(a.qs, nx)[pos] = (uint8_t)src;
     int32_t *tf = pick(a.tf, nx);
     const uint32_t t0 = (off + kTileE - 1) / kTileE, t1 = (off + d - 1) / kTileE;
     for (uint32_t t = t0; t <= t1; t++) tf[t] = (int32_t)pos;
 }
 
-__device__ __forceinline__ void found(SSmem &sm, bool pred, int32_t v, int32_t rs, uint32_t d) {
+template <bool kMulti>
+__device__ __forceinline__ void found(SSmem<kMulti> &sm, bool pred, int32_t v, uint32_t src, int32_t rs, uint32_t d) {
     const unsigned mask = __ballot_sync(0xffffffffu, pred);
     if (!mask) return;
     const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
@@ -106,11 +143,13 @@ __device__ __forceinline__ void found(SSmem &sm, bool pred, int32_t v, int32_t r
         const uint32_t i = base + __popc(mask & lanemask_lt());
         sm.out[i] = make_uint2((uint32_t)rs, d);
         sm.outv[i] = v;
+        if (kMulti) sm.outs[i] = (uint8_t)src;
     }
 }
 
 // The tile's found vertices -> the next queue, one atomic per tile.
-__device__ __forceinline__ void flush(const SArgs &a, SSmem &sm, unsigned long long *ctr, int nx) {
+template <bool kMulti>
+__device__ __forceinline__ void flush(const SArgs &a, SSmem<kMulti> &sm, unsigned long long *ctr, int nx) {
     __syncthreads();
     const uint32_t n = sm.nout;
     if (n == 0) return;  // the same for every thread
@@ -142,14 +181,15 @@ __device__ __forceinline__ void flush(const SArgs &a, SSmem &sm, unsigned long l
 #pragma unroll
     for (int k = 0; k < kItems; k++)
         if (i0 + k < n) {
-            write_entry(a, nx, (uint32_t)(base >> 32) + i0 + k, sm.outv[i0 + k], e[k].x, e[k].y, off);
+            write_entry<kMulti>(a, nx, (uint32_t)(base >> 32) + i0 + k, sm.outv[i0 + k], kMulti ? sm.outs[i0 + k] : 0u,
+                                e[k].x, e[k].y, off);
             off += e[k].y;
         }
 }
 
 // par: the claim bitmap of this superstep.
-template <bool kBm>
-__device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_t n, uint32_t m, float T, int par,
+template <bool kMulti, bool kBm>
+__device__ __forceinline__ void push(const SArgs &a, SSmem<kMulti> &sm, int cur, uint32_t n, uint32_t m, float T, int par,
                                      SCtr *ctr) {
     const uint32_t tiles = (m + kTileE - 1) / kTileE;
     const uint2 *q = pick(a.q, cur);
@@ -164,13 +204,17 @@ __device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_
         for (int j = threadIdx.x; j < k; j += kThreads) {
             const uint2 e = __ldcg(&q[i0 + j]);
             const int32_t u = __ldcg(&qv[i0 + j]);
+            const uint32_t pb = kMulti ? (uint32_t)__ldcg(&pick(a.qs, cur)[i0 + j]) * (uint32_t)a.V : 0u;
+            const uint32_t p = pb + (uint32_t)u;
             sm.off[j] = e.y;
             sm.row[j] = (int32_t)e.x;
-            sm.du[j] = __ldcg(&a.dist[u]);
-            old[u >> 5] = 0u;  // every bit set there is of a vertex in this queue
+            sm.du[j] = __ldcg(&a.dist[p]);
+            if (kMulti) sm.pb[j] = pb;
+            old[p >> 5] = 0u;  // every bit set there is of a vertex in this queue
         }
         __syncthreads();
         int32_t v[kItems];
+        uint32_t pb[kItems];
         float nd[kItems], dv[kItems];
         {
             const uint32_t e0 = c0 + threadIdx.x * kItems;
@@ -179,9 +223,11 @@ __device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_
             for (int r = 0; r < kItems; r++) {
                 const uint32_t e = e0 + r;
                 v[r] = -1;
+                pb[r] = 0u;
                 nd[r] = 0.f;
                 if (e < c1) {
                     while (j + 1 < k && sm.off[j + 1] <= e) j++;
+                    if (kMulti) pb[r] = sm.pb[j];
                     const int32_t at = sm.row[j] + (int32_t)e;
                     v[r] = __ldg(&a.col[at]);
                     nd[r] = sm.du[j] + __ldg(&a.wt[at]);
@@ -189,26 +235,28 @@ __device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_
             }
         }
 #pragma unroll
-        for (int r = 0; r < kItems; r++) dv[r] = v[r] >= 0 ? __ldcg(&a.dist[v[r]]) : 0.f;
+        for (int r = 0; r < kItems; r++) dv[r] = v[r] >= 0 ? __ldcg(&a.dist[pb[r] + (uint32_t)v[r]]) : 0.f;
 #pragma unroll
         for (int r = 0; r < kItems; r++) {
             bool own = false;
             int32_t rs = 0, re = 0;
             if (nd[r] < dv[r]) {
-                atomicMin((unsigned *)&a.dist[v[r]], __float_as_uint(nd[r]));
-                const uint32_t bit = 1u << (v[r] & 31);
+                const uint32_t p = pb[r] + (uint32_t)v[r];
+                atomicMin((unsigned *)&a.dist[p], __float_as_uint(nd[r]));
+                const uint32_t bit = 1u << (p & 31);
                 if (nd[r] >= T) {
                     far = true;
-                    atomicOr(&a.far[v[r] >> 5], bit);  // a test of the bit first costs more
+                    atomicOr(&a.far[p >> 5], bit);  // a test of the bit first costs more
                 } else if (kBm) {
-                    atomicOr(&claim[v[r] >> 5], bit);
+                    atomicOr(&claim[p >> 5], bit);
                 } else {
                     rs = __ldg(&a.row[v[r]]);
                     re = __ldg(&a.row[v[r] + 1]);
-                    own = !(atomicOr(&claim[v[r] >> 5], bit) & bit);
+                    own = !(atomicOr(&claim[p >> 5], bit) & bit);
                 }
             }
-            if (!kBm) found(sm, own && re > rs, v[r], rs, (uint32_t)(re - rs));
+            if (!kBm)
+                found(sm, own && re > rs, v[r], kMulti && own ? pb[r] / (uint32_t)a.V : 0u, rs, (uint32_t)(re - rs));
         }
         if (kBm) __syncthreads();  // the tile's entries are reloaded next
         else flush(a, sm, &ctr->q, cur ^ 1);
@@ -224,7 +272,7 @@ __device__ __forceinline__ void push(const SArgs &a, SSmem &sm, int cur, uint32_
 // took 30 to 60 us.)  kSplit: the far bitmap -- those below T leave it, and of
 // these the ones not below T0 are queued; the least distance kept goes to
 // ctr->far_min.  Else a claim bitmap, cleared.
-template <bool kSplit>
+template <bool kMulti, bool kSplit>
 __device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t *bm, float T0, float T, int nx,
                                          SCtr *ctr) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -240,12 +288,12 @@ __device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t
         const uint32_t x[4] = {next.x, next.y, next.z, next.w};
         next = words(u + step);
         if (!__syncthreads_or((x[0] | x[1] | x[2] | x[3]) != 0u)) continue;
-        const int32_t v0 = (int32_t)(u * 128) + lane;
+        const uint32_t p0 = (uint32_t)(u * 128) + lane;
         bool take[4];
         if (kSplit) {
             float d[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) d[k] = (x[k] >> lane) & 1u ? __ldcg(&a.dist[v0 + 32 * k]) : inf_f();
+            for (int k = 0; k < 4; k++) d[k] = (x[k] >> lane) & 1u ? __ldcg(&a.dist[p0 + 32 * k]) : inf_f();
             uint32_t keep[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -263,15 +311,18 @@ __device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t
             if (lane == 0 && (x[0] | x[1] | x[2] | x[3]) != 0u)
                 reinterpret_cast<uint4 *>(bm)[u] = make_uint4(0u, 0u, 0u, 0u);
         }
-        int32_t rs[4];
-        uint32_t dg[4], sum = 0, cnt = 0;
+        int32_t rs[4], v[4];
+        uint32_t dg[4], src[4], sum = 0, cnt = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             rs[k] = 0;
             dg[k] = 0;
+            const uint32_t p = p0 + 32 * k;
+            src[k] = kMulti ? p / (uint32_t)a.V : 0u;
+            v[k] = (int32_t)(p - src[k] * (uint32_t)a.V);
             if (take[k]) {
-                rs[k] = __ldg(&a.row[v0 + 32 * k]);
-                dg[k] = (uint32_t)(__ldg(&a.row[v0 + 32 * k + 1]) - rs[k]);
+                rs[k] = __ldg(&a.row[v[k]]);
+                dg[k] = (uint32_t)(__ldg(&a.row[v[k] + 1]) - rs[k]);
             }
         }
 #pragma unroll
@@ -284,7 +335,7 @@ __device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t
 #pragma unroll
         for (int k = 0; k < 4; k++)
             if (dg[k] > 0) {
-                write_entry(a, nx, pos, v0 + 32 * k, (uint32_t)rs[k], dg[k], off);
+                write_entry<kMulti>(a, nx, pos, v[k], src[k], (uint32_t)rs[k], dg[k], off);
                 pos++;
                 off += dg[k];
             }
@@ -295,8 +346,9 @@ __device__ __forceinline__ void to_queue(const SArgs &a, CoopRound &cr, uint32_t
     }
 }
 
+template <bool kMulti>
 __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
-    __shared__ SSmem sm;
+    __shared__ SSmem<kMulti> sm;
     __shared__ CoopRound cr;
     __shared__ unsigned long long s_n[kThreads / 32], s_m[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -308,25 +360,47 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
         return coop_barrier(&a.sh->bar, target, a.polls, &a.out->err);
     };
     int cur = 0, par = 0, it = 0, supersteps = 0, splits = 0, err = 0;
-    const int32_t rs0 = __ldg(&a.row[a.source]), deg0 = __ldg(&a.row[a.source + 1]) - rs0;
-    for (int64_t v = gt; v < a.V; v += gn) a.dist[v] = v == a.source ? 0.f : kMedusaMax;
+    const uint32_t pairs = kMulti ? (uint32_t)a.nsrc * (uint32_t)a.V : (uint32_t)a.V;
+    for (int64_t p = gt; p < pairs; p += gn) a.dist[p] = kMedusaMax;
     for (int64_t w = gt; w < a.W; w += gn) {
         a.claim[0][w] = 0u;
         a.claim[1][w] = 0u;
         a.far[w] = 0u;
     }
-    for (int64_t t = gt; t * kTileE < deg0; t += gn) a.tf[0][t] = 0;
-    if (gt == 0) {
-        a.q[0][0] = make_uint2((uint32_t)rs0, 0u);
-        a.qv[0][0] = a.source;
-        a.sh->ctr[0] = SCtr{0ull, 0u, kInf};
-    }
     if (tid == 0) sm.nout = 0;
-    uint32_t n = deg0 > 0 ? 1u : 0u, m = (uint32_t)deg0;
+    if (!sync()) return;
+    // the sources' queue, by the first warp
+    if (gt < 32) {
+        uint32_t qn = 0, qm = 0;
+        for (int32_t i0 = 0; i0 < a.nsrc; i0 += 32) {
+            const int32_t i = i0 + lane;
+            const int32_t v = i < a.nsrc ? (kMulti ? a.sources[i] : a.source) : -1;
+            int32_t rs = 0, re = 0;
+            if (v >= 0) {
+                rs = __ldg(&a.row[v]);
+                re = __ldg(&a.row[v + 1]);
+                a.dist[(uint32_t)i * (uint32_t)a.V + (uint32_t)v] = 0.f;
+            }
+            const uint32_t d = (uint32_t)(re - rs);
+            const unsigned in = __ballot_sync(0xffffffffu, d > 0);
+            const uint32_t incl = warp_incl_scan_u32(d);
+            if (d > 0)
+                write_entry<kMulti>(a, 0, qn + __popc(in & lanemask_lt()), v, (uint32_t)i, (uint32_t)rs, d,
+                                    qm + incl - d);
+            qn += __popc(in);
+            qm += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) {
+            *a.front = ((unsigned long long)qn << 32) | qm;
+            a.sh->ctr[0] = SCtr{0ull, 0u, kInf};
+        }
+    }
+    if (!sync()) return;
+    const unsigned long long f0 = __ldcg(a.front);
+    uint32_t n = (uint32_t)(f0 >> 32), m = (uint32_t)f0;
     unsigned long long work = 0;
     float T = a.delta > 0.f ? a.delta : inf, fmin = inf;
     bool far = false;
-    if (!sync()) return;
     for (;; it++) {
         if (n == 0 && !far) break;
         if (it >= a.cap) {
@@ -342,7 +416,7 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
             if (fmin < inf) T = fmaxf(T, fmin + a.delta);
             if (!(T > T0)) T = __uint_as_float(__float_as_uint(T0) + 1u);
             if (fmin < inf && !(T > fmin)) T = __uint_as_float(__float_as_uint(fmin) + 1u);
-            to_queue<true>(a, cr, a.far, T0, T, cur, ctr);
+            to_queue<kMulti, true>(a, cr, a.far, T0, T, cur, ctr);
             if (!sync()) return;
             fmin = __uint_as_float(__ldcg(&ctr->far_min));
             far = fmin < inf;
@@ -351,11 +425,11 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
             work += m;
             const bool bm = m >= kBmMin;
             if (bm) {
-                push<true>(a, sm, cur, n, m, T, par, ctr);
+                push<kMulti, true>(a, sm, cur, n, m, T, par, ctr);
                 if (!sync()) return;
-                to_queue<false>(a, cr, pick(a.claim, par), 0.f, 0.f, cur ^ 1, ctr);
+                to_queue<kMulti, false>(a, cr, pick(a.claim, par), 0.f, 0.f, cur ^ 1, ctr);
             } else {
-                push<false>(a, sm, cur, n, m, T, par, ctr);
+                push<kMulti, false>(a, sm, cur, n, m, T, par, ctr);
             }
             if (!sync()) return;
             far = far || __ldcg(&ctr->far) != 0u;
@@ -369,11 +443,12 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
     }
     // reached vertices and their out-edges
     unsigned long long rn = 0, rm = 0;
-    for (int64_t v = gt; v < a.V; v += gn)
-        if (__ldcg(&a.dist[v]) < kMedusaMax) {
-            rn++;
-            rm += (uint32_t)(__ldg(&a.row[v + 1]) - __ldg(&a.row[v]));
-        }
+    for (int64_t v = gt; v < a.V; v += gn) {
+        uint32_t c = 0;
+        for (int32_t i = 0; i < a.nsrc; i++) c += __ldcg(&a.dist[(uint32_t)i * (uint32_t)a.V + (uint32_t)v]) < kMedusaMax;
+        rn += c;
+        if (c) rm += (unsigned long long)c * (uint32_t)(__ldg(&a.row[v + 1]) - __ldg(&a.row[v]));
+    }
     rn = warp_sum(rn);
     rm = warp_sum(rm);
     if (lane == 0) {
@@ -405,26 +480,39 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
 
 }  // namespace
 
-void SsspCoopState::ensure(const Graph &g) {
-    if (built) return;
-    const size_t tiles = (size_t)(g.E / kSsspCoopTile) + 2, W = (((size_t)g.V + 31) / 32 + 3) & ~(size_t)3;
+void SsspCoopState::ensure(const Graph &g, int32_t nsrc) {
+    if (!built) {
+        sh.reserve(sizeof(SShared));
+        front.reserve(sizeof(unsigned long long));
+        srcs.reserve(sizeof(int32_t) * kSsspCoopSources);
+        double mean = 0.0;
+        bool bad = false;
+        sssp_weight_stats(g, &mean, &bad);
+        mean_w = (float)mean;
+        weights_ok = !bad;
+        built = true;
+    }
+    if (nsrc <= room) return;
+    const size_t pairs = (size_t)nsrc * (size_t)g.V, tiles = (size_t)nsrc * (size_t)g.E / kSsspCoopTile + 2;
+    const size_t W = ((pairs + 31) / 32 + 3) & ~(size_t)3;
     for (int i = 0; i < 2; i++) {
         claim[i].reserve(sizeof(uint32_t) * W);
-        q[i].reserve(sizeof(uint2) * (size_t)g.V);
-        qv[i].reserve(sizeof(int32_t) * (size_t)g.V);
+        q[i].reserve(sizeof(uint2) * pairs);
+        qv[i].reserve(sizeof(int32_t) * pairs);
+        if (nsrc > 1) qs[i].reserve(pairs);
         tf[i].reserve(sizeof(int32_t) * tiles);
     }
     far.reserve(sizeof(uint32_t) * W);
-    sh.reserve(sizeof(SShared));
-    double mean = 0.0;
-    bool bad = false;
-    sssp_weight_stats(g, &mean, &bad);
-    mean_w = (float)mean;
-    weights_ok = !bad;
-    built = true;
+    room = nsrc;
 }
 
-bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st) {
+int32_t sssp_coop_sources(const Graph &g) {
+    int64_t n = std::min<int64_t>(kSsspCoopSources, std::max<int64_t>(1, kPairs / std::max<int32_t>(g.V, 1)));
+    n = std::min<int64_t>(n, 0xffffffffll / std::max<int64_t>(g.E, 1));  // out-edges of a queue in 32 bits
+    return (int32_t)std::max<int64_t>(n, 1);
+}
+
+bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, int32_t nsrc) {
     // the loop graph's and the asynchronous kernel's own parameters ask for them
     for (int t : {MB_TUNE_SSSP_BM_PUSH_MIN, MB_TUNE_PUSH_BLOCKS_PER_SM, MB_TUNE_VERTEX_BLOCKS_PER_SM,
                   MB_TUNE_TAIL_EDGES, MB_TUNE_BULK_STAGE, MB_TUNE_SMALL_PUSH_EDGES, MB_TUNE_SSSP_ASYNC,
@@ -433,20 +521,32 @@ bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st) {
     if (ctx.schedule_policy != MB_POLICY_FIXED || !ctx.use_graphs || ctx.tracing || ctx.persist || !ctx.tail ||
         ctx.max_step >= 0 || ctx.sssp_delta != 0.f)
         return false;
-    if (async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
-    st.ensure(g);
+    if (nsrc == 1 && async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
+    if (nsrc > 1) {
+        if (ctx.tunable[MB_TUNE_MSS_DELTA] >= 0) return false;  // the lines' buckets
+        // on a large graph with a huge hub most sources' frontiers meet in a
+        // few supersteps, and a line of 32 distances per edge is the cheaper
+        // form (skewed R-MAT 2^20 / 2^24 x 16: 7.0 against 8.8-9.9 ms)
+        if (g.max_outdeg > g.E / 1024 && g.E >= (1 << 22)) return false;
+    }
+    st.ensure(g, 1);
     return st.weights_ok;
 }
 
-void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, int32_t source, float *dist, mb_stats *stats,
-                   const EmitFn *after) {
+void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
+                   mb_stats *stats, const EmitFn *after) {
     static_assert(sizeof(SsspCoopOut) <= Context::kSmallBytes - Context::kCtrlOff, "readback too small");
     cudaStream_t s = ctx.stream;
     volatile SsspCoopOut *out = (volatile SsspCoopOut *)ctx.ctrl_readback();
     out->err = 0;
+    st.ensure(g, nsrc);
+    const bool multi = nsrc > 1;
     SArgs a{};
     a.V = g.V;
-    a.W = ((((int64_t)g.V + 31) / 32) + 3) & ~3ll;  // whole units of to_queue
+    a.W = ((((int64_t)g.V * nsrc + 31) / 32) + 3) & ~3ll;
+    a.nsrc = nsrc;
+    a.sources = st.srcs.as<int32_t>();
+    a.front = st.front.as<unsigned long long>();
     a.row = g.row.as<int32_t>();
     a.col = g.col.as<int32_t>();
     a.wt = g.wt.as<float>();
@@ -455,25 +555,29 @@ void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, int32_t source, fl
         a.claim[i] = st.claim[i].as<uint32_t>();
         a.q[i] = st.q[i].as<uint2>();
         a.qv[i] = st.qv[i].as<int32_t>();
+        a.qs[i] = st.qs[i].as<uint8_t>();
         a.tf[i] = st.tf[i].as<int32_t>();
     }
     a.far = st.far.as<uint32_t>();
     a.sh = st.sh.as<SShared>();
     a.out = (SsspCoopOut *)ctx.ctrl_readback();
-    a.source = source;
-    a.cap = step_cap(ctx, (int64_t)g.V * 4 + 16);
-    a.delta = g.E >= kBucketMinE ? kBucketWidth * st.mean_w : 0.f;
+    a.source = sources[0];
+    a.cap = step_cap(ctx, ((int64_t)g.V * 4 + 16) * nsrc);
+    a.delta = multi ? pairs_width(g, nsrc) * st.mean_w : g.E >= kBucketMinE ? kBucketWidth * st.mean_w : 0.f;
     a.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
     int per_sm = 0;
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sssp_coop, kThreads, 0));
+    const void *kernel = multi ? (const void *)k_sssp_coop<true> : (const void *)k_sssp_coop<false>;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
     if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative SSSP kernel does not fit on an SM");
     // no more CTAs than tiles: fewer arrive at the barriers of small graphs
-    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kCtas), std::max<int64_t>(g.E / kTileE, 16));
+    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kCtas), std::max<int64_t>(g.E * nsrc / kTileE, 16));
     const cudaEvent_t e0 = ctx.event(0), e1 = ctx.event(1);
+    if (multi)
+        MB_CUDA(cudaMemcpyAsync(st.srcs.p, sources, sizeof(int32_t) * (size_t)nsrc, cudaMemcpyHostToDevice, s));
     MB_CUDA(cudaEventRecord(e0, s));
     MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(SShared), s));
     void *params[] = {&a};
-    MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_sssp_coop, dim3(grid), dim3(kThreads), params, 0, s));
+    MB_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), params, 0, s));
     MB_CUDA(cudaEventRecord(e1, s));
     if (after) (*after)(s);
     MB_CUDA(cudaStreamSynchronize(s));

@@ -15,30 +15,39 @@ struct SsspCoopState {
     bool built = false;
     bool weights_ok = false;  // no negative or NaN weight
     float mean_w = 0.f;
-    DevBuf dist, claim[2], far, q[2], qv[2], tf[2], sh;
+    int32_t room = 0;  // sources the buffers below hold at once
+    DevBuf claim[2], far, q[2], qv[2], qs[2], tf[2], sh, front, srcs;
     ~SsspCoopState() { release(); }
     void release() {
         for (int i = 0; i < 2; i++) {
             claim[i].release();
             q[i].release();
             qv[i].release();
+            qs[i].release();
             tf[i].release();
         }
-        dist.release();
         far.release();
         sh.release();
+        front.release();
+        srcs.release();
         built = false;
+        room = 0;
     }
-    void ensure(const Graph &g);
+    void ensure(const Graph &g, int32_t nsrc);
 };
 
-// Whether the context's settings and the graph leave a whole SSSP to
-// run_sssp_coop (makes the state when they do).
-bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st);
+constexpr int32_t kSsspCoopSources = 32;  // at most, in one run
 
-// One SSSP from `source` into `dist` (device memory, V entries).
+// Whether the context's settings and the graph leave SSSP from nsrc sources to
+// run_sssp_coop (makes the state when they do).
+bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, int32_t nsrc);
+
+// Sources that one run takes at a time.
+int32_t sssp_coop_sources(const Graph &g);
+
+// SSSP from nsrc sources (host array) into dist[s * V + v] (device memory).
 // after: queued behind the run, before its host synchronisation.
-void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, int32_t source, float *dist, mb_stats *stats,
-                   const EmitFn *after);
+void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
+                   mb_stats *stats, const EmitFn *after);
 
 }  // namespace mb
