@@ -408,7 +408,8 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                hop distances; one cooperative launch); 0 the
                                direction-optimising BSP supersteps; default: 1 on graphs
                                without hubs (largest out-degree <= 64) of at most 6
-                               edges per vertex.  Identical levels */
+                               edges per vertex and more than 10240 vertices or 65536
+                               edges (smaller ones: a one-CTA kernel).  Identical levels */
 #define MB_TUNE_BFS_ASYNC_DELTA 21 /* threshold step of the asynchronous BFS, in hops
                                      (default 8) */
 #define MB_TUNE_ASYNC_BELOW 22 /* > 0: the asynchronous SSSP (when on) takes over only

@@ -797,7 +797,14 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
             return;
         }
         const int64_t t_async = ctx->c.tunable[MB_TUNE_BFS_ASYNC];
-        const bool bfs_async = (t_async > 0 || (t_async < 0 && mb::async_by_default(g->g, true))) &&
+        // Hub-free graphs that fit one CTA go to its kernel, whatever their
+        // diameter (ms, asynchronous / one CTA: 10^4 vertices in a line 23.1 /
+        // 6.3, 100 x 100 0.53 / 0.18, 21 x 21 x 21 torus 0.19 / 0.08, uniform
+        // 2^12 with 5 edges per vertex 0.13 / 0.04); the larger ones do not, for
+        // a level of the whole grid costs 5 us or more (line of 40,000 91 / 147,
+        // 1000 x 1000 torus 4.4 / 7.4, 128^3 torus 1.3 / 1.7).
+        const bool one_cta = mb::bfs_small(g->g) && mb::bfs_coop_applies(ctx->c);
+        const bool bfs_async = (t_async > 0 || (t_async < 0 && mb::async_by_default(g->g, true) && !one_cta)) &&
                                (ctx->c.schedule_policy == MB_POLICY_FIXED ||
                                 ctx->c.schedule_policy == MB_POLICY_LEARNED) &&
                                !ctx->c.persist;

@@ -53,6 +53,23 @@ def test_levels_equal_the_oracle(gpu_ctx, V, E, rule):
     g.close()
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 2), (1, 10240), (100, 102), (100, 103), (128, 80)])
+def test_hub_free_lattices(gpu_ctx, rows, cols):
+    """Both sides of the one-CTA kernel's vertex limit, long diameters."""
+    V = rows * cols
+    i = np.arange(V, dtype=np.int32).reshape(rows, cols)
+    a = np.concatenate([i[:, :-1].ravel(), i[:-1].ravel()])
+    b = np.concatenate([i[:, 1:].ravel(), i[1:].ravel()])
+    src, dst = np.concatenate([a, b]), np.concatenate([b, a])
+    g = gpu_ctx.graph_from_edges(V, src, dst)
+    s = V // 3
+    want = (np.abs(i // cols - s // cols) + np.abs(i % cols - s % cols)).astype(np.int32).ravel()
+    got, st = g.bfs([s])
+    np.testing.assert_array_equal(got[0], want)
+    assert st["vertices_reached"] == V and st["edges_traversed"] == len(src)
+    g.close()
+
+
 def test_pull_list_lengths(gpu_ctx):
     """In-lists whose only visited source is the last one."""
     lengths = [1, 2, 4, 5, 31, 32, 33, 34, 159, 160, 161, 1000]
