@@ -471,7 +471,8 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
             }
             continue;
         }
-        if (reported != ph) {
+        // without a threshold there is no next phase to open
+        if (reported != ph && T < inf) {
             reported = ph;
             above = warp_min_f(above);
             if (lane == 0) async_idle(c, S, s_idle, ph, T, delta, above, cap);
