@@ -6,7 +6,10 @@
 //   k_bfs_small: one CTA, the frontier queues and the visited bits in shared
 //     memory, __syncthreads between supersteps.  Graphs of at most
 //     kBfsSmallV vertices and kBfsSmallE edges (push only: one CTA relaxes
-//     about an edge per clock, so larger graphs are faster on the whole GPU);
+//     about an edge per clock, so larger graphs are faster on the whole GPU),
+//     0.75 us per superstep; several sources take a CTA each (ms, 32 sources,
+//     the batched kernels / here: 10^4 vertices in a line 220 / 6.7, 100 x 100 grid
+//     3.8 / 0.22, mild R-MAT 10^4 / 6.5 10^4 0.29 / 0.09, 10^3 / 4 10^3 0.28 / 0.02);
 //   k_bfs_coop: one cooperative grid, one grid barrier per superstep.  Every
 //     CTA reads the superstep's counters after the barrier and takes the same
 //     decision, so no thread decides for the others between two barriers.
@@ -38,6 +41,14 @@ static_assert(kBfsSmallE <= kSmallMask && kBfsSmallV < (1 << (32 - kSmallShift))
 
 // ---- one CTA ----------------------------------------------------------------------
 
+struct SmallArgs {
+    int32_t V, E, W, cap;
+    const int32_t *row, *col;
+    int32_t *level;
+    BfsCoopOut *out;  // host memory, one per source
+    int32_t sources[kBfsSmallSources];
+};
+
 // Shared memory: the visited bits, the levels, two queues, and with kStaged
 // the graph itself (offsets and columns, read once): a superstep then waits
 // for no memory outside the SM.
@@ -46,7 +57,7 @@ __host__ __device__ inline size_t small_words(int32_t V, int64_t E, bool staged)
     return w4 + 5 * v4 + (staged ? v4 + 4 + (size_t)E : 0);
 }
 template <bool kStaged>
-__global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(CoopArgs a) {
+__global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(const __grid_constant__ SmallArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t v4 = ((uint32_t)a.V + 3u) & ~3u;
     uint32_t *vis = smem;  // W words
@@ -54,39 +65,45 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(CoopArgs a) {
     uint2 *q0 = reinterpret_cast<uint2 *>(level + v4);
     uint2 *q1 = q0 + v4;
     int32_t *srow = reinterpret_cast<int32_t *>(q1 + v4), *scol = srow + v4 + 4;
-    __shared__ uint32_t s_q[2];  // queued vertices << kSmallShift | their out-edges
+    // queued vertices << kSmallShift | their out-edges; a superstep fills the
+    // slot after its own, which the one before cleared, so one barrier is enough
+    __shared__ uint32_t s_q[3];
     __shared__ uint32_t s_reached;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int32_t rs0 = __ldg(&a.row[a.source]), deg0 = __ldg(&a.row[a.source + 1]) - rs0;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int32_t source = a.sources[blockIdx.x];
+    const int32_t rs0 = __ldg(&a.row[source]), deg0 = __ldg(&a.row[source + 1]) - rs0;
     if (kStaged) {
-        const int32_t E = (int32_t)a.E;
         for (int32_t i = tid; i <= a.V; i += kSmallThreads) srow[i] = __ldg(&a.row[i]);
 #pragma unroll 8
-        for (int32_t i = tid; i < E; i += kSmallThreads) scol[i] = __ldg(&a.col[i]);
+        for (int32_t i = tid; i < a.E; i += kSmallThreads) scol[i] = __ldg(&a.col[i]);
     }
     const int32_t *row = kStaged ? srow : a.row, *col = kStaged ? scol : a.col;
-    for (int i = tid; i < a.W; i += kSmallThreads) vis[i] = i == (a.source >> 5) ? 1u << (a.source & 31) : 0u;
-    for (int32_t v = tid; v < a.V; v += kSmallThreads) level[v] = v == a.source ? 0 : -1;
+    for (int i = tid; i < a.W; i += kSmallThreads) vis[i] = i == (source >> 5) ? 1u << (source & 31) : 0u;
+    for (int32_t v = tid; v < a.V; v += kSmallThreads) level[v] = v == source ? 0 : -1;
     if (tid == 0) {
         s_reached = 0;
         q0[0] = make_uint2((uint32_t)rs0, 0u);
         s_q[0] = deg0 > 0 ? (1u << kSmallShift) + (uint32_t)deg0 : 0u;
-        s_q[1] = 0u;
+        s_q[1] = s_q[2] = 0u;
     }
     __syncthreads();
     int32_t step = 0, err = 0;
-    unsigned long long edges = (uint32_t)deg0, work = 0;
+    int slot = 0, next = 1;
+    unsigned long long edges = 0;  // of every vertex queued, so of every one reached
     for (;;) {
         const uint2 *q = step & 1 ? q1 : q0;
         uint2 *qn = step & 1 ? q0 : q1;
-        const uint32_t c = s_q[step & 1], n = c >> kSmallShift, m = c & kSmallMask;
+        const uint32_t c = s_q[slot], n = c >> kSmallShift, m = c & kSmallMask;
         if (n == 0) break;
         if (step >= a.cap) {
             err = ERR_STEP_CAP;
             break;
         }
-        uint32_t *ctr = &s_q[(step & 1) ^ 1];
-        for (uint32_t b = 0; b < m; b += kSmallThreads * kSmallU) {
+        uint32_t *ctr = &s_q[next];
+        const int after = next == 2 ? 0 : next + 1;
+        if (tid == 0) s_q[after] = 0u;
+        // a warp without edges goes to the barrier: 32 idle warps took 1700 clocks
+        for (uint32_t b = 0; b + (uint32_t)wid * 32u < m; b += kSmallThreads * kSmallU) {
             int32_t v[kSmallU], rs[kSmallU], re[kSmallU];
             bool own[kSmallU];
 #pragma unroll
@@ -133,27 +150,25 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(CoopArgs a) {
                     base += (1u << kSmallShift) + (uint32_t)(re[r] - rs[r]);
                 }
         }
-        work += m;
+        edges += m;
         step++;
         __syncthreads();
-        edges += s_q[step & 1] & kSmallMask;
-        if (tid == 0) s_q[(step & 1) ^ 1] = 0u;
-        __syncthreads();
+        slot = next;
+        next = after;
     }
     uint32_t reached = 0;
+    int32_t *out = a.level + (size_t)blockIdx.x * (size_t)a.V;
     for (int i = tid; i < a.W; i += kSmallThreads) reached += __popc(vis[i]);
     reached = warp_sum(reached);
     if (lane == 0 && reached) atomicAdd(&s_reached, reached);
-    for (int32_t v = tid; v < a.V; v += kSmallThreads) a.level[v] = level[v];
+    for (int32_t v = tid; v < a.V; v += kSmallThreads) out[v] = level[v];
     __syncthreads();
     if (tid == 0) {
-        a.out->supersteps = step;
-        a.out->pushes = step;
-        a.out->pulls = 0;
-        a.out->err = err;
-        a.out->reached = s_reached;
-        a.out->edges = edges;
-        a.out->work = work;
+        BfsCoopOut &o = a.out[blockIdx.x];
+        o.supersteps = step;
+        o.err = err;
+        o.reached = s_reached;
+        o.edges = edges;
     }
 }
 
@@ -196,11 +211,54 @@ bool bfs_coop_applies(const Context &ctx) {
            ctx.max_step < 0;
 }
 
+void run_bfs_small(Context &ctx, Graph &g, const int32_t *sources, int32_t nsrc, int32_t *levels, mb_stats *stats,
+                   const EmitFn *after) {
+    static_assert(sizeof(BfsCoopOut) * kBfsSmallSources <= Context::kSmallBytes - Context::kCtrlOff,
+                  "readback too small");
+    cudaStream_t s = ctx.stream;
+    BfsCoopOut *out = (BfsCoopOut *)ctx.ctrl_readback();
+    SmallArgs a{};
+    a.V = g.V;
+    a.E = (int32_t)g.E;
+    a.W = (g.V + 31) / 32;
+    a.cap = step_cap(ctx, (int64_t)g.V + 4);
+    a.row = g.row.as<int32_t>();
+    a.col = g.col.as<int32_t>();
+    a.level = levels;
+    a.out = out;
+    for (int32_t i = 0; i < nsrc; i++) a.sources[i] = sources[i];
+    const bool staged = small_words(g.V, g.E, true) * 4 <= kSmallSmem;
+    const size_t smem = small_words(g.V, g.E, staged) * 4;
+    const void *fn = staged ? (const void *)k_bfs_small<true> : (const void *)k_bfs_small<false>;
+    MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
+    const cudaEvent_t e0 = ctx.event(0), e1 = ctx.event(1);
+    MB_CUDA(cudaEventRecord(e0, s));
+    void *params[] = {&a};
+    MB_CUDA(cudaLaunchKernel(fn, dim3(nsrc), dim3(kSmallThreads), params, smem, s));
+    MB_CUDA(cudaEventRecord(e1, s));
+    if (after) (*after)(s);
+    MB_CUDA(cudaStreamSynchronize(s));
+    float ms = 0;
+    MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    mb_stats total{};
+    for (int32_t i = 0; i < nsrc; i++) {
+        const BfsCoopOut &o = out[i];
+        if (o.err & ERR_STEP_CAP) fail(MB_ERR_TIMEOUT, "bfs: superstep cap reached");
+        total.supersteps = std::max(total.supersteps, o.supersteps);
+        total.edges_traversed += (int64_t)o.edges;
+        total.vertices_reached += (int64_t)o.reached;
+    }
+    total.device_ms = ms;
+    total.schedule_count[MB_SCHED_PUSH_EDGE_QUEUE] = total.supersteps;
+    total.kernel_launches = 1;
+    total.edges_scanned = total.edges_traversed;  // each once
+    if (stats) *stats = total;
+}
+
 void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int32_t *level, mb_stats *stats,
                   const EmitFn *after) {
     static_assert(sizeof(BfsCoopOut) <= Context::kSmallBytes - Context::kCtrlOff, "readback too small");
     cudaStream_t s = ctx.stream;
-    const bool small = bfs_small(g);
     volatile BfsCoopOut *out = (volatile BfsCoopOut *)ctx.ctrl_readback();
     out->err = 0;
     CoopArgs a{};
@@ -220,52 +278,40 @@ void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int3
     a.cap = step_cap(ctx, (int64_t)g.V + 4);
     a.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
     const cudaEvent_t e0 = ctx.event(0), e1 = ctx.event(1);
-    {
-        if (small) {
-            const bool staged = small_words(g.V, g.E, true) * 4 <= kSmallSmem;
-            const size_t smem = small_words(g.V, g.E, staged) * 4;
-            const void *fn = staged ? (const void *)k_bfs_small<true> : (const void *)k_bfs_small<false>;
-            MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-            MB_CUDA(cudaEventRecord(e0, s));
-            void *params[] = {&a};
-            MB_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(kSmallThreads), params, smem, s));
-        } else {
-            st.ensure(g);
-            for (int i = 0; i < 2; i++) {
-                a.vis[i] = st.vis[i].as<uint32_t>();
-                a.q[i] = st.q[i].as<uint2>();
-                a.tf[i] = st.tf[i].as<int32_t>();
-            }
-            a.sh = st.sh.as<CoopShared>();
-            int per_sm = 0;
-            MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_coop, kCoopThreads, 0));
-            if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative BFS kernel does not fit on an SM");
-            // no more CTAs than tiles: fewer arrive at the barriers of small graphs
-            const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kBfsCoopCtas),
-                                                    std::max<int64_t>(g.E / kCoopTile, 16));
-            MB_CUDA(cudaEventRecord(e0, s));
-            MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(CoopShared), s));
-            void *params[] = {&a};
-            MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_bfs_coop, dim3(grid), dim3(kCoopThreads), params, 0, s));
-        }
-        MB_CUDA(cudaEventRecord(e1, s));
-        if (after) (*after)(s);
-        MB_CUDA(cudaStreamSynchronize(s));
-        float ms = 0;
-        MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (out->err & ERR_BARRIER) fail(MB_ERR_TIMEOUT, "bfs: a grid barrier timed out");
-        if (out->err & ERR_STEP_CAP) fail(MB_ERR_TIMEOUT, "bfs: superstep cap reached");
-        if (stats) {
-            *stats = mb_stats{};
-            stats->supersteps = out->supersteps;
-            stats->edges_traversed = (int64_t)out->edges;
-            stats->vertices_reached = (int64_t)out->reached;
-            stats->device_ms = ms;
-            stats->schedule_count[MB_SCHED_PUSH_EDGE_QUEUE] = out->pushes;
-            stats->schedule_count[MB_SCHED_PULL_THREAD] = out->pulls;
-            stats->kernel_launches = 1;
-            stats->edges_scanned = (int64_t)out->work;
-        }
+    st.ensure(g);
+    for (int i = 0; i < 2; i++) {
+        a.vis[i] = st.vis[i].as<uint32_t>();
+        a.q[i] = st.q[i].as<uint2>();
+        a.tf[i] = st.tf[i].as<int32_t>();
+    }
+    a.sh = st.sh.as<CoopShared>();
+    int per_sm = 0;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_coop, kCoopThreads, 0));
+    if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative BFS kernel does not fit on an SM");
+    // no more CTAs than tiles: fewer arrive at the barriers of small graphs
+    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kBfsCoopCtas),
+                                            std::max<int64_t>(g.E / kCoopTile, 16));
+    MB_CUDA(cudaEventRecord(e0, s));
+    MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(CoopShared), s));
+    void *params[] = {&a};
+    MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_bfs_coop, dim3(grid), dim3(kCoopThreads), params, 0, s));
+    MB_CUDA(cudaEventRecord(e1, s));
+    if (after) (*after)(s);
+    MB_CUDA(cudaStreamSynchronize(s));
+    float ms = 0;
+    MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if (out->err & ERR_BARRIER) fail(MB_ERR_TIMEOUT, "bfs: a grid barrier timed out");
+    if (out->err & ERR_STEP_CAP) fail(MB_ERR_TIMEOUT, "bfs: superstep cap reached");
+    if (stats) {
+        *stats = mb_stats{};
+        stats->supersteps = out->supersteps;
+        stats->edges_traversed = (int64_t)out->edges;
+        stats->vertices_reached = (int64_t)out->reached;
+        stats->device_ms = ms;
+        stats->schedule_count[MB_SCHED_PUSH_EDGE_QUEUE] = out->pushes;
+        stats->schedule_count[MB_SCHED_PULL_THREAD] = out->pulls;
+        stats->kernel_launches = 1;
+        stats->edges_scanned = (int64_t)out->work;
     }
 }
 

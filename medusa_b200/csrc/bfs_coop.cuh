@@ -8,6 +8,7 @@ constexpr int kBfsCoopTile = 1024;
 constexpr int kBfsCoopCtas = 4;  // CTAs per SM of the cooperative grid
 constexpr int32_t kBfsSmallV = 10240;  // 20 bytes of shared memory per vertex
 constexpr int64_t kBfsSmallE = 1 << 16;
+constexpr int32_t kBfsSmallSources = 128;  // at most, in one launch
 
 struct BfsCoopOut {
     int32_t supersteps, pushes, pulls, err;
@@ -30,12 +31,17 @@ struct BfsCoopState {
     void ensure(const Graph &g);
 };
 
-// Whether the one-CTA kernel runs the graph; it stores the levels in one
-// sweep, so `level` may also be pinned host memory then.
+// Whether the graph fits the one-CTA kernel.
 inline bool bfs_small(const Graph &g) { return g.V <= kBfsSmallV && g.E <= kBfsSmallE; }
 
 // Whether the context's settings leave a whole BFS to run_bfs_coop.
 bool bfs_coop_applies(const Context &ctx);
+
+// A graph that fits one CTA: BFS from nsrc <= kBfsSmallSources sources (host
+// array), a CTA each, into levels[s * V + v], which is written in one sweep and
+// so may also be pinned host memory.
+void run_bfs_small(Context &ctx, Graph &g, const int32_t *sources, int32_t nsrc, int32_t *levels, mb_stats *stats,
+                   const EmitFn *after);
 
 // One BFS from `source` into `level` (device memory, V entries).
 // after: queued behind the run, before its host synchronisation.

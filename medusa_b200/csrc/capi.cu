@@ -757,6 +757,44 @@ int mb_batch_destroy(mb_batch *b) {
     return MB_OK;
 }
 
+}  // extern "C"
+
+// Runs of a graph that fits one CTA, `most` sources in a launch (a CTA each).
+// run: run_bfs_small or run_sssp_small, less the context and the graph.
+template <class T, class Run>
+static mb_stats small_runs(mb_ctx *ctx, mb_graph *g, const std::vector<int32_t> &src, int32_t most, T *result,
+                           const Run &run) {
+    // results for a host array: the kernel stores up to 256 KB in pinned
+    // memory itself, more is copied
+    constexpr size_t kPinnedMax = 256 << 10;
+    const bool here = on_this_device(result), host = !here && !mb::is_device_ptr(result);
+    const int32_t nsrc = (int32_t)src.size();
+    mb_stats total{};
+    for (int32_t b0 = 0; b0 < nsrc; b0 += most) {
+        const int32_t nb = std::min(most, nsrc - b0);
+        T *out = result + (size_t)b0 * g->g.V;
+        const size_t bytes = sizeof(T) * (size_t)nb * g->g.V;
+        const bool pinned = host && bytes <= kPinnedMax;
+        T *dev = here ? out : (T *)(pinned ? ctx->c.pinned_reserve(bytes) : apps(g).run_out.reserve(bytes));
+        const mb::EmitFn copy = [&](cudaStream_t s) {
+            MB_CUDA(cudaMemcpyAsync(out, dev, bytes, cudaMemcpyDefault, s));
+        };
+        mb_stats st{};
+        run(src.data() + b0, nb, dev, &st, here || pinned ? nullptr : &copy);
+        if (pinned) std::memcpy(out, dev, bytes);
+        total.supersteps = std::max(total.supersteps, st.supersteps);
+        total.edges_traversed += st.edges_traversed;
+        total.vertices_reached += st.vertices_reached;
+        total.device_ms += st.device_ms;
+        total.kernel_launches += st.kernel_launches;
+        total.edges_scanned += st.edges_scanned;
+        for (int k = 0; k < MB_NUM_SCHEDULES; k++) total.schedule_count[k] += st.schedule_count[k];
+    }
+    return total;
+}
+
+extern "C" {
+
 int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc,
            int32_t *levels_out, mb_stats *stats) {
     return guarded(ctx, [&] {
@@ -770,7 +808,24 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
         for (int32_t s : src)
             if (s < 0 || s >= V) mb::fail(MB_ERR_INVALID, "source vertex out of range");
         mb_stats total{};
-        if (nsrc > 1 && ctx->c.batching) {
+        const bool batch = nsrc > 1 && ctx->c.batching;
+        const int64_t t_async = ctx->c.tunable[MB_TUNE_BFS_ASYNC];
+        // A graph that fits one CTA goes to its kernel, hub-free or not, whatever
+        // its diameter (ms, asynchronous / one CTA: 10^4 vertices in a line 23.1 /
+        // 4.2, 100 x 100 0.53 / 0.15, 21 x 21 x 21 torus 0.19 / 0.08, uniform
+        // 2^12 with 5 edges per vertex 0.13 / 0.04).  Larger hub-free graphs do
+        // not leave the asynchronous kernel for one launch, for a level of the
+        // whole grid costs 5 us or more (line of 40,000 91 / 147, 1000 x 1000
+        // torus 4.4 / 7.4, 128^3 torus 1.3 / 1.7).
+        if (mb::bfs_small(g->g) && mb::bfs_coop_applies(ctx->c) && (batch || t_async <= 0)) {
+            total = small_runs(ctx, g, src, batch ? mb::kBfsSmallSources : 1, levels_out,
+                               [&](const int32_t *from, int32_t n, int32_t *out, mb_stats *st, const mb::EmitFn *after) {
+                                   mb::run_bfs_small(ctx->c, g->g, from, n, out, st, after);
+                               });
+            if (stats) *stats = total;
+            return;
+        }
+        if (batch) {
             // batches of up to 64 sources, one masked traversal each
             mb::MsBfsState &ms = apps(g).msbfs;
             ms.ensure(g->g);  // before reserving ms.out (a rebuild releases it)
@@ -796,15 +851,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
             if (stats) *stats = total;
             return;
         }
-        const int64_t t_async = ctx->c.tunable[MB_TUNE_BFS_ASYNC];
-        // Hub-free graphs that fit one CTA go to its kernel, whatever their
-        // diameter (ms, asynchronous / one CTA: 10^4 vertices in a line 23.1 /
-        // 6.3, 100 x 100 0.53 / 0.18, 21 x 21 x 21 torus 0.19 / 0.08, uniform
-        // 2^12 with 5 edges per vertex 0.13 / 0.04); the larger ones do not, for
-        // a level of the whole grid costs 5 us or more (line of 40,000 91 / 147,
-        // 1000 x 1000 torus 4.4 / 7.4, 128^3 torus 1.3 / 1.7).
-        const bool one_cta = mb::bfs_small(g->g) && mb::bfs_coop_applies(ctx->c);
-        const bool bfs_async = (t_async > 0 || (t_async < 0 && mb::async_by_default(g->g, true) && !one_cta)) &&
+        const bool bfs_async = (t_async > 0 || (t_async < 0 && mb::async_by_default(g->g, true))) &&
                                (ctx->c.schedule_policy == MB_POLICY_FIXED ||
                                 ctx->c.schedule_policy == MB_POLICY_LEARNED) &&
                                !ctx->c.persist;
@@ -816,15 +863,11 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
             if (coop) {
                 int32_t *out = levels_out + (size_t)i * V;
                 const size_t bytes = sizeof(int32_t) * (size_t)V;
-                // a small graph's levels go to a host array through pinned memory
-                const bool pinned = !out_here && !mb::is_device_ptr(levels_out) && mb::bfs_small(g->g);
-                int32_t *dev = out_here ? out : pinned ? (int32_t *)ctx->c.pinned_reserve(bytes)
-                                                       : (int32_t *)apps(g).run_out.reserve(bytes);
+                int32_t *dev = out_here ? out : (int32_t *)apps(g).run_out.reserve(bytes);
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(int32_t) * (size_t)V, cudaMemcpyDefault, s));
                 };
-                mb::run_bfs_coop(ctx->c, g->g, apps(g).bfs_coop, src[i], dev, &st, out_here || pinned ? nullptr : &copy);
-                if (pinned) std::memcpy(out, dev, bytes);
+                mb::run_bfs_coop(ctx->c, g->g, apps(g).bfs_coop, src[i], dev, &st, out_here ? nullptr : &copy);
             } else {
             // the levels' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {
@@ -864,7 +907,17 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
         for (int32_t s : src)
             if (s < 0 || s >= V) mb::fail(MB_ERR_INVALID, "source vertex out of range");
         mb_stats total{};
-        if (nsrc > 1 && ctx->c.batching && mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop, nsrc)) {
+        const bool batch = nsrc > 1 && ctx->c.batching;
+        const bool coop = mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop, batch ? nsrc : 1);
+        if (coop && mb::sssp_small(g->g)) {
+            total = small_runs(ctx, g, src, batch ? mb::kSsspSmallSources : 1, dist_out,
+                               [&](const int32_t *from, int32_t n, float *out, mb_stats *st, const mb::EmitFn *after) {
+                                   mb::run_sssp_small(ctx->c, g->g, apps(g).sssp_coop, from, n, out, st, after);
+                               });
+            if (stats) *stats = total;
+            return;
+        }
+        if (batch && coop) {
             const bool here = on_this_device(dist_out);
             const int32_t most = mb::sssp_coop_sources(g->g);
             for (int32_t b0 = 0; b0 < nsrc; b0 += most) {
@@ -888,7 +941,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
-        if (nsrc > 1 && ctx->c.batching) {
+        if (batch) {
             // batches of up to 32 sources, one masked traversal each
             mb::MsSsspState &ms = apps(g).mssssp;
             ms.ensure(g->g);  // before reserving ms.out (a rebuild releases it)
@@ -915,7 +968,6 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
-        const bool coop = mb::sssp_coop_applies(ctx->c, g->g, apps(g).sssp_coop, 1);
         const bool out_here = coop && on_this_device(dist_out);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};

@@ -521,7 +521,8 @@ bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, in
     if (ctx.schedule_policy != MB_POLICY_FIXED || !ctx.use_graphs || ctx.tracing || ctx.persist || !ctx.tail ||
         ctx.max_step >= 0 || ctx.sssp_delta != 0.f)
         return false;
-    if (nsrc == 1 && async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
+    const bool small = sssp_small(g);
+    if (nsrc == 1 && !small && async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
     if (nsrc > 1) {
         if (ctx.tunable[MB_TUNE_MSS_DELTA] >= 0) return false;  // the lines' buckets
         // on a large graph with a huge hub most sources' frontiers meet in a

@@ -5,6 +5,9 @@
 namespace mb {
 
 constexpr int kSsspCoopTile = 512;
+constexpr int32_t kSsspSmallV = 10240;  // 20 bytes of shared memory per vertex
+constexpr int64_t kSsspSmallE = 49152, kSsspSmallHubE = 40960;  // without hubs, with
+constexpr int32_t kSsspSmallSources = 128;  // at most, in one launch
 
 struct SsspCoopOut {
     int32_t supersteps, splits, err, pad;
@@ -49,5 +52,12 @@ int32_t sssp_coop_sources(const Graph &g);
 // after: queued behind the run, before its host synchronisation.
 void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
                    mb_stats *stats, const EmitFn *after);
+
+// A graph that fits one CTA, nsrc <= kSsspSmallSources sources (a CTA each):
+// the same, but the distances are stored in one sweep, so `dist` may also be
+// pinned host memory.
+bool sssp_small(const Graph &g);
+void run_sssp_small(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
+                    mb_stats *stats, const EmitFn *after);
 
 }  // namespace mb
