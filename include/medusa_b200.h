@@ -397,7 +397,8 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                 graphs without a negative or NaN weight.  Identical
                                 distances */
 #define MB_TUNE_ASYNC_DELTA 18 /* width by which the asynchronous SSSP's threshold rises
-                                 (default: 24 x mean weight / mean out-degree, at least the
+                                 (default: 24 x mean weight / mean out-degree -- 72 x with
+                                 fewer than 4 edges per vertex --, at least the
                                  mean weight, on graphs without hubs; 0 -- no threshold --
                                  for the tail on graphs with hubs) */
 #define MB_TUNE_ASYNC_BLOCKS_PER_SM 19 /* CTAs of 256 threads per SM of the asynchronous
@@ -411,7 +412,7 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                edges per vertex and more than 10240 vertices or 65536
                                edges (smaller ones: a one-CTA kernel).  Identical levels */
 #define MB_TUNE_BFS_ASYNC_DELTA 21 /* threshold step of the asynchronous BFS, in hops
-                                     (default 8) */
+                                     (default 8; 24 with fewer than 4 edges per vertex) */
 #define MB_TUNE_ASYNC_BELOW 22 /* > 0: the asynchronous SSSP (when on) takes over only
                                  once the frontier, after reaching this many out-edges,
                                  has fewer -- the large supersteps run as BSP pushes and

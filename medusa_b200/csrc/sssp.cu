@@ -48,6 +48,7 @@ struct SsspArgs {
     // the asynchronous kernel's dirty bitmap over vertex ids [0, V) and hub
     // chunk ids [V, V + nchunks) (a.nbm when the graph has no hub)
     uint32_t *adirty;
+    bool look_first;              // read a distance before the atomic that may lower it
     int64_t WA;                   // its words
     const int32_t *hub_cbase;     // first chunk of each hub
     const int32_t *chunk_src;     // hub of the chunk at each position (id - V)
@@ -1102,9 +1103,10 @@ __global__ void k_sssp_init(SsspArgs a) {
         unsigned long long *w = &a.as->p[0].v;
         constexpr int kWords = (int)(offsetof(AsyncState, pt) / 8);
         for (int i = threadIdx.x; i < kWords; i += blockDim.x) w[i] = 0ull;
-        if (threadIdx.x < 2) a.as->idle[threadIdx.x].v = 0ull;
+        if (threadIdx.x < 2) a.as->idle[threadIdx.x].v = kAsyncIdle0;
         if (threadIdx.x == 2) a.as->bar.v = 0ull;
         if (threadIdx.x == 3) a.as->abort_.v = 0ull;
+        if (threadIdx.x == 4) a.as->open.v = 0ull;
     }
     __syncthreads();
     if (threadIdx.x == 0) choose_next(c, APP_SSSP, a.f.V, a.f.E);
@@ -1204,7 +1206,11 @@ float sssp_default_delta(const Graph &g, double mean_w) {
 float sssp_async_delta(const Graph &g, double mean_w) {
     if (g.E == 0) return 0.f;
     const double mean_deg = (double)g.E / (double)g.V;
-    return (float)std::max(mean_w, mean_w * 24.0 / std::max(1.0, mean_deg));
+    // road-like graphs: their frontiers are too small for narrow buckets (ms,
+    // 24 / 72 mean weights over the mean out-degree: grids of 1448 x 1448 1.04 /
+    // 0.90, 300 x 300 0.53 / 0.44; but uniform, 4 V 0.39 / 0.45, 16 V 0.58 / 1.32)
+    const double k = mean_deg < 4.0 ? 72.0 : 24.0;
+    return (float)std::max(mean_w, mean_w * k / std::max(1.0, mean_deg));
 }
 
 // Hub chunk tables of the asynchronous kernel for graph g (once).
@@ -1296,7 +1302,7 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
                                                                : (hub_free ? st.async_delta : 0.f);
     if (unit)
         async_delta = ctx.tunable[MB_TUNE_BFS_ASYNC_DELTA] >= 0 ? (float)ctx.tunable[MB_TUNE_BFS_ASYNC_DELTA]
-                                                                : kBfsAsyncDelta;
+                                                                : bfs_async_delta(g);
     // made on the first run whether or not it is asynchronous: the pointers
     // below are captured in the run's loop graph, which must not change
     // when a later run switches the kernel on
@@ -1304,6 +1310,10 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
     const int64_t nchunks = st.nchunks > 0 ? st.nchunks : 0;
     a.nc32 = nchunks ? st.nc32 : 0;
     a.adirty = nchunks ? st.adirty.as<uint32_t>() : a.nbm;
+    // The read saves atomics where most relaxations fail, but lengthens the chain
+    // of a hop (ms, with / without: SSSP on uniform 2^20 / 2^24 0.56 / 0.59, 2^20 / 2^23
+    // 0.52 / 0.52, 2^23 / 4 10^7 2.45 / 2.40, the 1448^2 grid 1.07 / 1.04, BFS on it 0.67 / 0.64).
+    a.look_first = g.E > 8 * (int64_t)g.V;
     a.WA = ((int64_t)g.V + 32 * (int64_t)a.nc32 + 31) / 32;
     a.hub_cbase = st.hub_cbase.as<int32_t>();
     a.chunk_src = st.chunk_src.as<int32_t>();

@@ -26,7 +26,8 @@ struct AsyncState {
     AsyncLine p[kAsyncSlots];  // monotone: dirty bits a warp may set, added before it sets any
     AsyncLine d[kAsyncSlots];  // monotone: the part of that it did not set, plus finished claims
     AsyncLine pt;              // (phase << 32) | float bits of the threshold (phase 0: the start's)
-    AsyncLine idle[2];         // CTAs whose warps all went idle in the phase of that parity
+    AsyncLine idle[2];         // CTAs whose warps are all idle in the phase of that parity
+    AsyncLine open;            // the last phase opened, claimed by the warp that opens it
     AsyncLine mn[2];           // least distance seen above the threshold in that phase (float bits)
     AsyncLine t0;              // least distance of the starting frontier (float bits)
     AsyncLine bar;             // start barrier: CTAs arrived

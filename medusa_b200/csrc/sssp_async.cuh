@@ -29,18 +29,26 @@
 //    itself set the bit of a vertex below T claims it back and relaxes it
 //    next (local continuation).  A claim is an atomicAnd that returned the
 //    bit set, so every set bit has exactly one claimer;
-//  - termination: AsyncState::p counts the bits a warp may set (added, and
-//    its return awaited, before the warp sets any) and AsyncState::d the
-//    part it did not set plus every finished claim.  Both only grow, and
-//    sum(p) - sum(d) is never below the bits set plus the claims in flight.
-//    A warp reads every d, then every p: equal sums mean that at a moment
-//    between the two reads no bit was set and no claim in flight, and from
-//    then on nothing can set one, so every warp leaves;
-//  - a warp that finds nothing below T reports itself idle once per phase
-//    (the CTA's warps in shared memory, then one global count per CTA); the
-//    last CTA raises T by delta (or to the least distance seen above T plus
-//    delta) and opens the next phase.  T only orders the claims: every order
-//    reaches the same fixpoint, the exact distances;
+//  - termination: a warp holds credit, the bits it may set.  AsyncState::p
+//    counts what warps took (added, and its return awaited, before the warp
+//    sets a bit of it), AsyncState::d what they gave back.  A bit set spends
+//    one, a finished claim earns one, and a warp that finds no work gives back
+//    all it holds.  Both counts only grow, and sum(p) - sum(d) is never below
+//    the bits set plus the claims in flight.  A warp reads every d, then every
+//    p: equal sums mean that at a moment between the two reads no bit was set,
+//    no claim in flight and no credit held, and from then on nothing can set a
+//    bit, so every warp leaves.  (Two counter atomics per batch of claims, one
+//    of them awaited, cost the 1448^2 grid 0.68 against 0.64 ms for BFS, 1.13
+//    against 1.00 for SSSP, a line of 40,000 95 against 81.);
+//  - a warp that finds nothing below T reports itself idle, and takes that
+//    back when it finds work in the same phase (the CTA's warps in shared
+//    memory, then one global count of CTAs); when every CTA is idle at once,
+//    T rises by delta (or to the least distance seen above T plus delta) and
+//    the next phase opens.  T only orders the claims: every order reaches the
+//    same fixpoint, the exact distances.  (Reports that stood for the phase let
+//    T run away while the first frontiers were small: SSSP on uniform 2^20 /
+//    2^24 took 0.51 ms in some runs, 1.05-1.1 with 4.5 relaxations per edge in
+//    the others; now 0.56-0.60 in all.);
 //  - every wait is bounded: the start barrier and a warp's run of idle
 //    passes give up after wait_polls (default kAsyncSpins), set ERR_ASYNC
 //    and make every warp leave; a warp with more claiming passes than the
@@ -60,6 +68,9 @@ constexpr int kAsyncWarps = kAsyncThreads / 32;
 #define MB_ASYNC_SLEEP_MAX 4  // idle sleep 128 ns << min(idle passes, this)
 #endif
 constexpr int kAsyncU = MB_ASYNC_U;  // strips of 32 edges in flight per warp
+// The idle counts start here: one CTA's minus may be performed before its plus,
+// and the sign bit has to stay zero.
+constexpr uint32_t kAsyncIdle0 = 1u << 16;
 constexpr long kAsyncSpins = 1l << 22;
 constexpr uint32_t kInfBits = 0x7f800000u;
 static_assert(kAsyncSlots == 32, "one work counter slot per lane");
@@ -102,10 +113,11 @@ __device__ __forceinline__ bool async_finished(AsyncState *S) {
 #define MB_ASYNC_CHUNK 64
 #endif
 constexpr int32_t kAsyncChunk = MB_ASYNC_CHUNK;
-// Default threshold step of the asynchronous BFS, in hops: 8 measured best
-// on the 1448^2 grid (1 -> 94 phases, 1.53 ms; 4 -> 25 phases, 0.85 ms; 8 ->
-// 13 phases, 0.73 ms; every vertex still relaxed once).
-constexpr float kBfsAsyncDelta = 8.f;
+// Default threshold step of the asynchronous BFS, in hops.  8 / 16 / 24, ms: on
+// road-like graphs (fewer than 4 edges per vertex) wide ones, grids of 1448 x
+// 1448 0.64 / 0.60 / 0.55, 300 x 300 0.39 / 0.35 / 0.32; uniform 2^20 with 4
+// edges per vertex 0.24 / 0.26 / 0.26, 2^23 with 5 1.38 / 1.49 / 1.62.
+inline float bfs_async_delta(const Graph &g) { return g.E < 4 * (int64_t)g.V ? 24.f : 8.f; }
 // Relax what this warp claimed: lane l holds one dirty id (or v < 0) -- a
 // vertex (its out-edges), a hub (the bits of its chunks) or a chunk (its
 // out-edges).  Every item (an edge, or a chunk bit) may set one dirty bit.
@@ -118,10 +130,11 @@ constexpr float kBfsAsyncDelta = 8.f;
 #define MB_ASYNC_LOCAL 1
 #endif
 constexpr uint32_t kAsyncNext = 64;
+constexpr uint32_t kAsyncCredit = 1024;  // taken beyond what a batch needs
 
 template <bool kUnit>
 __device__ __forceinline__ uint32_t async_relax(const SsspArgs &a, AsyncState *S, int slot, int32_t v,
-                                                float T, int32_t *nxt, uint32_t *nn) {
+                                                float T, int32_t *nxt, uint32_t *nn, uint32_t &credit) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     uint32_t *dirty = a.adirty;
@@ -155,9 +168,14 @@ __device__ __forceinline__ uint32_t async_relax(const SsspArgs &a, AsyncState *S
     const uint32_t total = __shfl_sync(FULL, incl, 31);
     const int32_t base_e = base - (int32_t)(incl - deg);  // item k of the owner: base_e(owner) + k
     const uint32_t hubs = __ballot_sync(FULL, hub);
-    unsigned long long pre = 0;
-    if (lane == 0 && total) pre = atomicAdd(&S->p[slot].v, (unsigned long long)total);
-    const int32_t order = (int32_t)(__shfl_sync(FULL, pre, 0) >> 63);  // zero
+    int32_t order = 0;
+    if (credit < total) {
+        const uint32_t more = total - credit + kAsyncCredit;
+        unsigned long long pre = 0;
+        if (lane == 0) pre = atomicAdd(&S->p[slot].v, (unsigned long long)more);
+        order = (int32_t)(__shfl_sync(FULL, pre, 0) >> 63);  // zero
+        credit += more;
+    }
     uint32_t newly = 0;
     for (uint32_t b0 = 0; b0 < total; b0 += 32 * kAsyncU) {
         int32_t x[kAsyncU];
@@ -188,7 +206,7 @@ __device__ __forceinline__ uint32_t async_relax(const SsspArgs &a, AsyncState *S
             nd[u] = ok[u] ? ds + (kUnit ? 1.f : __ldg(&a.wt[e])) : 0.f;
         }
 #pragma unroll
-        for (int u = 0; u < kAsyncU; u++) dx[u] = ok[u] ? ld_dist(a, x[u]) : 0.f;
+        for (int u = 0; u < kAsyncU; u++) dx[u] = ok[u] ? (a.look_first ? ld_dist(a, x[u]) : 3.0e38f) : 0.f;
         bool keep[kAsyncU];
 #if MB_ASYNC_LOCAL == 2
         // a vertex that dropped below T is kept by this warp WITHOUT setting
@@ -246,31 +264,33 @@ __device__ __forceinline__ uint32_t async_relax(const SsspArgs &a, AsyncState *S
             }
         }
     }
-    newly = warp_sum(newly);
-    // performed after every bit set above (its operand depends on them)
-    if (lane == 0 && (total | claimed))
-        atomicAdd(&S->d[slot].v, (unsigned long long)(total - newly) + (unsigned long long)__popc(claimed));
+    credit += (uint32_t)__popc(claimed) - warp_sum(newly);
     return total - warp_sum(hub ? deg : 0u);
 }
 
-// Lane 0 of a warp whose pass found nothing below the threshold, once per
-// phase: count the warp idle; the CTA's last warp counts the CTA, and the
-// grid's last CTA opens the next phase.
-__device__ __forceinline__ void async_idle(Ctrl *c, AsyncState *S, uint32_t *s_idle, uint32_t ph,
-                                           float T, float delta, float above, int cap) {
+// Lane 0 of a warp whose pass found nothing below the threshold: counts the
+// warp idle; the CTA's last warp counts the CTA, and the grid's last CTA opens
+// the next phase.  *s_idle: the CTA's idle warps, under the phase they reported
+// (phase << 8 | warps).  zero: async_busy's result, so that its change is
+// performed first.  False: the CTA is in a later phase already.
+__device__ __forceinline__ bool async_idle(Ctrl *c, AsyncState *S, uint32_t *s_idle, uint32_t ph,
+                                           float T, float delta, float above, int cap, uint32_t zero) {
     uint32_t dep = 0;
     if (above < __uint_as_float(kInfBits))
         dep = atomicMin((unsigned *)&S->mn[ph & 1].v, __float_as_uint(above));
     // distances are non-negative: dep >> 31 is zero
-    const uint32_t k = atomicAdd(&s_idle[ph & 1], 1u + (dep >> 31)) + 1u;
-    if (k != (uint32_t)kAsyncWarps) return;
-    // this CTA's warps all reported phase ph; none reports ph + 1 before the
-    // phase opens, which needs this CTA's count below
-    const uint32_t r = atomicExch(&s_idle[(ph + 1) & 1], 0u);
+    const uint32_t tag = (ph & 0xffffffu) << 8;
+    uint32_t old = *(volatile uint32_t *)s_idle, now;
+    do {
+        now = old;
+        if ((int32_t)((now & ~255u) - tag) > 0) return false;
+        old = atomicCAS(s_idle, now, ((now & ~255u) == tag ? now : tag) + 1u + (dep >> 31) + zero);
+    } while (old != now);
+    if (((now & ~255u) == tag ? (now & 255u) : 0u) + 1u != (uint32_t)kAsyncWarps) return true;
     __threadfence();
-    const uint32_t g = atomicAdd((unsigned *)&S->idle[ph & 1].v, 1u + (r >> 31)) + 1u;
-    if (g != gridDim.x) return;
-    // every CTA idle in phase ph: raise the threshold
+    if (atomicAdd((unsigned *)&S->idle[ph & 1].v, 1u) + 1u != kAsyncIdle0 + gridDim.x) return true;
+    // every CTA idle in phase ph: one of those that saw it raises the threshold
+    if (atomicCAS((unsigned *)&S->open.v, ph, ph + 1u) != ph) return true;
     const uint32_t mb = atomicExch((unsigned *)&S->mn[ph & 1].v, kInfBits);
     const float m = __uint_as_float(mb);
     float tn = T + delta;
@@ -279,12 +299,27 @@ __device__ __forceinline__ void async_idle(Ctrl *c, AsyncState *S, uint32_t *s_i
     // step past the least distance seen above T, so that vertex is below tn
     if (!(tn > T)) tn = __uint_as_float(__float_as_uint(T) + 1u);
     if (m < __uint_as_float(kInfBits) && !(tn > m)) tn = __uint_as_float(mb + 1u);
-    const uint32_t r2 = atomicExch((unsigned *)&S->idle[(ph + 1) & 1].v, 0u);
+    const uint32_t r2 = atomicExch((unsigned *)&S->idle[(ph + 1) & 1].v, kAsyncIdle0);
     const uint32_t nph = ph + 1u + (r2 >> 31) + (mb >> 31);  // both shifts zero
     atomicExch(&S->pt.v, ((unsigned long long)nph << 32) | __float_as_uint(tn));
     atomicAdd(&c->splits, 1);
     atomicAdd(&c->supersteps, 1);
     if ((int64_t)nph > (int64_t)cap) async_abort(c, S, ERR_STEP_CAP);
+    return true;
+}
+
+// Lane 0 of a warp that reported phase ph and has found work again.  Returns
+// zero once the grid's count has changed.
+__device__ __forceinline__ uint32_t async_busy(AsyncState *S, uint32_t *s_idle, uint32_t ph) {
+    const uint32_t tag = (ph & 0xffffffu) << 8;
+    uint32_t old = *(volatile uint32_t *)s_idle, now;
+    do {
+        now = old;
+        if ((now & ~255u) != tag) return 0u;
+        old = atomicCAS(s_idle, now, now - 1u);
+    } while (old != now);
+    if ((now & 255u) != (uint32_t)kAsyncWarps) return 0u;
+    return atomicSub((unsigned *)&S->idle[ph & 1].v, 1u) >> 31;
 }
 
 // kUnit: every weight 1 (BFS levels as hop distances; a.wt is not read).
@@ -295,7 +330,7 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
     count_launch(c);
     AsyncState *S = a.as;
     uint32_t *dirty = a.adirty;
-    __shared__ uint32_t s_idle[2];
+    __shared__ uint32_t s_idle;
     __shared__ int s_ok;
     __shared__ volatile int s_done;  // set by the CTA's checker warp: every warp leaves
     // claimed vertices waiting for a full batch of 32, and the vertices the
@@ -313,8 +348,10 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
     const float inf = __uint_as_float(kInfBits);
     const int64_t W = a.WA;
     const int32_t V = a.f.V;
-    if (threadIdx.x < 2) s_idle[threadIdx.x] = 0u;
-    if (threadIdx.x == 0) s_done = 0;
+    if (threadIdx.x == 0) {
+        s_idle = 0u;
+        s_done = 0;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0)  // finish_superstep credits the frontier's edges
         atomicAdd((unsigned long long *)&c->work, 0ull - (unsigned long long)c->front_m);
     // 1. the queue frontier's vertices become dirty
@@ -369,8 +406,10 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
     const float T0 = delta > 0.f ? t0 + delta : inf;
     // 3. claim and relax until no work is left
     uint32_t reported = 0xffffffffu;
+    uint32_t zero = 0u;
     long idle = 0, busy = 0;
     unsigned long long relaxed = 0;
+    uint32_t credit = 0;  // counted in p, not yet in d: bits this warp may still set (warp-uniform)
     const bool checker = (threadIdx.x >> 5) == 0;
     for (;;) {
         if (s_done) break;
@@ -419,7 +458,7 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
                     continue;
                 }
                 if (nb >= 32 || (all && nb > 0)) {
-                    relaxed += async_relax<kUnit>(a, S, slot, lane < (int)nb ? bv[lane] : -1, T, nxt, &nn);
+                    relaxed += async_relax<kUnit>(a, S, slot, lane < (int)nb ? bv[lane] : -1, T, nxt, &nn, credit);
                     const uint32_t done = min(nb, 32u);
                     const uint32_t rest = nb - done;
                     const int32_t t = lane < (int)rest ? bv[32 + lane] : -1;
@@ -452,6 +491,10 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
                 if (lane == 0) old = atom_and_acquire(&dirty[w], ~mask);
                 const uint32_t claimed = __shfl_sync(FULL, old, 0) & mask;
                 if (!claimed) continue;
+                if (!found && reported == ph) {
+                    if (lane == 0) zero = async_busy(S, &s_idle, ph);
+                    reported = 0xffffffffu;
+                }
                 found = true;
                 if ((claimed >> lane) & 1u) bv[nb + __popc(claimed & lanemask_lt())] = id;
                 nb += __popc(claimed);
@@ -471,12 +514,16 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
             }
             continue;
         }
+        if (credit) {  // an idle warp sets no bits
+            if (lane == 0) atomicAdd(&S->d[slot].v, (unsigned long long)credit);
+            credit = 0;
+        }
         // without a threshold there is no next phase to open
         if (reported != ph && T < inf) {
-            reported = ph;
             above = warp_min_f(above);
-            if (lane == 0) async_idle(c, S, s_idle, ph, T, delta, above, cap);
-            __syncwarp();
+            bool in = true;
+            if (lane == 0) in = async_idle(c, S, &s_idle, ph, T, delta, above, cap, zero);
+            if (__shfl_sync(FULL, in, 0)) reported = ph;
         }
         if (++idle > budget) {
             if (lane == 0) {
