@@ -230,23 +230,20 @@ __global__ void __launch_bounds__(kPrThreads) k_pr_pull(PrArgs a) {
     }
 }
 
-// A warp's first unit is its number; the next ones come from the counter, so
-// that CTAs which start late (the hub scans hold SMs) take no share of their
-// own.  Longest groups first.
-template <int kG, bool kSmall>
-__global__ void __launch_bounds__(256, kSmall ? kSellCtasSmall : kSellCtas) k_pr_sell(SellArgs a) {
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+// One unit per warp, longest groups first, and as many CTAs as that takes: the
+// hardware hands them to the SMs as these get free, beside the hub scans too.
+// (A resident grid whose warps took their next unit from a counter, one atomic
+// a unit on the same address, us per superstep: R-MAT 2^24 / 2^28 957, now
+// 943; 4 10^6 / 6 10^7 250 in the fixed order, now 232; uniform 9 10^5 / 1.4 10^7 67,
+// now 57; 9 10^5 / 3.6 10^6 28, now 18.)
+template <int kG>
+__global__ void __launch_bounds__(256, kSellCtas) k_pr_sell(SellArgs a) {
     const uint32_t units = (uint32_t)a.nlong + (uint32_t)(a.ngroups - a.nlong + kG - 1) / kG;
-    uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     zero_vertices(a);
-    while (u < units) {
-        uint32_t t = 0;  // the next unit's number is on its way during this one
-        if ((threadIdx.x & 31) == 0 && a.ctr) t = atomicAdd(a.ctr, 1u);
-        if (u < (uint32_t)a.nlong) sell_long<kSmall ? kSellUSmall : kSellU>(a, u);
-        else sell_short<kG>(a, a.nlong + (int64_t)(u - a.nlong) * kG);
-        if (!a.ctr) break;
-        u = warps + __shfl_sync(0xffffffffu, t, 0);
-    }
+    if (u >= units) return;
+    if (u < (uint32_t)a.nlong) sell_long<kSellU>(a, u);
+    else sell_short<kG>(a, a.nlong + (int64_t)(u - a.nlong) * kG);
 }
 
 // All supersteps in one cooperative launch, for graphs whose groups fit one
@@ -707,8 +704,15 @@ __global__ void k_stage_fill(const int2 *items, const int32_t *meg_off, int32_t 
 
 // ---- contribution layout ------------------------------------------------------
 // Sort key of a vertex: its out-degree class, four per octave, the largest
-// degrees first; vertices without out-edges last.
+// degrees first (flat: one class, for graphs without hubs), and in a class its
+// in-degree, the order of the sliced ELL; vertices without out-edges last.
+// The classes keep the hot contributions in few lines; the order in a class
+// makes a warp's 32 new contributions a few runs of them (in id order instead,
+// us per superstep: uniform 6 10^6 / 6 10^7 285, here 268; R-MAT 4 10^6 / 6 10^7
+// 284 / 280, 2^24 / 2^28 965 / 957).
 constexpr int kDegClasses = 128;
+constexpr int kInKeyBits = 16;
+constexpr uint32_t kInKeyMask = (1u << kInKeyBits) - 1u;
 __host__ __device__ inline uint32_t degree_key(uint32_t d) {
     if (d == 0) return kDegClasses;
     uint32_t e = 0;
@@ -716,17 +720,20 @@ __host__ __device__ inline uint32_t degree_key(uint32_t d) {
     const uint32_t frac = e >= 2 ? (d >> (e - 2)) & 3u : (d << (2 - e)) & 3u;
     return kDegClasses - 1 - (4 * e + frac);
 }
-__global__ void k_deg_keys(const int32_t *outdeg, int32_t V, uint32_t *key, uint32_t *val) {
+__global__ void k_deg_keys(const int32_t *outdeg, const int32_t *rrow, int32_t V, bool flat, uint32_t *key,
+                           uint32_t *val) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
          v += (int64_t)gridDim.x * blockDim.x) {
-        key[v] = degree_key((uint32_t)outdeg[v]);
+        const uint32_t c = flat && outdeg[v] > 0 ? 0u : degree_key((uint32_t)outdeg[v]);
+        const uint32_t in = min((uint32_t)(rrow[v + 1] - rrow[v]), kInKeyMask);
+        key[v] = (c << kInKeyBits) | (kInKeyMask - in);
         val[v] = (uint32_t)v;
     }
 }
 __global__ void k_pos(const uint32_t *key, const uint32_t *val, int32_t V, int32_t *pos) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V;
          i += (int64_t)gridDim.x * blockDim.x)
-        pos[val[i]] = key[i] < kDegClasses ? (int32_t)i : -1;
+        pos[val[i]] = (key[i] >> kInKeyBits) < kDegClasses ? (int32_t)i : -1;
 }
 
 __global__ void k_map_pos(const int32_t *src, int64_t E, const int32_t *pos, int32_t *out) {
@@ -887,9 +894,9 @@ void PrState::ensure(Context &ctx, const Graph &g) {
         key.reserve(sizeof(uint32_t) * (size_t)V);
         val.reserve(sizeof(uint32_t) * (size_t)V);
         pos.reserve(sizeof(int32_t) * (size_t)V);
-        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), V, key.as<uint32_t>(), val.as<uint32_t>());
+        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), g.rrow.as<int32_t>(), V, g.max_outdeg <= 64, key.as<uint32_t>(), val.as<uint32_t>());
         MB_CHECK_LAUNCH();
-        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8, s);
+        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8 + kInKeyBits, s);
         k_pos<<<gridV, 256, 0, s>>>(key.as<uint32_t>(), val.as<uint32_t>(), V, pos.as<int32_t>());
         MB_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
@@ -956,7 +963,6 @@ void PrState::build_sell(Context &ctx, const Graph &g, int32_t max_rows, const i
     cudaStream_t s = ctx.stream;
     const int gridV = grid_for(V, 256, ctx.num_sms * 16);
     max_rows = std::min(max_rows, g.max_indeg);
-    out.max_rows = max_rows;
     int bits = 1;
     while (bits < 32 && ((int64_t)1 << bits) < (int64_t)max_rows + 2) bits++;
     DevBuf key, val, cnt;
@@ -1132,8 +1138,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         return ctx.num_sms * std::max(per_sm, 1);
     };
     const int grid_pull = resident((const void *)k_pr_pull<true>, kPrThreads);
-    // short sliced-ELL groups a warp takes at once: the tunable, else 4
-    const int vpl = ctx.tunable[MB_TUNE_PR_LIGHT_VPL] > 0 ? (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL] : 4;
+    // short sliced-ELL groups a warp takes at once: the tunable, else 1 (1 / 2 / 4,
+    // us per superstep: uniform 9 10^5 with 4 / 8 / 16 edges per vertex 17.9 / 16.8 /
+    // 20.7, 30.4 / 30.7 / 38.7, 56.6 / 58.7 / 62.7; R-MAT 4 10^6 / 6 10^7 232 / 233 / 238,
+    // 3 10^6 / 3 10^7 80 / 78 / 81)
+    const int vpl = ctx.tunable[MB_TUNE_PR_LIGHT_VPL] > 0 ? (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL] : 1;
     const int pair = ctx.tunable[MB_TUNE_PR_SHORT_PAIR] > 0 ? (int)ctx.tunable[MB_TUNE_PR_SHORT_PAIR]
                                                              : kShortPairDefault;
     // each variant's grid is its own resident block count (registers differ)
@@ -1141,14 +1150,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                                    (const void *)k_heavy_blocks<false, 4>},
                                   {(const void *)k_heavy_blocks<true, 1>, (const void *)k_heavy_blocks<true, 2>,
                                    (const void *)k_heavy_blocks<true, 4>}};
-    const void *sell_fn[2][3] = {
-        {(const void *)k_pr_sell<1, false>, (const void *)k_pr_sell<2, false>, (const void *)k_pr_sell<4, false>},
-        {(const void *)k_pr_sell<1, true>, (const void *)k_pr_sell<2, true>, (const void *)k_pr_sell<4, true>}};
+    const void *sell_fn[3] = {(const void *)k_pr_sell<1>, (const void *)k_pr_sell<2>, (const void *)k_pr_sell<4>};
     const int pi = pair == 1 ? 0 : pair == 2 ? 1 : 2, vi = vpl == 1 ? 0 : vpl == 2 ? 1 : 2;
     const int64_t heavy_threads = heavy_units(st.nitems, st.nlong, pair) * 32;
     const int grid_heavy[2] = {grid_for(heavy_threads, 256, resident(heavy_fn[0][pi], 256)),
                                grid_for(heavy_threads, 256, resident(heavy_fn[1][pi], 256))};
-    const int grid_sell[2] = {resident(sell_fn[0][vi], 256), resident(sell_fn[1][vi], 256)};
     auto heavy = [&](bool from_msg, cudaStream_t cs, const PrArgs &a) {
         PrArgs arg = a;
         void *params[] = {&arg};
@@ -1182,11 +1188,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         }
         void *params[] = {&a};
         const int64_t units = (int64_t)l.nlong + (l.ngroups - l.nlong + vpl - 1) / vpl;
-        const int small = l.max_rows <= kPrLight && units > (int64_t)grid_sell[0] * (256 / 32) &&
-                          units <= (int64_t)grid_sell[1] * (256 / 32);
-        const int grid = grid_for(units * 32, 256, grid_sell[small]);
-        a.ctr = (int64_t)grid * (256 / 32) < units ? st.ctr.as<uint32_t>() + it : nullptr;
-        MB_CUDA(cudaLaunchKernel(sell_fn[small][vi], grid, 256, params, 0, cs));
+        MB_CUDA(cudaLaunchKernel(sell_fn[vi], (unsigned)((units + 7) / 8), 256, params, 0, cs));
     };
     const int grid_vtx = ctx.num_sms * 8;
     const int hub_ctas = ctx.tunable[MB_TUNE_PR_HUB_CTAS] > 0 ? (int)ctx.tunable[MB_TUNE_PR_HUB_CTAS]
@@ -1227,13 +1229,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         if (grid_res > resident(res_fn, res_threads)) res_fn = (const void *)k_pr_resident<8>;
         if (grid_res > resident(res_fn, res_threads)) grid_res = 0;
     }
-    st.ctr.reserve(sizeof(uint32_t) * (size_t)std::max(iters, 1));
     if (grid_res && !st.bar.p) {
         st.bar.reserve(256);
         MB_CUDA(cudaMemsetAsync(st.bar.p, 0, 256, s));
     }
     auto emit = [&](cudaStream_t cs) {
-        if (!unfused && !grid_res) MB_CUDA(cudaMemsetAsync(st.ctr.p, 0, sizeof(uint32_t) * (size_t)std::max(iters, 1), cs));
         if (init_vec)
             k_pr_init_vec<<<grid_vtx, 256, 0, cs>>>(g.outdeg.as<int32_t>(), st.pos.as<int32_t>(), g.V, init_vec,
                                                     st.contrib[0].as<float>());

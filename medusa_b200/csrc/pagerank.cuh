@@ -9,7 +9,6 @@ namespace mb {
 struct PrSell {
     DevBuf v, pd, rows, base, src, zv, zpd;
     int32_t ngroups = 0, nlong = 0, nz = 0;
-    int32_t max_rows = 0;  // no vertex in it has more in-edges
     void release() {
         v.release(); pd.release(); rows.release(); base.release(); src.release();
         zv.release(); zpd.release();
@@ -29,7 +28,7 @@ struct PrState {
     // where each vertex's contribution sits in contrib[] (-1: no out-edges):
     // ordered by out-degree class, the sources with the most out-edges first
     DevBuf pos;
-    DevBuf ctr;  // the sliced ELL's work counters, one per superstep
+    DevBuf ctr;  // the many-graph kernel's work counters, one per superstep
     DevBuf bar;  // the one-launch run's barrier
     bool fixed_built = false;  // the fixed order's lists below
     int32_t nitems = 0, nhub = 0;

@@ -50,7 +50,6 @@ struct SellArgs {
     int32_t ngroups, nlong; // groups [0, nlong) have more than kSellShort rows
     const float *contrib_in;
     float *contrib_out, *rank_out;
-    uint32_t *ctr;          // units taken by late warps, zero before the launch (null: every unit has its warp)
     // vertices without in-edges: their sum is 0 in every superstep, so their
     // contributions are written once to each of the two buffers (zfirst), their
     // ranks with the others'
@@ -70,12 +69,10 @@ __device__ __forceinline__ void zero_vertices(const SellArgs &a) {
     }
 }
 constexpr int kSellShort = 8;
-// Two builds of the kernel: 16 rows in flight and at least 5 CTAs per SM, or
-// 8 and 8 CTAs, where that takes every unit at once and the first does not (light
-// vertices only: a long group's chain wants the deeper prefetch; R-MAT
-// 2^24 / 2^28: 0.955 against 1.011 ms a superstep; uniform 2^18 / 2^22: 25.8
-// against 22.8 us).
-constexpr int kSellU = 16, kSellCtas = 5, kSellUSmall = 8, kSellCtasSmall = 8;
+// 16 rows in flight and at least 5 CTAs of 256 threads per SM (8 rows and 8 CTAs:
+// R-MAT 2^24 / 2^28 0.955 against 1.011 ms a superstep, uniform 9 10^5 / 3.6 10^6 21
+// against 27 us).
+constexpr int kSellU = 16, kSellCtas = 5;
 
 // One group: kSellU rows (coalesced index loads, then the gathers) in
 // flight; each lane folds its own vertex's slots in order.  Padding slots
