@@ -547,6 +547,9 @@ static void union_build(Context &ctx, Batch &b) {
     MB_CHECK_LAUNCH();
     MB_CUDA(cudaStreamSynchronize(s));
     PrState &pr = u->pr;
+    // by id within a class: a graph's contributions stay together (64 graphs of
+    // 2^10 to 2^16 vertices 2.24 against 2.39 ms)
+    pr.by_indegree = false;
     pr.ensure(ctx, g);
     pr.ensure_fixed(ctx, g);
     u->c0.reserve(sizeof(float) * (size_t)g.V);

@@ -725,7 +725,7 @@ __global__ void k_deg_keys(const int32_t *outdeg, const int32_t *rrow, int32_t V
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
          v += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t c = flat && outdeg[v] > 0 ? 0u : degree_key((uint32_t)outdeg[v]);
-        const uint32_t in = min((uint32_t)(rrow[v + 1] - rrow[v]), kInKeyMask);
+        const uint32_t in = rrow ? min((uint32_t)(rrow[v + 1] - rrow[v]), kInKeyMask) : 0u;
         key[v] = (c << kInKeyBits) | (kInKeyMask - in);
         val[v] = (uint32_t)v;
     }
@@ -894,7 +894,8 @@ void PrState::ensure(Context &ctx, const Graph &g) {
         key.reserve(sizeof(uint32_t) * (size_t)V);
         val.reserve(sizeof(uint32_t) * (size_t)V);
         pos.reserve(sizeof(int32_t) * (size_t)V);
-        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), g.rrow.as<int32_t>(), V, g.max_outdeg <= 64, key.as<uint32_t>(), val.as<uint32_t>());
+        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), by_indegree ? g.rrow.as<int32_t>() : nullptr, V,
+                                         g.max_outdeg <= 64, key.as<uint32_t>(), val.as<uint32_t>());
         MB_CHECK_LAUNCH();
         radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8 + kInKeyBits, s);
         k_pos<<<gridV, 256, 0, s>>>(key.as<uint32_t>(), val.as<uint32_t>(), V, pos.as<int32_t>());

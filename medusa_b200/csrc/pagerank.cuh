@@ -28,6 +28,7 @@ struct PrState {
     // where each vertex's contribution sits in contrib[] (-1: no out-edges):
     // ordered by out-degree class, the sources with the most out-edges first
     DevBuf pos;
+    bool by_indegree = true;  // the contributions' order within a class (k_deg_keys), else by id
     DevBuf ctr;  // the many-graph kernel's work counters, one per superstep
     DevBuf bar;  // the one-launch run's barrier
     bool fixed_built = false;  // the fixed order's lists below
