@@ -40,8 +40,8 @@
 //    bit, so every warp leaves.  (Two counter atomics per batch of claims, one
 //    of them awaited, cost the 1448^2 grid 0.68 against 0.64 ms for BFS, 1.13
 //    against 1.00 for SSSP, a line of 40,000 95 against 81.);
-//  - a warp that finds nothing below T reports itself idle, and takes that
-//    back when it finds work in the same phase (the CTA's warps in shared
+//  - a warp that finds nothing below T reports itself idle, and (idle_back)
+//    takes that back when it finds work in the same phase (the CTA's warps in shared
 //    memory, then one global count of CTAs); when every CTA is idle at once,
 //    T rises by delta (or to the least distance seen above T plus delta) and
 //    the next phase opens.  T only orders the claims: every order reaches the
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
                 if (lane == 0) old = atom_and_acquire(&dirty[w], ~mask);
                 const uint32_t claimed = __shfl_sync(FULL, old, 0) & mask;
                 if (!claimed) continue;
-                if (!found && reported == ph) {
+                if (a.idle_back && !found && reported == ph) {
                     if (lane == 0) zero = async_busy(S, &s_idle, ph);
                     reported = 0xffffffffu;
                 }
