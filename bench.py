@@ -356,7 +356,8 @@ def run_medusa(args):
                    "parallelism": "replicas" if world > 1 else "single GPU",
                    "schedule_policy": "fixed (direction-optimising rule)",
                    "loop": ("host-driven loop (one flag read per superstep)" if args.hostloop
-                            else "one CUDA graph per BSP loop (device-side convergence)"),
+                            else "one launch per run where the default rules allow, else one CUDA graph "
+                                 "per BSP loop (device-side convergence)"),
                    "autotuned": {k: float(v) for k, v in tuned.items()}},
         "bfs": {"gteps": round(sb_last["edges_traversed"] / sb_last["device_ms"] / 1e6, 3),
                 "ms": round(sb_last["device_ms"], 4), "supersteps": sb_last["supersteps"],

@@ -118,8 +118,8 @@ int mb_set_schedule_replay(mb_ctx *ctx, const int8_t *schedules, int32_t n);
 /* SSSP near-far (delta-stepping) bucket width: vertices whose new distance
  * is below the current threshold are expanded next, the rest wait in a far
  * pile until the threshold (raised by delta each time the near frontier runs
- * dry) passes them.  delta > 0: that width; 0 (the default): plain frontier
- * Bellman-Ford; < 0: 32 x mean weight / mean out-degree of the graph.
+ * dry) passes them.  delta > 0: that width; 0 (the default): none in the
+ * superstep loop (the one-launch kernels have buckets of their own); < 0: 32 x mean weight / mean out-degree of the graph.
  * Distances are identical for every delta.  No reference counterpart (the
  * reference relaxes every edge every superstep, SSSP/CPUFunctorHoster.cpp:58-99). */
 int mb_set_sssp_delta(mb_ctx *ctx, float delta);
@@ -296,8 +296,8 @@ int mb_vis_edge_lines(mb_ctx *ctx, const mb_graph *g, const float *pos, float *l
  * supersteps from 1/V (as mb_pagerank in MB_PR_ORDER_FIXED, bit for bit) and
  * then one BFS (as mb_bfs) from
  * sources[i] (nullable: vertex 0), all in ONE persistent cooperative launch
- * fed by a device work queue; each graph is worked by a team of CTAs sized
- * by its edge count.  Outputs are concatenated: graph i's ranks and levels
+ * over their disjoint union (with a batch tunable set, or without
+ * supersteps: a team of CTAs per graph, fed by a device work queue).  Outputs are concatenated: graph i's ranks and levels
  * at [vbase[i], vbase[i+1]) (mb_batch_vertex_offsets); host or device. */
 typedef struct mb_batch mb_batch;
 int mb_batch_generate(mb_ctx *ctx, int32_t n, const mb_gen_params *params, mb_batch **out);
@@ -419,7 +419,8 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                  0: from the first superstep; default: 0 on graphs
                                  without hubs (largest out-degree <= 64), else
                                  max(2^18, E/16) */
-#define MB_TUNE_MSS_DELTA 23 /* batched SSSP (2..32 sources): near-far width -- the
+#define MB_TUNE_MSS_DELTA 23 /* batched SSSP (2..32 sources; setting it also keeps the
+                               batch from the one-launch kernels): near-far width -- the
                                frontier holds only the (vertex, source) pairs below a
                                threshold that rises by this much whenever none is
                                left; 0: plain frontier Bellman-Ford; default: 0.3 x

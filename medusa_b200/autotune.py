@@ -164,7 +164,7 @@ def tune_traversals(ctx, g, source=0, reps=3):
 
 
 def tune_pagerank(ctx, g, iters=10, reps=3, out=None):
-    """Light vertices per lane of the fused pull, and, in the reference's
+    """Short sliced-ELL groups per warp, and, in the reference's
     order, the in-degree above which a vertex is summed by one CTA's integer
     scan (else short heavy blocks per warp of the fixed order), timing
     `iters` PageRank supersteps on g (out: a rank buffer to reuse, e.g. a
