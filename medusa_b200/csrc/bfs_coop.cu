@@ -183,9 +183,9 @@ __global__ void __launch_bounds__(kCoopThreads, kBfsCoopCtas) k_bfs_coop(CoopArg
         a.level[a.source] = 0;
     }
     if (threadIdx.x == 0) sm.nout = 0;
-    uint32_t target = gridDim.x;
-    if (!coop_sync(a, target)) return;
-    coop_bfs(a, sm, target, deg0 > 0 ? 1u : 0u, (uint32_t)deg0);
+    uint32_t barriers = 0;
+    if (!coop_sync(a, ++barriers)) return;
+    coop_bfs(a, sm, barriers, deg0 > 0 ? 1u : 0u, (uint32_t)deg0);
 }
 
 }  // namespace

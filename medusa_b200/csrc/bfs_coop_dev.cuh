@@ -21,7 +21,7 @@ struct CoopShared {  // device memory of a run, zero before it
     unsigned long long toq;  // the queue built from a pull's vertices
     unsigned long long reached;
     uint32_t ticket;
-    alignas(128) uint32_t bar;  // polled: a line of its own
+    alignas(128) BarWord bar;  // polled: a line of its own
 };
 
 struct CoopArgs {
@@ -40,8 +40,8 @@ struct CoopArgs {
 
 // ---- one cooperative grid -----------------------------------------------------------
 
-__device__ __forceinline__ bool coop_sync(const CoopArgs &a, uint32_t target) {
-    return coop_barrier(&a.sh->bar, target, a.polls, &a.out->err);
+__device__ __forceinline__ bool coop_sync(const CoopArgs &a, uint32_t k) {
+    return coop_barrier(&a.sh->bar, k, a.polls, &a.out->err);
 }
 
 struct CoopSmem {
@@ -309,7 +309,7 @@ __device__ __forceinline__ void coop_toq(const CoopArgs &a, CoopSmem &sm, const 
 // visited bits set, tile table filled), then -1 for the vertices not reached and
 // the report; false if a barrier gave up.  sm.nout is 0 and the frontier
 // visible to every CTA (a barrier passed).
-__device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32_t &target, uint32_t n,
+__device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32_t &barriers, uint32_t n,
                                          unsigned long long m) {
     __shared__ unsigned long long s_r[kCoopThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -336,8 +336,7 @@ __device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32
         const int32_t lvl = step + 1;
         if (pull) {
             coop_pull(a, a.vis[vb], a.vis[vb ^ 1], lvl, ctr);
-            target += gridDim.x;
-            if (!coop_sync(a, target)) return false;
+            if (!coop_sync(a, ++barriers)) return false;
             prev_n = n;
             n = __ldcg(&ctr->n);
             m = __ldcg(&ctr->m);
@@ -348,16 +347,14 @@ __device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32
         } else {
             if (!queue) {
                 coop_toq(a, sm, a.vis[vb], a.vis[vb ^ 1], &a.sh->toq, a.q[cur], a.tf[cur]);
-                target += gridDim.x;
-                if (!coop_sync(a, target)) return false;
+                if (!coop_sync(a, ++barriers)) return false;
                 const unsigned long long c = __ldcg(&a.sh->toq);
                 n = (uint32_t)(c >> 32);
                 queue = true;
             }
             work += m;
             coop_push(a, sm, a.q[cur], a.tf[cur], n, (uint32_t)m, a.vis[vb], lvl, ctr, a.q[cur ^ 1], a.tf[cur ^ 1]);
-            target += gridDim.x;
-            if (!coop_sync(a, target)) return false;
+            if (!coop_sync(a, ++barriers)) return false;
             if (gt == 0) a.sh->toq = 0ull;  // read by every CTA before this barrier
             const unsigned long long c = __ldcg(&ctr->q);
             n = (uint32_t)(c >> 32);

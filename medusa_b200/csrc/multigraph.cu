@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a)
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t gt = (int64_t)blockIdx.x * kCoopThreads + tid, gn = (int64_t)gridDim.x * kCoopThreads;
     const uint32_t gw = (uint32_t)(gt >> 5), warps = (uint32_t)(gn >> 5);
-    uint32_t target = 0;
+    uint32_t barriers = 0;
     for (int64_t w = gt; w < a.bfs.W; w += gn) a.bfs.vis[0][w] = 0u;
     if (tid == 0) sm.nout = 0;
     // 1. PageRank
@@ -411,8 +411,7 @@ __global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a)
             }
             u = warps + __shfl_sync(0xffffffffu, t, 0);
         }
-        target += gridDim.x;
-        if (!coop_sync(a.bfs, target)) return;
+        if (!coop_sync(a.bfs, ++barriers)) return;
     }
     // 2. one BFS from every graph's source; CTA 0 makes the frontier
     if (blockIdx.x == 0 && tid < 32) {
@@ -440,10 +439,9 @@ __global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a)
         }
         if (lane == 0) *a.front = ((unsigned long long)n << 32) | m;
     }
-    target += gridDim.x;
-    if (!coop_sync(a.bfs, target)) return;
+    if (!coop_sync(a.bfs, ++barriers)) return;
     const unsigned long long f = __ldcg(a.front);
-    coop_bfs(a.bfs, sm, target, (uint32_t)(f >> 32), (uint32_t)f);
+    coop_bfs(a.bfs, sm, barriers, (uint32_t)(f >> 32), (uint32_t)f);
 }
 
 }  // namespace
