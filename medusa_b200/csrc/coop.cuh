@@ -1,5 +1,5 @@
 // coop.cuh -- the grid barrier and the bounded waits of the one-launch kernels
-// (bfs_coop.cu, sssp_coop.cu).
+// (bfs_coop.cu, sssp_coop.cu, multigraph.cu, pagerank.cu).
 #pragma once
 #include "barrier_word.h"
 #include "engine.cuh"

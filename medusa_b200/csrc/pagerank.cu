@@ -29,6 +29,7 @@
 // array at msgDstID, then the same combine+update reading the messages.
 #include <algorithm>
 #include <vector>
+#include "coop.cuh"
 #include "pagerank.cuh"
 #include "pr_order.cuh"
 #include "pr_sell.cuh"
@@ -262,39 +263,11 @@ struct ResidentArgs {
     const int32_t *zv;  // vertices without in-edges
     const int2 *zpd;
     int32_t nz, iters;
-    uint32_t *bar;      // arrivals (top bit: a wait gave up), and CTAs done, on lines of their own;
+    BarWord *bar;       // arrivals (barrier_word.h), and 128 bytes further the CTAs done;
                         // zero before the launch, which leaves them so
-    volatile int *err;
+    int32_t *err;
     long polls;
 };
-__device__ __forceinline__ bool resident_sync(const ResidentArgs &a, uint32_t target) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        constexpr uint32_t kGaveUp = 1u << 31;
-        __threadfence();
-        atomicAdd(a.bar, 1u);
-        int ok = 0;
-        for (long it = 0;; it++) {
-            uint32_t v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-            if (v >= kGaveUp) break;
-            if (v >= target) {
-                ok = 1;
-                break;
-            }
-            if (it >= a.polls) {
-                *a.err = 1;
-                atomicOr(a.bar, kGaveUp);
-                break;
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok;
-}
 template <int kResU>
 __global__ void __launch_bounds__(kResThreads, kResU == 8 ? 2 : 1) k_pr_resident(SellArgs a, ResidentArgs r) {
     const int lane = threadIdx.x & 31;
@@ -304,15 +277,11 @@ __global__ void __launch_bounds__(kResThreads, kResU == 8 ? 2 : 1) k_pr_resident
     const int32_t rows = in ? __ldg(&a.rows[g]) : 0;
     const int2 pd = in ? __ldg(&a.pd[(int64_t)g * 32 + lane]) : make_int2(-1, 0);
     const int32_t *src = a.src + (in ? (int64_t)__ldg(&a.base[g]) * 32 + lane : 0);
-    uint32_t target = 0;
     for (int it = 0; it < r.iters; it++) {
         int32_t idx[kResU];
 #pragma unroll
         for (int u = 0; u < kResU; u++) idx[u] = u < rows ? __ldg(src + u * 32) : -1;
-        if (it > 0) {
-            target += gridDim.x;
-            if (!resident_sync(r, target)) return;
-        }
+        if (it > 0 && !coop_barrier(r.bar, (uint32_t)it, r.polls, r.err)) return;
         const float *cin = it & 1 ? r.contrib[1] : r.contrib[0];
         float *cout = it & 1 ? r.contrib[0] : r.contrib[1];
         float *rank = it == r.iters - 1 ? r.rank : nullptr;
@@ -347,9 +316,9 @@ __global__ void __launch_bounds__(kResThreads, kResU == 8 ? 2 : 1) k_pr_resident
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&r.bar[32], 1u) == gridDim.x - 1) {  // no CTA waits any more
-        r.bar[0] = 0u;
-        r.bar[32] = 0u;
+    if (threadIdx.x == 0 && atomicAdd(&r.bar[16], (BarWord)1) == gridDim.x - 1) {  // no CTA waits any more
+        r.bar[0] = 0;
+        r.bar[16] = 0;
     }
 }
 
@@ -1218,8 +1187,8 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     const PrSell &all = ref_order ? st.sell : st.light;
     int grid_res = 0, res_threads = kResThreads;
     const void *res_fn = (const void *)k_pr_resident<16>;
-    volatile int *res_err = (volatile int *)ctx.ctrl_readback();
-    *res_err = 0;
+    int32_t *res_err = (int32_t *)ctx.ctrl_readback();
+    *(volatile int32_t *)res_err = 0;
     if (!unfused && iters > 1 && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
         // small graphs in smaller CTAs, one per SM: 177 groups in 6 CTAs of 32
         // warps were bound by 6 SMs' gathers
@@ -1252,7 +1221,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             r.zpd = all.zpd.as<int2>();
             r.nz = all.nz;
             r.iters = iters;
-            r.bar = st.bar.as<uint32_t>();
+            r.bar = st.bar.as<BarWord>();
             r.err = res_err;
             r.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : 1l << 22;
             void *params[] = {&a, &r};
@@ -1379,11 +1348,11 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             MB_CUDA(cudaEventRecord(e1, s));
         }
         MB_CUDA(cudaEventSynchronize(e1));
-        if (grid_res && *res_err) {
+        if (grid_res && *(volatile int32_t *)res_err) {
             MB_CUDA(cudaMemsetAsync(st.bar.p, 0, 256, s));
             MB_CUDA(cudaStreamSynchronize(s));
+            fail(MB_ERR_TIMEOUT, "pagerank: a barrier between two supersteps timed out");
         }
-        if (grid_res && *res_err) fail(MB_ERR_TIMEOUT, "pagerank: a barrier between two supersteps timed out");
         float ms = 0;
         MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         if (stats) {
