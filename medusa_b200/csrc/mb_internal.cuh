@@ -18,6 +18,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <string>
 #include <vector>
 #include "../../include/medusa_b200.h"
@@ -138,6 +139,13 @@ void graph_from_gtgraph(Context &ctx, Graph &g, const char *text, int64_t len, u
 
 // ---- context ------------------------------------------------------------------
 struct Context {
+    // what a plan kept on a graph is keyed by: no two contexts of a process
+    // share it, while an address may come back after a context is destroyed
+    const uint64_t id = next_id();
+    static uint64_t next_id() {
+        static std::atomic<uint64_t> last{0};
+        return ++last;
+    }
     int device = 0;
     bool pool_counted = false;  // counted among the device's contexts (pool.cu)
     cudaStream_t stream = nullptr;

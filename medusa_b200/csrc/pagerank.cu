@@ -1315,11 +1315,10 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     MB_CUDA(cudaEventCreate(&e1));
     try {
         if (ctx.use_graphs) {
-            if (!st.exec || st.g_iters != iters || st.g_init != init || st.g_init_vec != init_vec ||
+            if (!st.exec || st.g_ctx != ctx.id || st.g_iters != iters || st.g_init != init || st.g_init_vec != init_vec ||
                 st.g_sched != sched ||
                 st.g_order != ctx.pr_order || st.g_tune != ctx.tune_gen) {
-                if (st.exec) cudaGraphExecDestroy(st.exec);
-                st.exec = nullptr;
+                st.drop_exec();
                 cudaGraph_t gr;
                 MB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
                 try {
@@ -1332,6 +1331,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
                 cudaError_t e = cudaGraphInstantiate(&st.exec, gr, 0);
                 cudaGraphDestroy(gr);
                 MB_CUDA(e);
+                st.g_ctx = ctx.id;
                 st.g_iters = iters;
                 st.g_init = init;
                 st.g_init_vec = init_vec;

@@ -56,7 +56,10 @@ struct PrState {
     // the warp-per-hub scans on another, beside the big hubs' CTAs
     cudaStream_t side3 = nullptr;
     cudaEvent_t ev_join3 = nullptr;
-    cudaGraphExec_t exec = nullptr;  // captured run (init + iters supersteps)
+    // captured run (init + iters supersteps), and the context that captured it:
+    // its error word, poll limit and tunables are in the capture
+    cudaGraphExec_t exec = nullptr;
+    uint64_t g_ctx = 0;
     int32_t g_iters = -1, g_sched = -1, g_order = -1;
     uint64_t g_tune = ~0ull;  // tunables generation of the captured run
     float g_init = 0.f;
@@ -70,10 +73,12 @@ struct PrState {
         if (!ev_join3) MB_CUDA(cudaEventCreateWithFlags(&ev_join3, cudaEventDisableTiming));
     }
     ~PrState() { release(); }
-    void release() {
+    void drop_exec() {
         if (exec) cudaGraphExecDestroy(exec);
         exec = nullptr;
         g_iters = -1;
+    }
+    void release() {
         rank.release(); contrib[0].release(); contrib[1].release(); msg.release();
         init_stage.release();
         pos.release(); hcol.release(); light.release(); ctr.release(); bar.release();
@@ -92,6 +97,7 @@ struct PrState {
         built = false;
     }
     void release_exact() {
+        drop_exec();  // it may read the buffers that go
         sell.release();
         x_hub_v.release();
         x_stage.release(); stage_src.release(); stage_off.release(); stage_items.release();
