@@ -50,10 +50,6 @@ constexpr uint32_t kBmMin = 1 << 20;  // 2^19 and less: 2-4% slower
 // (10^4 / 10^5: 0.118 without, 0.146 with).
 constexpr float kBucketWidth = 0.85f;
 constexpr int64_t kBucketMinE = 1 << 18;
-// Several sources: (source, vertex) pairs of a run, 128 MB of distances.
-// 32 sources at 2^23 / 2^24 / 2^25 pairs: mild R-MAT 2^20 / 2^24 15.7 / 14.1 / 13.2 ms,
-// 2^22 / 2^26 59.0 / 55.6 / 54.0.
-constexpr int64_t kPairs = 1 << 25;
 // Bucket width in mean weights with several sources.  The more out-edges a
 // run's frontiers hold, the less a superstep's own cost matters, and the
 // narrower the best bucket; a sparse graph without hubs (roads) needs
@@ -503,11 +499,7 @@ void SsspCoopState::ensure(const Graph &g, int32_t nsrc) {
     room = nsrc;
 }
 
-int32_t sssp_coop_sources(const Graph &g) {
-    int64_t n = std::min<int64_t>(kSsspCoopSources, std::max<int64_t>(1, kPairs / std::max<int32_t>(g.V, 1)));
-    n = std::min<int64_t>(n, 0xffffffffll / std::max<int64_t>(g.E, 1));  // out-edges of a queue in 32 bits
-    return (int32_t)std::max<int64_t>(n, 1);
-}
+int32_t sssp_coop_sources(const Graph &g) { return pairs_sources(g.V, g.E); }
 
 bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, int32_t nsrc) {
     // the loop graph's and the asynchronous kernel's own parameters ask for them

@@ -1,6 +1,7 @@
 // sssp_coop.cuh -- a whole SSSP in one launch (internal).
 #pragma once
 #include "engine.cuh"
+#include "pairs_limit.h"
 
 namespace mb {
 
@@ -38,8 +39,6 @@ struct SsspCoopState {
     }
     void ensure(const Graph &g, int32_t nsrc);
 };
-
-constexpr int32_t kSsspCoopSources = 32;  // at most, in one run
 
 // Whether the context's settings and the graph leave SSSP from nsrc sources to
 // run_sssp_coop (makes the state when they do).
