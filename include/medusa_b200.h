@@ -146,7 +146,10 @@ int mb_set_graph_capture(mb_ctx *ctx, int enable);
 
 /* ---- graph storage ----------------------------------------------------------- */
 /* Build a device-resident graph (CSR + reverse CSR + message slots) from an
- * edge list in insertion order.  w may be NULL (unweighted).
+ * edge list in insertion order.  w may be NULL (unweighted).  Host arrays, or
+ * device arrays: those of this device are read in place, on the context's
+ * stream, so the caller first waits for whatever writes them (arrays that
+ * change during the call give an error or a graph of no use).
  * Replaces GTGraph::get_parition's single-partition path + GraphIR::AddEdge +
  * InitHostDS + InitDeviceDS (MultipleGPU/PartitionManager.cu:116-534,
  * MedusaRT/GraphConverter.cu:180-196, MultipleGPU/MultiPublicAPI.h:43-96,144-308)

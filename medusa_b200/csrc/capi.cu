@@ -493,7 +493,7 @@ int mb_graph_from_edges(mb_ctx *ctx, int32_t V, int64_t E, const int32_t *src, c
         use_device(ctx);
         mb::DevBuf bs, bd, bw;
         try {
-            // device arrays are read in place
+            // device arrays are read in place, each once
             const size_t n = 4 * (size_t)E;
             const void *ps = E > 0 ? stage_in(bs, src, n, ctx->c.stream) : nullptr;
             const void *pd = E > 0 ? stage_in(bd, dst, n, ctx->c.stream) : nullptr;
