@@ -87,9 +87,11 @@ mb::AppStates &apps(mb_graph *g) {
     return *g->g.apps;
 }
 
-// Memory that kernels on the current device may use in place.
+// An array of 4-byte elements that kernels on the current device may use in
+// place: an address off the elements' alignment, which a copy takes, faults in
+// a kernel.
 bool on_this_device(const void *p) {
-    if (!mb::is_device_ptr(p)) return false;
+    if ((reinterpret_cast<uintptr_t>(p) & 3) || !mb::is_device_ptr(p)) return false;
     cudaPointerAttributes a;
     int device = 0;
     MB_CUDA(cudaPointerGetAttributes(&a, p));
@@ -735,14 +737,14 @@ int mb_batch_run(mb_ctx *ctx, mb_batch *b, int32_t pr_iters, const int32_t *sour
         std::vector<int32_t> src;
         if (sources) src = fetch_i32(sources, n);
         const size_t nv = (size_t)b->b.total_V;
-        const bool dev_r = mb::is_device_ptr(ranks_out), dev_l = mb::is_device_ptr(levels_out);
+        const bool dev_r = on_this_device(ranks_out), dev_l = on_this_device(levels_out);
         float *r = ranks_out;
         int32_t *l = levels_out;
         if (!dev_r) r = (float *)b->b.rank.reserve(sizeof(float) * std::max<size_t>(nv, 1));
         if (!dev_l) l = (int32_t *)b->b.level.reserve(sizeof(int32_t) * std::max<size_t>(nv, 1));
         mb::batch_run(ctx->c, b->b, pr_iters, sources ? src.data() : nullptr, r, l, stats);
-        if (!dev_r) MB_CUDA(cudaMemcpyAsync(ranks_out, r, sizeof(float) * nv, cudaMemcpyDeviceToHost, ctx->c.stream));
-        if (!dev_l) MB_CUDA(cudaMemcpyAsync(levels_out, l, sizeof(int32_t) * nv, cudaMemcpyDeviceToHost, ctx->c.stream));
+        if (!dev_r) MB_CUDA(cudaMemcpyAsync(ranks_out, r, sizeof(float) * nv, cudaMemcpyDefault, ctx->c.stream));
+        if (!dev_l) MB_CUDA(cudaMemcpyAsync(levels_out, l, sizeof(int32_t) * nv, cudaMemcpyDefault, ctx->c.stream));
         MB_CUDA(cudaStreamSynchronize(ctx->c.stream));
     });
 }
@@ -829,7 +831,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
             // batches of up to 64 sources, one masked traversal each
             mb::MsBfsState &ms = apps(g).msbfs;
             ms.ensure(g->g);  // before reserving ms.out (a rebuild releases it)
-            const bool dev_out = mb::is_device_ptr(levels_out);
+            const bool dev_out = on_this_device(levels_out);
             for (int32_t b0 = 0; b0 < nsrc; b0 += 64) {
                 const int32_t nb = std::min<int32_t>(64, nsrc - b0);
                 int32_t *dst = levels_out + (size_t)b0 * V;
@@ -839,7 +841,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                 mb::run_msbfs(ctx->c, g->g, ms, src.data() + b0, nb, dev, &st);
                 if (!dev_out)
                     MB_CUDA(cudaMemcpyAsync(dst, dev, sizeof(int32_t) * (size_t)nb * V,
-                                            cudaMemcpyDeviceToHost, ctx->c.stream));
+                                            cudaMemcpyDefault, ctx->c.stream));
                 total.supersteps = std::max(total.supersteps, st.supersteps);
                 total.edges_traversed += st.edges_traversed;
                 total.vertices_reached += st.vertices_reached;
@@ -945,7 +947,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             // batches of up to 32 sources, one masked traversal each
             mb::MsSsspState &ms = apps(g).mssssp;
             ms.ensure(g->g);  // before reserving ms.out (a rebuild releases it)
-            const bool dev_out = mb::is_device_ptr(dist_out);
+            const bool dev_out = on_this_device(dist_out);
             for (int32_t b0 = 0; b0 < nsrc; b0 += 32) {
                 const int32_t nb = std::min<int32_t>(32, nsrc - b0);
                 float *dst = dist_out + (size_t)b0 * V;
@@ -955,7 +957,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
                 mb::run_mssssp(ctx->c, g->g, ms, src.data() + b0, nb, dev, &st);
                 if (!dev_out)
                     MB_CUDA(cudaMemcpyAsync(dst, dev, sizeof(float) * (size_t)nb * V,
-                                            cudaMemcpyDeviceToHost, ctx->c.stream));
+                                            cudaMemcpyDefault, ctx->c.stream));
                 total.supersteps = std::max(total.supersteps, st.supersteps);
                 total.edges_traversed += st.edges_traversed;
                 total.vertices_reached += st.vertices_reached;
