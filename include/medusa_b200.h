@@ -258,7 +258,9 @@ int mb_set_pagerank_order(mb_ctx *ctx, int32_t order);
 
 /* Device layout of a graph, for code compiled against the header-only
  * operator API (include/medusa/medusa.h), whose functor kernels read it in
- * place.  Pointers stay valid until mb_graph_destroy.  row/col/esrc/wt: the
+ * place.  Pointers stay valid until mb_graph_destroy and are cudaMalloc's own
+ * (for cudaIpcGetMemHandle, or a peer GPU), memory allowing: a graph's first
+ * view moves its arrays out of the library's memory pool.  row/col/esrc/wt: the
  * CSR in the reference's AA edge order (SSSP/EdgeDataType.cu:138-186; esrc is
  * srcVertexID, wt is null for an unweighted graph); rrow/rcol: the reverse
  * CSR, whose position j is message slot j; mslot: msgDstID; outdeg:

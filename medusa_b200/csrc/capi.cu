@@ -4,6 +4,7 @@
 // of the last error is kept per context (and per thread for calls made
 // without a usable context).  Array arguments may be host or device pointers.
 #include <cstring>
+#include <mutex>
 #include <new>
 #include "bfs.cuh"
 #include "bfs_coop.cuh"
@@ -29,6 +30,11 @@ struct AppStates {
     MsSsspState mssssp;
     PrState pr;
     int stepped = -1;  // the app of the stepped run in progress (mb_superstep), or -1
+    // the captured runs, which hold the addresses of the graph's arrays
+    void drop_plans() {
+        for (LoopGraph *l : {&bfs.lg, &bfs_async.lg, &sssp.lg, &msbfs.lg}) l->reset();
+        pr.drop_exec();
+    }
 };
 int64_t generate_edges_host(const mb_gen_params &p, int32_t *src, int32_t *dst, float *w);
 void graph_generate(Context &ctx, Graph &g, const mb_gen_params &p, uint32_t flags);
@@ -46,6 +52,10 @@ struct mb_batch {
 };
 struct mb_graph {
     mb::Graph g;
+    // held by every call that reads the graph's arrays or its plans:
+    // mb_graph_device_view may move the arrays
+    mutable std::mutex use;
+    bool viewed = false;
 };
 
 namespace {
@@ -107,9 +117,11 @@ std::vector<int32_t> fetch_i32(const int32_t *p, int64_t n) {
     return out;
 }
 
-void check_graph(mb_ctx *ctx, const mb_graph *g) {
+// The graph checked, and held for the call.
+std::unique_lock<std::mutex> check_graph(mb_ctx *ctx, const mb_graph *g) {
     if (!ctx || !g) mb::fail(MB_ERR_INVALID, "null context or graph");
     if (g->g.device != ctx->c.device) mb::fail(MB_ERR_INVALID, "graph lives on another device");
+    return std::unique_lock<std::mutex>(g->use);
 }
 
 }  // namespace
@@ -258,7 +270,7 @@ int mb_vis_node_quads(mb_ctx *ctx, int32_t V, const float *pos, const int32_t *r
 
 int mb_vis_edge_lines(mb_ctx *ctx, const mb_graph *g, const float *pos, float *lines) {
     return guarded(ctx, [&] {
-        check_graph(ctx, g);
+        const auto held = check_graph(ctx, g);
         if (!pos || !lines) mb::fail(MB_ERR_INVALID, "bad arguments");
         use_device(ctx);
         mb::DevBuf bp, bl;
@@ -379,7 +391,7 @@ int mb_scheduler_collect(mb_ctx *ctx, const mb_graph *gc, int32_t app, int32_t s
                          float *features, float *times, int32_t *fixed_sched,
                          int32_t max_samples, int32_t *n_out) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (app < 0 || app > 2)
             mb::fail(MB_ERR_INVALID, "app must be 0 (BFS), 1 (SSSP) or 2 (batched BFS)");
         if (!features || !times || !n_out || max_samples < 0) mb::fail(MB_ERR_INVALID, "bad output");
@@ -589,8 +601,27 @@ int mb_generate_edges_host(const mb_gen_params *p, int32_t *src, int32_t *dst, f
     });
 }
 
-int mb_graph_device_view(const mb_graph *g, mb_graph_view *v) {
-    if (!g || !v) return set_error(nullptr, MB_ERR_INVALID, "null argument");
+int mb_graph_device_view(const mb_graph *gc, mb_graph_view *v) {
+    if (!gc || !v) return set_error(nullptr, MB_ERR_INVALID, "null argument");
+    mb_graph *g = const_cast<mb_graph *>(gc);
+    const std::unique_lock<std::mutex> held(g->use);
+    if (!g->viewed) {
+        // from here on the addresses are the caller's too: out of the pool
+        int device = -1;
+        cudaGetDevice(&device);
+        const int rc = guarded(nullptr, [&] {
+            MB_CUDA(cudaSetDevice(g->g.device));
+            MB_CUDA(cudaDeviceSynchronize());
+            mb::PoolIdle idle;
+            if (g->g.apps) g->g.apps->drop_plans();
+            for (mb::DevBuf *b : {&g->g.row, &g->g.col, &g->g.esrc, &g->g.wt, &g->g.rrow, &g->g.rcol, &g->g.rwt,
+                                  &g->g.mslot, &g->g.outdeg})
+                mb::pool_detach(*b);
+            g->viewed = true;
+        });
+        if (device >= 0) cudaSetDevice(device);
+        if (rc != MB_OK) return rc;
+    }
     v->num_vertices = g->g.V;
     v->num_edges = g->g.E;
     v->row = g->g.row.as<int32_t>();
@@ -634,7 +665,7 @@ int mb_graph_info(const mb_graph *g, int32_t *V, int64_t *E) {
 int mb_graph_export(mb_ctx *ctx, const mb_graph *g, int32_t *row, int32_t *col, float *w,
                     int32_t *rrow, int32_t *rcol, int32_t *mslot) {
     return guarded(ctx, [&] {
-        check_graph(ctx, g);
+        const auto held = check_graph(ctx, g);
         use_device(ctx);
         const mb::Graph &G = g->g;
         const size_t vb = sizeof(int32_t) * (size_t)(G.V + 1), eb = sizeof(int32_t) * (size_t)G.E;
@@ -800,7 +831,7 @@ extern "C" {
 int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc,
            int32_t *levels_out, mb_stats *stats) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (nsrc < 1 || !sources || !levels_out) mb::fail(MB_ERR_INVALID, "bad sources/output");
         use_device(ctx);
         mb_graph *g = const_cast<mb_graph *>(gc);
@@ -899,7 +930,7 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
 int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc, float *dist_out,
             mb_stats *stats) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (nsrc < 1 || !sources || !dist_out) mb::fail(MB_ERR_INVALID, "bad sources/output");
         use_device(ctx);
         mb_graph *g = const_cast<mb_graph *>(gc);
@@ -1005,7 +1036,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
 int mb_pagerank(mb_ctx *ctx, const mb_graph *gc, int32_t iters, float init, float *rank_out,
                 mb_stats *stats) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (iters < 0 || !rank_out) mb::fail(MB_ERR_INVALID, "bad iters/output");
         use_device(ctx);
         mb_graph *g = const_cast<mb_graph *>(gc);
@@ -1022,7 +1053,7 @@ int mb_pagerank(mb_ctx *ctx, const mb_graph *gc, int32_t iters, float init, floa
 int mb_superstep(mb_ctx *ctx, const mb_graph *gc, int32_t app, int32_t step, int32_t source,
                  int32_t schedule, int32_t *continue_out) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (!continue_out || step < 0) mb::fail(MB_ERR_INVALID, "bad step/output");
         if (schedule < -1 || schedule >= MB_NUM_SCHEDULES) mb::fail(MB_ERR_INVALID, "bad schedule");
         use_device(ctx);
@@ -1063,7 +1094,7 @@ int mb_superstep(mb_ctx *ctx, const mb_graph *gc, int32_t app, int32_t step, int
 
 int mb_superstep_result(mb_ctx *ctx, const mb_graph *gc, int32_t app, void *out, mb_stats *stats) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (!out) mb::fail(MB_ERR_INVALID, "null output");
         use_device(ctx);
         mb_graph *g = const_cast<mb_graph *>(gc);
@@ -1090,7 +1121,7 @@ int mb_superstep_result(mb_ctx *ctx, const mb_graph *gc, int32_t app, void *out,
 int mb_pagerank_from(mb_ctx *ctx, const mb_graph *gc, int32_t iters, const float *init_ranks,
                      float *rank_out, mb_stats *stats) {
     return guarded(ctx, [&] {
-        check_graph(ctx, gc);
+        const auto held = check_graph(ctx, gc);
         if (iters < 0 || !rank_out || !init_ranks) mb::fail(MB_ERR_INVALID, "bad iters/input/output");
         use_device(ctx);
         mb_graph *g = const_cast<mb_graph *>(gc);

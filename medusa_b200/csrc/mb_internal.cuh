@@ -56,6 +56,11 @@ struct ApiError {
 void *pool_alloc(size_t n);
 void pool_free(void *p);
 void pool_use_stream(cudaStream_t s);
+struct DevBuf;
+// Move b out of the pool, contents and all, into memory of its own
+// (cudaMalloc); it stays where it is when there is none to be had.  The device
+// is idle.
+void pool_detach(DevBuf &b);
 void pool_context(int device, int delta);  // a context of the device is made (+1) or destroyed (-1)
 struct PoolIdle {
     bool was;

@@ -9,7 +9,9 @@
 // is destroyed.  Buffers above kPoolMax come from cudaMalloc: past the kept
 // size the pool unmaps at every wait, and mapping anew there is slower (a
 // 2^24 / 2^28 graph with every buffer from the pool: built in 739 ms against
-// 223 ms).
+// 223 ms).  So do buffers whose addresses callers get (pool_detach): memory of
+// a pool can neither be opened by another process (cudaIpcGetMemHandle) nor
+// reached from a peer GPU by cudaDeviceEnablePeerAccess.
 //
 // Ordering.  Callers rely on what cudaMalloc and cudaFree give them: memory
 // usable on every stream at once, and no use in flight when it is handed on.
@@ -125,6 +127,32 @@ void pool_free(void *p) {
     }
     cudaFree(p);
     cudaGetLastError();
+}
+
+void pool_detach(DevBuf &b) {
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        bool pooled = false;
+        for (DevicePool &d : g_pools) pooled = pooled || d.live.count(b.p);
+        if (!pooled) return;
+    }
+    void *p = nullptr;
+    if (cudaMalloc(&p, b.bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaMemcpy(p, b.p, b.bytes, cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        cudaFree(p);
+        MB_CUDA(e);
+    }
+    pool_free(b.p);
+    b.p = p;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (device < kMaxDevices) g_pools[device].plain.insert(p);
 }
 
 void pool_use_stream(cudaStream_t s) { t_stream = s; }
