@@ -685,10 +685,12 @@ int mb_graph_destroy(mb_graph *g) {
     cudaSetDevice(g->g.device);
     cudaDeviceSynchronize();
     mb::PoolIdle idle;
+    const int device = g->g.device;
     delete g->g.apps;
     g->g.apps = nullptr;
     g->g.release();
     delete g;
+    mb::pool_trim(device);
     return MB_OK;
 }
 
@@ -785,8 +787,10 @@ int mb_batch_destroy(mb_batch *b) {
     cudaSetDevice(b->device);
     cudaDeviceSynchronize();
     mb::PoolIdle idle;
+    const int device = b->device;
     b->b.release();
     delete b;
+    mb::pool_trim(device);
     return MB_OK;
 }
 

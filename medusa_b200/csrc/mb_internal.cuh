@@ -61,6 +61,7 @@ struct DevBuf;
 // (cudaMalloc); it stays where it is when there is none to be had.  The device
 // is idle.
 void pool_detach(DevBuf &b);
+void pool_trim(int device);  // after a graph or a batch has gone
 void pool_context(int device, int delta);  // a context of the device is made (+1) or destroyed (-1)
 struct PoolIdle {
     bool was;

@@ -5,8 +5,9 @@
 // cudaMalloc / cudaFree map and unmap device memory each time: loading a
 // 2^20 / 2^24 edge list and one SSSP on it spent more than half of its
 // 28.3 ms there.  The pool keeps at most 1/16 of the device's memory mapped
-// between uses and gives all of it back when the last context of the device
-// is destroyed.  Buffers above kPoolMax come from cudaMalloc: past the kept
+// between uses, no more than kPoolSpare of it unused once a graph or a batch is
+// destroyed (so that other allocators of the process find the rest), and gives
+// all of it back when the last context of the device is destroyed.  Buffers above kPoolMax come from cudaMalloc: past the kept
 // size the pool unmaps at every wait, and mapping anew there is slower (a
 // 2^24 / 2^28 graph with every buffer from the pool: built in 739 ms against
 // 223 ms).  So do buffers whose addresses callers get (pool_detach): memory of
@@ -35,6 +36,7 @@ struct DevicePool {
 std::mutex g_mutex;
 constexpr int kMaxDevices = 64;
 constexpr size_t kPoolMax = (size_t)256 << 20;
+constexpr uint64_t kPoolSpare = (uint64_t)2 << 30;  // building 2^21 / 4 10^7 and one SSSP on it take 1.9 GB
 DevicePool g_pools[kMaxDevices];
 
 void drop_pool(DevicePool &d) {
@@ -156,6 +158,19 @@ void pool_detach(DevBuf &b) {
 }
 
 void pool_use_stream(cudaStream_t s) { t_stream = s; }
+
+void pool_trim(int device) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (device < 0 || device >= kMaxDevices) return;
+    DevicePool &d = g_pools[device];
+    uint64_t used = 0, reserved = 0;
+    if (d.pool && cudaStreamSynchronize(d.stream) == cudaSuccess &&
+        cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        reserved > used + kPoolSpare)
+        cudaMemPoolTrimTo(d.pool, used + kPoolSpare);
+    cudaGetLastError();
+}
 
 void pool_context(int device, int delta) {
     std::lock_guard<std::mutex> lock(g_mutex);
