@@ -871,9 +871,12 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                 const int32_t nb = std::min<int32_t>(64, nsrc - b0);
                 int32_t *dst = levels_out + (size_t)b0 * V;
                 int32_t *dev = dst;
-                if (!dev_out) dev = (int32_t *)ms.out.reserve(sizeof(int32_t) * (size_t)nb * V);
                 mb_stats st{};
-                mb::run_msbfs(ctx->c, g->g, ms, src.data() + b0, nb, dev, &st);
+                const auto run = [&] {
+                    if (!dev_out) dev = (int32_t *)ms.out.reserve(sizeof(int32_t) * (size_t)nb * V);
+                    mb::run_msbfs(ctx->c, g->g, ms, src.data() + b0, nb, dev, &st);
+                };
+                if (!mb::memory_for(run, [&] { ms.drop_keep(); })) run();
                 if (!dev_out)
                     MB_CUDA(cudaMemcpyAsync(dst, dev, sizeof(int32_t) * (size_t)nb * V,
                                             cudaMemcpyDefault, ctx->c.stream));
@@ -892,15 +895,21 @@ int mb_bfs(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsrc
                                (ctx->c.schedule_policy == MB_POLICY_FIXED ||
                                 ctx->c.schedule_policy == MB_POLICY_LEARNED) &&
                                !ctx->c.persist;
-        const bool coop = !bfs_async && mb::bfs_coop_applies(ctx->c);
+        bool coop = !bfs_async && mb::bfs_coop_applies(ctx->c);
         const bool out_here = coop && on_this_device(levels_out);
+        if (coop)
+            coop = mb::memory_for(
+                [&] {
+                    apps(g).bfs_coop.ensure(g->g);
+                    if (!out_here) apps(g).run_out.reserve(sizeof(int32_t) * (size_t)V);
+                },
+                [&] { apps(g).bfs_coop.release(); });
         if (bfs_async) apps(g).bfs.ensure(g->g);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};
             if (coop) {
                 int32_t *out = levels_out + (size_t)i * V;
-                const size_t bytes = sizeof(int32_t) * (size_t)V;
-                int32_t *dev = out_here ? out : (int32_t *)apps(g).run_out.reserve(bytes);
+                int32_t *dev = out_here ? out : apps(g).run_out.as<int32_t>();
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(int32_t) * (size_t)V, cudaMemcpyDefault, s));
                 };
@@ -954,9 +963,18 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
-        if (batch && coop) {
-            const bool here = on_this_device(dist_out);
-            const int32_t most = mb::sssp_coop_sources(g->g);
+        // the sources of a run, fewer where memory is short (then none: the lines)
+        const bool here = coop && on_this_device(dist_out);
+        int32_t most = coop ? std::min(batch ? mb::sssp_coop_sources(g->g) : 1, nsrc) : 0;
+        mb::SsspCoopState &cs = apps(g).sssp_coop;
+        while (most > 0 && !mb::memory_for(
+                               [&] {
+                                   cs.ensure(g->g, most);
+                                   if (!here) apps(g).run_out.reserve(sizeof(float) * (size_t)most * V);
+                               },
+                               [&] { cs.release_room(); }))
+            most /= 2;
+        if (batch && most > 0) {
             for (int32_t b0 = 0; b0 < nsrc; b0 += most) {
                 const int32_t nb = std::min(most, nsrc - b0);
                 const size_t bytes = sizeof(float) * (size_t)nb * V;
@@ -966,7 +984,7 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
                     MB_CUDA(cudaMemcpyAsync(out, dev, bytes, cudaMemcpyDefault, s));
                 };
                 mb_stats st{};
-                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, src.data() + b0, nb, dev, &st, here ? nullptr : &copy);
+                mb::run_sssp_coop(ctx->c, g->g, cs, src.data() + b0, nb, dev, &st, here ? nullptr : &copy);
                 total.supersteps = std::max(total.supersteps, st.supersteps);
                 total.edges_traversed += st.edges_traversed;
                 total.vertices_reached += st.vertices_reached;
@@ -1005,16 +1023,15 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
             if (stats) *stats = total;
             return;
         }
-        const bool out_here = coop && on_this_device(dist_out);
         for (int32_t i = 0; i < nsrc; i++) {
             mb_stats st{};
-            if (coop) {
+            if (most > 0) {
                 float *out = dist_out + (size_t)i * V;
-                float *dev = out_here ? out : (float *)apps(g).run_out.reserve(sizeof(float) * (size_t)V);
+                float *dev = here ? out : apps(g).run_out.as<float>();
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(float) * (size_t)V, cudaMemcpyDefault, s));
                 };
-                mb::run_sssp_coop(ctx->c, g->g, apps(g).sssp_coop, &src[i], 1, dev, &st, out_here ? nullptr : &copy);
+                mb::run_sssp_coop(ctx->c, g->g, cs, &src[i], 1, dev, &st, here ? nullptr : &copy);
             } else {
             // the distances' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {

@@ -90,6 +90,22 @@ struct DevBuf {
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
 
+// Whether reserve() finds device memory for what it reserves; where it does
+// not, give_back() returns what it got so far, and the caller takes a form
+// that needs less.
+template <class Reserve, class GiveBack>
+bool memory_for(Reserve &&reserve, GiveBack &&give_back) {
+    try {
+        reserve();
+        return true;
+    } catch (const CudaError &e) {
+        if (e.err != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();
+        give_back();
+        return false;
+    }
+}
+
 struct AppStates;  // per-app run state cached on a graph (capi.cu)
 
 struct Graph {

@@ -73,7 +73,7 @@ struct MsArgs {
     int64_t E;
     const int32_t *row, *col, *rrow, *rcol, *outdeg;
     unsigned long long *seen, *front[2], *nxt;
-    unsigned long long *keep;  // kMsKeep frontiers of V masks
+    unsigned long long *keep;  // kMsKeep frontiers of V masks, or null
     int32_t *touched;
     int32_t *qv[2];
     uint32_t *qo[2];
@@ -325,7 +325,7 @@ __device__ __forceinline__ void write_levels_warp(const MsArgs &a, int32_t v, un
 // once kMsKeep are kept.
 __device__ __forceinline__ unsigned long long *ms_keep(const MsArgs &a) {
     const int k = a.c->nkeep;
-    return k < kMsKeep ? a.keep + (size_t)k * a.V : nullptr;
+    return a.keep && k < kMsKeep ? a.keep + (size_t)k * a.V : nullptr;
 }
 
 // Counters of a pull (all 32 lanes; one set of atomics per warp).
@@ -585,9 +585,9 @@ __device__ void ms_begin(MsCtrl *c, int pull, int wide) {
     }
 }
 
-__device__ void ms_end(MsCtrl *c, int pull, int wide) {
+__device__ void ms_end(MsCtrl *c, int pull, int wide, bool keep) {
     if (wide) {
-        if (c->nkeep < kMsKeep) c->keep_lvl[c->nkeep++] = c->step + 1;
+        if (keep && c->nkeep < kMsKeep) c->keep_lvl[c->nkeep++] = c->step + 1;
         c->cur ^= 1;
         c->mode = 1;
         c->q[0] = c->q[1] = 0ull;
@@ -626,7 +626,7 @@ __global__ void k_ms_select(MsArgs a, int cap, cudaGraphConditionalHandle h_cont
         c->p.launches++;
         if (c->pending) {
             c->pending = 0;
-            ms_end(c, c->last_pull, c->last_wide);
+            ms_end(c, c->last_pull, c->last_wide, a.keep != nullptr);
         }
         c->iter++;
         if (c->iter > cap && !c->done) {
@@ -751,7 +751,6 @@ void MsBfsState::ensure(const Graph &g) {
     front[0].reserve(8 * vb);
     front[1].reserve(8 * vb);
     nxt.reserve(8 * vb);
-    keep.reserve(8 * vb * kMsKeep);
     touched.reserve(4 * vb);
     const size_t tiles = (size_t)(E / kTile) + 2;
     for (int i = 0; i < 2; i++) {
@@ -762,6 +761,8 @@ void MsBfsState::ensure(const Graph &g) {
     ctrl.reserve(sizeof(MsCtrl));
     stats.reserve(2 * sizeof(unsigned long long));
     srcs.reserve(64 * sizeof(int32_t));
+    // last: without memory for them every superstep stores its levels itself
+    memory_for([&] { keep.reserve(8 * vb * kMsKeep); }, [&] { keep.release(); });
     built = true;
 }
 

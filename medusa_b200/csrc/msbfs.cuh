@@ -17,6 +17,10 @@ struct MsBfsState {
     int32_t key_nsrc = 0;
     const float *key_mlp = nullptr;
     ~MsBfsState() { release(); }
+    void drop_keep() {
+        lg.reset();  // it has their address
+        keep.release();
+    }
     void release() {
         lg.reset();
         key_levels = nullptr;

@@ -580,7 +580,6 @@ static void union_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *s
         if (v < 0 || v >= b.graphs[i].V) fail(MB_ERR_INVALID, "batch: source vertex out of range");
         src[i] = (int32_t)(b.vbase[i] + v);
     }
-    union_build(ctx, b);
     BatchUnion &u = *b.uni;
     const Graph &g = u.g;
     PrState &pr = u.pr;
@@ -675,9 +674,12 @@ void batch_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *sources,
                int32_t *levels_dev, mb_stats *stats) {
     const int32_t n = (int32_t)b.graphs.size();
     if (pr_iters > 0 && b.total_V <= INT32_MAX && b.total_E <= INT32_MAX &&
-        ctx.tunable[MB_TUNE_BATCH_THREADS] < 0 && ctx.tunable[MB_TUNE_BATCH_EDGES_PER_CTA] < 0) {
-        union_run(ctx, b, pr_iters, sources, ranks_dev, levels_dev, stats);
-        return;
+        ctx.tunable[MB_TUNE_BATCH_THREADS] < 0 && ctx.tunable[MB_TUNE_BATCH_EDGES_PER_CTA] < 0 && !b.no_union) {
+        b.no_union = !memory_for([&] { union_build(ctx, b); }, [] {});
+        if (!b.no_union) {
+            union_run(ctx, b, pr_iters, sources, ranks_dev, levels_dev, stats);
+            return;
+        }
     }
     cudaStream_t s = ctx.stream;
     const int threads = (int)(ctx.tunable[MB_TUNE_BATCH_THREADS] > 0 ? ctx.tunable[MB_TUNE_BATCH_THREADS] : 256);

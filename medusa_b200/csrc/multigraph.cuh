@@ -40,6 +40,7 @@ struct BatchUnion {
 
 struct Batch {
     std::unique_ptr<BatchUnion> uni;
+    bool no_union = false;            // there was no memory for it
     std::vector<Graph> graphs;        // built with the single-graph builder
     std::vector<int64_t> vbase;       // n+1 prefix of vertex counts
     int64_t total_V = 0, total_E = 0;
@@ -49,6 +50,7 @@ struct Batch {
     ~Batch() { release(); }
     void release() {
         uni.reset();
+        no_union = false;
         for (auto &g : graphs) g.release();
         graphs.clear();
         desc.release(); team.release(); entries.release();

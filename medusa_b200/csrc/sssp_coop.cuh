@@ -22,7 +22,7 @@ struct SsspCoopState {
     int32_t room = 0;  // sources the buffers below hold at once
     DevBuf claim[2], far, q[2], qv[2], qs[2], tf[2], sh, front, srcs;
     ~SsspCoopState() { release(); }
-    void release() {
+    void release_room() {
         for (int i = 0; i < 2; i++) {
             claim[i].release();
             q[i].release();
@@ -31,11 +31,14 @@ struct SsspCoopState {
             tf[i].release();
         }
         far.release();
+        room = 0;
+    }
+    void release() {
+        release_room();
         sh.release();
         front.release();
         srcs.release();
         built = false;
-        room = 0;
     }
     void ensure(const Graph &g, int32_t nsrc);
 };
