@@ -1,12 +1,14 @@
-// barrier_word.h -- the word of the one-launch kernels' grid barriers.
+// barrier_word.h -- the counting of the one-launch kernels' grid barriers.
 //
-// The word counts arrivals over a whole run, and its top bit says that a wait
-// gave up.  It has 64 bits because a run has no bound of its own on its
-// supersteps: 592 CTAs pass 2^31 arrivals after 3.6 million of them, which a
-// BFS along a chain of vertices reaches, and a count that ran into the top bit
-// would end every wait without anyone having given up.
+// One word counts the arrivals of a whole run, another says that a wait gave
+// up.  A run has no bound of its own on its supersteps (592 CTAs pass 2^31
+// arrivals after 3.6 million of them, which a BFS along a chain of vertices
+// reaches), so the count wraps around, and a wait looks at its distance to the
+// target: arrivals are never further than a grid's CTAs from it.  (64-bit
+// arrivals cost 0.15 us more per barrier.)
 // No CUDA in here, so that a host program can run the same decisions.
 #pragma once
+#include <cstdint>
 
 #ifdef __CUDACC__
 #define MB_BAR_FN __host__ __device__ __forceinline__
@@ -16,13 +18,8 @@
 
 namespace mb {
 
-typedef unsigned long long BarWord;
-constexpr BarWord kBarGivenUp = 1ull << 63;
-enum BarWait { BAR_WAIT, BAR_PASSED, BAR_GIVEN_UP };
-
-// What a wait for `target` arrivals does after reading v.
-MB_BAR_FN BarWait bar_poll(BarWord v, BarWord target) {
-    return v >= kBarGivenUp ? BAR_GIVEN_UP : v >= target ? BAR_PASSED : BAR_WAIT;
-}
+// Arrivals at which barrier k of a run is passed; the first is 1.
+MB_BAR_FN uint32_t bar_target(uint32_t k, uint32_t grid) { return k * grid; }
+MB_BAR_FN bool bar_passed(uint32_t arrivals, uint32_t target) { return (int32_t)(arrivals - target) >= 0; }
 
 }  // namespace mb

@@ -21,7 +21,7 @@ struct CoopShared {  // device memory of a run, zero before it
     unsigned long long toq;  // the queue built from a pull's vertices
     unsigned long long reached;
     uint32_t ticket;
-    alignas(128) BarWord bar;  // polled: a line of its own
+    alignas(128) uint32_t bar[2];  // polled: a line of its own
 };
 
 struct CoopArgs {
@@ -41,7 +41,7 @@ struct CoopArgs {
 // ---- one cooperative grid -----------------------------------------------------------
 
 __device__ __forceinline__ bool coop_sync(const CoopArgs &a, uint32_t k) {
-    return coop_barrier(&a.sh->bar, k, a.polls, &a.out->err);
+    return coop_barrier(a.sh->bar, k, a.polls, &a.out->err);
 }
 
 struct CoopSmem {

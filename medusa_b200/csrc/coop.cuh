@@ -6,37 +6,35 @@
 
 namespace mb {
 
-__device__ __forceinline__ BarWord ld_acquire_gpu(const BarWord *p) {
-    BarWord v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid barrier of a cooperative launch: *bar counts arrivals over the run
-// (zero before it, barrier_word.h); barrier k, the first is 1, is passed when it
-// reaches k times the grid (k in 32 bits: the target's 64 would be one more
-// register of every thread across the whole run).  The wait is bounded: past `polls` polls the CTA gives the barrier
-// up, which ends every wait at once.  Whatever way a wait ends other than by
-// passing, the CTA records ERR_BARRIER in *err (host memory) and returns
+// Grid barrier of a cooperative launch: bar[0] counts arrivals over the run
+// (both words zero before it); barrier k, the first is 1, is passed when they
+// reach k times the grid (barrier_word.h).  The wait is bounded: past `polls`
+// polls the CTA says in bar[1] that it gave up, which the others see while they
+// wait.  Whatever way a wait ends other than by passing, the CTA records
+// ERR_BARRIER in *err (host memory) and returns
 // false; the caller leaves.  The acquire drops this SM's
 // stale L1 lines.  *bar wants a 128-byte line of its own: the waiting CTAs
 // poll it, and atomics on counters beside it queue up behind them (SSSP on
 // R-MAT 2^20 / 2^24: 1.27 -> 0.97 ms).
-__device__ __forceinline__ bool coop_barrier(BarWord *bar, uint32_t k, long polls, int32_t *err) {
+__device__ __forceinline__ bool coop_barrier(uint32_t *bar, uint32_t k, long polls, int32_t *err) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const BarWord target = (BarWord)k * gridDim.x;
+        const uint32_t target = bar_target(k, gridDim.x);
         __threadfence();
-        atomicAdd(bar, (BarWord)1);
-        BarWait w;
-        for (long it = 0; (w = bar_poll(ld_acquire_gpu(bar), target)) == BAR_WAIT; it++)
-            if (it >= polls) {
-                atomicOr(bar, kBarGivenUp);
-                w = BAR_GIVEN_UP;
+        atomicAdd(bar, 1u);
+        int ok = 0;
+        for (long it = 0;; it++) {
+            if (bar_passed(ld_acquire_gpu(bar), target)) {
+                ok = 1;
                 break;
             }
-        const int ok = w == BAR_PASSED;
+            if (it >= polls) {
+                atomicOr(bar + 1, 1u);
+                break;
+            }
+            if ((it & 63) == 63 && ld_acquire_gpu(bar + 1)) break;
+        }
         if (!ok) *(volatile int32_t *)err = ERR_BARRIER;
         __threadfence();
         s_ok = ok;

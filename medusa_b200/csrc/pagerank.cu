@@ -263,8 +263,8 @@ struct ResidentArgs {
     const int32_t *zv;  // vertices without in-edges
     const int2 *zpd;
     int32_t nz, iters;
-    BarWord *bar;       // arrivals (barrier_word.h), and 128 bytes further the CTAs done;
-                        // zero before the launch, which leaves them so
+    uint32_t *bar;      // the barrier's two words (coop.cuh), and 128 bytes further the CTAs
+                        // done; zero before the launch, which leaves them so
     int32_t *err;
     long polls;
 };
@@ -316,9 +316,9 @@ __global__ void __launch_bounds__(kResThreads, kResU == 8 ? 2 : 1) k_pr_resident
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&r.bar[16], (BarWord)1) == gridDim.x - 1) {  // no CTA waits any more
-        r.bar[0] = 0;
-        r.bar[16] = 0;
+    if (threadIdx.x == 0 && atomicAdd(&r.bar[32], 1u) == gridDim.x - 1) {  // no CTA waits any more
+        r.bar[0] = 0u;
+        r.bar[32] = 0u;
     }
 }
 
@@ -1221,7 +1221,7 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
             r.zpd = all.zpd.as<int2>();
             r.nz = all.nz;
             r.iters = iters;
-            r.bar = st.bar.as<BarWord>();
+            r.bar = st.bar.as<uint32_t>();
             r.err = res_err;
             r.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : 1l << 22;
             void *params[] = {&a, &r};

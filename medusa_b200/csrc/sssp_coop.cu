@@ -76,7 +76,7 @@ struct SShared {  // device memory of a run, zero before it
     SCtr ctr[3];
     unsigned long long reached, edges;
     uint32_t ticket;
-    alignas(128) BarWord bar;  // polled: a line of its own
+    alignas(128) uint32_t bar[2];  // polled: a line of its own
 };
 
 // kMulti: nsrc sources at once.  A vertex is then a (source, vertex) pair,
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
     const int64_t gt = (int64_t)blockIdx.x * kThreads + tid, gn = (int64_t)gridDim.x * kThreads;
     const float inf = inf_f();
     uint32_t barriers = 0;
-    auto sync = [&] { return coop_barrier(&a.sh->bar, ++barriers, a.polls, &a.out->err); };
+    auto sync = [&] { return coop_barrier(a.sh->bar, ++barriers, a.polls, &a.out->err); };
     int cur = 0, par = 0, it = 0, supersteps = 0, splits = 0, err = 0;
     const uint32_t pairs = kMulti ? (uint32_t)a.nsrc * (uint32_t)a.V : (uint32_t)a.V;
     for (int64_t p = gt; p < pairs; p += gn) a.dist[p] = kMedusaMax;

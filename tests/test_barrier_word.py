@@ -12,31 +12,24 @@ from conftest import ROOT
 SRC = r"""
 #include "barrier_word.h"
 using namespace mb;
-// Barriers [first, first + n) of a run on `grid` CTAs, each arrival followed by
-// a poll of every CTA that waits (one of them stands for all).  0: every wait
-// ended at its own last arrival; 1: one ended early; 2: one did not end;
-// 3: one gave up.
+// Barriers [first, first + n) of a run on `grid` CTAs, after each arrival a poll
+// of a CTA that waits at this barrier and of one that waits at the next.  0:
+// every wait ended at its own last arrival; 1: one ended early; 2: one did not end.
 extern "C" int run(long long first, long long n, int grid) {
     for (long long k = first; k < first + n; k++) {
-        BarWord word = (BarWord)k * grid;
-        const BarWord target = (BarWord)(k + 1) * grid;
+        uint32_t word = (uint32_t)((unsigned long long)k * grid);
+        const uint32_t here = bar_target((uint32_t)(k + 1), grid), next = bar_target((uint32_t)(k + 2), grid);
         for (int c = 0; c < grid; c++) {
             word += 1;
-            const BarWait w = bar_poll(word, target);
-            if (w == BAR_GIVEN_UP) return 3;
-            if (c + 1 < grid && w == BAR_PASSED) return 1;
-            if (c + 1 == grid && w != BAR_PASSED) return 2;
+            if (c + 1 < grid && bar_passed(word, here)) return 1;
+            if (c + 1 == grid && !bar_passed(word, here)) return 2;
+            if (bar_passed(word, next)) return 1;
         }
+        // CTAs that run ahead to the next barrier keep this one passed
+        for (int c = 0; c + 1 < grid; c++)
+            if (!bar_passed(word += 1, here)) return 2;
     }
     return 0;
-}
-// A wait that gives up: every later poll says so, whatever arrives.
-extern "C" int gives_up(long long arrivals, int grid) {
-    BarWord word = (BarWord)arrivals;
-    word |= kBarGivenUp;
-    for (int c = 0; c < grid; c++, word += 1)
-        if (bar_poll(word, word & ~kBarGivenUp) != BAR_GIVEN_UP) return 0;
-    return 1;
 }
 """
 
@@ -51,7 +44,6 @@ def word(tmp_path_factory):
                            "-o", lib])
     so = ctypes.CDLL(lib)
     so.run.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
-    so.gives_up.argtypes = [ctypes.c_longlong, ctypes.c_int]
     return so
 
 
@@ -60,8 +52,3 @@ def word(tmp_path_factory):
 def test_every_barrier_ends_with_its_own_last_arrival(word, grid, arrivals):
     first = max(arrivals // grid - 50, 0)
     assert word.run(first, 100, grid) == 0
-
-
-@pytest.mark.parametrize("arrivals", [0, 591, 1 << 31, 1 << 45])
-def test_a_barrier_given_up_ends_every_wait(word, arrivals):
-    assert word.gives_up(arrivals, 592) == 1
