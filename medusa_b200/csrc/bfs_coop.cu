@@ -23,6 +23,8 @@
 // hold a vertex's first edge, not its number: a push loads no offsets for its
 // tiles.  Levels go straight to the caller's device array; vertices not
 // reached get -1 at the end instead of a fill before.
+// Long runs of small frontiers go on in a second launch, of the kernel whose
+// CTA 0 runs them alone (coop_solo, bfs_coop_dev.cuh).
 // Measured (calls): R-MAT 2^10 / 2^13 161 -> 41 us; 2^24 / 2^28 596 -> 453 us
 // (a small superstep 6-7 us; the large ones push 57 G edges/s and pull at the
 // latency of their first list entries); first calls 5.9 -> 0.6 ms, for there is
@@ -172,8 +174,17 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_bfs_small(const __grid_con
     }
 }
 
+// kSolo: the rest of a run that the kernel without left (CoopResume).
+template <bool kSolo>
 __global__ void __launch_bounds__(kCoopThreads, kBfsCoopCtas) k_bfs_coop(CoopArgs a) {
     __shared__ CoopSmem sm;
+    uint32_t barriers = 0;
+    if (kSolo) {
+        if (threadIdx.x == 0) sm.nout = 0;
+        __syncthreads();
+        coop_bfs<true>(a, sm, barriers, 0u, 0ull, &a.sh->resume);
+        return;
+    }
     const int64_t gt = (int64_t)blockIdx.x * kCoopThreads + threadIdx.x, gn = (int64_t)gridDim.x * kCoopThreads;
     const int32_t rs0 = __ldg(&a.row[a.source]), deg0 = __ldg(&a.row[a.source + 1]) - rs0;
     for (int64_t w = gt; w < a.W; w += gn) a.vis[0][w] = w == (a.source >> 5) ? 1u << (a.source & 31) : 0u;
@@ -183,9 +194,8 @@ __global__ void __launch_bounds__(kCoopThreads, kBfsCoopCtas) k_bfs_coop(CoopArg
         a.level[a.source] = 0;
     }
     if (threadIdx.x == 0) sm.nout = 0;
-    uint32_t barriers = 0;
     if (!coop_sync(a, ++barriers)) return;
-    coop_bfs(a, sm, barriers, deg0 > 0 ? 1u : 0u, (uint32_t)deg0);
+    coop_bfs<false>(a, sm, barriers, deg0 > 0 ? 1u : 0u, (uint32_t)deg0, nullptr);
 }
 
 }  // namespace
@@ -261,6 +271,7 @@ void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int3
     cudaStream_t s = ctx.stream;
     volatile BfsCoopOut *out = (volatile BfsCoopOut *)ctx.ctrl_readback();
     out->err = 0;
+    out->handed = 0;
     CoopArgs a{};
     a.V = g.V;
     a.E = g.E;
@@ -285,19 +296,24 @@ void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int3
         a.tf[i] = st.tf[i].as<int32_t>();
     }
     a.sh = st.sh.as<CoopShared>();
-    int per_sm = 0;
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_coop, kCoopThreads, 0));
-    if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative BFS kernel does not fit on an SM");
-    // no more CTAs than tiles: fewer arrive at the barriers of small graphs
-    const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kBfsCoopCtas),
-                                            std::max<int64_t>(g.E / kCoopTile, 16));
+    auto launch = [&](const void *kernel) {
+        int per_sm = 0;
+        MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCoopThreads, 0));
+        if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "cooperative BFS kernel does not fit on an SM");
+        // no more CTAs than tiles: fewer arrive at the barriers of small graphs
+        const int grid = (int)std::min<int64_t>(ctx.num_sms * std::min(per_sm, kBfsCoopCtas),
+                                                std::max<int64_t>(g.E / kCoopTile, 16));
+        MB_CUDA(cudaMemsetAsync(st.sh.p, 0, offsetof(CoopShared, resume), s));
+        void *params[] = {&a};
+        MB_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kCoopThreads), params, 0, s));
+        MB_CUDA(cudaEventRecord(e1, s));
+        if (after) (*after)(s);
+        MB_CUDA(cudaStreamSynchronize(s));
+    };
     MB_CUDA(cudaEventRecord(e0, s));
-    MB_CUDA(cudaMemsetAsync(st.sh.p, 0, sizeof(CoopShared), s));
-    void *params[] = {&a};
-    MB_CUDA(cudaLaunchCooperativeKernel((const void *)k_bfs_coop, dim3(grid), dim3(kCoopThreads), params, 0, s));
-    MB_CUDA(cudaEventRecord(e1, s));
-    if (after) (*after)(s);
-    MB_CUDA(cudaStreamSynchronize(s));
+    launch((const void *)k_bfs_coop<false>);
+    const bool handed = !out->err && out->handed;
+    if (handed) launch((const void *)k_bfs_coop<true>);
     float ms = 0;
     MB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     if (out->err & ERR_BARRIER) fail(MB_ERR_TIMEOUT, "bfs: a grid barrier timed out");
@@ -310,7 +326,7 @@ void run_bfs_coop(Context &ctx, Graph &g, BfsCoopState &st, int32_t source, int3
         stats->device_ms = ms;
         stats->schedule_count[MB_SCHED_PUSH_EDGE_QUEUE] = out->pushes;
         stats->schedule_count[MB_SCHED_PULL_THREAD] = out->pulls;
-        stats->kernel_launches = 1;
+        stats->kernel_launches = 1 + handed;
         stats->edges_scanned = (int64_t)out->work;
     }
 }

@@ -13,6 +13,7 @@ constexpr int32_t kBfsSmallSources = 128;  // at most, in one launch
 struct BfsCoopOut {
     int32_t supersteps, pushes, pulls, err;
     unsigned long long reached, edges, work;
+    unsigned long long handed;  // left to the kernel with supersteps of one CTA
 };
 
 struct BfsCoopState {

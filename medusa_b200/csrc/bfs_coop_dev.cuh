@@ -16,12 +16,24 @@ struct alignas(128) CoopCtr {  // one per superstep in turn, three in all
     uint32_t n, pad;       // a pull's new vertices
     unsigned long long m;  // and their out-edges
 };
-struct CoopShared {  // device memory of a run, zero before it
+struct CoopSolo {  // what coop_solo leaves to the grid
+    uint32_t n, m, steps, pad;       // the frontier, and the supersteps run
+    unsigned long long edges, work;  // of those: out-edges found, edges looked at
+};
+struct CoopResume {  // where a run stands between two supersteps, the frontier in a queue
+    int32_t vb, cur, step, pushes, pulls;
+    uint32_t n, prev_n, pad;
+    unsigned long long m, edges, work;
+    int64_t unvisited;
+};
+struct CoopShared {  // device memory of a run, zero before each launch up to resume
     CoopCtr ctr[3];
+    CoopSolo solo[2];  // in turn
     unsigned long long toq;  // the queue built from a pull's vertices
     unsigned long long reached;
     uint32_t ticket;
     alignas(128) uint32_t bar[2];  // polled: a line of its own
+    alignas(128) CoopResume resume;
 };
 
 struct CoopArgs {
@@ -305,20 +317,165 @@ __device__ __forceinline__ void coop_toq(const CoopArgs &a, CoopSmem &sm, const 
     __syncthreads();  // sm.out is the pushes' next
 }
 
+// Supersteps of a frontier of at most a tile of out-edges, by this CTA alone:
+// a superstep of the grid costs 5 us, nearly all of it the barrier, however
+// small the frontier is.  Here __syncthreads stands between two of them, the
+// frontier stays in shared memory, and what is left is a chain of two L2 round
+// trips and a search.  Until the frontier has more out-edges, the rule asks for
+// a pull, nothing is left, or kSoloSteps supersteps have run: the other CTAs
+// wait at the barrier meanwhile, and their wait is bounded.
+// (Without it graphs of a long diameter with one hub, which the superstep loop
+// runs in its own one-CTA kernel, took twice as long as there: ms, loop / grid
+// alone / here, a line of 40,000 with a hub 77 / 147 / 27, grid 300 x 300 2.3 /
+// 3.0 / 1.95, 2^18 skewed R-MAT with 64 lines of 2000 7.3 / 11.7 / 3.1; 64 lines of
+// 10,000 in one batch, teams / grid alone / here, 28 / 53 / 14.5.)
+constexpr uint32_t kSoloSteps = 1024;
+// Small supersteps of the grid before it: one alone costs 3 us more here than
+// there, and a graph of a short diameter has but a few at each end (2^17 / 2^21
+// skewed R-MAT 74 us; 84 where one was enough).
+constexpr int kSoloAfter = 8;
+__device__ __forceinline__ bool coop_pull_next(unsigned long long m, int64_t unvisited, int32_t alpha, int32_t gamma,
+                                               int64_t E) {
+    return alpha > 0 && (int64_t)m * alpha > unvisited && (gamma == 0 || (int64_t)m * gamma >= E);
+}
+struct SoloArgs {  // in shared memory: what a call of its own needs, so that it takes no register of its caller
+    const int32_t *row, *col;
+    int32_t *level, *tf;  // tf, qn: the frontier it leaves
+    uint32_t *vis;
+    const uint2 *q;
+    uint2 *qn;
+    CoopSolo *out;
+    int64_t E, unvisited;
+    int32_t alpha, gamma, cap, step;
+    uint32_t n, m;
+};
+// A call, not inlined: inlined, its registers pushed the grid's pull and push
+// into spills.
+static __device__ __noinline__ void coop_solo(const SoloArgs &a, CoopSmem &sm) {
+    static_assert(sizeof(sm.off) + sizeof(sm.row) >= kCoopTile * sizeof(uint2) &&
+                      offsetof(CoopSmem, row) == sizeof(sm.off) && offsetof(CoopSmem, off) == 0,
+                  "two frontiers of a tile's vertices");
+    uint2 *buf[2] = {reinterpret_cast<uint2 *>(sm.off), sm.out};  // {first edge less off, off}
+    // queued vertices << 32 | their out-edges; a superstep fills the slot after
+    // its own, which the one before cleared, so one barrier is enough
+    __shared__ unsigned long long s_q[3];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint32_t n = a.n, m = a.m;
+    int64_t unvisited = a.unvisited;
+    const int32_t step = a.step;
+    for (uint32_t i = tid; i < n; i += kCoopThreads) {
+        const uint2 e = __ldcg(&a.q[i]);
+        buf[0][i] = make_uint2(e.x - e.y, e.y);
+    }
+    if (tid < 3) s_q[tid] = tid == 0 ? ((unsigned long long)n << 32) | m : 0ull;
+    __syncthreads();
+    uint32_t steps = 0;
+    unsigned long long edges = 0, work = 0;
+    int next = 1;
+    for (;;) {
+        const uint2 *f = steps & 1 ? buf[1] : buf[0];
+        uint2 *fn = steps & 1 ? buf[0] : buf[1];
+        const int after = next == 2 ? 0 : next + 1;
+        if (tid == 0) s_q[after] = 0ull;
+        const int32_t lvl = step + (int32_t)steps + 1;
+        work += m;
+        // a warp without edges goes to the barrier
+        for (uint32_t b = 0; b + (uint32_t)wid * 32u < m; b += kCoopThreads) {
+            const uint32_t e = b + tid;
+            int32_t v = -1, rs = 0;
+            uint32_t d = 0;
+            if (e < m) {
+                uint32_t lo = 0, hi = n;  // f[lo].y <= e < f[hi].y
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (f[mid].y <= e) lo = mid; else hi = mid;
+                }
+                v = __ldg(&a.col[(int32_t)(f[lo].x + e)]);
+                // the offsets load beside the claim, found or not
+                rs = __ldg(&a.row[v]);
+                const int32_t re = __ldg(&a.row[v + 1]);
+                const uint32_t bit = 1u << (v & 31);
+                if (!(atomicOr(&a.vis[v >> 5], bit) & bit)) {
+                    a.level[v] = lvl;
+                    d = (uint32_t)(re - rs);
+                }
+            }
+            const unsigned in = __ballot_sync(0xffffffffu, d > 0);
+            if (!in) continue;
+            const uint32_t incl = warp_incl_scan_u32(d);
+            unsigned long long base = 0;
+            if (lane == 31) base = atomicAdd(&s_q[next], ((unsigned long long)__popc(in) << 32) | incl);
+            base = __shfl_sync(0xffffffffu, base, 31);
+            if (d > 0) {
+                const uint32_t off = (uint32_t)base + incl - d;
+                fn[(uint32_t)(base >> 32) + __popc(in & lanemask_lt())] = make_uint2((uint32_t)rs - off, off);
+            }
+        }
+        __syncthreads();
+        steps++;
+        const unsigned long long c = s_q[next];
+        n = (uint32_t)(c >> 32);
+        m = (uint32_t)c;
+        edges += m;
+        unvisited -= (int64_t)m;
+        next = after;
+        if (n == 0 || m > kCoopTile || steps >= kSoloSteps || step + (int32_t)steps >= a.cap ||
+            coop_pull_next(m, unvisited, a.alpha, a.gamma, a.E))
+            break;
+    }
+    // the frontier to the other queue, with its tile table
+    const uint2 *f = steps & 1 ? buf[1] : buf[0];
+    for (uint32_t i = tid; i < n; i += kCoopThreads) {
+        const uint32_t off = f[i].y, end = i + 1 < n ? f[i + 1].y : m;
+        a.qn[i] = make_uint2(f[i].x + off, off);
+        const uint32_t t0 = (off + kCoopTile - 1) / kCoopTile, t1 = (end - 1) / kCoopTile;
+        for (uint32_t t = t0; t <= t1; t++) a.tf[t] = (int32_t)i;
+    }
+    if (tid == 0) {
+        a.out->n = n;
+        a.out->m = m;
+        a.out->steps = steps;
+        a.out->edges = edges;
+        a.out->work = work;
+    }
+    __syncthreads();  // sm.out is the pushes' next
+}
+
 // The supersteps from the frontier in q[0] (n vertices, m out-edges, levels and
 // visited bits set, tile table filled), then -1 for the vertices not reached and
 // the report; false if a barrier gave up.  sm.nout is 0 and the frontier
-// visible to every CTA (a barrier passed).
+// visible to every CTA (a barrier passed).  kSolo: small frontiers by one CTA;
+// without it a run that has come to them stops there (CoopResume), for a
+// kernel with it to go on from: both in one kernel cost the large supersteps
+// of R-MAT 2^24 / 2^28 4% in registers.
+template <bool kSolo>
 __device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32_t &barriers, uint32_t n,
-                                         unsigned long long m) {
+                                         unsigned long long m, const CoopResume *from) {
     __shared__ unsigned long long s_r[kCoopThreads / 32];
+    __shared__ SoloArgs s_solo;
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t gt = (int64_t)blockIdx.x * kCoopThreads + tid;
     int vb = 0, cur = 0, step = 0, pushes = 0, pulls = 0, err = 0;
+    uint32_t it = 0, solos = 0;  // supersteps of the grid, calls of coop_solo
+    int small = 0;               // supersteps in a row with a tile of edges or less
     bool queue = true;  // the frontier is in q[cur]; else what a pull added
     uint32_t prev_n = n;
     unsigned long long edges = m, work = 0;
     int64_t unvisited = a.E - (int64_t)m;
+    if (kSolo && from) {
+        vb = from->vb;
+        cur = from->cur;
+        step = from->step;
+        pushes = from->pushes;
+        pulls = from->pulls;
+        n = from->n;
+        prev_n = from->prev_n;
+        m = from->m;
+        edges = from->edges;
+        work = from->work;
+        unvisited = from->unvisited;
+        small = kSoloAfter;
+    }
     while (n > 0 && m > 0) {
         if (step >= a.cap) {
             err = ERR_STEP_CAP;
@@ -326,13 +483,44 @@ __device__ __forceinline__ bool coop_bfs(const CoopArgs &a, CoopSmem &sm, uint32
         }
         // the fixed rule (engine.cuh)
         bool pull;
-        if (queue)
-            pull = a.alpha > 0 && (int64_t)m * a.alpha > unvisited &&
-                   (a.gamma == 0 || (int64_t)m * a.gamma >= a.E);
-        else
-            pull = !((int64_t)n * a.beta < (int64_t)a.V && n < prev_n);
-        CoopCtr *ctr = &a.sh->ctr[step % 3];
-        if (gt == 0) a.sh->ctr[(step + 1) % 3] = CoopCtr{0ull, 0u, 0u, 0ull};  // last read before the barrier just passed
+        if (queue) pull = coop_pull_next(m, unvisited, a.alpha, a.gamma, a.E);
+        else pull = !((int64_t)n * a.beta < (int64_t)a.V && n < prev_n);
+        small = !pull && queue && m <= kCoopTile ? small + 1 : 0;
+        if (!kSolo && small > kSoloAfter) {
+            if (gt == 0) {
+                a.sh->resume = CoopResume{vb, cur, step, pushes, pulls, n, prev_n, 0u, m, edges, work, unvisited};
+                a.out->handed = 1ull;
+            }
+            return true;
+        }
+        if (kSolo && small > kSoloAfter) {
+            // read by every CTA before the barrier after the next solo
+            CoopSolo *so = &a.sh->solo[solos & 1];
+            if (blockIdx.x == 0) {
+                if (tid == 0)
+                    s_solo = SoloArgs{a.row,  a.col,     a.level, a.tf[cur ^ 1], a.vis[vb], a.q[cur], a.q[cur ^ 1],
+                                      so,     a.E,       unvisited, a.alpha,     a.gamma,   a.cap,    step,
+                                      n,      (uint32_t)m};
+                __syncthreads();
+                coop_solo(s_solo, sm);
+            }
+            if (!coop_sync(a, ++barriers)) return false;
+            prev_n = n = __ldcg(&so->n);
+            m = __ldcg(&so->m);
+            const uint32_t k = __ldcg(&so->steps);
+            const unsigned long long found = __ldcg(&so->edges);
+            edges += found;
+            unvisited -= (int64_t)found;
+            work += __ldcg(&so->work);
+            step += (int)k;
+            pushes += (int)k;
+            cur ^= 1;
+            solos++;
+            continue;
+        }
+        CoopCtr *ctr = &a.sh->ctr[it % 3];
+        it++;
+        if (gt == 0) a.sh->ctr[it % 3] = CoopCtr{0ull, 0u, 0u, 0ull};  // last read before the barrier just passed
         const int32_t lvl = step + 1;
         if (pull) {
             coop_pull(a, a.vis[vb], a.vis[vb ^ 1], lvl, ctr);

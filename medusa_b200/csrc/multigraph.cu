@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a)
     }
     if (!coop_sync(a.bfs, ++barriers)) return;
     const unsigned long long f = __ldcg(a.front);
-    coop_bfs(a.bfs, sm, barriers, (uint32_t)(f >> 32), (uint32_t)f);
+    coop_bfs<true>(a.bfs, sm, barriers, (uint32_t)(f >> 32), (uint32_t)f, nullptr);
 }
 
 }  // namespace
