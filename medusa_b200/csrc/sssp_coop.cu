@@ -46,10 +46,19 @@ constexpr uint32_t kBmMin = 1 << 20;  // 2^19 and less: 2-4% slower
 // Bucket width in mean weights.  0.5 / 0.7 / 0.85 / 1 / 1.5 / none, ms: mild R-MAT
 // 2^20 / 2^24 0.90 / 0.79 / 0.79 / 0.86 / 1.08 / 1.22; 2^23 / 10^8 3.31 / 3.80 / 3.43 /
 // 2.96 / 4.6 / 6.7; the skewed one 2^20 / 2^24 1.05 / 0.95 / 0.99 / 0.99 / 0.98 / 0.96.
-// Below kBucketMinE edges the supersteps saved by no buckets are worth more
-// (10^4 / 10^5: 0.118 without, 0.146 with).
-constexpr float kBucketWidth = 0.85f;
-constexpr int64_t kBucketMinE = 1 << 18;
+// Below kBucketMinE edges the supersteps that buckets add cost more than the
+// relaxations that they save, and where the edges per vertex are few there are
+// few relaxations to save.  ms, 0.85 / 2 / none / the superstep loop: mild R-MAT 2^16 x 8
+// edges per vertex 0.43 / 0.34 / 0.31 / 0.38, 2^18 x 4 0.65 / 0.52 / 0.41 / 0.45, 2^18 x 16
+// 0.52 / 0.55 / 0.54 / 0.56, 2^20 x 2 0.96 / 0.69 / 0.48 / 0.50, x 4 0.84 / 0.60 / 0.58 / 0.61, x 6
+// 0.81 / 0.68 / 0.74 / 0.72, x 8 0.79 / 0.79 / 0.94 / 0.88, 2^21 x 4 1.04 / 0.84 / 0.88 / 0.95, 2^24 x 4
+// 3.8 / 3.6 / 5.8 / 5.3, x 8 5.2 / 6.2 / 10.2 / 8.3; a tree of 2^19 with a hub 1.58 / 0.99 /
+// 0.39 / 0.47.
+constexpr int64_t kBucketMinE = 1 << 22;
+inline float single_width(const Graph &g) {
+    if (g.E < kBucketMinE) return 0.f;
+    return g.E < 7 * (int64_t)g.V ? 2.f : 0.85f;
+}
 // Bucket width in mean weights with several sources.  The more out-edges a
 // run's frontiers hold, the less a superstep's own cost matters, and the
 // narrower the best bucket; a sparse graph without hubs (roads) needs
@@ -553,7 +562,7 @@ void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sou
     a.out = (SsspCoopOut *)ctx.ctrl_readback();
     a.source = sources[0];
     a.cap = step_cap(ctx, ((int64_t)g.V * 4 + 16) * nsrc);
-    a.delta = multi ? pairs_width(g, nsrc) * st.mean_w : g.E >= kBucketMinE ? kBucketWidth * st.mean_w : 0.f;
+    a.delta = multi ? pairs_width(g, nsrc) * st.mean_w : single_width(g) * st.mean_w;
     a.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
     int per_sm = 0;
     const void *kernel = multi ? (const void *)k_sssp_coop<true> : (const void *)k_sssp_coop<false>;
