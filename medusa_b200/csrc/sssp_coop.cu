@@ -521,12 +521,18 @@ bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, in
         return false;
     const bool small = sssp_small(g);
     if (nsrc == 1 && !small && async_by_default(g, false)) return false;  // hub-free graphs: the asynchronous kernel
+    const bool skewed = g.max_outdeg > g.E / 1024;
+    // On the largest skewed graphs a few supersteps hold nearly all edges, which
+    // the loop's push and its asynchronous tail take faster, and buckets save
+    // nothing (ms, loop / here with buckets / without: R-MAT 2^24 / 2^28 5.7-5.9 /
+    // 6.1-7.0 / 7.5; 2^24 / 2^27 4.7 / 4.6 / 5.4; 2^23 / 2^27 4.0 / 3.8 / 4.2).
+    if (nsrc == 1 && skewed && g.E > ((int64_t)1 << 27)) return false;
     if (nsrc > 1) {
         if (ctx.tunable[MB_TUNE_MSS_DELTA] >= 0) return false;  // the lines' buckets
         // on a large graph with a huge hub most sources' frontiers meet in a
         // few supersteps, and a line of 32 distances per edge is the cheaper
         // form (skewed R-MAT 2^20 / 2^24 x 16: 7.0 against 8.8-9.9 ms)
-        if (g.max_outdeg > g.E / 1024 && g.E >= (1 << 22)) return false;
+        if (skewed && g.E >= (1 << 22)) return false;
     }
     st.ensure(g, 1);
     return st.weights_ok;
