@@ -529,10 +529,15 @@ bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, in
     if (nsrc == 1 && skewed && g.E > ((int64_t)1 << 27)) return false;
     if (nsrc > 1) {
         if (ctx.tunable[MB_TUNE_MSS_DELTA] >= 0) return false;  // the lines' buckets
-        // on a large graph with a huge hub most sources' frontiers meet in a
-        // few supersteps, and a line of 32 distances per edge is the cheaper
-        // form (skewed R-MAT 2^20 / 2^24 x 16: 7.0 against 8.8-9.9 ms)
-        if (skewed && g.E >= (1 << 22)) return false;
+        // On a graph with a huge hub most sources' frontiers meet in a few
+        // supersteps, and a line of 32 distances per edge is the cheaper form
+        // once there is enough of them: from 2^22 edges, or 2^25 of a run's sources
+        // together, on (ms, lines / pairs: skewed R-MAT 2^20 / 2^24 x 16 sources 7.0 /
+        // 8.8-9.9, 2^17 / 2^21 x 16 1.36 / 1.80, x 4 0.85 / 0.34, 2^16 / 2^20 x 32 1.05 / 1.40,
+        // x 16 0.99 / 0.69, 2^19 / 2^21 x 32 1.88 / 2.24; a star of 2^20 x 32 0.78 / 1.56, x 8
+        // 0.72 / 0.35).
+        const int64_t run = g.E * std::min(nsrc, kSsspCoopSources);  // out-edges of a run
+        if (skewed && !small && (g.E >= (1 << 22) || run >= (1 << 25))) return false;
     }
     st.ensure(g, 1);
     return st.weights_ok;
