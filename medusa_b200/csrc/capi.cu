@@ -1031,7 +1031,30 @@ int mb_sssp(mb_ctx *ctx, const mb_graph *gc, const int32_t *sources, int32_t nsr
                 const mb::EmitFn copy = [&](cudaStream_t s) {
                     MB_CUDA(cudaMemcpyAsync(out, dev, sizeof(float) * (size_t)V, cudaMemcpyDefault, s));
                 };
-                mb::run_sssp_coop(ctx->c, g->g, cs, &src[i], 1, dev, &st, here ? nullptr : &copy);
+                mb::SsspRest rest;
+                if (mb::run_sssp_coop(ctx->c, g->g, cs, &src[i], 1, dev, &st, here ? nullptr : &copy, &rest)) {
+                    const mb::EmitFn copy_rest = [&](cudaStream_t s) {
+                        MB_CUDA(cudaMemcpyAsync(out, apps(g).sssp.dist.p, sizeof(float) * (size_t)V,
+                                                cudaMemcpyDefault, s));
+                    };
+                    mb_stats more{};
+                    const mb_stats first = st;
+                    if (mb::memory_for(
+                            [&] {
+                                mb::run_sssp(ctx->c, g->g, apps(g).sssp, src[i], &more, mb::LOOP_ALL, -1, nullptr,
+                                             nullptr, &copy_rest, &rest);
+                            },
+                            [&] { apps(g).sssp.release(); })) {
+                        st = more;
+                        st.supersteps += first.supersteps;
+                        st.device_ms += first.device_ms;
+                        st.kernel_launches += first.kernel_launches;
+                        st.edges_scanned += first.edges_scanned;
+                        for (int k = 0; k < MB_NUM_SCHEDULES; k++) st.schedule_count[k] += first.schedule_count[k];
+                    } else {  // to the end as it began
+                        mb::run_sssp_coop(ctx->c, g->g, cs, &src[i], 1, dev, &st, here ? nullptr : &copy);
+                    }
+                }
             } else {
             // the distances' copy out rides on the run's own synchronisation
             const mb::EmitFn copy_out = [&](cudaStream_t s) {

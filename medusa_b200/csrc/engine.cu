@@ -102,7 +102,7 @@ void run_loop(Context &ctx, LoopSpec &sp, mb_stats *stats, int phase, int force,
     MB_CUDA(cudaEventCreate(&e0));
     MB_CUDA(cudaEventCreate(&e1));
     try {
-        if (ctx.use_graphs && !ctx.tracing) {
+        if (ctx.use_graphs && !ctx.tracing && !sp.host) {
             if (!st.lg.exec || st.owner != (const void *)&ctx || st.owner_mlp != (const void *)fa.mlp ||
                 st.owner_gen != ctx.tune_gen) {
                 const int cap = sp.cap, app = sp.app;

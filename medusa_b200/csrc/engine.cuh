@@ -729,6 +729,7 @@ struct LoopSpec {
     // its one host synchronisation (e.g. the copy of the run's output to the
     // caller), so that it costs no synchronisation of its own
     EmitFn after;
+    bool host = false;  // a whole run from the host's loop (a prologue of its own)
 };
 // The phases of a run driven one superstep at a time (mb_superstep): BEGIN
 // runs the prologue and picks the first superstep, STEP runs the picked one

@@ -28,6 +28,7 @@
 //     segmented min per destination, update
 //   7 full Bellman-Ford pull over every in-edge (the reference CPU form)
 #include "sssp.cuh"
+#include "sssp_coop.cuh"
 #include "bulk.cuh"
 
 namespace mb {
@@ -1113,6 +1114,40 @@ __global__ void k_sssp_init(SsspArgs a) {
     if (threadIdx.x == 0) choose_next(c, APP_SSSP, a.f.V, a.f.E);
 }
 
+// A run that the one-launch kernel left (SsspRest), after k_sssp_init: the rest
+// as a queue frontier for the asynchronous kernel.
+__global__ void k_adopt_begin(SsspArgs a, uint32_t n) {
+    Ctrl *c = a.f.ctrl;
+    count_launch(c);
+    c->q[0] = (unsigned long long)n << 32;
+    c->sched = MB_SCHED_PUSH_EDGE_QUEUE;
+    c->branch = kBranchAsync;
+    c->done = 0;
+    c->front_n = n;
+    c->front_m = 0;
+}
+__global__ void k_adopt(SsspArgs a, SsspRest r) {
+    Ctrl *c = a.f.ctrl;
+    count_launch(c);
+    int32_t *q = pick(a.f.qv, 0);
+    const int lane = threadIdx.x & 31;
+    const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gn = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = gt; i < r.n; i += gn) q[i] = r.near[i];
+    for (int64_t b = gt & ~31ll; b < a.f.V; b += gn) {
+        const int64_t v = b + lane;
+        const float d = v < a.f.V ? r.dist[v] : 0.f;
+        if (v < a.f.V) a.dist[v] = d;
+        // below T: relaxed at that distance, or in the near queue
+        const bool in = v < a.f.V && ((r.far[v >> 5] >> lane) & 1u) && d >= r.T;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (!m) continue;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(&c->q[0], (unsigned long long)__popc(m) << 32);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (in) q[(uint32_t)(base >> 32) + __popc(m & lanemask_lt())] = (int32_t)v;
+    }
+}
+
 __global__ void k_fill_dist(SsspArgs a) {
     count_launch(a.f.ctrl);
     float *d = a.dist;
@@ -1251,7 +1286,7 @@ static void async_chunks(Context &ctx, Graph &g, SsspState &st) {
 }
 
 void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *stats, int phase, int force,
-             int *cont, int32_t *bfs_levels, const EmitFn *after) {
+             int *cont, int32_t *bfs_levels, const EmitFn *after, const SsspRest *rest) {
     if (bfs_levels && (phase != LOOP_ALL || ctx.persist))
         fail(MB_ERR_INVALID, "asynchronous BFS: whole runs without the persistent grid only");
     st.ensure(g);
@@ -1371,8 +1406,13 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
         MB_CUDA(cudaMemsetAsync(a.nbm, 0, sizeof(uint32_t) * (size_t)a.f.W, s));
         if (a.adirty != a.nbm) MB_CUDA(cudaMemsetAsync(a.adirty, 0, sizeof(uint32_t) * (size_t)a.WA, s));
         k_sssp_init<<<1, 256, 0, s>>>(a);
+        if (rest) {
+            k_adopt_begin<<<1, 1, 0, s>>>(a, rest->n);
+            k_adopt<<<grid_vtx, 256, 0, s>>>(a, *rest);
+        }
         MB_CHECK_LAUNCH();
     };
+    sp.host = rest != nullptr;
     sp.branch = [&](int branch, cudaStream_t s) {
         if (branch == kBranchSplit) {
             k_far_split<<<grid_vtx, 256, 0, s>>>(a);

@@ -122,8 +122,10 @@ uint32_t sssp_bm_push_min(const Context &ctx, const Graph &g);
 // asynchronous kernel with every weight 1 (whole runs only; the state should
 // then serve BFS runs only, so that its loop graph stays the unit-weight one).
 // after: queued behind a whole run, before its host synchronisation.
+// rest: what run_sssp_coop left of a run from `source`, by the asynchronous kernel.
+struct SsspRest;
 void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *stats, int phase = 0,
              int force = -1, int *cont = nullptr, int32_t *bfs_levels = nullptr,
-             const EmitFn *after = nullptr);
+             const EmitFn *after = nullptr, const SsspRest *rest = nullptr);
 
 }  // namespace mb

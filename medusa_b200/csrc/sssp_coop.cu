@@ -6,7 +6,8 @@
 // IPDPS 2014) cut that to 1.3 to 2, but need three to five times the
 // supersteps, which the loop graph's 12-17 us per superstep made a loss.
 // Here the supersteps follow one another inside one cooperative grid with one
-// barrier each (6-8 us for a small one), so the buckets pay.
+// barrier each (6-8 us for a small one), so the buckets pay.  Where the steps
+// stay small for long, the asynchronous kernel takes the rest (SsspRest).
 //
 // A superstep relaxes the out-edges of the near queue.  A vertex whose
 // distance drops below the threshold T joins the next queue, once per
@@ -74,6 +75,17 @@ inline float pairs_width(const Graph &g, int32_t nsrc) {
     return e >= (double)(1 << 23) ? 2.5f : 5.f;
 }
 
+// The run stops when kHandSteps of its steps in a row have relaxed fewer than
+// kHandEdges edges each on average: on a graph of a long diameter a step here
+// is 5.4 us of barrier, where the asynchronous kernel follows each path by
+// itself.  ms, the superstep loop with that kernel for its tail / here to the end /
+// stopping: skewed R-MAT 2^18 with 64 lines of 2000 7.1 / 45 / 6.7, a line of 1.3 10^5
+// with a hub 412 / 588 / 200, the 1448^2 grid with a hub of 1000 3.4 / 4.1 / 2.4.  R-MAT
+// and uniform graphs have 10^5 edges a step and more in any such row; a ring of
+// 2 10^5 vertices with 80 edges each (1.2 10^4) is faster here (3.4; 8.6 in the loop).
+constexpr int kHandSteps = 64;
+constexpr uint32_t kHandEdges = 4096;
+
 __device__ __forceinline__ float inf_f() { return __uint_as_float(kInf); }
 
 struct alignas(128) SCtr {  // one per iteration in turn, three in all
@@ -108,6 +120,7 @@ struct SArgs {
     SsspCoopOut *out;  // host memory
     int32_t source, cap;
     float delta;       // 0: no buckets
+    bool hand;         // the run may stop (SsspRest)
     long polls;
 };
 
@@ -403,11 +416,27 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_sssp_coop(SArgs a) {
     unsigned long long work = 0;
     float T = a.delta > 0.f ? a.delta : inf, fmin = inf;
     bool far = false;
+    uint32_t mark = 0;  // work at the start of the row of steps
     for (;; it++) {
         if (n == 0 && !far) break;
         if (it >= a.cap) {
             err = ERR_STEP_CAP;
             break;
+        }
+        if (!kMulti && a.hand && it % kHandSteps == 0 && it > 0) {
+            if ((uint32_t)work - mark < kHandSteps * kHandEdges) {
+                if (gt == 0) {
+                    a.out->supersteps = supersteps;
+                    a.out->splits = splits;
+                    a.out->work = work;
+                    a.out->n = n;
+                    a.out->cur = cur;
+                    a.out->T = T;
+                    a.out->handed = 1;
+                }
+                return;
+            }
+            mark = (uint32_t)work;
         }
         SCtr *ctr = &a.sh->ctr[it % 3];
         // last read before the barrier just passed
@@ -543,12 +572,13 @@ bool sssp_coop_applies(const Context &ctx, const Graph &g, SsspCoopState &st, in
     return st.weights_ok;
 }
 
-void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
-                   mb_stats *stats, const EmitFn *after) {
+bool run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sources, int32_t nsrc, float *dist,
+                   mb_stats *stats, const EmitFn *after, SsspRest *rest) {
     static_assert(sizeof(SsspCoopOut) <= Context::kSmallBytes - Context::kCtrlOff, "readback too small");
     cudaStream_t s = ctx.stream;
     volatile SsspCoopOut *out = (volatile SsspCoopOut *)ctx.ctrl_readback();
     out->err = 0;
+    out->handed = 0;
     st.ensure(g, nsrc);
     const bool multi = nsrc > 1;
     SArgs a{};
@@ -575,6 +605,8 @@ void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sou
     a.cap = step_cap(ctx, ((int64_t)g.V * 4 + 16) * nsrc);
     a.delta = multi ? pairs_width(g, nsrc) * st.mean_w : single_width(g) * st.mean_w;
     a.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
+    // a caller's step cap counts supersteps, which the asynchronous kernel has none of
+    a.hand = rest && ctx.tunable[MB_TUNE_STEP_CAP] < 0;
     int per_sm = 0;
     const void *kernel = multi ? (const void *)k_sssp_coop<true> : (const void *)k_sssp_coop<false>;
     MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
@@ -605,6 +637,10 @@ void run_sssp_coop(Context &ctx, Graph &g, SsspCoopState &st, const int32_t *sou
         stats->kernel_launches = 1;
         stats->edges_scanned = (int64_t)out->work;
     }
+    if (!out->handed) return false;
+    *rest = SsspRest{dist, a.qv[out->cur], out->n, a.far, out->T};
+    if (stats) stats->edges_traversed = stats->vertices_reached = 0;  // counted at the end
+    return true;
 }
 
 }  // namespace mb
