@@ -359,7 +359,8 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
 #define MB_TUNE_BATCH_EDGES_PER_CTA 5 /* many-graph kernel: a graph gets one CTA per this
                                          many edges + vertices (default 65536) */
 #define MB_TUNE_PR_LIGHT_VPL 6 /* PageRank: groups of 32 vertices of at most 8 in-edges
-                                  that a warp folds at once, 1, 2 or 4 (default 1) */
+                                  that a warp folds at once, 1, 2 or 4 (default 1; 2 with fewer
+                                  than 8 edges per vertex) */
 #define MB_TUNE_PR_SHORT_PAIR 7 /* PageRank: heavy-vertex blocks of <= 512 in-edges
                                    folded at once by one warp, 1, 2 or 4 (default 2) */
 #define MB_TUNE_BFS_ALPHA 8 /* BFS fixed rule: bottom-up once frontier out-edges x alpha

@@ -1108,11 +1108,15 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
         return ctx.num_sms * std::max(per_sm, 1);
     };
     const int grid_pull = resident((const void *)k_pr_pull<true>, kPrThreads);
-    // short sliced-ELL groups a warp takes at once: the tunable, else 1 (1 / 2 / 4,
-    // us per superstep: uniform 9 10^5 with 4 / 8 / 16 edges per vertex 17.9 / 16.8 /
-    // 20.7, 30.4 / 30.7 / 38.7, 56.6 / 58.7 / 62.7; R-MAT 4 10^6 / 6 10^7 232 / 233 / 238,
-    // 3 10^6 / 3 10^7 80 / 78 / 81)
-    const int vpl = ctx.tunable[MB_TUNE_PR_LIGHT_VPL] > 0 ? (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL] : 1;
+    // short sliced-ELL groups a warp takes at once: the tunable, else 1, and 2 below
+    // 8 edges per vertex, where one leaves a warp few gathers (1 / 2 / 4, us per
+    // superstep: uniform 9 10^5 with 4 / 8 / 16 edges per vertex 17.9 / 16.8 / 20.7,
+    // 30.4 / 30.7 / 38.7, 56.6 / 58.7 / 62.7; R-MAT 4 10^6 / 6 10^7 232 / 233 / 238, 3 10^6 /
+    // 3 10^7 80 / 78 / 81; the 1448^2 grid 23.7 / 16.2 / 19.9, the 128^3 torus 24.6 / 17.5 /
+    // 23.2, a binary tree of 2^19 6.9 / 5.2 / 6.6)
+    const int vpl = ctx.tunable[MB_TUNE_PR_LIGHT_VPL] > 0 ? (int)ctx.tunable[MB_TUNE_PR_LIGHT_VPL]
+                    : g.E < 8 * (int64_t)g.V               ? 2
+                                                           : 1;
     const int pair = ctx.tunable[MB_TUNE_PR_SHORT_PAIR] > 0 ? (int)ctx.tunable[MB_TUNE_PR_SHORT_PAIR]
                                                              : kShortPairDefault;
     // each variant's grid is its own resident block count (registers differ)
