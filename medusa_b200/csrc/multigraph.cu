@@ -329,7 +329,47 @@ struct UnionArgs {
     int32_t nsrc;
     unsigned long long *front;  // their queue's count << 32 | out-edges
     CoopArgs bfs;
+    bool by_graph;       // the BFS graph by graph (union_by_graph), in `one`
+    MultiArgs one;
 };
+
+// The BFS of every graph by one CTA, as a team of one.  A level then is a
+// __syncthreads where the union's is a grid barrier, for a frontier that is
+// small in each graph but not in all of them together (sparse graphs of a long
+// diameter; ms, one superstep and the BFS, union / here: 200 grids of 30 x 30 0.53
+// / 0.36, 16 of 100 x 100 1.28 / 1.00).
+static __device__ __noinline__ void union_by_graph(const MultiArgs &a, CoopShared *sh, BfsCoopOut *out) {
+    __shared__ int s_g;
+    unsigned long long reached = 0, edges = 0;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_g = (int)atomicAdd(&a.work[0], 1u);
+        __syncthreads();
+        const int i = s_g;
+        if (i >= a.nentries) break;
+        const GDesc d = a.desc[i];
+        TeamState *ts = &a.team[i];
+        Member m;
+        m.k = 0;
+        m.t = 1;
+        m.tid = threadIdx.x;
+        m.nthr = blockDim.x;
+        m.warp = threadIdx.x >> 5;
+        m.nwarp = blockDim.x >> 5;
+        bfs_phase(a, d, ts, m);
+        __syncthreads();
+        reached += __ldcg(&ts->reached);
+        edges += __ldcg(&ts->reached_edges);
+    }
+    if (threadIdx.x != 0) return;
+    atomicAdd(&sh->reached, reached);
+    atomicAdd(&sh->toq, edges);  // unused otherwise here
+    __threadfence();
+    if (atomicAdd(&sh->ticket, 1u) == gridDim.x - 1) {
+        out->reached = atomicAdd(&sh->reached, 0ull);
+        out->edges = atomicAdd(&sh->toq, 0ull);
+    }
+}
 
 constexpr int kUnionCtas = 3;
 constexpr int kUnionU = 8;
@@ -418,6 +458,13 @@ __global__ void __launch_bounds__(kCoopThreads, kUnionCtas) k_union(UnionArgs a)
             u = warps + __shfl_sync(0xffffffffu, t, 0);
         }
         if (!coop_sync(a.bfs, ++barriers)) return;
+    }
+    if (a.by_graph) {
+        __shared__ MultiArgs s_one;
+        if (tid == 0) s_one = a.one;
+        __syncthreads();
+        union_by_graph(s_one, a.bfs.sh, a.bfs.out);
+        return;
     }
     // 2. one BFS from every graph's source; CTA 0 makes the frontier
     if (blockIdx.x == 0 && tid < 32) {
@@ -576,6 +623,30 @@ static void union_build(Context &ctx, Batch &b) {
     b.uni = std::move(u);
 }
 
+// Graph i as the teams' kernel reads it, without its team and source.
+static GDesc graph_desc(const Batch &b, int32_t i) {
+    const Graph &g = b.graphs[i];
+    GDesc d{};
+    d.V = g.V;
+    d.E = (int32_t)g.E;
+    d.row = g.row.as<int32_t>();
+    d.col = g.col.as<int32_t>();
+    d.rrow = g.rrow.as<int32_t>();
+    d.rcol = g.rcol.as<int32_t>();
+    d.vbase = b.vbase[i];
+    return d;
+}
+
+// Whether the union's BFS goes graph by graph: graphs that had a CTA each in
+// the teams' form, without hubs and with 2 to 6 edges per vertex (grids).  Lines and
+// trees have fewer: their frontiers stay small in the union too (64 lines of 1000
+// 1.45 ms there, 3.4 by graph), and denser graphs have short diameters.
+static bool union_bfs_by_graph(const Batch &b) {
+    for (const Graph &g : b.graphs)
+        if (g.E + g.V > (1 << 16) || g.max_outdeg > 64 || g.E < 2 * (int64_t)g.V || g.E > 6 * (int64_t)g.V) return false;
+    return b.graphs.size() > 1;
+}
+
 static void union_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *sources, float *ranks_dev,
                       int32_t *levels_dev, mb_stats *stats) {
     const int32_t n = (int32_t)b.graphs.size();
@@ -644,6 +715,26 @@ static void union_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *s
     f.gamma = kBfsGammaDefault;
     f.cap = INT32_MAX;  // every superstep reaches a vertex
     f.polls = ctx.tunable[MB_TUNE_WAIT_POLLS] >= 0 ? (long)ctx.tunable[MB_TUNE_WAIT_POLLS] : kBarrierSpins;
+    a.by_graph = union_bfs_by_graph(b);
+    std::vector<GDesc> desc;
+    if (a.by_graph) {
+        for (int32_t i = 0; i < n; i++) {
+            desc.push_back(graph_desc(b, i));
+            desc.back().source = sources ? sources[i] : 0;
+        }
+        MB_CUDA(cudaMemcpyAsync(b.desc.p, desc.data(), sizeof(GDesc) * n, cudaMemcpyHostToDevice, s));
+        MB_CUDA(cudaMemsetAsync(b.team.p, 0, sizeof(TeamState) * n, s));
+        MB_CUDA(cudaMemsetAsync(b.work.p, 0, 4 * sizeof(unsigned), s));
+        a.one.desc = b.desc.as<GDesc>();
+        a.one.team = b.team.as<TeamState>();
+        a.one.nentries = n;
+        a.one.queue[0] = b.queue[0].as<int32_t>();
+        a.one.queue[1] = b.queue[1].as<int32_t>();
+        a.one.level = levels_dev;
+        a.one.work = b.work.as<unsigned>();
+        a.one.wait_polls = f.polls;
+        out->edges = out->reached = 0;
+    }
     int per_sm = 0;
     MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_union, kCoopThreads, 0));
     if (per_sm < 1) fail(MB_ERR_UNSUPPORTED, "batch kernel does not fit on an SM");
@@ -702,13 +793,7 @@ void batch_run(Context &ctx, Batch &b, int32_t pr_iters, const int32_t *sources,
     for (int32_t i = 0; i < n; i++) {
         const Graph &g = b.graphs[i];
         GDesc &d = desc[i];
-        d.V = g.V;
-        d.E = (int32_t)g.E;
-        d.row = g.row.as<int32_t>();
-        d.col = g.col.as<int32_t>();
-        d.rrow = g.rrow.as<int32_t>();
-        d.rcol = g.rcol.as<int32_t>();
-        d.vbase = b.vbase[i];
+        d = graph_desc(b, i);
         d.team = (int32_t)std::min<int64_t>(std::max<int64_t>(1, (g.E + g.V + epc - 1) / epc), grid);
         d.source = sources ? sources[i] : 0;
         if (d.source < 0 || d.source >= g.V) fail(MB_ERR_INVALID, "batch: source vertex out of range");
