@@ -314,6 +314,12 @@ constexpr int kMsHubU = 4;
 __device__ __forceinline__ void write_levels_warp(const MsArgs &a, int32_t v, unsigned long long bits,
                                                   int32_t lvl) {
     unsigned long long any = warp_or64(bits);
+    if (!any) return;
+    // a few sources of their own in each lane: the lanes side by side
+    if (2 * __reduce_max_sync(0xffffffffu, __popcll(bits)) < __popcll(any)) {
+        write_levels(a, v, bits, lvl);
+        return;
+    }
     while (any) {
         const int s = __ffsll((long long)any) - 1;
         any &= any - 1;
@@ -367,6 +373,11 @@ __global__ void __launch_bounds__(256) k_ms_pull(MsArgs a) {
         const bool in = v < a.V;
         const unsigned long long old = in ? a.seen[v] : ~0ull;
         const unsigned long long need = live & ~old;
+        if (!__any_sync(0xffffffffu, need != 0ull)) {
+            if (in) front_nx[v] = 0ull;
+            if (in && keep) keep[v] = 0ull;
+            continue;
+        }
         unsigned long long acc = 0ull;
         int32_t j = 0, je = 0;
         bool hub = false;
@@ -798,6 +809,10 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
     a.c = st.ctrl.as<MsCtrl>();
     const size_t vb = (size_t)g.V;
     const int gv = ctx.num_sms * 8, gp = ctx.num_sms * 8;
+    // the pull's resident CTAs and no more: its warps share the vertices evenly
+    int per_sm = 0;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_pull, 256, 0));
+    const int gpull = ctx.num_sms * std::max(per_sm, 1);
     // every superstep reaches at least one new (vertex, source) pair
     const int cap = step_cap(ctx, (int64_t)g.V + 8);
 
@@ -812,7 +827,7 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
     };
     auto branch = [&](int b, cudaStream_t cs) {
         if (b == kMsBranchPull) {
-            k_ms_pull<<<gv, 256, 0, cs>>>(a);
+            k_ms_pull<<<gpull, 256, 0, cs>>>(a);
             if (g.max_indeg > kMsHubMin) k_ms_pull_hub<<<ctx.num_sms * 2, kMsHubThreads, 0, cs>>>(a);
         } else {
             if (b == kMsBranchDensePush || b == kMsBranchDenseWidePush) k_ms_dense2q<<<gv, 256, 0, cs>>>(a);
