@@ -65,8 +65,12 @@ constexpr int kMsKeep = 8;
 // touches so many vertices that a list of them (an atomic append each, and
 // a commit in list order with a scattered store per level) costs more than
 // one pass over all masks.  64 sources on R-MAT 2^22 / 2^26, the superstep
-// with 1.7M frontier edges: 0.48 ms as a list, 0.10 wide.
-constexpr int kMsWideDiv = 8;
+// with 1.7M frontier edges: 0.48 ms as a list, 0.10 wide.  But only where many
+// sources meet in a vertex, or the edges outnumber the vertices: each costs
+// three passes over all masks, and where every frontier vertex has one source
+// (grids, tori, rings) a list is the shorter (us per superstep, list / wide: 8 sources
+// on the 128^3 torus 56 / 94, 32 on a 700^2 grid 22 / 45, 8 on a ring of 2^20 31 / 36).
+constexpr int kMsWideDiv = 8, kMsWideWork = 16;
 
 struct MsArgs {
     int32_t V;
@@ -80,6 +84,7 @@ struct MsArgs {
     int32_t *tf[2];
     int32_t *levels;  // [nsrc][V]
     int32_t nsrc;
+    bool hubs;               // an out-degree above 64
     unsigned long long all;  // mask of the batch's sources
     const float *mlp;        // batched-traversal scheduler weights (nullptr: untrained)
     MsCtrl *c;
@@ -684,7 +689,8 @@ __global__ void k_ms_select(MsArgs a, int cap, cudaGraphConditionalHandle h_cont
     }
     const int pull = pull_family(s);
     c->sched = pull ? MB_SCHED_PULL_THREAD : MB_SCHED_PUSH_EDGE_QUEUE;
-    const int wide = pull || (unsigned long long)c->active_edges * kMsWideDiv >= (unsigned long long)a.V;
+    const unsigned long long fe = c->active_edges, V = (unsigned long long)a.V;
+    const int wide = pull || (fe * kMsWideDiv >= V && (fe >= V || (a.hubs && fe * a.nsrc >= kMsWideWork * V)));
     c->branch = pull ? kMsBranchPull
                      : wide ? (c->mode == 1 ? kMsBranchDenseWidePush : kMsBranchWidePush)
                             : (c->mode == 1 ? kMsBranchDensePush : kMsBranchPush);
@@ -804,6 +810,7 @@ void run_msbfs(Context &ctx, Graph &g, MsBfsState &st, const int32_t *sources, i
     }
     a.levels = levels_dev;
     a.nsrc = nsrc;
+    a.hubs = g.max_outdeg > 64;
     a.all = nsrc == 64 ? ~0ull : ((1ull << nsrc) - 1ull);
     a.mlp = ctx.model(MB_MODEL_BATCHED);
     a.c = st.ctrl.as<MsCtrl>();
