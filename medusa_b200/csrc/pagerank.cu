@@ -1193,7 +1193,12 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     const void *res_fn = (const void *)k_pr_resident<16>;
     int32_t *res_err = (int32_t *)ctx.ctrl_readback();
     *(volatile int32_t *)res_err = 0;
-    if (!unfused && iters > 1 && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
+    // A superstep of a small sparse graph is shorter than the barrier between two
+    // (us for ten, one launch / one each: 300 vertices with 2 / 4 edges 28 / 24, 28 / 24,
+    // 3000 with 2 / 4 / 8 / 16 30 / 27, 30 / 28, 31 / 29, 34 / 40, 10^4 with 2 / 4 32 / 30, 32 / 30,
+    // 4 10^4 34 / 34, 36 / 37, 7 10^4 35 / 38, 40 / 40).
+    const bool by_launch = g.E < (1 << 15) && g.E < 12 * (int64_t)g.V;
+    if (!unfused && iters > 1 && !by_launch && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
         // small graphs in smaller CTAs, one per SM: 177 groups in 6 CTAs of 32
         // warps were bound by 6 SMs' gathers
         const int64_t warps = std::min<int64_t>(kResThreads / 32,

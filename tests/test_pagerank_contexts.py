@@ -35,7 +35,7 @@ def test_a_wait_that_gives_up_is_the_running_contexts(order):
     b.set_pagerank_order(order)
     a.set_tunable("batch_threads", 256)  # as many changes as b's, and none to a run
     b.set_tunable("wait_polls", 0)
-    g = make(a, 4000, 30000, 1)
+    g = make(a, 4000, 60000, 1)
     want, _ = g.pagerank(7)
     gb = lend(b, g)
     with pytest.raises(api.MedusaError):
@@ -51,7 +51,7 @@ def test_a_wait_that_gives_up_is_the_running_contexts(order):
 
 def test_the_graph_outlives_the_context_that_captured():
     a, b = api.Context(0), api.Context(0)
-    g = make(a, 4000, 30000, 2)
+    g = make(a, 4000, 60000, 2)
     want, _ = g.pagerank(7)
     gb = lend(b, g)
     a.close()
