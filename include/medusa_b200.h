@@ -8,7 +8,7 @@
  * One mb_ctx per host thread; a context owns one CUDA stream and all device
  * scratch; a graph is device-resident until mb_graph_destroy.  Device buffers
  * come from a memory pool that the library keeps for the next ones: up to 1/16
- * of the device's memory, at most 2 GB of it unused once a graph or a batch has
+ * of the device's memory, at most 3 GB of it unused once a graph or a batch has
  * been destroyed, nothing after the last context.
  *
  * Sentinels match the reference: BFS unreached level = -1

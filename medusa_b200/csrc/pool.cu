@@ -36,7 +36,10 @@ struct DevicePool {
 std::mutex g_mutex;
 constexpr int kMaxDevices = 64;
 constexpr size_t kPoolMax = (size_t)256 << 20;
-constexpr uint64_t kPoolSpare = (uint64_t)2 << 30;  // building 2^21 / 4 10^7 and one SSSP on it take 1.9 GB
+// What building a graph of pooled arrays and one SSSP on it take at most: a
+// dozen buffers of kPoolMax.  With 2 GB a graph of 2^20 / 6.3 10^7 was built in 12.2 ms
+// and destroyed in 5.2, with this in 7.1 and 0.1.
+constexpr uint64_t kPoolSpare = (uint64_t)3 << 30;
 DevicePool g_pools[kMaxDevices];
 
 void drop_pool(DevicePool &d) {

@@ -1,4 +1,4 @@
-"""Device memory that the library holds after its graphs are gone: 2 GB at most
+"""Device memory that the library holds after its graphs are gone: 3 GB at most
 while a context lives, none after the last one."""
 import gc
 
@@ -19,11 +19,11 @@ def test_memory_of_destroyed_graphs_goes_back():
     torch.cuda.synchronize()
     ctx.graph_from_edges(1000, src[:100] % 1000, dst[:100] % 1000).close()
     free0 = torch.cuda.mem_get_info()[0]
-    graphs = [ctx.graph_from_edges(1 << 20, src, dst) for _ in range(10)]
+    graphs = [ctx.graph_from_edges(1 << 20, src, dst) for _ in range(12)]
     held = free0 - torch.cuda.mem_get_info()[0]
-    assert held > 3 << 30  # ten CSR pairs: 4 GB and more
+    assert held > 4 << 30  # twelve CSR pairs: 5 GB and more
     for g in graphs:
         g.close()
     left = free0 - torch.cuda.mem_get_info()[0]
-    assert left <= (2 << 30) + (64 << 20)
+    assert left <= (3 << 30) + (64 << 20)
     ctx.close()
