@@ -40,8 +40,8 @@
 //    bit, so every warp leaves.  (Two counter atomics per batch of claims, one
 //    of them awaited, cost the 1448^2 grid 0.68 against 0.64 ms for BFS, 1.13
 //    against 1.00 for SSSP, a line of 40,000 95 against 81.);
-//  - a warp that finds nothing below T reports itself idle, and (idle_back)
-//    takes that back when it finds work in the same phase (the CTA's warps in shared
+//  - a warp that finds nothing below T reports itself idle, and (idle_back,
+//    the first phases) takes that back when it finds work in the same phase (the CTA's warps in shared
 //    memory, then one global count of CTAs); when every CTA is idle at once,
 //    T rises by delta (or to the least distance seen above T plus delta) and
 //    the next phase opens.  T only orders the claims: every order reaches the
@@ -71,6 +71,12 @@ constexpr int kAsyncU = MB_ASYNC_U;  // strips of 32 edges in flight per warp
 // The idle counts start here: one CTA's minus may be performed before its plus,
 // and the sign bit has to stay zero.
 constexpr uint32_t kAsyncIdle0 = 1u << 16;
+// Reports are taken back in the first phases only, where the frontiers grow.  On
+// a graph of a long diameter every phase after them has some warp at work, and
+// waiting for all to be idle at once makes each longer (ms, all phases / these /
+// none: rings of 2^20 with 16 edges per vertex 10.5 / 9.3 / 9.1, of 5 10^5 with 60
+// 91 / 79 / 77; uniform 2^20 / 2^24, four phases in all, 0.64 / 0.65 / 0.79).
+constexpr uint32_t kAsyncBackPhases = 8;
 constexpr long kAsyncSpins = 1l << 22;
 constexpr uint32_t kInfBits = 0x7f800000u;
 static_assert(kAsyncSlots == 32, "one work counter slot per lane");
@@ -322,9 +328,11 @@ __device__ __forceinline__ uint32_t async_busy(AsyncState *S, uint32_t *s_idle, 
     return atomicSub((unsigned *)&S->idle[ph & 1].v, 1u) >> 31;
 }
 
+// Five CTAs per SM: left to itself the compiler takes 61 registers for one of the
+// two, which leaves four (uniform 2^20 / 2^24 0.74 ms against 0.65).
 // kUnit: every weight 1 (BFS levels as hop distances; a.wt is not read).
 template <bool kUnit>
-__global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int cap) {
+__global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int cap) {
     const unsigned FULL = 0xffffffffu;
     Ctrl *c = a.f.ctrl;
     count_launch(c);
@@ -491,7 +499,7 @@ __global__ void __launch_bounds__(kAsyncThreads) k_sssp_async(SsspArgs a, int ca
                 if (lane == 0) old = atom_and_acquire(&dirty[w], ~mask);
                 const uint32_t claimed = __shfl_sync(FULL, old, 0) & mask;
                 if (!claimed) continue;
-                if (a.idle_back && !found && reported == ph) {
+                if (a.idle_back && ph < kAsyncBackPhases && !found && reported == ph) {
                     if (lane == 0) zero = async_busy(S, &s_idle, ph);
                     reported = 0xffffffffu;
                 }
