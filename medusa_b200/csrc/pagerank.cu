@@ -680,8 +680,7 @@ __global__ void k_stage_fill(const int2 *items, const int32_t *meg_off, int32_t 
 // us per superstep: uniform 6 10^6 / 6 10^7 285, here 268; R-MAT 4 10^6 / 6 10^7
 // 284 / 280, 2^24 / 2^28 965 / 957).
 constexpr int kDegClasses = 128;
-constexpr int kInKeyBits = 16;
-constexpr uint32_t kInKeyMask = (1u << kInKeyBits) - 1u;
+constexpr int kInKeyBits = 16;  // of the in-degree, at most; fewer where the largest needs fewer
 __host__ __device__ inline uint32_t degree_key(uint32_t d) {
     if (d == 0) return kDegClasses;
     uint32_t e = 0;
@@ -689,20 +688,21 @@ __host__ __device__ inline uint32_t degree_key(uint32_t d) {
     const uint32_t frac = e >= 2 ? (d >> (e - 2)) & 3u : (d << (2 - e)) & 3u;
     return kDegClasses - 1 - (4 * e + frac);
 }
-__global__ void k_deg_keys(const int32_t *outdeg, const int32_t *rrow, int32_t V, bool flat, uint32_t *key,
-                           uint32_t *val) {
+__global__ void k_deg_keys(const int32_t *outdeg, const int32_t *rrow, int32_t V, bool flat, int in_bits,
+                           uint32_t *key, uint32_t *val) {
+    const uint32_t mask = (1u << in_bits) - 1u;
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
          v += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t c = flat && outdeg[v] > 0 ? 0u : degree_key((uint32_t)outdeg[v]);
-        const uint32_t in = rrow ? min((uint32_t)(rrow[v + 1] - rrow[v]), kInKeyMask) : 0u;
-        key[v] = (c << kInKeyBits) | (kInKeyMask - in);
+        const uint32_t in = in_bits ? min((uint32_t)(rrow[v + 1] - rrow[v]), mask) : 0u;
+        key[v] = (c << in_bits) | (mask - in);
         val[v] = (uint32_t)v;
     }
 }
-__global__ void k_pos(const uint32_t *key, const uint32_t *val, int32_t V, int32_t *pos) {
+__global__ void k_pos(const uint32_t *key, const uint32_t *val, int32_t V, int in_bits, int32_t *pos) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V;
          i += (int64_t)gridDim.x * blockDim.x)
-        pos[val[i]] = (key[i] >> kInKeyBits) < kDegClasses ? (int32_t)i : -1;
+        pos[val[i]] = (key[i] >> in_bits) < kDegClasses ? (int32_t)i : -1;
 }
 
 __global__ void k_map_pos(const int32_t *src, int64_t E, const int32_t *pos, int32_t *out) {
@@ -854,7 +854,7 @@ void PrState::ensure(Context &ctx, const Graph &g) {
     rank.reserve(sizeof(float) * (size_t)V);
     contrib[0].reserve(sizeof(float) * (size_t)V);
     contrib[1].reserve(sizeof(float) * (size_t)V);
-    // contribution layout: by out-degree class, id order within a class;
+    // contribution layout: by out-degree class, in-degree (or id) order within;
     // vertices without out-edges send nothing and have no position
     cudaStream_t s = ctx.stream;
     const int gridV = grid_for(V, 256, ctx.num_sms * 16);
@@ -863,11 +863,13 @@ void PrState::ensure(Context &ctx, const Graph &g) {
         key.reserve(sizeof(uint32_t) * (size_t)V);
         val.reserve(sizeof(uint32_t) * (size_t)V);
         pos.reserve(sizeof(int32_t) * (size_t)V);
-        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), by_indegree ? g.rrow.as<int32_t>() : nullptr, V,
-                                         g.max_outdeg <= 64, key.as<uint32_t>(), val.as<uint32_t>());
+        int in_bits = 0;
+        while (by_indegree && in_bits < kInKeyBits && (g.max_indeg >> in_bits) != 0) in_bits++;
+        k_deg_keys<<<gridV, 256, 0, s>>>(g.outdeg.as<int32_t>(), g.rrow.as<int32_t>(), V, g.max_outdeg <= 64, in_bits,
+                                         key.as<uint32_t>(), val.as<uint32_t>());
         MB_CHECK_LAUNCH();
-        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8 + kInKeyBits, s);
-        k_pos<<<gridV, 256, 0, s>>>(key.as<uint32_t>(), val.as<uint32_t>(), V, pos.as<int32_t>());
+        radix_sort_pairs(ctx, key.as<uint32_t>(), val.as<uint32_t>(), V, 8 + in_bits, s);
+        k_pos<<<gridV, 256, 0, s>>>(key.as<uint32_t>(), val.as<uint32_t>(), V, in_bits, pos.as<int32_t>());
         MB_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         key.release(); val.release();
@@ -1058,7 +1060,6 @@ void PrState::ensure_exact(Context &ctx, const Graph &g, int32_t hub_min) {
         off.release();
     }
     MB_CUDA(cudaStreamSynchronize(s));
-    ensure_streams();
     x_hub_min = hub_min;
     exact_built = true;
 }
@@ -1075,7 +1076,8 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     if (ref_order && !unfused) st.ensure_exact(ctx, g, hub_min);
     if (!ref_order) st.ensure_fixed(ctx, g);
     if (unfused) st.msg.reserve(sizeof(float) * (size_t)std::max<int64_t>(g.E, 1));
-    st.ensure_streams();
+    // only for the hubs' scans and the heavy blocks
+    if (!unfused && (ref_order ? st.x_nhub : st.nitems) > 0) st.ensure_streams();
     cudaStream_t s = ctx.stream;
     auto args = [&](int it) {
         const int parity = it & 1;
