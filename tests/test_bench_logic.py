@@ -100,3 +100,22 @@ def test_verify_against_bsp_compares_and_restores_the_tuned_settings():
     assert ctx.t["sssp_async"] == 1 and ctx.t["async_below"] == 1 << 20 and ctx.sssp_delta == 100.0
     r = bench.verify_against_bsp(ctx, api, G(), lv, torch.tensor([0.0, 1.0, 2.0, 4.0]))
     assert r == {"bfs_levels": True, "sssp_distances": False}
+
+
+def test_dominant_kernel_of_runs_in_one_launch():
+    """Runs in one launch are their own dominant kernel; a loop beside one
+    counts with its traced branch."""
+    V = 1000
+    sb = {"device_ms": 0.1, "kernel_launches": 1, "edges_traversed": 10 ** 6, "vertices_reached": 900}
+    ss = {"device_ms": 0.5, "kernel_launches": 2, "edges_traversed": 10 ** 6, "vertices_reached": 900}
+    r = bench.dominant_kernel(None, None, sb, ss, V, 6000.0, "measured")
+    assert r["kernel"] == "k_sssp_coop (SSSP in one launch)"
+    assert r["algorithmic_bytes_per_launch"] == 12 * 10 ** 6 + 20 * 900 + 4 * V
+    assert abs(r["share_of_step_time"] - 0.5 / 0.6) < 1e-3
+    trace = [rec(0, 0, 5, 10, 0.9), rec(1, 19, 2000, 10 ** 6, 0.2)]  # the BFS part of the trace is not the step's
+    loop = dict(ss, kernel_launches=40)
+    r = bench.dominant_kernel(FakeCtx(trace), FakeGraph(), sb, loop, V, 6000.0, "measured")
+    assert r["kernel"].startswith("k_push_edge_bm")
+    slow = dict(sb, device_ms=0.3)
+    r = bench.dominant_kernel(FakeCtx(trace), FakeGraph(), slow, loop, V, 6000.0, "measured")
+    assert r["kernel"] == "k_bfs_coop (BFS in one launch)"
