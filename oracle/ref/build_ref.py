@@ -23,7 +23,8 @@ reference's CPUMalloc (see ref_harness.cpp).  Output goes only to
 
 Usage: python oracle/ref/build_ref.py [--reference PATH] [--force]
 Exits 0 without doing anything when the reference tree is absent and the
-libraries already exist (the GPU box only uses prebuilt files).
+libraries already exist (a machine without it only uses prebuilt files), with 3 when
+neither is there, with 1 when the build fails.
 """
 import argparse
 import os
@@ -37,6 +38,7 @@ ORACLE = os.path.dirname(HERE)
 OUT = os.path.join(ORACLE, "_ref")
 SHIM = os.path.join(HERE, "shim")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+NO_REFERENCE = 3
 
 # app name in the reference tree -> (library tag, harness define)
 APPS = {
@@ -116,12 +118,12 @@ def main(argv=None):
     p.add_argument("--force", action="store_true")
     a = p.parse_args(argv)
     have = all(os.path.exists(lib_path(t)) for t, _ in APPS.values())
-    if not os.path.isdir(a.reference):
+    if not os.path.isdir(os.path.join(a.reference, "Algorithm")):
         if have:
             return 0
         print("reference tree not found at %s; oracle/_ref not built" % a.reference,
               file=sys.stderr)
-        return 1
+        return NO_REFERENCE
     if have and not a.force:
         newest_input = max(os.path.getmtime(os.path.join(HERE, f))
                            for f in ("ref_harness.cpp", "build_ref.py"))
