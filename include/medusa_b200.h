@@ -45,7 +45,10 @@ extern "C" {
 
 /* ---- schedule policies (which kernel runs each superstep) ---------------- */
 #define MB_POLICY_FIXED 0       /* the fixed rule: frontier-size thresholds */
-#define MB_POLICY_LEARNED 1     /* the trained MLP scheduler, run on the device */
+#define MB_POLICY_LEARNED 1     /* the trained MLP scheduler, run on the device, superstep
+                                   by superstep: these runs keep the superstep loop, where
+                                   the fixed rule runs a whole traversal in one launch, and
+                                   are slower than it on most graphs */
 #define MB_POLICY_FORCED 2      /* one schedule id for every superstep */
 #define MB_POLICY_ORACLE_BEST 3 /* replay a per-superstep schedule list */
 
@@ -305,7 +308,9 @@ int mb_vis_edge_lines(mb_ctx *ctx, const mb_graph *g, const float *pos, float *l
  * then one BFS (as mb_bfs) from
  * sources[i] (nullable: vertex 0), all in ONE persistent cooperative launch
  * over their disjoint union (with a batch tunable set, or without
- * supersteps: a team of CTAs per graph, fed by a device work queue).  Outputs are concatenated: graph i's ranks and levels
+ * supersteps, or where the union does not fit in memory: a team of CTAs per
+ * graph, fed by a device work queue).  The first run of a batch builds the
+ * union.  Outputs are concatenated: graph i's ranks and levels
  * at [vbase[i], vbase[i+1]) (mb_batch_vertex_offsets); host or device. */
 typedef struct mb_batch mb_batch;
 int mb_batch_generate(mb_ctx *ctx, int32_t n, const mb_gen_params *params, mb_batch **out);
@@ -395,9 +400,11 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                 asynchronous cooperative launch (no superstep barriers:
                                 warps relax the dirty vertices below a distance threshold
                                 that rises by MB_TUNE_ASYNC_DELTA whenever every warp is
-                                idle); 0 the BSP supersteps; default 1 (on graphs with
-                                hubs only for the tail, MB_TUNE_ASYNC_BELOW), unless the
-                                persistent grid is set; never with a near-far width (the
+                                idle); 0 the BSP supersteps; default 1 (in a loop
+                                graph's run on a graph with hubs only for the tail,
+                                MB_TUNE_ASYNC_BELOW; by default such graphs run in a
+                                kernel of their own, which leaves a long rest of small
+                                supersteps to this one), unless the persistent grid is set; never with a near-far width (the
                                 far pile is not the kernel's frontier).  Under
                                 MB_POLICY_FIXED and MB_POLICY_LEARNED (it is how schedule
                                 0 runs the rest of a traversal; the forced and replay

@@ -26,7 +26,9 @@
 // a group, hubs of thousands of in-edges one after another, and CTAs idle
 // behind the largest graphs.  The union's vertices go through the sliced ELL
 // and the heavy blocks of pagerank.cu, whatever graph they belong to, with one
-// grid barrier per superstep, and its BFS has one source per graph.  The sums'
+// grid barrier per superstep, and its BFS has one source per graph, or, on small
+// sparse graphs without hubs, runs graph by graph (union_by_graph).  The first
+// run builds the union; where there is no memory for it, the teams run.  The sums'
 // order is per vertex, so the ranks are the same bits.  64 graphs of 2^10 to
 // 2^16 vertices, 21.6M edges, 20 supersteps and one BFS each: 2.28 ms,
 // against 8.0.
@@ -317,7 +319,7 @@ struct UnionArgs {
     SellArgs sell;
     // heavy blocks (PrState): {j0, j1, vertex, hub slot or -1}
     const int4 *items;
-    const int32_t *hcol, *pos, *outdeg, *slot_hub, *hub_first, *hub_v;
+    const int32_t *hcol, *pos, *outdeg, *slot_hub, *hub_first;
     float *blk_sum;
     uint32_t *hub_done;  // blocks of a hub summed; zero before and after a superstep
     int32_t nitems, nlong;

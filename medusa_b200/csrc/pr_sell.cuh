@@ -38,7 +38,10 @@ __device__ __forceinline__ float ld_contrib(const float *c, int32_t i) {
 
 // ---- sliced ELL ------------------------------------------------------------------
 // Vertices sorted by in-degree (largest first), 32 per group: a group's rows
-// are its first vertex's in-degree, at most 31 slots of padding per group.
+// are its first vertex's in-degree, so a group pads by at most 31 slots per row
+// of the difference to its last vertex: over the groups of a sorted list these
+// differences add up to the largest in-degree (31 times that many slots in all,
+// beside the empty lanes of the last group).
 // Light vertices in both orders, and mid vertices (up to hub_min in-edges) in
 // the reference's order.
 struct SellArgs {

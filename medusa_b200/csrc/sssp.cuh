@@ -95,16 +95,17 @@ struct SsspState : FrontierState {
 };
 
 // Graphs without hubs (largest out-degree <= 64): MB_TUNE_SSSP_ASYNC = -1
-// runs the whole SSSP in the asynchronous kernel (on other graphs only the
-// tail after the frontier's peak, MB_TUNE_ASYNC_BELOW), unless near-far
-// buckets or the persistent grid were asked for.  MB_TUNE_BFS_ASYNC = -1:
-// the kernel for BFS on hub-free graphs that are also sparse (mean
-// out-degree <= 6).  Measured on B200 (ms, BSP -> asynchronous):
-// SSSP on the 1448^2 grid 2.5 -> 1.2, uniform 2^20 / 2^24 1.19 -> 0.74,
-// uniform 2^18 / 2^22 0.64 -> 0.43; BFS on the grid 1.34 -> 0.72, uniform
-// 2^20 with 4 edges per vertex 0.31 -> 0.27, but uniform 2^20 / 2^24 0.21 ->
-// 0.29 (the direction-optimising pulls skip most edges).  On R-MAT graphs
-// (hubs) the BSP supersteps are as fast or faster for both.
+// runs the whole SSSP in the asynchronous kernel.  On other graphs the
+// one-launch kernel (sssp_coop.cu) comes first and hands over to it where the
+// supersteps stay small for long (SsspRest); where the loop graph runs, only
+// the tail after the frontier's peak is asynchronous (MB_TUNE_ASYNC_BELOW),
+// unless near-far buckets or the persistent grid were asked for.
+// MB_TUNE_BFS_ASYNC = -1: the kernel for BFS on hub-free graphs that are also
+// sparse (mean out-degree <= 6).  Measured on B200 (ms, loop graph ->
+// asynchronous): SSSP on the 1448^2 grid 2.5 -> 1.01, uniform 2^20 / 2^24 1.19 ->
+// 0.58; BFS on the grid 1.34 -> 0.60, uniform 2^20 with 4 edges per vertex 0.31 ->
+// 0.24, but uniform 2^20 / 2^24 0.21 -> 0.29 (the direction-optimising pulls skip
+// most edges).
 inline bool async_by_default(const Graph &g, bool bfs) {
     if (g.V <= 0 || g.max_outdeg > 64) return false;
     return !bfs || (double)g.E <= 6.0 * (double)g.V;
