@@ -412,9 +412,10 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                 graphs without a negative or NaN weight.  Identical
                                 distances */
 #define MB_TUNE_ASYNC_DELTA 18 /* width by which the asynchronous SSSP's threshold rises
-                                 (default: 24 x mean weight / mean out-degree -- 72 x with
-                                 fewer than 4 edges per vertex --, at least the
-                                 mean weight, on graphs without hubs; 0 -- no threshold --
+                                 (default: 24 x mean weight / mean out-degree, at least the
+                                 mean weight, on graphs without hubs; with fewer than 4
+                                 edges per vertex 16 x on large ones, and 72 x while the
+                                 frontier is a front that moves along, as on roads; 0 -- no threshold --
                                  for the tail on graphs with hubs) */
 #define MB_TUNE_ASYNC_BLOCKS_PER_SM 19 /* CTAs of 256 threads per SM of the asynchronous
                                          SSSP (default: as many as fit, at most 8) */
@@ -427,7 +428,8 @@ int mb_get_trace(mb_ctx *ctx, mb_trace_rec *out, int32_t max, int32_t *n_out);
                                edges per vertex and more than 10240 vertices or 65536
                                edges (smaller ones: a one-CTA kernel).  Identical levels */
 #define MB_TUNE_BFS_ASYNC_DELTA 21 /* threshold step of the asynchronous BFS, in hops
-                                     (default 8; 24 with fewer than 4 edges per vertex) */
+                                     (default 8; 24, with fewer than 4 edges per vertex, while
+                                     the frontier is a front that moves along) */
 #define MB_TUNE_ASYNC_BELOW 22 /* > 0: the asynchronous SSSP (when on) takes over only
                                  once the frontier, after reaching this many out-edges,
                                  has fewer -- the large supersteps run as BSP pushes and

@@ -15,7 +15,7 @@ import numpy as np
 
 
 # threshold steps of the asynchronous SSSP tried (-1: the per-graph default,
-# 24 x mean weight / mean out-degree, 72 x on road-like graphs; 0: no threshold)
+# 24 x mean weight / mean out-degree, wider on road-like graphs; 0: no threshold)
 ASYNC_DELTAS = [-1, 0, 50, 200, 800, 3200]
 
 

@@ -1109,6 +1109,8 @@ __global__ void k_sssp_init(SsspArgs a) {
         if (threadIdx.x == 2) a.as->bar.v = 0ull;
         if (threadIdx.x == 3) a.as->abort_.v = 0ull;
         if (threadIdx.x == 4) a.as->open.v = 0ull;
+        if (threadIdx.x == 5) a.as->most.v = 0ull;
+        if (threadIdx.x >= 6 && threadIdx.x < 8) a.as->left[threadIdx.x - 6].v = 0ull;
     }
     __syncthreads();
     if (threadIdx.x == 0) choose_next(c, APP_SSSP, a.f.V, a.f.E);
@@ -1239,14 +1241,20 @@ float sssp_default_delta(const Graph &g, double mean_w) {
     return (float)(mean_w * kDeltaWarps / std::max(1.0, mean_deg));
 }
 
+// The asynchronous SSSP's step in mean weights over the mean out-degree, and with
+// fewer than 4 edges per vertex a wide one's (wide_step).  ms, 16 / 24 throughout:
+// uniform 2^24 x 3 3.1 / 4.3, x 3.9 3.2 / 5.3, 2^22 x 3.9 0.90 / 1.11, x 2 0.80 / 0.72, 2^20 x 3
+// 0.41 / 0.38, 2^19 x 2 0.35 / 0.29.  72 throughout: 2^24 x 3 7.9, 2^22 x 3.9 1.77, 2^20 x 3
+// 0.41; but grids of 1448 x 1448, 24 / 72, 1.29 / 1.17, 300 x 300 3.0 / 2.4.
+static double async_step(const Graph &g) {
+    return g.E < 4 * (int64_t)g.V && 2 * g.E >= 5 * (int64_t)g.V && g.V >= (1 << 21) ? 16.0 : 24.0;
+}
+constexpr double kAsyncWideStep = 72.0;
+
 float sssp_async_delta(const Graph &g, double mean_w) {
     if (g.E == 0) return 0.f;
     const double mean_deg = (double)g.E / (double)g.V;
-    // road-like graphs: their frontiers are too small for narrow buckets (ms,
-    // 24 / 72 mean weights over the mean out-degree: grids of 1448 x 1448 1.04 /
-    // 0.90, 300 x 300 0.53 / 0.44; but uniform, 4 V 0.39 / 0.45, 16 V 0.58 / 1.32)
-    const double k = mean_deg < 4.0 ? 72.0 : 24.0;
-    return (float)std::max(mean_w, mean_w * k / std::max(1.0, mean_deg));
+    return (float)std::max(mean_w, mean_w * async_step(g) / std::max(1.0, mean_deg));
 }
 
 // Hub chunk tables of the asynchronous kernel for graph g (once).
@@ -1336,9 +1344,12 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
                     : (t_async >= 0 ? (int32_t)t_async : (!ctx.persist ? 1 : 0)));
     float async_delta = ctx.tunable[MB_TUNE_ASYNC_DELTA] >= 0 ? (float)ctx.tunable[MB_TUNE_ASYNC_DELTA]
                                                                : (hub_free ? st.async_delta : 0.f);
-    if (unit)
-        async_delta = ctx.tunable[MB_TUNE_BFS_ASYNC_DELTA] >= 0 ? (float)ctx.tunable[MB_TUNE_BFS_ASYNC_DELTA]
-                                                                : bfs_async_delta(g);
+    const int64_t t_step = ctx.tunable[unit ? MB_TUNE_BFS_ASYNC_DELTA : MB_TUNE_ASYNC_DELTA];
+    if (unit) async_delta = t_step >= 0 ? (float)t_step : kBfsAsyncStep;
+    // a step that the caller sets is the step throughout
+    const float async_wide = t_step >= 0 || g.E >= 4 * (int64_t)g.V
+                                 ? 1.f
+                                 : (unit ? kBfsAsyncWide : (float)(kAsyncWideStep / async_step(g)));
     // made on the first run whether or not it is asynchronous: the pointers
     // below are captured in the run's loop graph, which must not change
     // when a later run switches the kernel on
@@ -1353,7 +1364,9 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
     // The read saves atomics where most relaxations fail, but lengthens the chain
     // of a hop (ms, with / without: SSSP on uniform 2^20 / 2^24 0.56 / 0.59, 2^20 / 2^23
     // 0.52 / 0.52, 2^23 / 4 10^7 2.45 / 2.40, the 1448^2 grid 1.07 / 1.04, BFS on it 0.67 / 0.64).
-    a.look_first = g.E > 8 * (int64_t)g.V;
+    // From 2^23 vertices on the distances and bitmaps crowd L2 (2^24 x 3 3.0 / 3.3, x 6 6.4 / 7.0,
+    // BFS 3.4 / 3.6).
+    a.look_first = g.E > 8 * (int64_t)g.V || g.V >= (1 << 23);
     a.WA = ((int64_t)g.V + 32 * (int64_t)a.nc32 + 31) / 32;
     a.hub_cbase = st.hub_cbase.as<int32_t>();
     a.chunk_src = st.chunk_src.as<int32_t>();
@@ -1364,7 +1377,7 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
         unit ? 0u : (uint32_t)std::min<int64_t>(t_below >= 0 ? t_below : below_dflt, 0xffffffffll);
     if (phase == LOOP_ALL)
         upload_params(ctx, st.ctrl.p, source, unit ? 0.f : delta, sssp_bm_push_min(ctx, g), async, async_delta,
-                      async_below);
+                      async_below, async_wide);
     if (phase == LOOP_BEGIN) {  // a stepped run: one superstep per call (no persistent kernels)
         const bool tail = ctx.tail, persist = ctx.persist;
         ctx.tail = ctx.persist = false;

@@ -10,7 +10,7 @@ void sssp_weight_stats(const Graph &g, double *mean_w, bool *bad);
 // edges per bucket at the mean degree, times the mean weight.
 float sssp_default_delta(const Graph &g, double mean_w);
 // Default threshold step of the asynchronous SSSP: 24 x mean weight / mean
-// out-degree, at least the mean weight.
+// out-degree (16 x on large graphs of 2.5 to 4 edges per vertex), at least the mean weight.
 float sssp_async_delta(const Graph &g, double mean_w);
 
 // Shared state of the asynchronous SSSP kernel (sssp.cu), one per run,
@@ -29,6 +29,8 @@ struct AsyncState {
     AsyncLine idle[2];         // CTAs whose warps are all idle in the phase of that parity
     AsyncLine open;            // the last phase opened, claimed by the warp that opens it
     AsyncLine mn[2];           // least distance seen above the threshold in that phase (float bits)
+    AsyncLine left[2];         // dirty vertices seen above the threshold in that phase
+    AsyncLine most;            // of which the next phase may be wide (0: none yet, wide_step)
     AsyncLine t0;              // least distance of the starting frontier (float bits)
     AsyncLine bar;             // start barrier: CTAs arrived
     AsyncLine abort_;          // nonzero: a wait gave up and every warp leaves

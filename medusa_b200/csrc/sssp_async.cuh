@@ -119,11 +119,30 @@ __device__ __forceinline__ bool async_finished(AsyncState *S) {
 #define MB_ASYNC_CHUNK 64
 #endif
 constexpr int32_t kAsyncChunk = MB_ASYNC_CHUNK;
-// Default threshold step of the asynchronous BFS, in hops.  8 / 16 / 24, ms: on
-// road-like graphs (fewer than 4 edges per vertex) wide ones, grids of 1448 x
+// Default threshold step of the asynchronous BFS, in hops, and how many of them
+// make a wide one (wide_step).  Steps of 8 / 16 / 24 throughout, ms: grids of 1448 x
 // 1448 0.64 / 0.60 / 0.55, 300 x 300 0.39 / 0.35 / 0.32; uniform 2^20 with 4
-// edges per vertex 0.24 / 0.26 / 0.26, 2^23 with 5 1.38 / 1.49 / 1.62.
-inline float bfs_async_delta(const Graph &g) { return g.E < 4 * (int64_t)g.V ? 24.f : 8.f; }
+// edges per vertex 0.24 / 0.26 / 0.26, 2^23 with 5 1.38 / 1.49 / 1.62, 2^24 with 3
+// 2.1 / 2.2 / 3.5.
+constexpr float kBfsAsyncStep = 8.f, kBfsAsyncWide = 3.f;
+// Whether the next phase may be wide (sparse graphs): where the vertices left above
+// the threshold are a small part of the graph, and at most kFrontGrowth times those
+// of the phase before (its square where that one was wide), the frontier is a front that
+// moves along (roads, grids), and narrow phases leave the grid idle.  On graphs whose
+// frontier multiplies from hop to hop a wide phase would take in most of the graph,
+// out of order.  (The edges per vertex alone do not tell: SSSP on uniform 2^24 with 3
+// 7.9 ms wide, 3.3 narrow.  Growth from one narrow phase to the next: grid 1448 x 1448 with
+// 0.25% random edges 2 to 3, 1000 x 1000 with 5% 20 to 30, uniform 1000 and more.)
+constexpr uint32_t kFrontGrowth = 8;
+__device__ __forceinline__ bool wide_step(AsyncState *S, uint32_t ph, int32_t V) {
+    const uint32_t left = atomicExch((unsigned *)&S->left[ph & 1].v, 0u);
+    const uint32_t most = ld_rlx32(&S->most.v);
+    const bool wide = most && left <= most && left <= (uint32_t)V / 8;
+    // below 2^31: the old value's sign bit is zero, and makes the result wait for the write
+    const uint32_t old = atomicExch((unsigned *)&S->most.v, min(left, 1u << 24) * (wide ? kFrontGrowth * kFrontGrowth
+                                                                                        : kFrontGrowth));
+    return wide != (bool)(old >> 31);
+}
 // Relax what this warp claimed: lane l holds one dirty id (or v < 0) -- a
 // vertex (its out-edges), a hub (the bits of its chunks) or a chunk (its
 // out-edges).  Every item (an edge, or a chunk bit) may set one dirty bit.
@@ -277,10 +296,16 @@ __device__ __forceinline__ uint32_t async_relax(const SsspArgs &a, AsyncState *S
 // Lane 0 of a warp whose pass found nothing below the threshold: counts the
 // warp idle; the CTA's last warp counts the CTA, and the grid's last CTA opens
 // the next phase.  *s_idle: the CTA's idle warps, under the phase they reported
-// (phase << 8 | warps).  zero: async_busy's result, so that its change is
+// (phase << 8 | warps).  *s_left: the dirty vertices that its warps saw above the
+// threshold (left: this warp's).  zero: async_busy's result, so that its change is
 // performed first.  False: the CTA is in a later phase already.
-__device__ __forceinline__ bool async_idle(Ctrl *c, AsyncState *S, uint32_t *s_idle, uint32_t ph,
-                                           float T, float delta, float above, int cap, uint32_t zero) {
+__device__ __forceinline__ bool async_idle(Ctrl *c, AsyncState *S, uint32_t *s_idle, uint32_t *s_left, uint32_t ph,
+                                           float T, float delta, float above, uint32_t left, int32_t V,
+                                           int cap, uint32_t zero) {
+    if (left) {
+        atomicAdd(s_left, left);
+        __threadfence_block();
+    }
     uint32_t dep = 0;
     if (above < __uint_as_float(kInfBits))
         dep = atomicMin((unsigned *)&S->mn[ph & 1].v, __float_as_uint(above));
@@ -293,12 +318,15 @@ __device__ __forceinline__ bool async_idle(Ctrl *c, AsyncState *S, uint32_t *s_i
         old = atomicCAS(s_idle, now, ((now & ~255u) == tag ? now : tag) + 1u + (dep >> 31) + zero);
     } while (old != now);
     if (((now & ~255u) == tag ? (now & 255u) : 0u) + 1u != (uint32_t)kAsyncWarps) return true;
+    const uint32_t cta_left = atomicExch(s_left, 0u);
+    if (cta_left) atomicAdd((unsigned *)&S->left[ph & 1].v, cta_left);
     __threadfence();
     if (atomicAdd((unsigned *)&S->idle[ph & 1].v, 1u) + 1u != kAsyncIdle0 + gridDim.x) return true;
     // every CTA idle in phase ph: one of those that saw it raises the threshold
     if (atomicCAS((unsigned *)&S->open.v, ph, ph + 1u) != ph) return true;
     const uint32_t mb = atomicExch((unsigned *)&S->mn[ph & 1].v, kInfBits);
     const float m = __uint_as_float(mb);
+    if (c->p.async_wide > 1.f && wide_step(S, ph, V)) delta *= c->p.async_wide;
     float tn = T + delta;
     if (m < __uint_as_float(kInfBits) && m + delta > tn) tn = m + delta;
     // where a sum rounds back (distances past 2^24, a small step), one float
@@ -338,7 +366,7 @@ __global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int
     count_launch(c);
     AsyncState *S = a.as;
     uint32_t *dirty = a.adirty;
-    __shared__ uint32_t s_idle;
+    __shared__ uint32_t s_idle, s_left;
     __shared__ int s_ok;
     __shared__ volatile int s_done;  // set by the CTA's checker warp: every warp leaves
     // claimed vertices waiting for a full batch of 32, and the vertices the
@@ -353,11 +381,13 @@ __global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int
     const int slot = (int)(gw & (kAsyncSlots - 1));
     const long budget = c->p.wait_polls >= 0 ? (long)c->p.wait_polls : kAsyncSpins;
     const float delta = c->p.async_delta;
+    const bool widen = c->p.async_wide > 1.f;
     const float inf = __uint_as_float(kInfBits);
     const int64_t W = a.WA;
     const int32_t V = a.f.V;
     if (threadIdx.x == 0) {
         s_idle = 0u;
+        s_left = 0u;
         s_done = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)  // finish_superstep credits the frontier's edges
@@ -437,6 +467,7 @@ __global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int
         const float T = ph ? __uint_as_float((uint32_t)pt) : T0;
         bool found = false;
         float above = inf;
+        uint32_t left = 0;  // dirty, above T (warp-uniform)
         uint32_t nb = 0;  // vertices in bv (warp-uniform)
         uint32_t nn = 0;  // vertices in nxt (warp-uniform)
         // relax full batches of bv (all of it when `all`), taking the kept
@@ -494,6 +525,7 @@ __global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int
                 const bool below = has && d < T;
                 if (has && !below) above = fminf(above, d);
                 const uint32_t mask = __ballot_sync(FULL, below);
+                left += (uint32_t)__popc(x & ~mask);
                 if (!mask) continue;
                 uint32_t old = 0;
                 if (lane == 0) old = atom_and_acquire(&dirty[w], ~mask);
@@ -530,7 +562,7 @@ __global__ void __launch_bounds__(kAsyncThreads, 5) k_sssp_async(SsspArgs a, int
         if (reported != ph && T < inf) {
             above = warp_min_f(above);
             bool in = true;
-            if (lane == 0) in = async_idle(c, S, &s_idle, ph, T, delta, above, cap, zero);
+            if (lane == 0) in = async_idle(c, S, &s_idle, &s_left, ph, T, delta, above, widen ? left : 0u, V, cap, zero);
             if (__shfl_sync(FULL, in, 0)) reported = ph;
         }
         if (++idle > budget) {
