@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(256, kSellCtas) k_pr_sell(SellArgs a) {
 // supersteps, and no superstep waits for a launch.  Contributions are read
 // with plain loads (other SMs write them during the launch; the barrier's
 // acquire drops stale L1 lines).  A barrier that gives up writes *err (host
-// memory) and ends the launch.  Uniform 2^18 / 2^22, ten supersteps: 20.4 us
+// memory) and ends the launch.  Uniform 2^18 / 2^22, ten supersteps: 17.9 us
 // each, against 22.8 in launches of their own (the gathers alone: 14).
 // 8 rows in flight at 32 registers (64 warps per SM), or 16 where half the
 // warps are enough: the fewer rounds, the shorter a small graph's superstep.
@@ -1201,10 +1201,14 @@ void run_pagerank(Context &ctx, Graph &g, PrState &st, int32_t iters, float init
     // 4 10^4 34 / 34, 36 / 37, 7 10^4 35 / 38, 40 / 40).
     const bool by_launch = g.E < (1 << 15) && g.E < 12 * (int64_t)g.V;
     if (!unfused && iters > 1 && !by_launch && (ref_order ? st.x_nhub == 0 : st.nitems == 0) && all.ngroups > 0) {
-        // small graphs in smaller CTAs, one per SM: 177 groups in 6 CTAs of 32
-        // warps were bound by 6 SMs' gathers
-        const int64_t warps = std::min<int64_t>(kResThreads / 32,
-                                                std::max<int64_t>(4, (all.ngroups + ctx.num_sms - 1) / ctx.num_sms));
+        // the groups spread evenly over the SMs: small graphs in smaller CTAs, one
+        // per SM (177 groups in 6 CTAs of 32 warps were bound by 6 SMs' gathers), more
+        // than 32 groups per SM in two: with full CTAs some SMs had two and others one (us
+        // per superstep, launches of their own / full CTAs / so, 21 edges per vertex: 155851
+        // vertices 19.0 / 23.3 / 13.8, 215578 22.2 / 24.5 / 18.3, 2^18 28.4 / 25.3 / 22.5)
+        const int64_t per_sm = (all.ngroups + ctx.num_sms - 1) / ctx.num_sms;
+        const int64_t full = kResThreads / 32, ctas = per_sm > full ? 2 : 1;
+        const int64_t warps = std::min<int64_t>(full, std::max<int64_t>(4, (per_sm + ctas - 1) / ctas));
         res_threads = (int)warps * 32;
         grid_res = (int)std::min<int64_t>((all.ngroups + warps - 1) / warps, INT32_MAX);
         if (grid_res > resident(res_fn, res_threads)) res_fn = (const void *)k_pr_resident<8>;
