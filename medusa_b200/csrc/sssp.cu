@@ -1360,7 +1360,10 @@ void run_sssp(Context &ctx, Graph &g, SsspState &st, int32_t source, mb_stats *s
     // On small graphs a phase that opens early costs less than waiting for the
     // last warp (ms, taken back / not: uniform 6 10^4 / 9 10^5 0.25 / 0.22, 10^5 / 10^6
     // 0.25 / 0.23, 1.5 10^5 / 1.5 10^6 0.26 / 0.31, 2^20 / 2^24 0.58 / up to 1.1).
-    a.idle_back = g.E >= (1 << 20);
+    // Nor where there are few edges per vertex: the first phases are short there (ms,
+    // taken back / not: trees of 10^6 vertices 0.31 / 0.26, 2 10^6 0.49 / 0.36, BFS 0.29 / 0.25,
+    // 0.38 / 0.34; uniform 2^22 x 2 0.80 / 0.76, but x 3.9 0.90 / 1.07, and x 2.5 with twice the relaxations).
+    a.idle_back = g.E >= (1 << 20) && 4 * g.E >= 9 * (int64_t)g.V;
     // The read saves atomics where most relaxations fail, but lengthens the chain
     // of a hop (ms, with / without: SSSP on uniform 2^20 / 2^24 0.56 / 0.59, 2^20 / 2^23
     // 0.52 / 0.52, 2^23 / 4 10^7 2.45 / 2.40, the 1448^2 grid 1.07 / 1.04, BFS on it 0.67 / 0.64).

@@ -57,3 +57,13 @@ def test_moving_fronts_take_wide_steps(gpu_ctx, rows, cols, random_edges, weight
     st, sb = run(gpu_ctx, graph, weights)
     if (rows, cols) == (300, 300):  # 600 hops: 76 phases of 8, and some 28 of 24
         assert sb["supersteps"] < 50 and st["supersteps"] < 40, (st, sb)
+
+
+@pytest.mark.parametrize("V,fan", [(70001, 2), (550000, 40), (1 << 20, 3)])
+def test_trees(gpu_ctx, V, fan):
+    v = np.arange(1, V)
+    p = (v - 1) // fan
+    s, d = np.concatenate([p, v]).astype(np.int32), np.concatenate([v, p]).astype(np.int32)
+    st, sb = run(gpu_ctx, (V, s, d), "int")
+    # every vertex has one path: nothing is relaxed twice
+    assert st["edges_scanned"] == sb["edges_scanned"] == 2 * (V - 1)
