@@ -104,8 +104,8 @@ struct SsspState : FrontierState {
 // unless near-far buckets or the persistent grid were asked for.
 // MB_TUNE_BFS_ASYNC = -1: the kernel for BFS on hub-free graphs that are also
 // sparse (mean out-degree <= 6).  Measured on B200 (ms, loop graph ->
-// asynchronous): SSSP on the 1448^2 grid 2.5 -> 1.01, uniform 2^20 / 2^24 1.19 ->
-// 0.58; BFS on the grid 1.34 -> 0.60, uniform 2^20 with 4 edges per vertex 0.31 ->
+// asynchronous): SSSP on the 1448^2 grid 2.5 -> 1.03, uniform 2^20 / 2^24 1.19 ->
+// 0.58; BFS on the grid 1.34 -> 0.62, uniform 2^20 with 4 edges per vertex 0.31 ->
 // 0.24, but uniform 2^20 / 2^24 0.21 -> 0.29 (the direction-optimising pulls skip
 // most edges).
 inline bool async_by_default(const Graph &g, bool bfs) {
